@@ -3,7 +3,8 @@
 ``listed()`` names the cases, ``draw(rng)`` makes further ones of the same ranges, ``prepare(case, seed)`` is what a program
 holds before the call (operands on the GPU, converted weights, kernel handles and kernel arguments), ``run(state)`` is one
 pass through the public entry points, ``work(case)`` the bytes and operations the path cannot do without, and
-``tolerance(case)`` how far another correct implementation of the same precision may be off.
+``tolerance(case)`` how far another correct implementation of the same precision may be off, and ``exact(case, seed)`` the same
+results in 64 bits, by plain torch.
 
 The kinds of call (``case["kind"]``):
 
@@ -139,26 +140,46 @@ EPILOGUES = {"none": {}, "bias": {"epilogue": t0.EPI_BIAS_ADD_STORE_F32}, "bias_
              "silu": {"tile_epilogue": ["silu"]}}
 
 
-def prepare(case, seed):
-    rt, kind = _rt(), case["kind"]
+def _inputs(case, seed):
+    """The operands of a case, made from the seed alone: what both ``prepare`` and ``exact`` start from."""
+    kind = case["kind"]
     gen = torch.Generator(device="cuda")
     gen.manual_seed(seed)
-    s = {"kind": kind, "rt": rt}
     if kind == "dequant":
         rows, cols = case["rows"], case["cols"]
         groups = rows * cols // GROUP
-        s.update(rows=rows, cols=cols, bf16=case["out"] == "bf16", packed=_words(gen, rows * cols // 8),
-                 scales=torch.rand(groups, generator=gen, device="cuda") * 0.019 + 0.001,
-                 zeros=torch.randint(0, 16, (groups,), generator=gen, device="cuda", dtype=torch.int32),
+        return {"packed": _words(gen, rows * cols // 8), "scales": torch.rand(groups, generator=gen, device="cuda") * 0.019 + 0.001,
+                "zeros": torch.randint(0, 16, (groups,), generator=gen, device="cuda", dtype=torch.int32)}
+    m, n, k = case["m"], case["n"], case["k"]
+    if kind in ("gemm", "dispatch"):
+        nn = case.get("layout") == "nn"
+        s = {"x": _uniform(gen, m, k), "b": _uniform(gen, k, n) if nn else _uniform(gen, n, k)}
+        if kind == "gemm":
+            s["bias"] = torch.randn(n, generator=gen, device="cuda")
+        return s
+    if kind == "train":
+        return {"x": torch.randn(m, k, generator=gen, device="cuda"), "w": torch.randn(k, n, generator=gen, device="cuda") / math.sqrt(k),
+                "dy": torch.randn(m, n, generator=gen, device="cuda")}
+    problems = []
+    for _ in range(case.get("count", 1)):
+        w = _w4(gen, n, k)
+        problems.append((w, torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)))
+    return {"problems": problems}
+
+
+def prepare(case, seed):
+    rt, kind = _rt(), case["kind"]
+    given = _inputs(case, seed)
+    s = {"kind": kind, "rt": rt}
+    if kind == "dequant":
+        rows, cols = case["rows"], case["cols"]
+        s.update(given, rows=rows, cols=cols, bf16=case["out"] == "bf16",
                  y=torch.empty(rows, cols, device="cuda", dtype=torch.bfloat16 if case["out"] == "bf16" else torch.float32))
     elif kind in ("gemm", "dispatch"):
         m, n, k = case["m"], case["n"], case["k"]
-        nn = case.get("layout") == "nn"
-        s.update(m=m, n=n, k=k, x=_uniform(gen, m, k), b=_uniform(gen, k, n) if nn else _uniform(gen, n, k),
-                 y=torch.empty(m, n, device="cuda", dtype=torch.bfloat16 if case.get("out") == "bf16" else torch.float32))
+        s.update(given, m=m, n=n, k=k, y=torch.empty(m, n, device="cuda", dtype=torch.bfloat16 if case.get("out") == "bf16" else torch.float32))
         if kind == "gemm":
-            s["bias"] = torch.randn(n, generator=gen, device="cuda")
-            s["options"] = dict(EPILOGUES[case["epilogue"]], transpose=t0.NN if nn else t0.NT, out_bf16=case["out"] == "bf16")
+            s["options"] = dict(EPILOGUES[case["epilogue"]], transpose=t0.NN if case["layout"] == "nn" else t0.NT, out_bf16=case["out"] == "bf16")
         else:
             spec = t0.tile_auto_select(m, k, n)
             s["kernel"] = rt.ensure_kernel_t0(spec)
@@ -166,15 +187,13 @@ def prepare(case, seed):
             s["grid"] = t0.tile_compute_grid(spec, m, n)
     elif kind == "train":
         m, n, k = case["m"], case["n"], case["k"]
-        s.update(m=m, n=n, k=k, x=torch.randn(m, k, generator=gen, device="cuda"), w=torch.randn(k, n, generator=gen, device="cuda") / math.sqrt(k),
-                 dy=torch.randn(m, n, generator=gen, device="cuda"))
+        s.update(given, m=m, n=n, k=k)
         s.update(y=torch.empty(m, n, device="cuda"), dx=torch.empty(m, k, device="cuda"), dw=torch.empty(k, n, device="cuda"))
     else:
-        m, n, k, count = case["m"], case["n"], case["k"], case.get("count", 1)
+        m, n, k = case["m"], case["n"], case["k"]
         s.update(m=m, n=n, k=k, a=[], w=[], y=[])
-        for _ in range(count):
-            packed, scales, zeros = _w4(gen, n, k)
-            s["a"].append(torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16))
+        for (packed, scales, zeros), a in given["problems"]:
+            s["a"].append(a)
             s["y"].append(torch.empty(m, n, device="cuda"))
             if kind == "prefill":
                 s["w"].append((packed, scales, zeros))
@@ -252,3 +271,36 @@ def tolerance(case):
     # grows with the length of the sum: measured against f64, 1.9e-7 at K = 256 and 1e-9 K from K = 1000 on (7.5e-6 at K = 7680)
     k = max(case["m"], case["n"], case["k"]) if case["kind"] == "train" else case["k"]
     return {"rel": max(4e-6, 4e-9 * k)}
+
+
+# --------------------------------------------------------------------------- the same results in 64 bits
+
+def _nibbles(words, dim):
+    """The eight codes of each 32-bit word, lowest first, in place of dimension `dim`."""
+    codes = torch.stack([(words >> (4 * i)) & 15 for i in range(8)], dim + 1)
+    return codes.reshape(*words.shape[:dim], words.shape[dim] * 8, *words.shape[dim + 1:])
+
+
+def exact(case, seed):
+    kind, given = case["kind"], _inputs(case, seed)
+    if kind == "dequant":
+        codes = _nibbles(given["packed"], 0).reshape(-1, GROUP)
+        return ((codes - given["zeros"][:, None]).double() * given["scales"][:, None].double()).reshape(case["rows"], case["cols"])
+    if kind in ("gemm", "dispatch"):
+        b = given["b"].double()
+        y = given["x"].double() @ (b if case.get("layout") == "nn" else b.T)
+        epilogue = case.get("epilogue", "none")
+        if "bias" in epilogue:
+            y += given["bias"].double()
+        if epilogue == "bias_relu":
+            y = y.clamp_(min=0)
+        return y * torch.sigmoid(y) if epilogue == "silu" else y
+    if kind == "train":                           # the operands are rounded to bf16, the products are not
+        x, w, dy = (given[name].to(torch.bfloat16).double() for name in ("x", "w", "dy"))
+        return [x @ w, dy @ w.T, x.T @ dy]
+    out = []
+    for (packed, scales, zeros), a in given["problems"]:
+        z = _nibbles(zeros, 1)[:, :case["n"]].repeat_interleave(GROUP, 0)
+        w = ((_nibbles(packed, 0) - z).float() * scales.float().repeat_interleave(GROUP, 0)).to(torch.bfloat16)
+        out.append(a.double() @ w.double())
+    return out
