@@ -309,16 +309,7 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
                             if (s < n_split) { acc.x += part[u][s].x; acc.y += part[u][s].y; acc.z += part[u][s].z; acc.w += part[u][s].w; }
                         if (row >= p.M || col >= p.N) continue;
                         float o[4] = {acc.x, acc.y, acc.z, acc.w};
-                        if (p.n_ops) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) o[j] = apply_chain(o[j], (p.bias && col + j < p.N) ? __ldg(p.bias + col + j) : 0.0f, p);
-                        } else if (p.epilogue != T0_EPI_STORE_F32) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                o[j] += (p.bias && col + j < p.N) ? __ldg(p.bias + col + j) : 0.0f;
-                                if (p.epilogue == T0_EPI_BIAS_ADD_RELU_STORE_F32) o[j] = fmaxf(o[j], 0.0f);
-                            }
-                        }
+                        apply_epilogue(o, col, p);
                         const size_t off = (size_t)row * p.N + col;
                         if (vec && col + 4 <= p.N) {
                             *(float4*)((float*)y_out + off) = make_float4(o[0], o[1], o[2], o[3]);
