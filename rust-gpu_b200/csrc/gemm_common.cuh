@@ -31,7 +31,7 @@ struct KParams {
     uint32_t sk_stages, sk_alias; // split-K cluster kernel: ring depth; 1 = the accumulator is parked over the ring (one tile per cluster)
     uint32_t tail_start;         // pair kernel: work items from here on are half-width tiles (two per output tile); = total when unused
     uint32_t out_bf16, epilogue, n_ops;
-    uint32_t tma_store;          // full f32 chunks leave through the output tensor map
+    uint32_t tma_store;          // the output leaves through its tensor map
     uint32_t drop_load;          // self-test of the failure path: the producer of CTA 0 leaves out its first operand load
     uint32_t n_problems;         // split-K cluster kernel, grouped launch: problems of one shape in this launch (0 or 1 = a single problem)
     uint32_t n_peers;            // gathered output: every TMA-stored chunk also goes to this many other buffers (other GPUs' memory)
@@ -163,111 +163,92 @@ struct ClockProbe {
     }
 };
 
-constexpr uint32_t kEpiStageBytes = 4096;   // per epilogue warp: one 32 x 32 f32 chunk on its way to global memory
+constexpr uint32_t kEpiStageBytes = 4096;   // one block on its way to global memory: 32 rows x 128 bytes
 
-// One 32-row x 32-column chunk of the accumulator (this lane holds row `row_base + lane`): epilogue, then the store.
+// Chunk `c` of a tile: 32 rows x 32 columns of the accumulator (this lane holds row `row_base + lane`): epilogue, then the store.
 // A lane holds 32 consecutive columns of ONE row, so storing straight from registers makes every warp instruction touch
 // 32 different 128-byte lines (16 bytes of each): 256 line accesses per chunk, which made the epilogue of a 128 x 256 tile
-// cost about 5 us.  Full chunks therefore go through `stage` (this warp's 4 KiB of shared memory, 16-byte slots XOR-swizzled
-// so that neither the row-wise write nor the line-wise read has bank conflicts) and leave as whole lines: a warp instruction
-// stores four complete 128-byte row segments.  Ragged chunks (N edge, unaligned y or N) keep the element-wise path.
-// With `map_y` (an f32 output the TMA unit can address: 16-byte aligned base and row pitch) the staged block leaves as ONE
-// tiled TMA store instead of eight loads from the block and eight line-wise stores: the block's XOR pattern is the 128-byte
-// swizzle of the tensor map, rows beyond M are clipped by the copy.  `stage` is the warp's pair of blocks (1024-byte aligned,
-// kEpiStageBytes each).  `n_stores` is the warp's running count of committed TMA stores, carried across chunks AND tiles: store
-// i leaves from block i & 1, and before block i & 1 is rewritten the warp waits until every committed store but the latest
-// (which left from the other block) has read its source.  Counting only committed stores keeps that true when a tile has
-// an odd number of full chunks, a single chunk, or rows the copy would clip entirely.  The caller waits for its stores
-// (ptx::bulk_wait_group_all by lane 0) before shared memory goes away.
-__device__ __forceinline__ void store_chunk(const KParams& p, const uint32_t (&r)[32], uint32_t row_base, uint32_t lane, uint32_t col0,
-                                            uint32_t split, bool vec32, bool vec16, uint8_t* stage, uint32_t& n_stores, const CUtensorMap* map_y = nullptr,
+// cost about 5 us.  Chunks therefore go through `stage` (this warp's two 4 KiB blocks of shared memory, 1024-byte aligned,
+// 16-byte slots XOR-swizzled with the row so that neither side has bank conflicts).
+// With `map_y` (an output the TMA unit can address: 16-byte aligned base and row pitch) a block leaves as ONE tiled TMA store:
+// its XOR pattern is the 128-byte swizzle of the tensor map, rows beyond M and columns beyond N are clipped by the copy.  An f32
+// block is one chunk (32 columns), a bf16 block two (64 columns), filled by an even chunk and the odd one after it.
+// `n_stores` is the warp's running count of committed TMA stores, carried across chunks AND tiles: store i leaves from block
+// i & 1, and before block i & 1 is rewritten the warp waits until every committed store but the latest (which left from the
+// other block) has read its source.  Counting only committed stores keeps that true when a tile has an odd number of blocks, a
+// single one, or rows the copy would clip entirely.  The caller waits for its stores (ptx::bulk_wait_group_all by lane 0)
+// before shared memory goes away.
+// Without a map (N or the base not a multiple of 16 bytes, 32-wide bf16 tiles) the block is read back row by row, lane =
+// column: every store instruction writes 32 consecutive elements of one row, whatever the alignment.
+__device__ __forceinline__ void store_chunk(const KParams& p, const uint32_t (&r)[32], uint32_t row_base, uint32_t lane, uint32_t c, uint32_t col0,
+                                            uint32_t split, uint8_t* stage, uint32_t& n_stores, const CUtensorMap* map_y = nullptr,
                                             void* y_base = nullptr) {
-    void* const y_out = y_base ? y_base : p.y;       // a grouped launch names the problem's output
+    if (row_base >= p.M) return;                 // warp-uniform: no row of the chunk exists
     float v[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
     apply_epilogue(v, col0, p);
-    const size_t plane = (size_t)split * p.plane_stride;
-    const bool full = col0 + 32 <= p.N;          // warp-uniform
-    if (!p.out_bf16 && vec32 && full) {
-        // [32 rows][8 slots of 16 bytes], slot index XOR (row & 7); explicit shared-space accesses (the pointer went
-        // through an integer for alignment, so the compiler would otherwise use generic loads and stores)
-        if (map_y && row_base >= p.M) return;                 // warp-uniform: a box that starts below the last row has nothing to write
-        const uint32_t sb = ptx::smem_u32(stage) + (map_y ? (n_stores & 1u) * kEpiStageBytes : 0u);
-        if (map_y) {
-            if (lane == 0) ptx::bulk_wait_group_read_but_one();   // the latest committed store left from the other block
-            __syncwarp();
+    // explicit shared-space accesses: the pointer went through an integer for alignment, so the compiler would otherwise use
+    // generic loads and stores
+    const uint32_t sb = ptx::smem_u32(stage) + (map_y ? (n_stores & 1u) * kEpiStageBytes : 0u);
+    const uint32_t half = p.out_bf16 ? (c & 1u) : 0u;     // which half of a bf16 block
+    if (map_y && half == 0) {
+        if (lane == 0) ptx::bulk_wait_group_read_but_one();   // the latest committed store left from the other block
+        __syncwarp();
+    }
+    if (map_y && p.out_bf16) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            __nv_bfloat162 h[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
+            const uint32_t* q = (const uint32_t*)h;
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sb + (lane * 8 + ((half * 4 + j) ^ (lane & 7))) * 16), "r"(q[0]), "r"(q[1]), "r"(q[2]),
+                         "r"(q[3])
+                         : "memory");
         }
+        if (half == 0 && col0 + 32 < p.N) return;             // the odd chunk completes the block
+    } else {
 #pragma unroll
         for (uint32_t j = 0; j < 8; ++j)
             asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sb + (lane * 8 + (j ^ (lane & 7))) * 16), "f"(v[4 * j]), "f"(v[4 * j + 1]),
                          "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
                          : "memory");
-        if (map_y) {
-            ptx::fence_proxy_async_smem();                    // the copy reads the block through the async proxy
-            __syncwarp();
-            if (lane == 0) {
-                ptx::tma_store_3d(map_y, sb, (int32_t)col0, (int32_t)row_base, (int32_t)split);
-                // gathered output: the same block to the other GPUs' buffers (plain TMA stores to peer memory over NVLink),
-                // in the same bulk group, so the block is reused only after all of them have read it
-                for (uint32_t i = 0; i < p.n_peers; ++i) {
-                    // the maps were written to global memory by a copy before this launch: before the first use, order this
-                    // thread's tensor-map reads after that write (the slot is rewritten when the destinations change)
-                    if (n_stores == 0) ptx::fence_proxy_tensormap_acquire(p.peer_maps + i);
-                    ptx::tma_store_3d(p.peer_maps + i, sb, (int32_t)col0, (int32_t)row_base, (int32_t)split);
-                }
-                ptx::bulk_commit_group();
+    }
+    if (map_y) {
+        ptx::fence_proxy_async_smem();                        // the copy reads the block through the async proxy
+        __syncwarp();
+        if (lane == 0) {
+            const int32_t x = (int32_t)(col0 - half * 32);
+            ptx::tma_store_3d(map_y, sb, x, (int32_t)row_base, (int32_t)split);
+            // gathered output: the same block to the other GPUs' buffers (plain TMA stores to peer memory over NVLink),
+            // in the same bulk group, so the block is reused only after all of them have read it
+            for (uint32_t i = 0; i < p.n_peers; ++i) {
+                // the maps were written to global memory by a copy before this launch: before the first use, order this
+                // thread's tensor-map reads after that write (the slot is rewritten when the destinations change)
+                if (n_stores == 0) ptx::fence_proxy_tensormap_acquire(p.peer_maps + i);
+                ptx::tma_store_3d(p.peer_maps + i, sb, x, (int32_t)row_base, (int32_t)split);
             }
-            ++n_stores;
-            return;
+            ptx::bulk_commit_group();
         }
-        __syncwarp();
-        const uint32_t slot = lane & 7;
-#pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-            const uint32_t rr = i * 4 + (lane >> 3), row = row_base + rr;
-            float4 q;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(sb + (rr * 8 + (slot ^ (rr & 7))) * 16) : "memory");
-            if (row < p.M) *(float4*)((float*)y_out + plane + (size_t)row * p.N + col0 + 4 * slot) = q;
-        }
-        __syncwarp();
+        ++n_stores;
         return;
     }
-    if (p.out_bf16 && vec16 && full) {
-        uint4* s4 = (uint4*)stage;               // [32 rows][4 slots of 16 bytes], slot index XOR ((row >> 1) & 3)
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            uint4 q;
-            __nv_bfloat162 h0 = __floats2bfloat162_rn(v[8 * j], v[8 * j + 1]);
-            __nv_bfloat162 h1 = __floats2bfloat162_rn(v[8 * j + 2], v[8 * j + 3]);
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * j + 4], v[8 * j + 5]);
-            __nv_bfloat162 h3 = __floats2bfloat162_rn(v[8 * j + 6], v[8 * j + 7]);
-            q.x = *(uint32_t*)&h0; q.y = *(uint32_t*)&h1; q.z = *(uint32_t*)&h2; q.w = *(uint32_t*)&h3;
-            s4[lane * 4 + (j ^ ((lane >> 1) & 3))] = q;
+    __syncwarp();
+    const uint32_t col = col0 + lane;
+    const uint32_t rows = min(32u, p.M - row_base);
+    void* const y_out = y_base ? y_base : p.y;       // a grouped launch names the problem's output
+    const size_t off = (size_t)split * p.plane_stride + (size_t)row_base * p.N + col;
+#pragma unroll 8
+    for (uint32_t rr = 0; rr < 32; ++rr) {
+        float q;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(q) : "r"(sb + (rr * 8 + ((lane >> 2) ^ (rr & 7))) * 16 + (lane & 3) * 4) : "memory");
+        if (rr < rows && col < p.N) {
+            if (p.out_bf16) ((__nv_bfloat16*)y_out)[off + (size_t)rr * p.N] = __float2bfloat16_rn(q);
+            else ((float*)y_out)[off + (size_t)rr * p.N] = q;
         }
-        __syncwarp();
-        const uint32_t slot = lane & 3;
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            const uint32_t rr = i * 8 + (lane >> 2), row = row_base + rr;
-            const uint4 q = s4[rr * 4 + (slot ^ ((rr >> 1) & 3))];
-            if (row < p.M) *(uint4*)((__nv_bfloat16*)y_out + plane + (size_t)row * p.N + col0 + 8 * slot) = q;
-        }
-        __syncwarp();
-        return;
     }
-    const uint32_t row = row_base + lane;
-    if (row >= p.M) return;
-    const size_t off = plane + (size_t)row * p.N + col0;
-    if (!p.out_bf16) {
-        float* dst = (float*)y_out + off;
-        for (int j = 0; j < 32; ++j)
-            if (col0 + j < p.N) dst[j] = v[j];
-    } else {
-        __nv_bfloat16* dst = (__nv_bfloat16*)y_out + off;
-        for (int j = 0; j < 32; ++j)
-            if (col0 + j < p.N) dst[j] = __float2bfloat16_rn(v[j]);
-    }
+    __syncwarp();
 }
 
 // ------------------------------------------------------------------ launch (host)
@@ -358,19 +339,28 @@ inline int make_map_3d_plain(CUtensorMap* map, const void* base, uint32_t elem_b
     return T0_OK;
 }
 
-// 3-D view [planes][M][N] of the f32 output (or of split-K planes `plane_stride` elements apart), box 32 x 32, 128-byte
-// swizzle: what the epilogue's TMA store writes through.  Needs a 16-byte aligned base and N % 4 == 0.
-inline int make_map_out_f32(CUtensorMap* map, const void* base, uint32_t M, uint32_t N, uint32_t planes, uint64_t plane_stride) {
+// 3-D view [planes][M][N] of the output (or of split-K planes `plane_stride` elements apart), box 32 rows x 128 bytes, 128-byte
+// swizzle: what the epilogue's TMA store writes through.  Needs a 16-byte aligned base and row pitch.
+inline int make_map_out(CUtensorMap* map, const void* base, uint32_t M, uint32_t N, uint32_t planes, uint64_t plane_stride, bool bf16) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return fail(T0_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t es = bf16 ? 2 : 4;
     cuuint64_t dims[3] = {N, M, planes > 1 ? planes : 1};
-    cuuint64_t strides[2] = {(cuuint64_t)N * 4, planes > 1 ? (cuuint64_t)plane_stride * 4 : (cuuint64_t)M * N * 4};
-    cuuint32_t box[3] = {32, 32, 1};
+    cuuint64_t strides[2] = {(cuuint64_t)N * es, planes > 1 ? (cuuint64_t)plane_stride * es : (cuuint64_t)M * N * es};
+    cuuint32_t box[3] = {(cuuint32_t)(128 / es), 32, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(T0_ERR_CUDA, "cuTensorMapEncodeTiled (f32 output %u x %u) failed: %d", M, N, (int)r);
+    CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(T0_ERR_CUDA, "cuTensorMapEncodeTiled (output %u x %u) failed: %d", M, N, (int)r);
     return T0_OK;
+}
+
+// Whether the TMA unit can address this output: base, row pitch (and plane pitch) multiples of 16 bytes, and tiles at least as
+// wide as a box (a 64-column bf16 box over 32-wide tiles would write the neighbour's columns).
+inline bool tma_output_ok(const GemmLaunch& g, uint32_t split, uint32_t tile_n) {
+    static const bool no_tma_store = getenv("T0_NO_TMA_STORE") != nullptr;
+    const uint32_t unit = g.out_bf16 ? 8 : 4;
+    return !no_tma_store && g.n % unit == 0 && ((uintptr_t)g.y & 15) == 0 && (split == 1 || g.plane_stride % unit == 0) && tile_n >= 8 * unit;
 }
 
 // Gathered output: one output tensor map per extra destination, copied to `g.peer_map_slot` on the launch stream (a small
@@ -380,13 +370,13 @@ inline int stage_peer_maps(const GemmLaunch& g, KParams& p, uint32_t split, cuda
     p.peer_maps = nullptr;
     if (g.n_peer_y == 0) return T0_OK;
     if (g.n_peer_y > 7 || !g.peer_map_slot) return fail(T0_ERR_INVALID, "gathered output: %u destinations (at most 7) or no slot for their tensor maps", g.n_peer_y);
-    if (!p.tma_store || split != 1 || g.n % 32 != 0)
+    if (!p.tma_store || g.out_bf16 || split != 1 || g.n % 32 != 0)
         return fail(T0_ERR_UNSUPPORTED, "a gathered output needs the TMA-store epilogue on every chunk: f32 output, N %% 32 == 0 (N=%u), 16-byte aligned buffers, no split-K", g.n);
     if (!g.peer_maps_staged) {
         CUtensorMap maps[7];
         for (uint32_t i = 0; i < g.n_peer_y; ++i) {
             if (!g.peer_y[i] || ((uintptr_t)g.peer_y[i] & 15)) return fail(T0_ERR_INVALID, "gathered output: destination %u is null or not 16-byte aligned", i);
-            int rc = make_map_out_f32(&maps[i], g.peer_y[i], g.m, g.n, 1, 0);
+            int rc = make_map_out(&maps[i], g.peer_y[i], g.m, g.n, 1, 0, false);
             if (rc != T0_OK) return rc;
         }
         cudaError_t e = cudaMemcpyAsync(g.peer_map_slot, maps, g.n_peer_y * sizeof(CUtensorMap), cudaMemcpyHostToDevice, stream);

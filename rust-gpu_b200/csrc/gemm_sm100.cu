@@ -183,8 +183,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             void* y_out = p.y;
             const CUtensorMap* my = &map_y;
             if constexpr (kGrouped) { y_out = group.y[prob]; my = &group.maps[3 * prob + 2]; }
-            const bool vec32 = (p.N % 4 == 0) && (((uintptr_t)y_out & 15) == 0);
-            const bool vec16 = (p.N % 8 == 0) && (((uintptr_t)y_out & 15) == 0);
             const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
             if (!ptx::mbar_wait(ptx::smem_u32(&tmem_full_bar[buf]), acc_phase, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(w & 0xFFFFFF));
@@ -199,7 +197,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 uint32_t r[32];
                 ptx::tmem_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + buf * BN + c * 32, r);
                 ptx::tmem_ld_wait();
-                store_chunk(p, r, row_base, lane, col0, wi.split, vec32, vec16, epi_stage + quarter * 2 * kEpiStageBytes, n_stores,
+                store_chunk(p, r, row_base, lane, c, col0, wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores,
                             p.tma_store ? my : nullptr, y_out);
             }
             ptx::tc_fence_before_sync();
@@ -289,11 +287,9 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     const uint64_t total = (uint64_t)p.tiles_m * p.tiles_n * split;
     if (total > 0x7FFFFFFFull) return fail(T0_ERR_UNSUPPORTED, "too many tiles");
     const uint32_t grid = (uint32_t)std::min<uint64_t>(total, g.n_sms ? g.n_sms : 148);
-    // f32 output the TMA unit can address (16-byte aligned base, row pitch and plane pitch): full chunks leave as TMA stores
-    static const bool no_tma_store = getenv("T0_NO_TMA_STORE") != nullptr;
     CUtensorMap my = ma;   // a valid map either way; only read when p.tma_store is set
-    if (!no_tma_store && !g.out_bf16 && g.n % 4 == 0 && ((uintptr_t)g.y & 15) == 0 && (split == 1 || g.plane_stride % 4 == 0)) {
-        rc = make_map_out_f32(&my, g.y, g.m, g.n, split, g.plane_stride);
+    if (tma_output_ok(g, split, bn)) {
+        rc = make_map_out(&my, g.y, g.m, g.n, split, g.plane_stride, g.out_bf16);
         if (rc != T0_OK) return rc;
         p.tma_store = 1;
     }
@@ -339,9 +335,8 @@ int launch_gemm_sm100_grouped(const GemmLaunch* gs, uint32_t count, cudaStream_t
     p.scale = g0.scale; p.clamp_min = g0.clamp_min; p.clamp_max = g0.clamp_max;
     memcpy(p.ops, g0.ops, sizeof p.ops);
     p.n_problems = count;
-    static const bool no_tma_store = getenv("T0_NO_TMA_STORE") != nullptr;
-    bool tma_store = !no_tma_store && !g0.out_bf16 && g0.n % 4 == 0;
-    for (uint32_t i = 0; i < count; ++i) tma_store = tma_store && (((uintptr_t)gs[i].y & 15) == 0);
+    bool tma_store = true;
+    for (uint32_t i = 0; i < count; ++i) tma_store = tma_store && tma_output_ok(gs[i], 1, bn);
     p.tma_store = tma_store ? 1 : 0;
     static GroupOperands3 group;         // 12.5 KB: kept off the stack, filled under the lock, copied by the launch
     static std::mutex group_mu;
@@ -360,7 +355,7 @@ int launch_gemm_sm100_grouped(const GemmLaunch* gs, uint32_t count, cudaStream_t
         if (rc != T0_OK) return rc;
         group.maps[3 * i + 2] = group.maps[3 * i];          // a valid map either way; only read when p.tma_store is set
         if (tma_store) {
-            rc = make_map_out_f32(&group.maps[3 * i + 2], g.y, g.m, g.n, 1, 0);
+            rc = make_map_out(&group.maps[3 * i + 2], g.y, g.m, g.n, 1, 0, g.out_bf16);
             if (rc != T0_OK) return rc;
         }
         group.y[i] = g.y;

@@ -191,8 +191,6 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
         const uint32_t quarter = warp & 3;          // tensor-memory lanes 32*quarter .. +31 are the ones this warp may read
-        const bool vec32 = (p.N % 4 == 0) && (((uintptr_t)p.y & 15) == 0);
-        const bool vec16 = (p.N % 8 == 0) && (((uintptr_t)p.y & 15) == 0);
         uint32_t iter = 0, n_stores = 0;     // n_stores: this warp's committed TMA stores, see store_chunk
         for (uint32_t w = pair_id; w < total_work; w += n_pairs, ++iter) {
             const bool tail = w >= tail_start;
@@ -214,7 +212,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                 uint32_t r[32];
                 ptx::tmem_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + buf * kPairN + c * 32, r);
                 ptx::tmem_ld_wait();
-                store_chunk(p, r, row_base, lane, col0, wi.split, vec32, vec16, epi_stage + quarter * 2 * kEpiStageBytes, n_stores, p.tma_store ? &map_y : nullptr);
+                store_chunk(p, r, row_base, lane, c, col0, wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores, p.tma_store ? &map_y : nullptr);
             }
             ptx::tc_fence_before_sync();
             __syncwarp();
@@ -337,11 +335,9 @@ int launch_gemm_sm100_pair(const GemmLaunch& g, cudaStream_t stream) {
     if (rc != T0_OK) return rc;
     const uint64_t total = (uint64_t)p.tiles_m * p.tiles_n * split;
     if (total > 0x7FFFFFFFull) return fail(T0_ERR_UNSUPPORTED, "too many tiles");
-    // f32 output the TMA unit can address (16-byte aligned base, row pitch and plane pitch): full chunks leave as TMA stores
-    static const bool no_tma_store = getenv("T0_NO_TMA_STORE") != nullptr;
     CUtensorMap my = ma;   // a valid map either way; only read when p.tma_store is set
-    if (!no_tma_store && !g.out_bf16 && g.n % 4 == 0 && ((uintptr_t)g.y & 15) == 0 && (split == 1 || g.plane_stride % 4 == 0)) {
-        rc = make_map_out_f32(&my, g.y, g.m, g.n, split, g.plane_stride);
+    if (tma_output_ok(g, split, pair_n)) {
+        rc = make_map_out(&my, g.y, g.m, g.n, split, g.plane_stride, g.out_bf16);
         if (rc != T0_OK) return rc;
         p.tma_store = 1;
     }

@@ -228,7 +228,7 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
         const uint32_t quarter = warp & 3;
         const uint32_t n_split = p.split_k;
         const uint32_t cols_per = BN / n_split;             // columns of the tile this CTA reduces and stores
-        const bool vec_shape = (p.N % 4 == 0) && !p.out_bf16;
+        const bool vec_shape = p.N % 4 == 0;
         const uint32_t parked = ptx::smem_u32(parked_bar), readb = ptx::smem_u32(read_bar);
         bool ok = true;
         uint32_t iter = 0;
@@ -238,7 +238,7 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
             const WorkItem wi = decode_work(tile * p.split_k, p);
             void* y_out = p.y;
             if constexpr (kGrouped) y_out = group.y[prob];
-            const bool vec = vec_shape && (((uintptr_t)y_out & 15) == 0);
+            const bool vec = vec_shape && (((uintptr_t)y_out & 15) == 0);      // four columns of a row start on a 16-byte (bf16: 8-byte) boundary
             const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
             if (ok && !ptx::mbar_wait(ptx::smem_u32(&tmem_full_bar[buf]), acc_phase, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(w & 0xFFFFFF));
@@ -312,7 +312,12 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
                         apply_epilogue(o, col, p);
                         const size_t off = (size_t)row * p.N + col;
                         if (vec && col + 4 <= p.N) {
-                            *(float4*)((float*)y_out + off) = make_float4(o[0], o[1], o[2], o[3]);
+                            if (p.out_bf16) {
+                                const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
+                                *(uint2*)((__nv_bfloat16*)y_out + off) = *(const uint2*)h;
+                            } else {
+                                *(float4*)((float*)y_out + off) = make_float4(o[0], o[1], o[2], o[3]);
+                            }
                         } else {
                             for (int j = 0; j < 4; ++j) {
                                 if (col + j >= p.N) break;

@@ -1,0 +1,71 @@
+"""GPU tests of the edges of the kernels' tiles, splits and copies: where a store is clipped, a tile is cut between CTAs, a row does
+not start on a whole word.  Integer-valued operands make the products exact in f32 (every partial sum is an integer below 2^24), so
+those comparisons are bit for bit; the others state their bound.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GUARD = 512
+
+
+def ints(rng, *shape, lim=4):
+    return rng.integers(-lim, lim + 1, shape).astype(np.float32)
+
+
+def bf16_bits(v):
+    u = np.ascontiguousarray(v, np.float32).view(np.uint32).astype(np.uint64)
+    return ((u + 0x7FFF + ((u >> 16) & 1)) >> 16).astype(np.uint16)
+
+
+def from_bf16(u):
+    return (u.astype(np.uint32) << 16).view(np.float32)
+
+
+def run_gemm(t0, rt, x, b, m, n, k, out_bf16=False, bias=None, x_skip=0, b_skip=0, **kw):
+    """x [m,k] and b as given (f32 values that bf16 holds exactly), *_skip elements into their buffers; the output and its guard."""
+    xd = rt.upload(np.concatenate([np.zeros(x_skip, np.uint16), bf16_bits(x).ravel()]))
+    bd = rt.upload(np.concatenate([np.zeros(b_skip, np.uint16), bf16_bits(b).ravel()]))
+    size = 2 if out_bf16 else 4
+    y = rt.alloc(m * n * size + GUARD)
+    y.write(np.full(m * n * size + GUARD, 0xA5, np.uint8))
+    bb = rt.upload(bias) if bias is not None else None
+    rt.gemm(xd.gpu_addr() + 2 * x_skip, bd.gpu_addr() + 2 * b_skip, y.gpu_addr(), m, n, k, out_bf16=out_bf16, bias=bb.gpu_addr() if bb else 0, **kw)
+    rt.synchronize()
+    raw = y.read(m * n * size + GUARD, np.uint8)
+    for buf in [xd, bd, y] + ([bb] if bb else []):
+        buf.free()
+    assert np.all(raw[m * n * size:] == 0xA5), "wrote past the output"
+    body = raw[:m * n * size]
+    return from_bf16(body.view(np.uint16)).reshape(m, n) if out_bf16 else body.view(np.float32).reshape(m, n)
+
+
+@pytest.mark.parametrize("out_bf16", [False, True])
+@pytest.mark.parametrize("n", [8, 33, 36, 72, 130, 264, 520])
+@pytest.mark.parametrize("pair,tile_n", [(2, 32), (2, 64), (2, 128), (2, 256), (1, 128), (1, 256)])
+def test_output_edges_of_every_tile(t0, rt, pair, tile_n, n, out_bf16):
+    # widths that end inside a 32-column chunk, after an even chunk of a bf16 block, and that no 16-byte rule fits
+    m, k = 150, 96
+    rng = np.random.default_rng(n)
+    x, b, bias = ints(rng, m, k), ints(rng, n, k), ints(rng, n, lim=100)
+    got = run_gemm(t0, rt, x, b, m, n, k, out_bf16, bias, tile_n=tile_n, pair_cta=pair, epilogue=t0.EPI_BIAS_ADD_RELU_STORE_F32)
+    want = np.maximum(x @ b.T + bias, 0)
+    assert np.array_equal(got, from_bf16(bf16_bits(want)) if out_bf16 else want)
+
+
+@pytest.mark.parametrize("pair,tile_n,split_k", [(2, 64, 1), (2, 256, 1), (1, 256, 1), (2, 128, 4)])
+@pytest.mark.parametrize("out_bf16", [False, True])
+def test_epilogue_chain_on_every_kernel(t0, rt, pair, tile_n, split_k, out_bf16):
+    m, n, k = 150, 328, 512
+    rng = np.random.default_rng(5)
+    x, b = ints(rng, m, k, lim=1), ints(rng, n, k, lim=1)
+    bias = rng.uniform(-2, 2, n).astype(np.float32)
+    got = run_gemm(t0, rt, x, b, m, n, k, out_bf16, bias, tile_n=tile_n, pair_cta=pair, split_k=split_k, scale=0.125,
+                   tile_epilogue=["scale", "bias", "silu", "neg", "gelu"])
+    v = (x @ b.T).astype(np.float64) * 0.125 + bias
+    v = -(v / (1 + np.exp(-v)))
+    v = v / (1 + np.exp(-1.702 * v))
+    # f32 elementwise: a few roundings of 2^-24 each, exp2 of an argument of up to ~40 adds |argument| * 2^-24 to the relative error
+    tol = 1e-5 * np.abs(v) + 1e-6
+    assert np.all(np.abs(got - v) <= tol + (2.0 ** -8 * np.abs(v) if out_bf16 else 0))
