@@ -36,7 +36,9 @@ struct GroupOperands3 {
     void* y[kMaxGroupedGemms];
 };
 
-template <uint32_t BN, bool B_MN, bool kGrouped = false>
+// B_MN = B is given as B[K,N] (N contiguous), A_MN = A is given as A[K,M] (M contiguous): boxes of 64(k) x 64 columns, read by the
+// UMMA through MN-major descriptors.
+template <uint32_t BN, bool B_MN, bool kGrouped = false, bool A_MN = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_y, const KParams p,
@@ -45,7 +47,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     constexpr uint32_t kBStageBytes = BN * BK * 2;
     constexpr uint32_t kStageBytes = kAStageBytes + kBStageBytes;
     constexpr uint32_t kTmemCols = 2 * BN;   // two accumulator buffers; 64..512, a power of two
-    constexpr uint32_t kIdesc = ptx::make_idesc_bf16_f32(BM, BN, B_MN ? 1u : 0u);
+    constexpr uint32_t kIdesc = ptx::make_idesc_bf16_f32(BM, BN, B_MN ? 1u : 0u, A_MN ? 1u : 0u);
 
     extern __shared__ uint8_t smem_raw[];
     // 128-byte swizzled tiles need 1024-byte alignment
@@ -119,8 +121,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     // self-test of the failure path: this stage is never filled, so the issuer's bounded wait must run out
                     if (p.drop_load && blockIdx.x == 0 && w == 0 && kb == 0) { if (++stage == kStages) { stage = 0; phase ^= 1; } continue; }
                     ptx::mbar_arrive_expect_tx(fb, kStageBytes);
-                    ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
-                                     (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)wi.split);
+                    if constexpr (!A_MN) {
+                        ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
+                                         (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)wi.split);
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < BM / 64; ++j)
+                            ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), ma, fb,
+                                             (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                    }
                     if constexpr (!B_MN) {
                         ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
                                          (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)wi.split);
@@ -160,7 +169,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
                         // K-major, 128B swizzle: 8-row groups 1024 B apart; a 16-element K step is 32 B
-                        const uint64_t da = ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
+                        const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
+                                                 : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
                         // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
                         const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
                                                  : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
@@ -224,10 +234,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 // ------------------------------------------------------------------ host side
 
-template <uint32_t BN, bool B_MN, bool kGrouped = false>
+template <uint32_t BN, bool B_MN, bool kGrouped = false, bool A_MN = false>
 int launch_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const KParams& p, uint32_t grid, cudaStream_t stream,
                     const std::conditional_t<kGrouped, GroupOperands3, NoGroup>& group = {}) {
-    auto kern = gemm_bf16_tcgen05_kernel<BN, B_MN, kGrouped>;
+    auto kern = gemm_bf16_tcgen05_kernel<BN, B_MN, kGrouped, A_MN>;
     const uint32_t smem = gemm_smem_bytes(BN);
     static bool attr_set[64] = {};   // per instantiation, per device
     int dev = 0;
@@ -258,8 +268,9 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     const uint32_t split = g.split_k ? g.split_k : 1;
     if (g.k % split) return fail(T0_ERR_UNSUPPORTED, "K=%u not divisible by split_k=%u", g.k, split);
     const uint32_t kps = g.k / split;
-    const uint32_t ldx = g.ldx ? g.ldx : g.k;
+    const uint32_t ldx = g.ldx ? g.ldx : (g.at ? g.m : g.k);
     const uint32_t ldb = g.ldb ? g.ldb : (g.nn ? g.n : g.k);
+    if (g.at && !g.nn) return fail(T0_ERR_UNSUPPORTED, "a transposed first operand goes with B[K,N]");
     if ((ldx % 8) || (ldb % 8) || (split > 1 && (kps % 8)))
         return fail(T0_ERR_UNSUPPORTED, "row strides (%u, %u) and, with split-K, K per split (%u) must be multiples of 8 for the TMA path", ldx, ldb, kps);
     if (((uintptr_t)g.x & 15) || ((uintptr_t)g.b & 15)) return fail(T0_ERR_UNSUPPORTED, "operand pointers must be 16-byte aligned");
@@ -279,7 +290,7 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     memcpy(p.ops, g.ops, sizeof p.ops);
 
     CUtensorMap ma, mb;
-    int rc = make_map_kmajor(&ma, g.x, g.m, ldx, kps, split, BM);
+    int rc = g.at ? make_map_nmajor(&ma, g.x, g.m, ldx, kps, split) : make_map_kmajor(&ma, g.x, g.m, ldx, kps, split, BM);
     if (rc != T0_OK) return rc;
     rc = g.nn ? make_map_nmajor(&mb, g.b, g.n, ldb, kps, split) : make_map_kmajor(&mb, g.b, g.n, ldb, kps, split, bn);
     if (rc != T0_OK) return rc;
@@ -296,6 +307,13 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     rc = stage_peer_maps(g, p, split, stream);
     if (rc != T0_OK) return rc;
 
+    if (g.at) {
+        switch (bn) {
+            case 64: return launch_instance<64, true, false, true>(ma, mb, my, p, grid, stream);
+            case 128: return launch_instance<128, true, false, true>(ma, mb, my, p, grid, stream);
+            default: return launch_instance<256, true, false, true>(ma, mb, my, p, grid, stream);
+        }
+    }
     if (g.nn) {
         switch (bn) {
             case 64: return launch_instance<64, true>(ma, mb, my, p, grid, stream);

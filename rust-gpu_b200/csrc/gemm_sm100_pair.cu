@@ -29,8 +29,8 @@ __host__ __device__ constexpr uint32_t pair_stages(uint32_t pair_n) { return pai
 // kPairN = output columns per pair (256, or 128 when 256-wide tiles would quantise badly over the SMs)
 // B_MN = B is given as B[K,N] (N contiguous): each CTA then loads its half of the columns as 64(k) x 64(n) boxes and the
 // UMMA reads B through an MN-major descriptor, exactly as the single-CTA kernel does; `map_b_half` is unused (the boxes
-// are 64 columns wide whatever the tile).
-template <uint32_t kPairN, bool B_MN>
+// are 64 columns wide whatever the tile).  A_MN = A is given as A[K,M] (M contiguous): the same boxes and descriptors for A.
+template <uint32_t kPairN, bool B_MN, bool A_MN = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                               const __grid_constant__ CUtensorMap map_b_half, const __grid_constant__ CUtensorMap map_y, const KParams p) {
@@ -39,12 +39,12 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
     constexpr uint32_t kStageBytes = kAStageBytes + kBStageBytes;  // per CTA
     constexpr uint32_t kStages = pair_stages(kPairN);
     constexpr uint32_t kTmemCols = 2 * kPairN;                     // two accumulator buffers
-    constexpr uint32_t kIdesc = ptx::make_idesc_bf16_f32(kPairM, kPairN, B_MN ? 1u : 0u);
+    constexpr uint32_t kIdesc = ptx::make_idesc_bf16_f32(kPairM, kPairN, B_MN ? 1u : 0u, A_MN ? 1u : 0u);
     // Tail of the tile list: when the last wave would leave more than half of the pairs idle, its tiles are cut into two
     // half-width tiles (work items >= p.tail_start; item tail_start + 2i + h is half h of tile tail_start + i), so the wave
     // costs a half-width tile instead of a full one.  B then comes through a tensor map with a box half as tall.
     constexpr uint32_t kHalfN = kPairN / 2;
-    constexpr uint32_t kIdescHalf = ptx::make_idesc_bf16_f32(kPairM, kHalfN, B_MN ? 1u : 0u);
+    constexpr uint32_t kIdescHalf = ptx::make_idesc_bf16_f32(kPairM, kHalfN, B_MN ? 1u : 0u, A_MN ? 1u : 0u);
     constexpr uint32_t kBHalfStageBytes = (kHalfN / 2) * BK * 2;
 
     extern __shared__ uint8_t smem_raw[];
@@ -123,8 +123,15 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                     if (p.drop_load && pair_id == 0 && w == 0 && kb == 0) { if (++stage == kStages) { stage = 0; phase ^= 1; } continue; }
                     if (cta_rank == 0) ptx::mbar_arrive_expect_tx(fb_local, 2 * (kAStageBytes + (tail ? kBHalfStageBytes : kBStageBytes)));   // bytes of both CTAs
                     const uint32_t fb = ptx::mapa(fb_local, 0);   // the even CTA's barrier, from either CTA
-                    ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes), &map_a, fb,
-                                          (int32_t)(kb * BK), (int32_t)(wi.m_blk * kPairM + cta_rank * BM), (int32_t)wi.split);
+                    if constexpr (!A_MN) {
+                        ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes), &map_a, fb,
+                                              (int32_t)(kb * BK), (int32_t)(wi.m_blk * kPairM + cta_rank * BM), (int32_t)wi.split);
+                    } else {
+#pragma unroll
+                        for (uint32_t j = 0; j < BM / 64; ++j)
+                            ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), &map_a, fb,
+                                                  (int32_t)(wi.m_blk * kPairM + cta_rank * BM + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                    }
                     if constexpr (B_MN) {
                         // this CTA's columns of B[K,N]: one 64(k) x 64(n) box (a [k][128 B] block) per 64 columns
                         const uint32_t cols = tail ? kHalfN / 2 : kBHalfRows;
@@ -169,7 +176,8 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                     const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
-                        const uint64_t da = ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
+                        const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
+                                                 : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
                         // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
                         const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
                                                  : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
@@ -250,10 +258,10 @@ uint32_t gemm_pair_smem_bytes(uint32_t pair_n) {
 
 namespace {
 
-template <uint32_t kPairN, bool B_MN>
+template <uint32_t kPairN, bool B_MN, bool A_MN = false>
 int launch_pair_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb_half, const CUtensorMap& my, KParams p, uint64_t total, uint32_t n_sms,
                          cudaStream_t stream) {
-    auto kern = gemm_bf16_tcgen05_pair_kernel<kPairN, B_MN>;
+    auto kern = gemm_bf16_tcgen05_pair_kernel<kPairN, B_MN, A_MN>;
     const uint32_t smem = gemm_pair_smem_bytes(kPairN);
     static bool attr_set[64] = {};
     static int max_pairs[64] = {};
@@ -295,8 +303,9 @@ int launch_gemm_sm100_pair(const GemmLaunch& g, cudaStream_t stream) {
     const uint32_t split = g.split_k ? g.split_k : 1;
     if (g.k % split) return fail(T0_ERR_UNSUPPORTED, "K=%u not divisible by split_k=%u", g.k, split);
     const uint32_t kps = g.k / split;
-    const uint32_t ldx = g.ldx ? g.ldx : g.k;
+    const uint32_t ldx = g.ldx ? g.ldx : (g.at ? g.m : g.k);
     const uint32_t ldb = g.ldb ? g.ldb : (g.nn ? g.n : g.k);
+    if (g.at && !g.nn) return fail(T0_ERR_UNSUPPORTED, "a transposed first operand goes with B[K,N]");
     if ((ldx % 8) || (ldb % 8) || (split > 1 && (kps % 8)))
         return fail(T0_ERR_UNSUPPORTED, "row strides (%u, %u) and, with split-K, K per split (%u) must be multiples of 8 for the TMA path", ldx, ldb, kps);
     if (((uintptr_t)g.x & 15) || ((uintptr_t)g.b & 15)) return fail(T0_ERR_UNSUPPORTED, "operand pointers must be 16-byte aligned");
@@ -321,7 +330,7 @@ int launch_gemm_sm100_pair(const GemmLaunch& g, cudaStream_t stream) {
     memcpy(p.ops, g.ops, sizeof p.ops);
 
     CUtensorMap ma, mb;
-    int rc = make_map_kmajor(&ma, g.x, g.m, ldx, kps, split, BM);
+    int rc = g.at ? make_map_nmajor(&ma, g.x, g.m, ldx, kps, split) : make_map_kmajor(&ma, g.x, g.m, ldx, kps, split, BM);
     if (rc != T0_OK) return rc;
     CUtensorMap mb_half;
     if (g.nn) {
@@ -344,6 +353,9 @@ int launch_gemm_sm100_pair(const GemmLaunch& g, cudaStream_t stream) {
     rc = stage_peer_maps(g, p, split, stream);
     if (rc != T0_OK) return rc;
     const uint32_t n_sms = g.n_sms ? g.n_sms : 148;
+    if (g.at)
+        return pair_n == 256 ? launch_pair_instance<256, true, true>(ma, mb, mb_half, my, p, total, n_sms, stream)
+                             : launch_pair_instance<128, true, true>(ma, mb, mb_half, my, p, total, n_sms, stream);
     if (g.nn)
         return pair_n == 256 ? launch_pair_instance<256, true>(ma, mb, mb_half, my, p, total, n_sms, stream)
                              : launch_pair_instance<128, true>(ma, mb, mb_half, my, p, total, n_sms, stream);

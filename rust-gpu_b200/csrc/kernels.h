@@ -12,7 +12,7 @@ namespace t0 {
 enum : int { kStatusOk = 0, kStatusProducerTimeout = 0x01000000, kStatusMmaTimeout = 0x02000000, kStatusEpilogueTimeout = 0x03000000 };
 
 struct GemmLaunch {
-    const void* x;        // bf16 [M,K]
+    const void* x;        // bf16 [M,K]; [K,M] with at
     const void* b;        // bf16 [N,K] (NT) or [K,N] (NN)
     void* y;              // f32 [M,N] (or planes) / bf16 [M,N]
     const float* bias;    // f32 [N] or null
@@ -22,6 +22,7 @@ struct GemmLaunch {
     uint32_t split_k;     // >= 1
     uint64_t plane_stride;  // elements between split planes
     bool nn, out_bf16, swap_grid;
+    bool at;              // x is given transposed, [K,M] with M contiguous (row stride ldx, 0 = M); only together with nn
     uint8_t epilogue;     // T0_EPI_*
     uint8_t n_ops;        // TileIR chain (overrides epilogue when > 0)
     uint8_t ops[T0_TILE_MAX_EPILOGUE];

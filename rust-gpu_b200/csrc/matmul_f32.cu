@@ -7,11 +7,11 @@
 // is dX = dY * W^T, `gemm_backward_weight` (:264-312) is dW = X^T * dY, `matmul_with_wt_bf16` (:93-133) takes the weight
 // already transposed and in bf16.  src/universal/math/mod.rs:24-47 is the BLAS trait, math/blas.rs:18-100 its CPU body.
 //
-// Here the conversions are one pass on the device (f32 -> bf16, optionally transposing), the GEMM reads the operands
-// where they lie (NN layout for w, so no transpose of the weight at all; ragged edges are handled by TMA zero fill and
-// masked stores), and nothing is padded, copied back or round-tripped through the host.
+// Here the conversion of both operands is one pass on the device (f32 -> bf16, rows padded to whole 16-byte units) and the GEMM
+// reads them where they lie: w as B[K,N], X^T for dW as A[K,M], so nothing is ever transposed; ragged edges are handled by
+// TMA zero fill and clipped stores, and nothing is copied back or round-tripped through the host.
 #include "runtime_internal.h"
-#include "kernels.h"
+#include "gemm_common.cuh"
 
 using namespace t0;
 
@@ -23,50 +23,50 @@ __device__ __forceinline__ uint16_t bf16_rne_bits(float v) {
     return (uint16_t)((bits + 0x7FFFu + ((bits >> 16) & 1u)) >> 16);
 }
 
-// dst[r][c] = bf16(src[r * ld_src + c]), dense rows x cols
-__global__ void cvt_f32_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, uint32_t rows, uint32_t cols, uint32_t ld_src) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if ((cols % 8 == 0) && (ld_src % 4 == 0) && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0) {
-        // eight elements per thread: two 16-byte streaming loads (the f32 source is read once), one 16-byte store
-        const uint32_t units_per_row = cols / 8;
-        const uint64_t units = (uint64_t)rows * units_per_row;
-        for (uint64_t u = gtid; u < units; u += stride) {
-            const uint32_t r = (uint32_t)(u / units_per_row), c = (uint32_t)(u - (uint64_t)r * units_per_row) * 8;
-            const float4* s4 = (const float4*)(src + (size_t)r * ld_src + c);
-            const float4 lo = __ldcs(s4), hi = __ldcs(s4 + 1);
-            uint4 o;
-            o.x = (uint32_t)bf16_rne_bits(lo.x) | ((uint32_t)bf16_rne_bits(lo.y) << 16);
-            o.y = (uint32_t)bf16_rne_bits(lo.z) | ((uint32_t)bf16_rne_bits(lo.w) << 16);
-            o.z = (uint32_t)bf16_rne_bits(hi.x) | ((uint32_t)bf16_rne_bits(hi.y) << 16);
-            o.w = (uint32_t)bf16_rne_bits(hi.z) | ((uint32_t)bf16_rne_bits(hi.w) << 16);
-            *(uint4*)(dst + (size_t)r * cols + c) = o;
-        }
-        return;
+// One operand of a conversion launch: dst[r * ld_dst + c] = bf16(src[r * ld_src + c]), c < cols, in units of eight destination
+// elements of one row (ld_dst is a multiple of 8 and dst 16-byte aligned; columns from cols to ld_dst are written as zero).
+struct CvtOperand {
+    const float* src;
+    uint16_t* dst;
+    uint32_t rows, cols, ld_src, ld_dst;
+};
+
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) { return (uint32_t)bf16_rne_bits(lo) | ((uint32_t)bf16_rne_bits(hi) << 16); }
+
+__device__ __forceinline__ void cvt_unit(const CvtOperand& o, bool vec, uint32_t r, uint32_t c) {
+    const float* s = o.src + (size_t)r * o.ld_src + c;
+    float v[8];
+    if (vec) {
+        const float4 lo = __ldcs((const float4*)s), hi = __ldcs((const float4*)s + 1);      // the f32 source is read once
+        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) v[i] = c + i < o.cols ? s[i] : 0.0f;
     }
-    const uint64_t total = (uint64_t)rows * cols;
-    for (uint64_t i = gtid; i < total; i += stride) {
-        const uint32_t r = (uint32_t)(i / cols), c = (uint32_t)(i - (uint64_t)r * cols);
-        dst[i] = bf16_rne_bits(src[(size_t)r * ld_src + c]);
-    }
+    *(uint4*)(o.dst + (size_t)r * o.ld_dst + c) = make_uint4(bf16_pair(v[0], v[1]), bf16_pair(v[2], v[3]), bf16_pair(v[4], v[5]), bf16_pair(v[6], v[7]));
 }
 
-// dst[c][r] = bf16(src[r][c]): 32 x 32 tiles through shared memory so both sides are coalesced
-__global__ void cvt_f32_bf16_transpose_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, uint32_t rows, uint32_t cols) {
-    __shared__ float tile[32][33];
-    const uint32_t tiles_c = (cols + 31) / 32, tiles_r = (rows + 31) / 32;
-    for (uint32_t t = blockIdx.x; t < tiles_c * tiles_r; t += gridDim.x) {
-        const uint32_t tr = t / tiles_c, tc = t - tr * tiles_c;
-        for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-            const uint32_t r = tr * 32 + i, c = tc * 32 + threadIdx.x;
-            tile[i][threadIdx.x] = (r < rows && c < cols) ? src[(size_t)r * cols + c] : 0.0f;
+// Both operands of a product in one launch: two 16-byte loads and one 16-byte store per unit.  Bound by memory.  It starts under
+// the tail of the kernel before it and lets the product start under its own (programmatic dependent launch); until the wait
+// returns it touches no global memory, since the kernel before may still write the sources or read the scratch.
+// A training step of a 1024 -> 4096 layer on 2048 rows ran six conversion launches, one of them transposing: 127 us; with one
+// launch per product and X^T read by the tensor cores as it lies, 105 us.
+__global__ void __launch_bounds__(256) cvt_operands_kernel(const CvtOperand a, const CvtOperand b) {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const CvtOperand& o = i == 0 ? a : b;
+        const bool vec = (o.cols % 8 == 0) && (o.ld_src % 4 == 0) && ((uintptr_t)o.src & 15) == 0;
+        const uint32_t per_row = o.ld_dst / 8;
+        const uint64_t units = (uint64_t)o.rows * per_row;
+        for (; u < units; u += stride) {
+            const uint32_t r = units >> 32 ? (uint32_t)(u / per_row) : (uint32_t)u / per_row;      // a 64-bit division only where it is needed
+            cvt_unit(o, vec, r, (uint32_t)(u - (uint64_t)r * per_row) * 8);
         }
-        __syncthreads();
-        for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-            const uint32_t c = tc * 32 + i, r = tr * 32 + threadIdx.x;
-            if (c < cols && r < rows) dst[(size_t)c * rows + r] = bf16_rne_bits(tile[threadIdx.x][i]);
-        }
-        __syncthreads();
+        u -= units;
     }
 }
 
@@ -102,32 +102,37 @@ uint32_t blocks_for(uint64_t n, uint32_t per_block, uint32_t sms) {
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sms * 8));
 }
 
-int convert(t0_runtime* rt, Scratch& s, uint64_t src, uint32_t rows, uint32_t cols, uint32_t ld_src, bool transpose, uint64_t* out) {
-    const size_t bytes = std::max<size_t>((size_t)rows * cols * 2, 16);
-    int rc = ensure_scratch(rt, s, bytes);
+uint32_t pitch(uint32_t cols) { return (cols + 7) & ~7u; }      // row stride of a converted operand: whole 16-byte units for the TMA maps
+
+// The bf16 copy of src[rows][cols] (row stride ld_src) goes to `dense`, or, where rows have to be padded, to `padded` (the buffer of the
+// padded operand copies of the bf16 entries): makes room and describes the conversion.
+int plan_cvt(t0_runtime* rt, Scratch& dense, Scratch& padded, uint64_t src, uint32_t rows, uint32_t cols, uint32_t ld_src, CvtOperand* o) {
+    Scratch& s = pitch(cols) == cols ? dense : padded;
+    int rc = ensure_scratch(rt, s, std::max<size_t>((size_t)rows * pitch(cols) * 2, 16));
     if (rc != T0_OK) return rc;
-    if ((uint64_t)rows * cols) {
-        if (!transpose) {
-            cvt_f32_bf16_kernel<<<blocks_for((uint64_t)rows * cols, 2048, rt->sm_count), 256, 0, rt->stream>>>((const float*)src, (uint16_t*)s.ptr, rows, cols, ld_src);
-        } else {
-            const uint64_t tiles = (uint64_t)((rows + 31) / 32) * ((cols + 31) / 32);
-            cvt_f32_bf16_transpose_kernel<<<blocks_for(tiles, 1, rt->sm_count), dim3(32, 8), 0, rt->stream>>>((const float*)src, (uint16_t*)s.ptr, rows, cols);
-        }
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return fail(T0_ERR_CUDA, "f32 -> bf16 conversion launch failed: %s", cudaGetErrorString(e));
-        rt->launches.fetch_add(1);
-    }
-    *out = (uint64_t)(uintptr_t)s.ptr;
+    *o = CvtOperand{(const float*)src, (uint16_t*)s.ptr, rows, cols, ld_src, pitch(cols)};
     return T0_OK;
 }
 
-int gemm_bf16(t0_runtime* rt, uint64_t a, uint64_t b, uint64_t y, uint32_t m, uint32_t n, uint32_t k, int transpose) {
-    t0_gemm_args ga;
-    memset(&ga, 0, sizeof ga);
-    ga.x = a; ga.b = b; ga.y = y;
-    ga.m = m; ga.n = n; ga.k = k;
-    ga.transpose = (uint8_t)transpose; ga.swap_grid = 1;
-    return t0_gemm_launch(rt, &ga);
+// `b` may have no rows (one operand only).
+int launch_cvt(t0_runtime* rt, const CvtOperand& a, const CvtOperand& b) {
+    const uint64_t units = (uint64_t)a.rows * (a.ld_dst / 8) + (uint64_t)b.rows * (b.ld_dst / 8);
+    if (units == 0) return T0_OK;
+    cudaError_t e = gemm::launch_pdl(cvt_operands_kernel, blocks_for(units, 256, rt->sm_count), 256, 0, rt->stream, a, b);
+    if (e != cudaSuccess) return fail(T0_ERR_CUDA, "f32 -> bf16 conversion launch failed: %s", cudaGetErrorString(e));
+    rt->launches.fetch_add(1);
+    return T0_OK;
+}
+
+// y[m,n] = bf16(a) * bf16(b): both operands converted in one launch, then the product.  a is [m,k], or [k,m] with `at`; b is [k,n]
+// with `nn`, else [n,k].
+int product(t0_runtime* rt, uint64_t a, uint32_t lda, bool at, uint64_t b, uint32_t ldb, bool nn, uint64_t y, uint32_t m, uint32_t n, uint32_t k) {
+    CvtOperand oa, ob;
+    int rc = at ? plan_cvt(rt, rt->scratch_cvt_a, rt->scratch_a, a, k, m, lda, &oa) : plan_cvt(rt, rt->scratch_cvt_a, rt->scratch_a, a, m, k, lda, &oa);
+    if (rc == T0_OK) rc = nn ? plan_cvt(rt, rt->scratch_cvt_b, rt->scratch_b, b, k, n, ldb, &ob) : plan_cvt(rt, rt->scratch_cvt_b, rt->scratch_b, b, n, k, ldb, &ob);
+    if (rc == T0_OK) rc = launch_cvt(rt, oa, ob);
+    if (rc != T0_OK) return rc;
+    return gemm_strided(rt, (uint64_t)(uintptr_t)oa.dst, oa.ld_dst, at, (uint64_t)(uintptr_t)ob.dst, ob.ld_dst, nn, y, m, n, k);
 }
 
 int check_ptrs(t0_runtime* rt, std::initializer_list<uint64_t> ptrs) {
@@ -147,11 +152,7 @@ int t0_matmul_f32(t0_runtime* rt, uint64_t x, uint64_t w, uint64_t y, uint32_t m
     if (rc != T0_OK) return rc;
     if (m == 0 || n == 0) return T0_OK;
     DeviceGuard guard(rt->device);
-    uint64_t xa = 0, wb = 0;
-    rc = convert(rt, rt->scratch_cvt_a, x, m, k, k, false, &xa);
-    if (rc == T0_OK) rc = convert(rt, rt->scratch_cvt_b, w, k, n, n, false, &wb);
-    if (rc != T0_OK) return rc;
-    return gemm_bf16(rt, xa, wb, y, m, n, k, T0_NN);                 // y = x * w, w read as B[K,N]
+    return product(rt, x, k, false, w, n, true, y, m, n, k);         // y = x * w, w read as B[K,N]
 }
 
 int t0_matmul_f32_with_wt_bf16(t0_runtime* rt, uint64_t x, uint64_t wt_bf16, uint64_t y, uint32_t m, uint32_t k, uint32_t n) {
@@ -159,10 +160,11 @@ int t0_matmul_f32_with_wt_bf16(t0_runtime* rt, uint64_t x, uint64_t wt_bf16, uin
     if (rc != T0_OK) return rc;
     if (m == 0 || n == 0) return T0_OK;
     DeviceGuard guard(rt->device);
-    uint64_t xa = 0;
-    rc = convert(rt, rt->scratch_cvt_a, x, m, k, k, false, &xa);
+    CvtOperand oa, none = {};
+    rc = plan_cvt(rt, rt->scratch_cvt_a, rt->scratch_a, x, m, k, k, &oa);
+    if (rc == T0_OK) rc = launch_cvt(rt, oa, none);
     if (rc != T0_OK) return rc;
-    return gemm_bf16(rt, xa, wt_bf16, y, m, n, k, T0_NT);
+    return gemm_strided(rt, (uint64_t)(uintptr_t)oa.dst, oa.ld_dst, false, wt_bf16, 0, false, y, m, n, k);
 }
 
 int t0_matmul_f32_backward_data(t0_runtime* rt, uint64_t dy, uint64_t w, uint64_t dx, uint32_t m, uint32_t k, uint32_t n) {
@@ -170,11 +172,7 @@ int t0_matmul_f32_backward_data(t0_runtime* rt, uint64_t dy, uint64_t w, uint64_
     if (rc != T0_OK) return rc;
     if (m == 0 || k == 0) return T0_OK;
     DeviceGuard guard(rt->device);
-    uint64_t a = 0, b = 0;
-    rc = convert(rt, rt->scratch_cvt_a, dy, m, n, n, false, &a);
-    if (rc == T0_OK) rc = convert(rt, rt->scratch_cvt_b, w, k, n, n, false, &b);
-    if (rc != T0_OK) return rc;
-    return gemm_bf16(rt, a, b, dx, m, k, n, T0_NT);                  // dX[M,K] = dY[M,N] * W[K,N]^T: contraction over N
+    return product(rt, dy, n, false, w, n, false, dx, m, k, n);      // dX[M,K] = dY[M,N] * W[K,N]^T: contraction over N
 }
 
 int t0_matmul_f32_backward_weight(t0_runtime* rt, uint64_t x, uint64_t dy, uint64_t dw, uint32_t m, uint32_t k, uint32_t n) {
@@ -182,11 +180,7 @@ int t0_matmul_f32_backward_weight(t0_runtime* rt, uint64_t x, uint64_t dy, uint6
     if (rc != T0_OK) return rc;
     if (k == 0 || n == 0) return T0_OK;
     DeviceGuard guard(rt->device);
-    uint64_t a = 0, b = 0;
-    rc = convert(rt, rt->scratch_cvt_a, x, m, k, k, true, &a);       // X^T [K, M]
-    if (rc == T0_OK) rc = convert(rt, rt->scratch_cvt_b, dy, m, n, n, false, &b);
-    if (rc != T0_OK) return rc;
-    return gemm_bf16(rt, a, b, dw, k, n, m, T0_NN);                  // dW[K,N] = X^T[K,M] * dY[M,N]: contraction over M
+    return product(rt, x, k, true, dy, n, true, dw, k, n, m);        // dW[K,N] = X^T[K,M] * dY[M,N]: contraction over M, X read as it lies
 }
 
 int t0_blas_gemm_f32(t0_runtime* rt, uint32_t m, uint32_t n, uint32_t k, float alpha, uint64_t a, uint32_t lda, uint64_t b, uint32_t ldb,
@@ -196,10 +190,6 @@ int t0_blas_gemm_f32(t0_runtime* rt, uint32_t m, uint32_t n, uint32_t k, float a
     if (m == 0 || n == 0) return T0_OK;
     if (lda < k || ldb < n || ldc < n) return fail(T0_ERR_INVALID, "leading dimensions (%u, %u, %u) smaller than the rows they stride (%u, %u, %u)", lda, ldb, ldc, k, n, n);
     DeviceGuard guard(rt->device);
-    uint64_t xa = 0, xb = 0;
-    rc = convert(rt, rt->scratch_cvt_a, a, m, k, lda, false, &xa);
-    if (rc == T0_OK) rc = convert(rt, rt->scratch_cvt_b, b, k, n, ldb, false, &xb);
-    if (rc != T0_OK) return rc;
     const bool direct = alpha == 1.0f && beta == 0.0f && ldc == n;
     uint64_t t = c;
     if (!direct) {
@@ -207,7 +197,7 @@ int t0_blas_gemm_f32(t0_runtime* rt, uint32_t m, uint32_t n, uint32_t k, float a
         if (rc != T0_OK) return rc;
         t = (uint64_t)(uintptr_t)rt->scratch_cvt_c.ptr;
     }
-    rc = gemm_bf16(rt, xa, xb, t, m, n, k, T0_NN);
+    rc = product(rt, a, lda, false, b, ldb, true, t, m, n, k);
     if (rc != T0_OK || direct) return rc;
     axpby_kernel<<<blocks_for((uint64_t)m * n, 1024, rt->sm_count), 256, 0, rt->stream>>>((const float*)t, (float*)c, m, n, ldc, alpha, beta);
     cudaError_t e = cudaGetLastError();

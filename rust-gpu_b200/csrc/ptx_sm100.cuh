@@ -276,12 +276,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
 }
 
 // Instruction descriptor for kind::f16 with bf16 A/B and f32 accumulation, M x N tile.
-// b_mn_major = 1 when B is stored N-contiguous in shared memory.
-__host__ __device__ constexpr uint32_t make_idesc_bf16_f32(uint32_t m, uint32_t n, uint32_t b_mn_major) {
+// b_mn_major = 1 when B is stored N-contiguous in shared memory, a_mn_major = 1 when A is stored M-contiguous.
+__host__ __device__ constexpr uint32_t make_idesc_bf16_f32(uint32_t m, uint32_t n, uint32_t b_mn_major, uint32_t a_mn_major = 0) {
     return (1u << 4)            // D format f32
          | (1u << 7)            // A format bf16
          | (1u << 10)           // B format bf16
-         | (0u << 15)           // A K-major
+         | (a_mn_major << 15)   // A major
          | (b_mn_major << 16)   // B major
          | ((n >> 3) << 17)
          | ((m >> 4) << 24);

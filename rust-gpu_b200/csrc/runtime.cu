@@ -12,8 +12,10 @@ namespace {
 struct GemmRequest {
     uint64_t x, b, y, bias;
     uint32_t m, n, k;
+    uint32_t ldx, ldb;         // row strides in elements, multiples of 8 (0 = dense)
     uint32_t tile_n, split_k;
     bool nn, out_bf16, planes, swap_grid;
+    bool at;                   // x is [K,M] (with nn)
     int pair;                  // 0 = choose by shape, 1 = CTA-pair kernel, 2 = single-CTA kernel
     uint64_t plane_stride;     // elements; only when planes
     uint8_t epilogue, n_ops;
@@ -77,7 +79,8 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     memset(&g, 0, sizeof g);
     g.x = (const void*)q.x; g.b = (const void*)q.b;
     g.m = q.m; g.n = q.n; g.k = q.k;
-    g.nn = q.nn; g.swap_grid = q.swap_grid;
+    g.ldx = q.ldx; g.ldb = q.ldb;
+    g.nn = q.nn; g.at = q.at; g.swap_grid = q.swap_grid;
     g.status = rt->d_status; g.probe = rt->d_probe; g.n_sms = (uint32_t)rt->sm_count;
     g.wait_limit_ns = rt->wait_limit_ns.load(std::memory_order_relaxed);
     g.drop_load = rt->drop_next_load.exchange(0) != 0;
@@ -94,8 +97,9 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
 
     // --- staging for shapes the TMA path cannot address (row stride or base not 16-byte aligned)
     const uint32_t kps = q.k / split;
-    const bool x_bad = (q.k % 8) || (q.x & 15);
-    const bool b_bad = q.nn ? ((q.n % 8) || (q.b & 15)) : ((q.k % 8) || (q.b & 15));
+    const bool x_bad = ((q.ldx ? q.ldx : q.at ? q.m : q.k) % 8) || (q.x & 15);
+    const bool b_bad = ((q.ldb ? q.ldb : q.nn ? q.n : q.k) % 8) || (q.b & 15);
+    if ((x_bad && (q.at || q.ldx)) || (b_bad && q.ldb)) return fail(T0_ERR_UNSUPPORTED, "operands given with a row stride must be 16-byte aligned, stride and base");
     if ((x_bad || b_bad || (kps % 8)) && split > 1)
         return fail(T0_ERR_UNSUPPORTED, "split-K needs K/split_k %% 8 == 0 and 16-byte aligned operands (K=%u, split_k=%u)", q.k, split);
     const uint32_t k_pad = (q.k + 7) & ~7u;
@@ -181,6 +185,27 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     rt->launches.fetch_add(1);
     return T0_OK;
 }
+
+}  // namespace
+
+namespace t0 {
+
+// The product of two bf16 operands with row strides (elements, multiples of 8) into a dense f32 [m,n]: the library's own choice of
+// kernel.  `at`: the first operand is [k,m]; `nn`: the second is [k,n].  Called with the runtime checked and its device current.
+int gemm_strided(t0_runtime* rt, uint64_t a, uint32_t lda, bool at, uint64_t b, uint32_t ldb, bool nn, uint64_t y, uint32_t m, uint32_t n, uint32_t k) {
+    GemmRequest q;
+    memset(&q, 0, sizeof q);
+    q.x = a; q.b = b; q.y = y;
+    q.m = m; q.n = n; q.k = k;
+    q.ldx = lda; q.ldb = ldb;
+    q.at = at; q.nn = nn; q.swap_grid = true;
+    q.scale = 1.0f;
+    return run_gemm(rt, q);
+}
+
+}  // namespace t0
+
+namespace {
 
 // Bytes available from `addr` to the end of the live allocation containing it, or SIZE_MAX when the
 // address belongs to no allocation of this runtime (foreign device memory).

@@ -69,3 +69,24 @@ def test_epilogue_chain_on_every_kernel(t0, rt, pair, tile_n, split_k, out_bf16)
     # f32 elementwise: a few roundings of 2^-24 each, exp2 of an argument of up to ~40 adds |argument| * 2^-24 to the relative error
     tol = 1e-5 * np.abs(v) + 1e-6
     assert np.all(np.abs(got - v) <= tol + (2.0 ** -8 * np.abs(v) if out_bf16 else 0))
+
+
+@pytest.mark.parametrize("m,k,n", [(3, 5, 7), (64, 64, 64), (100, 72, 200), (513, 264, 1000), (2048, 384, 640), (1024, 1024, 2056), (65, 1001, 30)])
+def test_f32_products_are_exact_on_integers(t0, rt, m, k, n):
+    # forward and both gradients; X^T is read as it lies (the tensor cores take it M-major), widths off the 16-byte rule are padded
+    rng = np.random.default_rng(m)
+    x, w, dy = ints(rng, m, k), ints(rng, k, n), ints(rng, m, n)
+    xd, wd, dyd = rt.upload(x), rt.upload(w), rt.upload(dy)
+    for call, rows, cols, want in ((lambda y: rt.matmul_f32(xd.gpu_addr(), wd.gpu_addr(), y, m, k, n), m, n, x @ w),
+                                   (lambda y: rt.matmul_f32_backward_data(dyd.gpu_addr(), wd.gpu_addr(), y, m, k, n), m, k, dy @ w.T),
+                                   (lambda y: rt.matmul_f32_backward_weight(xd.gpu_addr(), dyd.gpu_addr(), y, m, k, n), k, n, x.T @ dy)):
+        y = rt.alloc(rows * cols * 4 + GUARD)
+        y.write(np.full(rows * cols * 4 + GUARD, 0xA5, np.uint8))
+        call(y.gpu_addr())
+        rt.synchronize()
+        raw = y.read(rows * cols * 4 + GUARD, np.uint8)
+        assert np.array_equal(raw[:rows * cols * 4].view(np.float32).reshape(rows, cols), want)
+        assert np.all(raw[rows * cols * 4:] == 0xA5), "wrote past the output"
+        y.free()
+    for b in (xd, wd, dyd):
+        b.free()
