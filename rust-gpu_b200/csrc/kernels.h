@@ -68,8 +68,15 @@ int launch_splitk_reduce(const float* planes, void* y, const float* bias, uint32
                          bool out_bf16, uint8_t epilogue, uint8_t n_ops, const uint8_t* ops, float scale, float clamp_min,
                          float clamp_max, cudaStream_t stream);
 
-// dst[r][0..dst_cols) = src[r][0..cols) zero-extended, 16-bit elements (staging copy for shapes TMA cannot address).
-int launch_pad_copy_u16(const void* src, void* dst, uint32_t rows, uint32_t cols, uint32_t dst_cols, cudaStream_t stream);
+// dst[r][0..dst_cols) = src[r][0..cols) zero-extended, 16-bit elements (staging copy for shapes TMA cannot address).  dst_cols is a
+// multiple of 8 and dst 16-byte aligned; src and cols are anything.
+struct PadCopy {
+    const uint16_t* src;
+    uint16_t* dst;
+    uint32_t rows, cols, dst_cols;
+};
+// Up to two copies in one launch (rows = 0: none).
+int launch_pad_copy_u16(const PadCopy& a, const PadCopy& b, cudaStream_t stream);
 
 int launch_fill_uniform_bf16(void* dst, uint64_t n, uint64_t seed, uint64_t first, cudaStream_t stream);
 int launch_fill_u32(void* dst, uint64_t n, uint64_t seed, uint64_t first, cudaStream_t stream);

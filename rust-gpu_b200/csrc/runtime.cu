@@ -103,29 +103,23 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     if ((x_bad || b_bad || (kps % 8)) && split > 1)
         return fail(T0_ERR_UNSUPPORTED, "split-K needs K/split_k %% 8 == 0 and 16-byte aligned operands (K=%u, split_k=%u)", q.k, split);
     const uint32_t k_pad = (q.k + 7) & ~7u;
+    PadCopy pad[2] = {};
     if (x_bad) {
         int rc = ensure_scratch(rt, rt->scratch_a, (size_t)q.m * k_pad * 2);
         if (rc != T0_OK) return rc;
-        rc = launch_pad_copy_u16((const void*)q.x, rt->scratch_a.ptr, q.m, q.k, k_pad, rt->stream);
-        if (rc != T0_OK) return rc;
-        rt->launches.fetch_add(1);
+        pad[0] = PadCopy{(const uint16_t*)q.x, (uint16_t*)rt->scratch_a.ptr, q.m, q.k, k_pad};
         g.x = rt->scratch_a.ptr; g.ldx = k_pad;
     }
     if (b_bad) {
-        if (q.nn) {
-            const uint32_t n_pad = (q.n + 7) & ~7u;
-            int rc = ensure_scratch(rt, rt->scratch_b, (size_t)q.k * n_pad * 2);
-            if (rc != T0_OK) return rc;
-            rc = launch_pad_copy_u16((const void*)q.b, rt->scratch_b.ptr, q.k, q.n, n_pad, rt->stream);
-            if (rc != T0_OK) return rc;
-            g.b = rt->scratch_b.ptr; g.ldb = n_pad;
-        } else {
-            int rc = ensure_scratch(rt, rt->scratch_b, (size_t)q.n * k_pad * 2);
-            if (rc != T0_OK) return rc;
-            rc = launch_pad_copy_u16((const void*)q.b, rt->scratch_b.ptr, q.n, q.k, k_pad, rt->stream);
-            if (rc != T0_OK) return rc;
-            g.b = rt->scratch_b.ptr; g.ldb = k_pad;
-        }
+        const uint32_t rows = q.nn ? q.k : q.n, cols = q.nn ? q.n : q.k, cols_pad = (cols + 7) & ~7u;
+        int rc = ensure_scratch(rt, rt->scratch_b, (size_t)rows * cols_pad * 2);
+        if (rc != T0_OK) return rc;
+        pad[1] = PadCopy{(const uint16_t*)q.b, (uint16_t*)rt->scratch_b.ptr, rows, cols, cols_pad};
+        g.b = rt->scratch_b.ptr; g.ldb = cols_pad;
+    }
+    if (x_bad || b_bad) {
+        int rc = launch_pad_copy_u16(pad[0], pad[1], rt->stream);
+        if (rc != T0_OK) return rc;
         rt->launches.fetch_add(1);
     }
 

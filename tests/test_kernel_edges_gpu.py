@@ -90,3 +90,15 @@ def test_f32_products_are_exact_on_integers(t0, rt, m, k, n):
         y.free()
     for b in (xd, wd, dyd):
         b.free()
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+@pytest.mark.parametrize("m,n,k", [(5, 9, 3), (64, 65, 77), (130, 111, 250), (257, 1030, 129)])
+@pytest.mark.parametrize("x_skip,b_skip", [(0, 0), (1, 0), (0, 3), (1, 1), (2, 4)])
+def test_operands_at_any_element_address(t0, rt, layout, m, n, k, x_skip, b_skip):
+    # rows that start at odd elements, bases inside a word: the staging copy reads whole words and shifts
+    rng = np.random.default_rng(m + k)
+    x, b = ints(rng, m, k), ints(rng, n, k)
+    nn = layout == "nn"
+    got = run_gemm(t0, rt, x, b.T if nn else b, m, n, k, x_skip=x_skip, b_skip=b_skip, transpose=t0.NN if nn else t0.NT)
+    assert np.array_equal(got, x @ b.T)
