@@ -338,12 +338,11 @@ int t0_rt_new(int device, t0_runtime** out) {
     T0_CUDA(cudaStreamCreateWithFlags(&rt->stream, cudaStreamNonBlocking));
     T0_CUDA(cudaEventCreate(&rt->ev_start));
     T0_CUDA(cudaEventCreate(&rt->ev_stop));
-    T0_CUDA(cudaMalloc(&rt->d_status, sizeof(int)));
-    T0_CUDA(cudaMemset(rt->d_status, 0, sizeof(int)));
     T0_CUDA(cudaMalloc(&rt->d_probe, (2 + 64) * sizeof(unsigned long long)));   // clock words + eight launches' trace stamps
     T0_CUDA(cudaMemset(rt->d_probe, 0, (2 + 64) * sizeof(unsigned long long)));
-    T0_CUDA(cudaMallocHost(&rt->h_status, sizeof(int)));
+    T0_CUDA(cudaHostAlloc(&rt->h_status, sizeof(int), cudaHostAllocMapped));
     *rt->h_status = 0;
+    T0_CUDA(cudaHostGetDevicePointer(&rt->d_status, rt->h_status, 0));
     *out = rt.release();
     return T0_OK;
 }
@@ -356,7 +355,6 @@ void t0_rt_free(t0_runtime* rt) {
     t0_rt_pool_clear(rt);
     for (Scratch* s : {&rt->scratch_a, &rt->scratch_b, &rt->scratch_planes, &rt->scratch_w4, &rt->scratch_w, &rt->scratch_cvt_a, &rt->scratch_cvt_b, &rt->scratch_cvt_c})
         if (s->ptr) cudaFree(s->ptr);
-    if (rt->d_status) cudaFree(rt->d_status);
     if (rt->d_probe) cudaFree(rt->d_probe);
     if (rt->d_peer_maps) cudaFree(rt->d_peer_maps);
     if (rt->h_status) cudaFreeHost(rt->h_status);
