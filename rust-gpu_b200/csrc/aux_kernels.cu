@@ -17,11 +17,6 @@ struct EpiParams {
     uint8_t ops[T0_TILE_MAX_EPILOGUE];
 };
 
-__device__ __forceinline__ float sigmoid_seq(float x) {
-    const float e = exp2f((-x) * 1.44269504088896340736f);
-    return __frcp_rn(e + 1.0f);
-}
-
 __device__ __forceinline__ float apply_epilogue(float v, uint32_t col, const EpiParams& e) {
     if (e.n_ops) {
         for (uint32_t o = 0; o < e.n_ops; ++o) {
@@ -29,8 +24,8 @@ __device__ __forceinline__ float apply_epilogue(float v, uint32_t col, const Epi
                 case T0_TEPI_BIAS_ADD: if (e.bias) v = v + __ldg(e.bias + col); break;
                 case T0_TEPI_SCALE: v = v * e.scale; break;
                 case T0_TEPI_RELU: v = fmaxf(v, 0.0f); break;
-                case T0_TEPI_SILU: v = v * sigmoid_seq(v); break;
-                case T0_TEPI_GELU: v = v * sigmoid_seq(v * 1.702f); break;
+                case T0_TEPI_SILU: v = v * gemm::sigmoid_seq(v); break;
+                case T0_TEPI_GELU: v = v * gemm::sigmoid_seq(v * 1.702f); break;
                 case T0_TEPI_ABS: v = fabsf(v); break;
                 case T0_TEPI_NEG: v = -v; break;
                 case T0_TEPI_CLAMP: v = fminf(fmaxf(v, e.clamp_min), e.clamp_max); break;
