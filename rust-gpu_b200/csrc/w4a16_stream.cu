@@ -12,13 +12,18 @@
 //     one list, cut into equal contiguous ranges, one per CTA (one CTA per SM), so that launch, pipeline fill and the band
 //     fix-up at the end of a range are paid once per launch instead of once per problem;
 //   * warp 16 (one lane) streams the tiles of the range into a ring of stages with one 16 KiB bulk copy each;
-//   * warps 17..20 prepare, one step each in turn and a few steps ahead of the consumers, what else a step needs in the
+//   * warps 17..19 prepare, one step each in turn and a few steps ahead of the consumers, what else a step needs in the
 //     same stage: the activations of the step as mma.sync B fragments, and per column pair the words {128+z, s} the
 //     dequantisation uses, so that a consumer gets them with one 16-byte load and no decoding;
-//   * warps 0..15 (consumers) own 16 columns of the band each: two LDS.128 fetch a lane's eight packed words of a step;
-//     nibble pairs become bf16x2 with one LOP3 (0x4300 | q is the bf16 128+q), minus (128+z), times s - bit-identical
-//     to the oracle because (q-z)*s is rounded once - and every dequantised word IS the 16 x 16 A fragment of one
-//     mma.sync.m16n8k16 whose 8-column B operand is the activations;
+//   * warps 0..15 (consumers): warps 2i and 2i + 1 own columns 32i .. 32i + 31 of the band, each one k half of every step: two
+//     LDS.128 fetch a lane's eight packed words; nibble pairs become bf16x2 with one LOP3 (0x4300 | q is the bf16 128+q), minus
+//     (128+z), times s - bit-identical to the oracle because (q-z)*s is rounded once - and every dequantised word IS the
+//     16 x 16 A fragment of one mma.sync.m16n8k16 whose 8-column B operand is the activations.  The two halves meet in shared
+//     memory when a band ends.
+//     What bounds this loop is the instructions around the arithmetic as much as the arithmetic (15 per packed word of 8 codes, 8 words
+//     per warp and step) and, with two row groups, the rate of mma.sync (leaving the dequantisation out changes nothing at M = 16).  A
+//     warp that owned 16 columns and the whole k of a step read all the activation fragments of the step for half the columns, and 21
+//     warps left 80 registers a thread: 12 problems of M = 1, N = 11008, K = 4096 took 80.4 us, 70.5 so; two of them 19.3 and 18.7.
 //   * a band that lies wholly inside a range is stored directly; a band shared by several CTAs is finished by whichever
 //     CTA arrives last (per-band arrival counter, partial pieces in scratch, added in k order: deterministic, repeated
 //     calls agree bit for bit); no CTA ever waits for another.  A spare lane of the producer warp counts a range's leading
@@ -32,18 +37,21 @@ using namespace t0::w4;
 
 namespace {
 
-constexpr int kStConsumers = 16;                      // consumer warps: warp w owns columns 16w .. 16w+15 of the band, all k of a step
-constexpr int kStHelpers = 4;                         // warps that prepare activations and scale / zero-point words
+constexpr int kStConsumers = 16;                      // consumer warps: warp w owns columns 32 (w / 2) .. + 31 of the band, k half w % 2 of every step
+constexpr int kStHelpers = 3;                         // warps that prepare activations and scale / zero-point words
 constexpr int kStProducerWarp = kStConsumers;
 constexpr int kStHelperWarp0 = kStConsumers + 1;
-constexpr int kStThreads = (kStHelperWarp0 + kStHelpers) * 32;    // 672 = 21 warps
+constexpr int kStThreads = (kStHelperWarp0 + kStHelpers) * 32;    // 640: five warps per scheduler, which leaves 96 registers a thread
 constexpr int kStSzBytes = 2048;                      // per stage: [16 warps][8 g] uint4 {128+z(col), s(col), 128+z(col+8), s(col+8)} as bf16x2 pairs
 constexpr int kStAFragBytes = 2048;                   // per stage and group of eight rows: [2 j][2 pr][32 lanes] uint4 B fragments
 constexpr int kStMaxProblems = 32;                    // problems per launch (the table travels as a kernel parameter)
 
 __host__ __device__ constexpr int st_stage_bytes(int m_groups) { return kWeightBytes + kStSzBytes + m_groups * kStAFragBytes; }
-__host__ __device__ constexpr int st_stages(int m_groups) { return m_groups == 1 ? 11 : 10; }
-__host__ __device__ constexpr size_t st_smem_bytes(int m_groups) { return 128 + (size_t)st_stages(m_groups) * st_stage_bytes(m_groups) + 512; }
+__host__ __device__ constexpr int st_stages(int m_groups) { return m_groups == 1 ? 10 : 9; }
+__host__ __device__ constexpr int st_exchange_bytes(int m_groups) { return kStConsumers * m_groups * 512; }     // one accumulator fragment per warp and row group
+__host__ __device__ constexpr size_t st_smem_bytes(int m_groups) {
+    return 128 + (size_t)st_stages(m_groups) * st_stage_bytes(m_groups) + 256 + st_exchange_bytes(m_groups);
+}
 
 struct StProblem {
     const uint16_t* a;         // [M][K] bf16
@@ -66,8 +74,6 @@ struct StParams {
     unsigned long long* stamps;   // optional trace: 4 nanosecond stamps per CTA (entry, first step landed, loop done, exit)
     uint64_t wait_limit_ns;
     uint32_t n_problems, total_units;
-    uint32_t probe;            // timing experiments, only in builds with -DT0_W4_PROBE (results are then wrong on purpose):
-                               // 1 = consumers skip the arithmetic, 2 = the producer copies nothing, 3 = both
 };
 
 struct Cursor { uint32_t p, band, ks; };
@@ -88,6 +94,8 @@ __device__ __forceinline__ void advance(const StParams& P, Cursor& c) {
     }
 }
 
+// the two warps of a column pair (barriers 2..9; 1 is the consumers')
+__device__ __forceinline__ void st_pair_sync(uint32_t pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 2) : "memory"); }
 __device__ __forceinline__ void st_consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStConsumers * 32) : "memory"); }
 // explicit shared-space accesses: the ring's address went through an integer for alignment, so plain pointers would make
 // the compiler use generic loads and 64-bit address arithmetic
@@ -111,16 +119,12 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
     const uint32_t empty_bar = full_bar + kSt * 8;
     const uint32_t head_written_bar = empty_bar + kSt * 8;               // all 16 consumer warps have stored their part of the head piece
     const uint32_t head_counted_bar = head_written_bar + 8;              // the head piece is counted in and s_head_last is valid
+    const uint32_t exchange = full_bar + 256;                            // [16 warps][kMGroups][32 lanes] float4
     __shared__ int s_flags[4];
     volatile int* abort_flag = &s_flags[0];
     int* s_last = &s_flags[1];
     int* s_head_last = &s_flags[2];                                      // 1 when this CTA turned out to be the last contributor of its head band
 
-#ifdef T0_W4_PROBE
-    const uint32_t probe = P.probe;
-#else
-    constexpr uint32_t probe = 0;
-#endif
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t U0 = range_begin(blockIdx.x, gridDim.x, P.total_units);
     const uint32_t U1 = range_begin(blockIdx.x + 1, gridDim.x, P.total_units);
@@ -142,10 +146,10 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
     }
     __syncthreads();
     ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();      // global memory is touched only after the previous grid in the stream is done
-    if (tid == 0) stamp(0);
     const Cursor c0 = locate(P, U0);
     const uint32_t n_units = U1 - U0;
+    ptx::grid_dependency_wait();      // global memory is read and written only after the previous grid in the stream is done
+    if (tid == 0) stamp(0);
     // A head piece: the range starts inside a band and goes on into the next one.  Counting it in (fence, atomic round
     // trip) is the head warp's job, so no consumer warp falls behind the others while the range goes on.
     const uint32_t head_end = U0 - c0.ks + P.prob[c0.p].ksteps;    // one past the last unit of the first band
@@ -184,12 +188,8 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
                 // step loaded into the same stage a ring later.
                 ptx::fence_proxy_async_smem();
                 const uint32_t fb = full_bar + stage * 8;
-                if (probe & 2) {
-                    ptx::mbar_arrive(fb);
-                } else {
-                    ptx::mbar_arrive_expect_tx(fb, kWeightBytes);
-                    ptx::bulk_load(ring + stage * kSB, src, kWeightBytes, fb);
-                }
+                ptx::mbar_arrive_expect_tx(fb, kWeightBytes);
+                ptx::bulk_load(ring + stage * kSB, src, kWeightBytes, fb);
                 if (++stage == kSt) { stage = 0; phase ^= 1; }
                 // the tiles of one problem are consecutive in memory in the order the range walks them
                 src += kWeightBytes;
@@ -202,7 +202,7 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
         return;
     }
     if (warp >= kStHelperWarp0) {
-        // ------------------------------------------------------------ helpers: step i of the range is prepared by helper i % 4
+        // ------------------------------------------------------------ helpers: step i of the range is prepared by helper i % kStHelpers
         const uint32_t h = warp - kStHelperWarp0;
         if (h >= n_units) return;
         Cursor c = c0;
@@ -222,16 +222,6 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
                 zbase = pr.zeros_t + w2 * 8;
             }
             const uint32_t stage = i % kSt, round = i / kSt;
-            if (probe & 4) {      // timing experiment: no preparation, only the hand-off
-                uint32_t okp = 1;
-                if (lane == 0 && !ptx::mbar_wait_relaxed(empty_bar + stage * 8, (round & 1) ^ 1, abort_flag, P.wait_limit_ns, 400)) okp = 0;
-                okp = __shfl_sync(0xFFFFFFFFu, okp, 0);
-                if (!okp) break;
-                if (lane == 0) ptx::mbar_arrive(full_bar + stage * 8);
-                i += kStHelpers;
-                if (i >= n_units) break;
-                continue;
-            }
             // loads first (they do not touch the stage), then the wait for the stage, then the stores
             // -- scale / zero-point words: entry e = 8w + g serves consumer warp w, lanes g: columns 16w + g and 16w + g + 8
             const size_t sz_row = (size_t)c.band * groups + c.ks / upg;
@@ -297,32 +287,26 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
 
     // ---------------------------------------------------------------- consumers (16 warps)
     const uint32_t g = lane >> 2, t = lane & 3;
-    // four accumulator sets, one per k step modulo 4: consecutive MMAs must not wait for each other's result
-    constexpr int kAccSets = 4;
-    float acc[kMGroups][kAccSets][4];
+    const uint32_t pair = warp >> 1, khalf = warp & 1;        // columns 32 pair .. + 31, k half of every step
+    // per row group and column group two accumulator sets, taken in turn: consecutive MMAs must not wait for each other's result
+    float acc[kMGroups][2][2][4];
 #pragma unroll
     for (int mg = 0; mg < kMGroups; ++mg)
 #pragma unroll
-        for (int a = 0; a < kAccSets; ++a)
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[mg][a][j] = 0.0f;
+            for (int j = 0; j < 4; ++j) acc[mg][a >> 1][a & 1][j] = 0.0f;
     uint32_t mask, magic;
     asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
     asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
     Cursor c = c0;
     bool ok = true;    // false after a wait expired: the warps keep walking (barriers stay matched) but do no work
-    const uint32_t col0 = warp * 16 + g;                      // this lane's two columns within the band: col0 and col0 + 8
-    // a lane's places in the current stage: eight packed words [w][j][lane] uint4, the scale / zero words of its column pair,
-    // its B fragments; the stage's barriers
-    uint32_t st_w = ring + warp * 1024 + lane * 16;
-    uint32_t st_sz = ring + kWeightBytes + (warp * 8 + g) * 16;
-    uint32_t st_af = ring + kWeightBytes + kStSzBytes + lane * 16;
-    uint32_t fb = full_bar, eb = empty_bar, stage = 0, phase = 0;
-#ifdef T0_W4_PROBE
-    bool first_step = true;
-    long long wait_cycles = 0;
-    const long long cyc0 = clock64();
-#endif
+    const uint32_t col0 = warp * 16 + g;                      // the lane's two columns within the band once the k halves are added: col0 and col0 + 8
+    // a lane's place in a stage's words ([16 column groups][2 k halves][32 lanes] uint4), scale / zero words and B fragments
+    const uint32_t lane_w = ring + pair * 2048 + khalf * 512 + lane * 16;
+    const uint32_t lane_sz = ring + kWeightBytes + (pair * 16 + g) * 16;
+    const uint32_t lane_af = ring + kWeightBytes + kStSzBytes + khalf * 1024 + lane * 16;
+    uint32_t stage = 0, phase = 0;
 
     // The CTA that contributes last to a band adds the pieces in k order (CTA order) and stores; nobody waits for anybody.
     // Only the first contributor can hold the band in slot 1 (its range began in the band before).
@@ -376,22 +360,36 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
         const uint32_t c_last = owner_of(last_unit - 1, gridDim.x, P.total_units);
         const uint32_t slot = (first_unit <= U0) ? 0u : 1u;   // the piece of the band holding this CTA's first unit is slot 0
         float* piece = P.partials + ((size_t)blockIdx.x * 2 + slot) * kPieceFloats;
+        // The two k halves meet: a warp gives the other's column group away and keeps its own (column group khalf of the pair).
+#pragma unroll
+        for (int mg = 0; mg < kMGroups; ++mg) {
+            float give[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) give[j] = khalf ? acc[mg][0][0][j] + acc[mg][0][1][j] : acc[mg][1][0][j] + acc[mg][1][1][j];
+            sts128(exchange + ((warp ^ 1) * kMGroups + mg) * 512 + lane * 16,
+                   make_uint4(__float_as_uint(give[0]), __float_as_uint(give[1]), __float_as_uint(give[2]), __float_as_uint(give[3])));
+        }
+        st_pair_sync(pair);
         // accumulator fragment: c0,c1 = (column col0, rows 2t, 2t+1), c2,c3 = (column col0 + 8, same rows)
 #pragma unroll
         for (int mg = 0; mg < kMGroups; ++mg) {
+            const uint4 got4 = lds128(exchange + (warp * kMGroups + mg) * 512 + lane * 16);
+            const uint32_t got[4] = {got4.x, got4.y, got4.z, got4.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const uint32_t m = mg * 8 + 2 * t + (j & 1), col = col0 + (j >> 1) * 8;
                 const uint32_t ncol = c.band * kBandCols + col;
-                const float v = (acc[mg][0][j] + acc[mg][1][j]) + (acc[mg][2][j] + acc[mg][3][j]);
+                const float own = khalf ? acc[mg][1][0][j] + acc[mg][1][1][j] : acc[mg][0][0][j] + acc[mg][0][1][j];
+                const float v = khalf ? __uint_as_float(got[j]) + own : own + __uint_as_float(got[j]);      // lower k half first
                 if (m < pr.M) {
                     if (!whole) piece[m * kBandCols + col] = v;
                     else if (ncol < pr.N) pr.y[(size_t)m * pr.N + ncol] = v;
                 }
 #pragma unroll
-                for (int a = 0; a < kAccSets; ++a) acc[mg][a][j] = 0.0f;
+                for (int a = 0; a < 4; ++a) acc[mg][a >> 1][a & 1][j] = 0.0f;
             }
         }
+        st_pair_sync(pair);                                    // both have read before either writes again
         if (!whole) {
             if (u_next < U1) {
                 // head piece, more steps follow: hand it to the counting lane and go on
@@ -412,65 +410,70 @@ w4a16_stream_kernel(const __grid_constant__ StParams P) {
         if (++c.band == pr.n_bands) { c.band = 0; ++c.p; }
     };
 
-    // every warp walks the ring at its own pace: it waits for the stage, reads its words, and tells the producer when it is done
+    // Every warp walks the ring at its own pace: it waits for the stage, reads it, and tells the producer when it is done.  The words of
+    // the next step are fetched before the arithmetic of this one when they are there already, so that a warp does not begin each
+    // step with an empty pipeline.
     uint32_t ksteps_cur = P.prob[c.p].ksteps;
-    for (uint32_t u = U0; u < U1; ++u) {
-#ifdef T0_W4_PROBE
-        const long long tw0 = clock64();
-#endif
-        if (ok && !ptx::mbar_wait(fb, phase, abort_flag, P.wait_limit_ns)) {
+    uint4 q[2];
+    auto wait_stage = [&](uint32_t u, uint32_t s, uint32_t ph) {
+        if (ok && !ptx::mbar_wait(full_bar + s * 8, ph, abort_flag, P.wait_limit_ns)) {
             if (lane == 0) atomicCAS(P.status, 0, kStatusMmaTimeout | (int)(u & 0xFFFFFF));
             ok = false;
         }
-#ifdef T0_W4_PROBE
-        if (!first_step) wait_cycles += clock64() - tw0;      // (the first step's wait is the pipeline fill)
-        if (first_step && tid == 0) stamp(1);
-        first_step = false;
-#endif
-        if (ok && !(probe & 1)) {
-            const uint4 q0 = lds128(st_w);
-            const uint4 q1 = lds128(st_w + 512);
-            const uint4 sz = lds128(st_sz);          // {128+z, s} of column col0, then of col0 + 8
-            const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    };
+    wait_stage(U0, 0, 0);
+    if (tid == 0) stamp(1);
+    q[0] = lds128(lane_w);
+    q[1] = lds128(lane_w + 1024);
+    for (uint32_t u = U0; u < U1; ++u) {
+        const uint32_t off = stage * kSB;
+        uint32_t next = stage + 1, next_phase = phase;
+        if (next == kSt) { next = 0; next_phase ^= 1; }
+        bool ready = false;
+        if (ok) {
+            uint4 sz[2], bf[kMGroups][2];
+            sz[0] = lds128(lane_sz + off);               // {128+z, s} of columns g, then g + 8, of the first column group
+            sz[1] = lds128(lane_sz + off + 128);         // ... of the second
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
+            for (int mg = 0; mg < kMGroups; ++mg)        // (rows that do not exist: stale bytes, whose products are never stored)
 #pragma unroll
-                for (int p2 = 0; p2 < 2; ++p2) {
-                    uint4 bf[kMGroups];
+                for (int p2 = 0; p2 < 2; ++p2) bf[mg][p2] = lds128(lane_af + off + mg * kStAFragBytes + p2 * 512);
+            ready = u + 1 < U1 && ptx::mbar_try_wait(full_bar + next * 8, next_phase);
+            uint4 n0 = q[0], n1 = q[1];
+            if (ready) {
+                n0 = lds128(lane_w + next * kSB);
+                n1 = lds128(lane_w + next * kSB + 1024);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                // k step 4 khalf + e: one word per column group
+#pragma unroll
+                for (int cg = 0; cg < 2; ++cg) {
+                    const uint32_t wd = e == 0 ? q[cg].x : e == 1 ? q[cg].y : e == 2 ? q[cg].z : q[cg].w;
+                    const uint32_t a0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), sz[cg].x), sz[cg].y);
+                    const uint32_t a1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), sz[cg].z), sz[cg].w);
+                    const uint32_t a2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), sz[cg].x), sz[cg].y);
+                    const uint32_t a3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), sz[cg].z), sz[cg].w);
 #pragma unroll
                     for (int mg = 0; mg < kMGroups; ++mg) {
-                        bf[mg] = lds128(st_af + ((mg * 2 + j) * 2 + p2) * 512);     // (rows that do not exist: stale bytes, whose products are never stored)
-                    }
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const uint32_t wd = words[j * 4 + p2 * 2 + e];
-                        const uint32_t a0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), sz.x), sz.y);
-                        const uint32_t a1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), sz.z), sz.w);
-                        const uint32_t a2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), sz.x), sz.y);
-                        const uint32_t a3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), sz.z), sz.w);
-#pragma unroll
-                        for (int mg = 0; mg < kMGroups; ++mg)
-                            mma_bf16_16816(acc[mg][p2 * 2 + e], a0, a1, a2, a3, e ? bf[mg].z : bf[mg].x, e ? bf[mg].w : bf[mg].y);
+                        const uint4& b = bf[mg][e >> 1];
+                        mma_bf16_16816(acc[mg][cg][e & 1], a0, a1, a2, a3, e & 1 ? b.z : b.x, e & 1 ? b.w : b.y);
                     }
                 }
             }
-        }
-        if (ok) {
+            q[0] = n0; q[1] = n1;
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(eb);          // this warp has read the stage
+            if (lane == 0) ptx::mbar_arrive(empty_bar + stage * 8);          // this warp has read the stage
         }
-        st_w += kSB; st_sz += kSB; st_af += kSB; fb += 8; eb += 8;
-        if (++stage == kSt) {
-            stage = 0; phase ^= 1;
-            st_w -= kSt * kSB; st_sz -= kSt * kSB; st_af -= kSt * kSB; fb -= kSt * 8; eb -= kSt * 8;
-        }
+        stage = next; phase = next_phase;
         if (++c.ks == ksteps_cur || u + 1 == U1) {
-#ifdef T0_W4_PROBE
-            if (u + 1 == U1 && tid == 0 && P.stamps) { P.stamps[gridDim.x * 4 + blockIdx.x] = (unsigned long long)(clock64() - cyc0); P.stamps[gridDim.x * 5 + blockIdx.x] = (unsigned long long)wait_cycles; }
-#endif
             if (u + 1 == U1 && tid == 0) stamp(2);
             flush_piece(u + 1);
             if (u + 1 < U1) ksteps_cur = P.prob[c.p].ksteps;
+        }
+        if (u + 1 < U1 && !ready) {
+            wait_stage(u + 1, stage, phase);
+            q[0] = lds128(lane_w + stage * kSB);
+            q[1] = lds128(lane_w + stage * kSB + 1024);
         }
     }
     if (has_head) {
@@ -596,9 +599,6 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
     const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
     P.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
     P.n_problems = (uint32_t)count; P.total_units = (uint32_t)total;
-#ifdef T0_W4_PROBE
-    if (const char* pm = getenv("T0_W4_PROBE")) P.probe = (uint32_t)atoi(pm);
-#endif
     const int m_groups = max_m <= 8 ? 1 : 2;
     static bool attr_set[64] = {};
     if (rt->device < 64 && !attr_set[rt->device]) {
@@ -640,18 +640,6 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
             fill += (double)(h[c * 4 + 1] - h[c * 4]); loop += (double)(h[c * 4 + 2] - h[c * 4 + 1]); tail += (double)(h[c * 4 + 3] - h[c * 4 + 2]);
             if (h[c * 4 + 3] - h[c * 4] > h[slow * 4 + 3] - h[slow * 4]) slow = c;
         }
-#ifdef T0_W4_PROBE
-        {
-            std::vector<unsigned long long> cy(grid);
-            T0_CUDA(cudaMemcpy(cy.data(), stamps.d + (size_t)grid * 4, cy.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-            std::vector<unsigned long long> wt(grid);
-            T0_CUDA(cudaMemcpy(wt.data(), stamps.d + (size_t)grid * 5, wt.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-            double csum = 0, wsum = 0;
-            for (uint32_t c = 0; c < grid; ++c) { csum += (double)cy[c]; wsum += (double)wt[c]; }
-            fprintf(stderr, "[w4a16 stream trace] main loop %.0f SM cycles per step (mean over CTAs), of which warp 0 waits %.0f for the stage; %.3f GHz\n",
-                    csum / grid / ((double)total / grid), wsum / grid / ((double)total / grid), csum / grid / (loop / grid));
-        }
-#endif
         fprintf(stderr, "[w4a16 stream trace] %zu problems, %llu steps on %u CTAs: first entry -> last exit %.2f us; per CTA mean: first step landed after %.2f us, "
                 "main loop %.2f us (%.3f us per step), flush+exit %.2f us; slowest CTA %u entered %.2f us after the first, loop %.2f us, flush+exit %.2f us\n",
                 count, (unsigned long long)total, grid, (t_max - t_min) * 1e-3, fill / grid * 1e-3, loop / grid * 1e-3, loop / grid * 1e-3 / ((double)total / grid),
