@@ -8,7 +8,7 @@
 // 32/64/128/256 columns, tile_k is one 128-byte swizzle atom (64 bf16), split-K is 1..8.  The score
 // is predicted time = max(tensor time with wave quantisation over the SMs, HBM time on the
 // algorithmic bytes) + launch (+ the split-K reduction pass).
-#include "common.h"
+#include "kernels.h"
 
 namespace t0 {
 uint32_t gemm_smem_bytes(uint32_t tile_n);        // gemm_sm100.cu
@@ -99,6 +99,45 @@ static std::vector<Candidate> schedule(uint32_t m, uint32_t n, uint32_t k) {
     }
     std::stable_sort(out.begin(), out.end(), [](const Candidate& a, const Candidate& b) { return a.pred_us < b.pred_us; });
     return out;
+}
+
+// Microseconds of one launch among others, fitted to measurements of every kernel alone (2048 x 1024 x 4096 ... 256^3, both layouts, one
+// to four rounds of tiles): a launch's fixed part (prologue, first operands, last epilogue, exit), the k blocks of the longest CTA, and
+// per round what of its epilogue stays exposed.  The search above scores whole configurations for the public entry points; its
+// split-K entries stand for the two-launch and cluster forms.
+GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms) {
+    struct Fit { uint32_t tile_n; double fixed, kblock, round; };
+    static const Fit single[] = {{256, 5.5, 0.40, 1.0}, {128, 4.8, 0.31, 0.4}, {64, 4.4, 0.28, 0.2}, {32, 4.4, 0.26, 0.1}};
+    static const uint32_t parts_tried[] = {1, 2, 3, 4, 6, 8};
+    const uint32_t kb = ceil_div(k, 64);
+    const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + 4.0 * (double)m * n) / 6.0e6;
+    GemmChoice best = {128, 1, false, min_split > 1};
+    double best_us = 1e30;
+    auto consider = [&](double us, GemmChoice c) {
+        us = std::max(us, 4.0 + bytes_us);
+        if (us < best_us) { best_us = us; best = c; }
+    };
+    if (m > 128 && n > 128 && min_split <= 1) {
+        // 256 x 256 per pair; the tiles of a last wave that at most half fills the GPU are cut in two
+        const uint32_t pairs = n_sms / 2;
+        const uint64_t tiles = (uint64_t)ceil_div(m, 256) * ceil_div(n, 256), rest = tiles % pairs;
+        const double rounds = (double)(tiles / pairs) + (rest == 0 ? 0.0 : (2 * rest <= pairs && tiles > pairs) ? 0.55 : 1.0);
+        consider(6.7 + rounds * (kb * 0.36 + 0.8), {256, 1, true, false});
+    }
+    for (const Fit& f : single) {
+        if (f.tile_n > 32 && n <= f.tile_n / 2) continue;           // more than half of the tile would be beyond N
+        if (nn && f.tile_n < 64) continue;                          // B[K,N] boxes are 64 columns wide
+        const uint64_t tiles = (uint64_t)ceil_div(m, 128) * ceil_div(n, f.tile_n);
+        for (uint32_t parts : parts_tried) {
+            if (parts > 1 && (tiles * parts > n_sms || kb < 2 * parts || f.tile_n == 256)) continue;      // parts pay while they find idle SMs
+            const bool halves = parts < min_split;                  // (two accumulators of up to 128 columns, double-buffered, fill tensor memory)
+            if (halves && (f.tile_n > 128 || 2 * parts < min_split)) continue;
+            const double rounds = std::ceil((double)(tiles * parts) / n_sms);
+            const double exchange = parts == 1 ? 0.0 : 1.6 + f.tile_n / 32.0 * (0.6 + 0.14 * parts);
+            consider(f.fixed + rounds * (ceil_div(kb, parts) * f.kblock + f.round) + exchange, {f.tile_n, parts, false, halves});
+        }
+    }
+    return best;
 }
 
 static t0_gemm_config legacy(uint32_t m, uint32_t k, uint32_t n) {

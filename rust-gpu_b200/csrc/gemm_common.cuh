@@ -34,6 +34,9 @@ struct KParams {
     uint32_t tma_store;          // the output leaves through its tensor map
     uint32_t drop_load;          // self-test of the failure path: the producer of CTA 0 leaves out its first operand load
     uint32_t n_problems;         // split-K cluster kernel, grouped launch: problems of one shape in this launch (0 or 1 = a single problem)
+    float4* pieces;              // split-K with a complete result: the parts' partial sums, in the lanes' own order (see gemm_sm100.cu)
+    uint32_t halves;             // tiles up to 128 wide: the second half of a part's k blocks goes to an accumulator of its own (see gemm_sm100.cu)
+    uint32_t* tickets;           // ... arrivals per tile and epilogue warp, zero between launches
     uint32_t n_peers;            // gathered output: every TMA-stored chunk also goes to this many other buffers (other GPUs' memory)
     const CUtensorMap* peer_maps; // their output tensor maps, in global memory (written by the host before the launch)
     float scale, clamp_min, clamp_max;
@@ -45,6 +48,13 @@ struct KParams {
 struct NoGroup { uint32_t unused; };
 
 struct WorkItem { uint32_t m_blk, n_blk, split; };
+
+// The k blocks of a part of K: a plane (split-K into planes, a third map dimension) or, for a complete result, a range of the whole K.
+struct KRange { uint32_t first, end, z; };
+__device__ __forceinline__ KRange k_range(uint32_t split, const KParams& p) {
+    if (!p.pieces) return {0, p.kb_per_split, split};
+    return {split * p.kb_per_split / p.split_k, (split + 1) * p.kb_per_split / p.split_k, 0};      // (kb_per_split is all of K here)
+}
 
 __device__ __forceinline__ WorkItem decode_work(uint32_t w, const KParams& p) {
     WorkItem it;

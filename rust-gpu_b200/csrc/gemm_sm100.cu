@@ -29,6 +29,40 @@ constexpr uint32_t kThreads = 192;
 
 __host__ __device__ constexpr uint32_t stages_for(uint32_t bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
 
+// First k block of a part's second accumulator (the end of the part when it has only one).
+template <uint32_t kAccs>
+__device__ __forceinline__ uint32_t k_mid(const KRange& kr, const KParams& p) {
+    return kAccs == 2 && p.halves ? kr.first + (kr.end - kr.first + 1) / 2 : kr.end;
+}
+// 32 columns of a warp's rows of the accumulator, of both where there are two.
+template <uint32_t BN>
+__device__ __forceinline__ void load_acc(uint32_t taddr, bool two_accs, uint32_t (&r)[32]) {
+    ptx::tmem_ld_32x32b_x32(taddr, r);
+    ptx::tmem_ld_wait();
+    if (two_accs) {                                    // warp-uniform
+        uint32_t r2[32];
+        ptx::tmem_ld_32x32b_x32(taddr + BN, r2);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+    }
+}
+
+// Waits (bounded) until all parts but the caller's own are counted as written in the high half of the counter.
+__device__ __forceinline__ bool wait_for_parts(const uint32_t* counter, uint32_t n_parts, volatile int* abort_flag, uint64_t limit_ns) {
+    uint64_t t_start = 0;
+    for (uint32_t spin = 1;; ++spin) {
+        uint32_t v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+        if ((v >> 16) + 1 == n_parts) return true;
+        if ((spin & 0x3F) == 0) {
+            const uint64_t now = ptx::globaltimer_ns();
+            if (t_start == 0) t_start = now;
+            if (*abort_flag || now - t_start > limit_ns) { *abort_flag = 1; return false; }
+        }
+    }
+}
+
 // Grouped launch: operand and output maps and the output addresses of up to kMaxGroupedGemms problems of one shape (12.5 KB
 // of kernel parameters).
 struct GroupOperands3 {
@@ -46,7 +80,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     constexpr uint32_t kStages = stages_for(BN);
     constexpr uint32_t kBStageBytes = BN * BK * 2;
     constexpr uint32_t kStageBytes = kAStageBytes + kBStageBytes;
-    constexpr uint32_t kTmemCols = 2 * BN;   // two accumulator buffers; 64..512, a power of two
+    // Two accumulator buffers.  Up to 128 columns a buffer holds two accumulators: with p.halves the first and second half of a part's
+    // k blocks are summed apart and added in f32 by the epilogue, which halves the length of the tensor cores' sums and so their error.
+    constexpr uint32_t kAccs = BN <= 128 ? 2 : 1;
+    constexpr uint32_t kTmemCols = 2 * BN * kAccs;   // 128..512, a power of two
     constexpr uint32_t kIdesc = ptx::make_idesc_bf16_f32(BM, BN, B_MN ? 1u : 0u, A_MN ? 1u : 0u);
 
     extern __shared__ uint8_t smem_raw[];
@@ -111,7 +148,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const CUtensorMap* ma = &map_a;
                 const CUtensorMap* mb = &map_b;
                 if constexpr (kGrouped) { ma = &group.maps[3 * prob]; mb = &group.maps[3 * prob + 1]; }
-                for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
+                const KRange kr = k_range(wi.split, p);
+                for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
                     if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
                         atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
                         ok = false;
@@ -123,22 +161,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     ptx::mbar_arrive_expect_tx(fb, kStageBytes);
                     if constexpr (!A_MN) {
                         ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
-                                         (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)wi.split);
+                                         (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)kr.z);
                     } else {
 #pragma unroll
                         for (uint32_t j = 0; j < BM / 64; ++j)
                             ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), ma, fb,
-                                             (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                                             (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
                     }
                     if constexpr (!B_MN) {
                         ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
-                                         (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)wi.split);
+                                         (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)kr.z);
                     } else {
                         // B[K,N]: one 64(k) x 64(n) box per 64 columns; each box is an [k][128 B] block
 #pragma unroll
                         for (uint32_t j = 0; j < BN / 64; ++j)
                             ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes + j * (BK * 128)), mb, fb,
-                                             (int32_t)(wi.n_blk * BN + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                                             (int32_t)(wi.n_blk * BN + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
                     }
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
@@ -156,14 +194,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const uint32_t tmem_d = tmem_base + buf * BN;
-                for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
+                const KRange kr = k_range(w % p.split_k, p);
+                const uint32_t kb_mid = k_mid<kAccs>(kr, p);
+                uint32_t tmem_d = tmem_base + buf * BN * kAccs;
+                for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
                     if (!ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
                         atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after_sync();
+                    if (kb == kb_mid) tmem_d += BN;
                     const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
                     const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
 #pragma unroll
@@ -174,7 +215,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
                         const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
                                                  : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
-                        ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, (kb | k4) != 0 ? 1u : 0u);
+                        ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, ((kb != kr.first && kb != kb_mid) || k4 != 0) ? 1u : 0u);
                     }
                     ptx::umma_commit(ptx::smem_u32(&empty_bar[stage]));
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -194,20 +235,93 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             const CUtensorMap* my = &map_y;
             if constexpr (kGrouped) { y_out = group.y[prob]; my = &group.maps[3 * prob + 2]; }
             const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
+            const uint32_t row_base = wi.m_blk * BM + quarter * 32;
+            // Split-K with a complete result.  The parts of a tile are added by whichever CTA gets to it last, each epilogue warp its own 32
+            // rows: a warp takes a ticket (low half of the counter); all but the last store their partial sums in the order their lanes
+            // hold them and count them as written (high half); the last one waits for those counts and adds the parts in split order, so
+            // the result does not depend on who was last.  The warps it waits for hold a ticket: they are running and wait for nobody.
+            const bool in_parts = p.pieces != nullptr && row_base < p.M;
+            uint32_t ticket = 0;
+            uint32_t* const counter = p.tickets + (w / p.split_k) * 4 + quarter;
+            if (in_parts && lane == 0) ticket = atomicAdd(counter, 1u) & 0xFFFFu;      // (its round trip passes under the main loop)
             if (!ptx::mbar_wait(ptx::smem_u32(&tmem_full_bar[buf]), acc_phase, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(w & 0xFFFFFF));
                 break;
             }
             ptx::tc_fence_after_sync();
-            const uint32_t row_base = wi.m_blk * BM + quarter * 32;
+            const KRange kr = k_range(wi.split, p);
+            const bool two_accs = k_mid<kAccs>(kr, p) < kr.end;
+            const uint32_t tmem_acc = tmem_base + ((quarter * 32) << 16) + buf * BN * kAccs;
+            constexpr uint32_t kPieceF4 = BM * BN / 4;                                 // of one part; BN / 32 chunks of 8 x 32 lanes per warp
+            float4* const piece0 = p.pieces + (size_t)(w - wi.split) * kPieceF4 + quarter * (kPieceF4 / 4) + lane;
+            if (in_parts) {
+                ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
+                if (ticket + 1 != p.split_k) {
+                    float4* const mine = piece0 + (size_t)wi.split * kPieceF4;
+#pragma unroll 1
+                    for (uint32_t c = 0; c < BN / 32; ++c) {
+                        if (wi.n_blk * BN + c * 32 >= p.N) break;
+                        uint32_t r[32];
+                        load_acc<BN>(tmem_acc + c * 32, two_accs, r);
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j)
+                            __stcg(mine + (c * 8 + j) * 32, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                                                                        __uint_as_float(r[4 * j + 3])));
+                    }
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        ptx::mbar_arrive(ptx::smem_u32(&tmem_empty_bar[buf]));
+                        __threadfence();                                               // the warp's part is visible before it is counted
+                        atomicAdd(counter, 0x10000u);
+                    }
+                    continue;
+                }
+                uint32_t good = 1;
+                if (lane == 0) {
+                    good = wait_for_parts(counter, p.split_k, abort_flag, p.wait_limit_ns) ? 1u : 0u;
+                    if (good) *counter = 0;                                            // ready for the next launch
+                    else atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(w & 0x7FFFFF));
+                    __threadfence();
+                }
+                good = __shfl_sync(0xFFFFFFFFu, good, 0);
+                if (!good) break;
+            }
 #pragma unroll 1
             for (uint32_t c = 0; c < BN / 32; ++c) {
                 const uint32_t col0 = wi.n_blk * BN + c * 32;
                 if (col0 >= p.N) break;   // warp-uniform
                 uint32_t r[32];
-                ptx::tmem_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + buf * BN + c * 32, r);
-                ptx::tmem_ld_wait();
-                store_chunk(p, r, row_base, lane, c, col0, wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores,
+                load_acc<BN>(tmem_acc + c * 32, two_accs, r);
+                if (in_parts) {
+                    float sum[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[j] = 0.0f;
+#pragma unroll 1
+                    for (uint32_t s0 = 0; s0 < p.split_k; s0 += 4) {
+                        // the loads of four parts are under way together: one round trip to L2 per chunk and four parts, not one per part
+                        float4 f[4][8];
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i) {
+                            const float4* theirs = piece0 + (size_t)(s0 + i) * kPieceF4 + c * 8 * 32;
+                            const bool other = s0 + i < p.split_k && s0 + i != wi.split;
+#pragma unroll
+                            for (uint32_t j = 0; j < 8; ++j) {
+                                f[i][j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+                                if (other) f[i][j] = __ldcg(theirs + j * 32);
+                            }
+                        }
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i) {
+                            if (s0 + i >= p.split_k) break;
+#pragma unroll
+                            for (uint32_t j = 0; j < 8; ++j) { sum[4 * j] += f[i][j].x; sum[4 * j + 1] += f[i][j].y; sum[4 * j + 2] += f[i][j].z; sum[4 * j + 3] += f[i][j].w; }
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[j]);
+                }
+                store_chunk(p, r, row_base, lane, c, col0, in_parts ? 0u : wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores,
                             p.tma_store ? my : nullptr, y_out);
             }
             ptx::tc_fence_before_sync();
@@ -254,6 +368,11 @@ int launch_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensor
 
 }  // namespace
 
+size_t gemm_pieces_bytes(uint32_t m, uint32_t n, uint32_t tile_n, uint32_t split) {
+    const uint32_t bn = snap_tile_n(tile_n);
+    return (size_t)ceil_div(m, BM) * ceil_div(n, bn) * split * BM * bn * sizeof(float);
+}
+
 uint32_t gemm_stage_count(uint32_t tile_n) { return stages_for(snap_tile_n(tile_n)); }
 
 uint32_t gemm_smem_bytes(uint32_t tile_n) {
@@ -265,13 +384,17 @@ uint32_t gemm_smem_bytes(uint32_t tile_n) {
 int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     if (g.m == 0 || g.n == 0) return T0_OK;
     if (g.k == 0) return fail(T0_ERR_INVALID, "K must be positive");
-    const uint32_t split = g.split_k ? g.split_k : 1;
-    if (g.k % split) return fail(T0_ERR_UNSUPPORTED, "K=%u not divisible by split_k=%u", g.k, split);
-    const uint32_t kps = g.k / split;
+    // parts of K: planes of the output (and of the operand maps), or, with scratch for the partial sums, ranges of the whole K
+    const bool parts = g.pieces != nullptr && g.split_k > 1;
+    const uint32_t planes = parts || g.split_k == 0 ? 1 : g.split_k, split = parts ? g.split_k : planes;
+    if (g.k % planes) return fail(T0_ERR_UNSUPPORTED, "K=%u not divisible by split_k=%u", g.k, split);
+    const uint32_t kps = g.k / planes;
+    if (parts && (!g.tickets || split > ceil_div(g.k, BK) || ceil_div(g.m, BM) * (uint64_t)ceil_div(g.n, snap_tile_n(g.tile_n)) > kMaxTicketTiles))
+        return fail(T0_ERR_UNSUPPORTED, "split-K in one launch: %u parts of %u k blocks", split, ceil_div(g.k, BK));
     const uint32_t ldx = g.ldx ? g.ldx : (g.at ? g.m : g.k);
     const uint32_t ldb = g.ldb ? g.ldb : (g.nn ? g.n : g.k);
     if (g.at && !g.nn) return fail(T0_ERR_UNSUPPORTED, "a transposed first operand goes with B[K,N]");
-    if ((ldx % 8) || (ldb % 8) || (split > 1 && (kps % 8)))
+    if ((ldx % 8) || (ldb % 8) || (planes > 1 && (kps % 8)))
         return fail(T0_ERR_UNSUPPORTED, "row strides (%u, %u) and, with split-K, K per split (%u) must be multiples of 8 for the TMA path", ldx, ldb, kps);
     if (((uintptr_t)g.x & 15) || ((uintptr_t)g.b & 15)) return fail(T0_ERR_UNSUPPORTED, "operand pointers must be 16-byte aligned");
     const uint32_t bn = snap_tile_n(g.tile_n);
@@ -288,19 +411,21 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     p.out_bf16 = g.out_bf16 ? 1 : 0; p.epilogue = g.epilogue; p.n_ops = g.n_ops;
     p.scale = g.scale; p.clamp_min = g.clamp_min; p.clamp_max = g.clamp_max;
     memcpy(p.ops, g.ops, sizeof p.ops);
+    if (parts) { p.pieces = (float4*)g.pieces; p.tickets = g.tickets; }
+    p.halves = g.halves ? 1 : 0;
 
     CUtensorMap ma, mb;
-    int rc = g.at ? make_map_nmajor(&ma, g.x, g.m, ldx, kps, split) : make_map_kmajor(&ma, g.x, g.m, ldx, kps, split, BM);
+    int rc = g.at ? make_map_nmajor(&ma, g.x, g.m, ldx, kps, planes) : make_map_kmajor(&ma, g.x, g.m, ldx, kps, planes, BM);
     if (rc != T0_OK) return rc;
-    rc = g.nn ? make_map_nmajor(&mb, g.b, g.n, ldb, kps, split) : make_map_kmajor(&mb, g.b, g.n, ldb, kps, split, bn);
+    rc = g.nn ? make_map_nmajor(&mb, g.b, g.n, ldb, kps, planes) : make_map_kmajor(&mb, g.b, g.n, ldb, kps, planes, bn);
     if (rc != T0_OK) return rc;
 
     const uint64_t total = (uint64_t)p.tiles_m * p.tiles_n * split;
     if (total > 0x7FFFFFFFull) return fail(T0_ERR_UNSUPPORTED, "too many tiles");
     const uint32_t grid = (uint32_t)std::min<uint64_t>(total, g.n_sms ? g.n_sms : 148);
     CUtensorMap my = ma;   // a valid map either way; only read when p.tma_store is set
-    if (tma_output_ok(g, split, bn)) {
-        rc = make_map_out(&my, g.y, g.m, g.n, split, g.plane_stride, g.out_bf16);
+    if (tma_output_ok(g, planes, bn)) {
+        rc = make_map_out(&my, g.y, g.m, g.n, planes, g.plane_stride, g.out_bf16);
         if (rc != T0_OK) return rc;
         p.tma_store = 1;
     }

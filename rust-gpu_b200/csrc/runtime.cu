@@ -14,6 +14,8 @@ struct GemmRequest {
     uint32_t m, n, k;
     uint32_t ldx, ldb;         // row strides in elements, multiples of 8 (0 = dense)
     uint32_t tile_n, split_k;
+    uint32_t parts;            // parts of K chosen by the library (0, 1 = none): added in the same launch, any K
+    bool halves;               // ... each summed in two accumulators
     bool nn, out_bf16, planes, swap_grid;
     bool at;                   // x is [K,M] (with nn)
     int pair;                  // 0 = choose by shape, 1 = CTA-pair kernel, 2 = single-CTA kernel
@@ -43,11 +45,18 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     GemmRequest q = q_in;
     if (q.m == 0 || q.n == 0) return T0_OK;
     // A caller that fixed nothing (tile width 0, kernel 0, no split, complete result wanted) gets the cost model's choice
-    // for the shape: tile, CTA pair or not, and split-K with the device-side reduction.  (The "widest tile that fills the
-    // machine" rule below picked 64-wide tiles for 128 x 11008 x 4096, 45 us against 28 us for the model's 128 x 128.)
+    // for the shape: tile, CTA pair or not, and into how many parts K is cut.
     if (q.tile_n == 0 && q.pair == 0 && q.split_k <= 1 && !q.planes && q.k >= 64) {
         t0_gemm_config c;
-        if (t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK) {
+        if (!getenv("T0_FORCE_CFG")) {
+            const bool known = t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK;
+            const uint32_t s = known && c.split_k > 1 && q.k % c.split_k == 0 ? c.split_k : 1;
+            const GemmChoice choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count);
+            q.tile_n = choice.tile_n;
+            q.parts = choice.parts;
+            q.halves = choice.halves;
+            q.pair = choice.pair ? 1 : 2;
+        } else if (t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK) {
             const uint32_t s = c.split_k > 1 ? c.split_k : 1;
             const bool split_ok = s == 1 || (q.k % s == 0 && (q.k / s) % 8 == 0 && q.k % 8 == 0 && !(q.x & 15) && !(q.b & 15) && (!q.nn || q.n % 8 == 0));
             if (split_ok) {
@@ -85,6 +94,7 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     g.wait_limit_ns = rt->wait_limit_ns.load(std::memory_order_relaxed);
     g.drop_load = rt->drop_next_load.exchange(0) != 0;
     g.split_k = split;
+    g.halves = q.halves;
     g.tile_n = q.tile_n ? snap_tile_n(q.tile_n) : choose_tile_n(rt, q.m, q.n, q.k, split);
     if (q.nn && g.tile_n < 64) g.tile_n = 64;
     // the CTA-pair kernel (256 x 256 tiles) pays off once there are enough tiles to fill the machine
@@ -123,24 +133,48 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
         rt->launches.fetch_add(1);
     }
 
-    const bool fused_reduce = split > 1 && !q.planes;
-    if (fused_reduce && !use_pair) {
+    bool fused_reduce = split > 1 && !q.planes;
+    static const bool no_cluster = getenv("T0_NO_CLUSTER_SPLITK") != nullptr;
+    // Split-K in one launch, the parts added by the CTA that finishes last (gemm_sm100.cu).  A split the caller asked for runs this way
+    // where its parts are whole k blocks (the parts, and so the sums, are then those of the planes form) and the launch is about one wave.
+    uint32_t parts = q.parts > 1 && !use_pair ? q.parts : 0;
+    if (fused_reduce && !use_pair && !no_cluster && q.k % (64u * split) == 0) parts = split;
+    if (parts) {
+        const uint64_t tiles = (uint64_t)ceil_div(q.m, 128) * ceil_div(q.n, g.tile_n);
+        const size_t bytes = gemm_pieces_bytes(q.m, q.n, g.tile_n, parts);
+        if (tiles > kMaxTicketTiles || tiles * parts > 4ull * (uint64_t)rt->sm_count) parts = 0;
+        // 128 x 128 tiles with most of their rows: 64 KB a part, which the CTAs of a cluster exchange faster (each adds a slice) than one of
+        // them reads the others' from L2: 16.7 against 17.8 us at 128 x 4096 x 4096 in four parts, but 17.9 against 16.8 at M = 64
+        if (parts && g.tile_n == 128 && q.m > 64 && !q.halves && !q.nn && !q.at && (parts == 2 || parts == 4) && q.k % (64u * parts) == 0 && !no_cluster) {
+            g.split_k = split = parts;
+            parts = 0;
+            fused_reduce = true;
+        }
+        if (parts && bytes > rt->scratch_planes.size) {
+            // nothing may be allocated while the stream is being captured: the forms without scratch then
+            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+            T0_CUDA(cudaStreamIsCapturing(rt->stream, &capturing));
+            if (capturing != cudaStreamCaptureStatusNone) parts = 0;
+            else if (int rc = ensure_scratch(rt, rt->scratch_planes, bytes)) return rc;
+        }
+    }
+    if (parts) { g.split_k = parts; g.pieces = rt->scratch_planes.ptr; g.tickets = rt->d_tickets; }
+    if (fused_reduce && !use_pair && !parts) {
         // one launch: the CTAs that share a tile form a cluster and add their partial sums through distributed shared
         // memory (T0_NO_CLUSTER_SPLITK=1 keeps the two-launch form below for comparison)
-        static const bool no_cluster = getenv("T0_NO_CLUSTER_SPLITK") != nullptr;
         GemmLaunch gc = g;
         gc.y = (void*)q.y; gc.plane_stride = 0; gc.bias = (const float*)q.bias;
         gc.out_bf16 = q.out_bf16; gc.epilogue = q.epilogue; gc.n_ops = q.n_ops;
         memcpy(gc.ops, q.ops, sizeof gc.ops);
         gc.scale = q.scale; gc.clamp_min = q.clamp_min; gc.clamp_max = q.clamp_max;
-        if (!no_cluster && !x_bad && !b_bad && gemm_splitk_cluster_supported(gc)) {
+        if (!no_cluster && gemm_splitk_cluster_supported(gc)) {
             int rc = launch_gemm_sm100_splitk(gc, rt->stream);
             if (rc != T0_OK) return rc;
             rt->launches.fetch_add(1);
             return T0_OK;
         }
     }
-    if (fused_reduce) {
+    if (fused_reduce && !parts) {
         // partial planes go to scratch; K4 sums them in split order and applies the epilogue
         const size_t mn = (size_t)q.m * q.n;
         int rc = ensure_scratch(rt, rt->scratch_planes, mn * split * sizeof(float));
@@ -169,7 +203,7 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
         rt->peer_maps_key = key;
     }
     g.y = (void*)q.y;
-    g.plane_stride = split > 1 ? (q.plane_stride ? q.plane_stride : (uint64_t)q.m * q.n) : 0;
+    g.plane_stride = split > 1 && !parts ? (q.plane_stride ? q.plane_stride : (uint64_t)q.m * q.n) : 0;
     g.bias = (const float*)q.bias;
     g.out_bf16 = q.out_bf16; g.epilogue = q.epilogue; g.n_ops = q.n_ops;
     memcpy(g.ops, q.ops, sizeof g.ops);
@@ -340,6 +374,8 @@ int t0_rt_new(int device, t0_runtime** out) {
     T0_CUDA(cudaEventCreate(&rt->ev_stop));
     T0_CUDA(cudaMalloc(&rt->d_probe, (2 + 64) * sizeof(unsigned long long)));   // clock words + eight launches' trace stamps
     T0_CUDA(cudaMemset(rt->d_probe, 0, (2 + 64) * sizeof(unsigned long long)));
+    T0_CUDA(cudaMalloc(&rt->d_tickets, kMaxTicketTiles * 4 * sizeof(uint32_t)));
+    T0_CUDA(cudaMemset(rt->d_tickets, 0, kMaxTicketTiles * 4 * sizeof(uint32_t)));
     T0_CUDA(cudaHostAlloc(&rt->h_status, sizeof(int), cudaHostAllocMapped));
     *rt->h_status = 0;
     T0_CUDA(cudaHostGetDevicePointer(&rt->d_status, rt->h_status, 0));
@@ -356,6 +392,7 @@ void t0_rt_free(t0_runtime* rt) {
     for (Scratch* s : {&rt->scratch_a, &rt->scratch_b, &rt->scratch_planes, &rt->scratch_w4, &rt->scratch_w, &rt->scratch_cvt_a, &rt->scratch_cvt_b, &rt->scratch_cvt_c})
         if (s->ptr) cudaFree(s->ptr);
     if (rt->d_probe) cudaFree(rt->d_probe);
+    if (rt->d_tickets) cudaFree(rt->d_tickets);
     if (rt->d_peer_maps) cudaFree(rt->d_peer_maps);
     if (rt->h_status) cudaFreeHost(rt->h_status);
     if (rt->ev_start) cudaEventDestroy(rt->ev_start);

@@ -102,3 +102,43 @@ def test_operands_at_any_element_address(t0, rt, layout, m, n, k, x_skip, b_skip
     nn = layout == "nn"
     got = run_gemm(t0, rt, x, b.T if nn else b, m, n, k, x_skip=x_skip, b_skip=b_skip, transpose=t0.NN if nn else t0.NT)
     assert np.array_equal(got, x @ b.T)
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+@pytest.mark.parametrize("tile_n,split_k", [(64, 2), (64, 8), (128, 2), (128, 4)])
+@pytest.mark.parametrize("m,n,k", [(40, 72, 512), (129, 200, 1024), (300, 640, 4096)])
+@pytest.mark.parametrize("out_bf16", [False, True])
+def test_cluster_split_k_in_both_layouts(t0, rt, layout, tile_n, split_k, m, n, k, out_bf16):
+    rng = np.random.default_rng(n)
+    x, b, bias = ints(rng, m, k), ints(rng, n, k), ints(rng, n, lim=100)
+    nn = layout == "nn"
+    before = rt.launch_count()
+    got = run_gemm(t0, rt, x, b.T if nn else b, m, n, k, out_bf16, bias, tile_n=tile_n, split_k=split_k, pair_cta=2,
+                   transpose=t0.NN if nn else t0.NT, epilogue=t0.EPI_BIAS_ADD_STORE_F32)
+    assert rt.launch_count() - before == 1
+    want = x @ b.T + bias
+    assert np.array_equal(got, from_bf16(bf16_bits(want)) if out_bf16 else want)
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+@pytest.mark.parametrize("m,n,k", [(32, 752, 3984), (16, 2048, 2048), (100, 296, 8192), (512, 512, 2048), (1024, 512, 4096), (2048, 1024, 4096), (128, 4096, 1024),
+                                   (1, 8, 64), (64, 1024, 200), (130, 136, 72)])
+def test_library_chosen_kernel(t0, rt, layout, m, n, k):
+    # nothing fixed by the caller: parts of K that are not of one length, sums in two accumulators, pairs, and tiny products
+    rng = np.random.default_rng(k)
+    x, b, bias = ints(rng, m, k), ints(rng, n, k), ints(rng, n, lim=100)
+    nn = layout == "nn"
+    for out_bf16 in (False, True):
+        got = run_gemm(t0, rt, x, b.T if nn else b, m, n, k, out_bf16, bias, transpose=t0.NN if nn else t0.NT, epilogue=t0.EPI_BIAS_ADD_STORE_F32)
+        want = x @ b.T + bias
+        assert np.array_equal(got, from_bf16(bf16_bits(want)) if out_bf16 else want)
+
+
+def test_parts_added_in_order_whoever_is_last(t0, rt):
+    # real-valued operands: the parts of a tile are added in split order, so repeated launches agree bit for bit
+    rng = np.random.default_rng(3)
+    m, n, k = 48, 512, 6144
+    x, b = from_bf16(bf16_bits(rng.uniform(-1, 1, (m, k)))), from_bf16(bf16_bits(rng.uniform(-1, 1, (n, k))))
+    first = run_gemm(t0, rt, x, b, m, n, k)
+    for _ in range(5):
+        assert np.array_equal(run_gemm(t0, rt, x, b, m, n, k), first)
