@@ -198,7 +198,8 @@ int t0_rt_selftest_drop_one_load(t0_runtime* rt);
  *     captured a product that finds the buffer too small takes a form without it (a cluster of CTAs, or K not cut);
  *   t0_w4a16_gemm outside the fused shapes: T0_SCRATCH_W4_WEIGHTS = K * N * 2;
  *   every fused W4A16 call (row layout and streaming layout): T0_SCRATCH_W4_FUSED, t0_rt_w4_fused_scratch_bytes(rt) bytes,
- *     a fixed size per device, so only the first fused call of a runtime allocates;
+ *     a fixed size per device, so only the first fused call of a runtime allocates (reserving it also makes room for the
+ *     partial sums of the grouped calls with 16 < M <= 128, which go without them while the stream is being captured);
  *   t0_matmul_f32*, t0_blas_gemm_f32: bf16 copies of the operands, T0_SCRATCH_F32_A / _B = elements * 2 (an operand whose
  *     rows are not a multiple of 8 elements: T0_SCRATCH_OPERAND_A / _B = rows * roundup(columns, 8) * 2), and, for
  *     alpha/beta other than 1/0 or ldc != n, T0_SCRATCH_F32_C = m * n * 4;

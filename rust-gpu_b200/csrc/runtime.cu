@@ -389,7 +389,7 @@ void t0_rt_free(t0_runtime* rt) {
     cudaStreamSynchronize(rt->stream);
     host_pipe_free(rt);
     t0_rt_pool_clear(rt);
-    for (Scratch* s : {&rt->scratch_a, &rt->scratch_b, &rt->scratch_planes, &rt->scratch_w4, &rt->scratch_w, &rt->scratch_cvt_a, &rt->scratch_cvt_b, &rt->scratch_cvt_c})
+    for (Scratch* s : {&rt->scratch_a, &rt->scratch_b, &rt->scratch_planes, &rt->scratch_w4, &rt->scratch_um, &rt->scratch_w, &rt->scratch_cvt_a, &rt->scratch_cvt_b, &rt->scratch_cvt_c})
         if (s->ptr) cudaFree(s->ptr);
     if (rt->d_probe) cudaFree(rt->d_probe);
     if (rt->d_tickets) cudaFree(rt->d_tickets);
@@ -449,7 +449,7 @@ int t0_rt_reserve_scratch(t0_runtime* rt, int which, size_t bytes) {
                 if (rc != T0_OK) return rc;
                 T0_CUDA(cudaMemsetAsync(rt->scratch_w4.ptr, 0, w4a16_counter_region_bytes(), rt->stream));
             }
-            return T0_OK;
+            return w4a16_umma_reserve(rt, (uint32_t)rt->sm_count, 128);
         }
         default: return fail(T0_ERR_INVALID, "unknown scratch kind %d", which);
     }

@@ -57,6 +57,7 @@ struct t0_runtime {
     Scratch scratch_a, scratch_b, scratch_planes;
     uint32_t* d_tickets = nullptr;           // split-K in one launch: arrivals per output tile and epilogue warp, zero between launches
     Scratch scratch_w4;          // W4A16: slab arrival counters + straddling pieces
+    Scratch scratch_um;          // tcgen05 W4A16, grouped: counters + partial sums of the cut tiles
     Scratch scratch_w;           // W4A16 general path: dequantised weights
     Scratch scratch_cvt_a, scratch_cvt_b, scratch_cvt_c;   // f32 entries: bf16 copies of the operands, f32 product before alpha/beta
     void* host_pipe = nullptr;   // host-operand GEMM pipeline (streams, events, staging sets), made on first use
@@ -65,6 +66,7 @@ struct t0_runtime {
 namespace t0 {
 
 void host_pipe_free(t0_runtime* rt);   // host_pipeline.cu
+int w4a16_umma_reserve(t0_runtime* rt, uint32_t ctas, uint32_t rows);   // w4a16_umma_cut.cu
 // runtime.cu: one bf16 product of operands with row strides, everything else chosen by the library
 int gemm_strided(t0_runtime* rt, uint64_t a, uint32_t lda, bool at, uint64_t b, uint32_t ldb, bool nn, uint64_t y, uint32_t m, uint32_t n, uint32_t k);
 

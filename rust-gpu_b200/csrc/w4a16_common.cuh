@@ -76,6 +76,14 @@ __device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t mask, uint32_t m
     return r;
 }
 
+// Grouped launch of the tcgen05 kernels: the four tensor maps (weights, scales, zero points, activations) and the output of up to 32
+// problems of one shape in the kernel parameters (16.6 KB).
+constexpr uint32_t kUmMaxGroup = 32;
+struct UmGroup {
+    CUtensorMap maps[4 * kUmMaxGroup];
+    float* y[kUmMaxGroup];
+};
+
 // Trace buffer of the T0_W4_TRACE debugging aid: freed on every path out of the entry point that made it.
 struct StampBuffer {
     unsigned long long* d = nullptr;

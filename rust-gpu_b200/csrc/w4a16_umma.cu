@@ -109,14 +109,6 @@ __device__ __forceinline__ float4 um_ld_cluster_f4(uint32_t addr) {
     return v;
 }
 
-// Grouped launch: the four tensor maps (weights, scales, zero points, activations) and the output of up to 32 problems of
-// one shape in the kernel parameters (16.6 KB).
-constexpr uint32_t kUmMaxGroup = 32;
-struct UmGroup {
-    CUtensorMap maps[4 * kUmMaxGroup];
-    float* y[kUmMaxGroup];
-};
-
 template <bool kGrouped>
 __global__ void __launch_bounds__(kUmThreads, 1)
 w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
@@ -825,6 +817,10 @@ __global__ void w4_to_tiled_kernel(const uint32_t* __restrict__ packed, const ui
 
 namespace t0 {
 
+bool w4a16_umma_cut_pays(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count);     // w4a16_umma_cut.cu
+uint32_t w4a16_umma_cut_rows(uint32_t M);
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count);
+
 // Whether the fused tcgen05 kernel takes this W4A16 problem.
 bool w4a16_umma_supported(uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t y, uint32_t M, uint32_t N, uint32_t K, uint32_t group) {
     if (M == 0 || M > 128 || N % 32 || K == 0 || K % kUmBK || group == 0 || group % kUmBK || K % group) return false;
@@ -832,24 +828,24 @@ bool w4a16_umma_supported(uint64_t a, uint64_t packed, uint64_t scales, uint64_t
     return true;
 }
 
-// The four tensor maps of one problem: packed words, scales, zero points, and the activations as the 128-row operand
-// (K-major boxes of 64, 128-byte swizzle, rows beyond M read as zero).
-static int um_maps(uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint32_t M, uint32_t N, uint32_t K, uint32_t group, CUtensorMap* out4) {
+// The four tensor maps of one problem: packed words, scales, zero points, and the activations (K-major boxes
+// of 64 k x a_rows, 128-byte swizzle, rows beyond M read as zero).
+static int um_maps(uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint32_t M, uint32_t N, uint32_t K, uint32_t group, CUtensorMap* out4, uint32_t a_rows = 128) {
     int rc = gemm::make_map_2d_plain(&out4[0], (const void*)packed, 4, K / 8, N, kUmBN, kUmBK / 8);
     if (rc == T0_OK) rc = gemm::make_map_2d_plain(&out4[1], (const void*)scales, 2, K / group, N, kUmBN, 1);
     if (rc == T0_OK) rc = gemm::make_map_2d_plain(&out4[2], (const void*)zeros, 4, K / group, N / 8, kUmBN / 8, 1);
-    if (rc == T0_OK) rc = gemm::make_map_kmajor(&out4[3], (const void*)a, M, K, K, 1, 128);
+    if (rc == T0_OK) rc = gemm::make_map_kmajor(&out4[3], (const void*)a, M, K, K, 1, a_rows);
     return rc;
 }
 
 // The same four maps over the tile-major buffer: 3-D views (column in tile, row, tile).
-static int um_maps_tiled(uint64_t a, uint64_t tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group, CUtensorMap* out4) {
+static int um_maps_tiled(uint64_t a, uint64_t tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group, CUtensorMap* out4, uint32_t a_rows = 128) {
     const TiledLayout L = tiled_layout(K, N, group);
     const uint8_t* base = (const uint8_t*)tiled;
     int rc = gemm::make_map_3d_plain(&out4[0], base + L.off_words, 4, kUmBN, L.rows, L.tiles, kUmBN * 4, (uint64_t)L.rows * kUmBN * 4, kUmBN, kUmBK / 8);
     if (rc == T0_OK) rc = gemm::make_map_3d_plain(&out4[1], base + L.off_scales, 2, kUmBN, L.groups, L.tiles, kUmBN * 2, (uint64_t)L.groups * kUmBN * 2, kUmBN, 1);
     if (rc == T0_OK) rc = gemm::make_map_3d_plain(&out4[2], base + L.off_zeros, 4, kUmBN / 8, L.groups, L.tiles, (kUmBN / 8) * 4, (uint64_t)L.groups * (kUmBN / 8) * 4, kUmBN / 8, 1);
-    if (rc == T0_OK) rc = gemm::make_map_kmajor(&out4[3], (const void*)a, M, K, K, 1, 128);
+    if (rc == T0_OK) rc = gemm::make_map_kmajor(&out4[3], (const void*)a, M, K, K, 1, a_rows);
     return rc;
 }
 
@@ -943,14 +939,16 @@ int launch_w4a16_umma_tiled_grouped(t0_runtime* rt, const t0_w4a16_args* args, u
     static UmGroup grp;
     static std::mutex grp_mu;
     std::lock_guard<std::mutex> lock(grp_mu);
+    const bool cut = w4a16_umma_cut_pays(rt, a0.n, a0.k, count);
     for (uint32_t i = 0; i < count; ++i) {
         const t0_w4a16_args& a = args[i];
         if (a.m != a0.m || a.n != a0.n || a.k != a0.k || a.group != a0.group) return fail(T0_ERR_INVALID, "grouped launch: problem %u differs from problem 0 in shape", i);
         if (!um_tiled_supported(a.a, a.packed, a.y, a.m, a.n, a.k, a.group)) return fail(T0_ERR_UNSUPPORTED, "grouped launch: problem %u is not a shape of the fused tcgen05 kernel", i);
-        int rc = um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, &grp.maps[4 * i]);
+        int rc = um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, &grp.maps[4 * i], cut ? w4a16_umma_cut_rows(a.m) : 128);
         if (rc != T0_OK) return rc;
         grp.y[i] = (float*)a.y;
     }
+    if (cut) return launch_w4a16_umma_cut(rt, grp, true, a0.m, a0.n, a0.k, a0.group, count);
     UmParams p = um_params(rt, a0.a, a0.y, a0.m, a0.n, a0.k, a0.group);
     p.n_problems = count;
     p.tiled = 1;
@@ -986,15 +984,17 @@ int launch_w4a16_umma_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_
     static UmGroup grp;                  // 16.6 KB: kept off the stack, filled under the lock, copied by the launch
     static std::mutex grp_mu;
     std::lock_guard<std::mutex> lock(grp_mu);
+    const bool cut = w4a16_umma_cut_pays(rt, a0.n, a0.k, count);
     for (uint32_t i = 0; i < count; ++i) {
         const t0_w4a16_args& a = args[i];
         if (a.m != a0.m || a.n != a0.n || a.k != a0.k || a.group != a0.group) return fail(T0_ERR_INVALID, "grouped launch: problem %u differs from problem 0 in shape", i);
         if (!w4a16_umma_supported(a.a, a.packed, a.scales, a.zeros, a.y, a.m, a.n, a.k, a.group))
             return fail(T0_ERR_UNSUPPORTED, "grouped launch: problem %u is not a shape of the fused tcgen05 kernel", i);
-        int rc = um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, &grp.maps[4 * i]);
+        int rc = um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, &grp.maps[4 * i], cut ? w4a16_umma_cut_rows(a.m) : 128);
         if (rc != T0_OK) return rc;
         grp.y[i] = (float*)a.y;
     }
+    if (cut) return launch_w4a16_umma_cut(rt, grp, false, a0.m, a0.n, a0.k, a0.group, count);
     UmParams p = um_params(rt, a0.a, a0.y, a0.m, a0.n, a0.k, a0.group);
     p.n_problems = count;
     static const bool smem_form = getenv("T0_W4_UMMA_SS") != nullptr;     // comparison switch: dequantised weights through shared memory

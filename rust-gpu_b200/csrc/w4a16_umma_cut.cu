@@ -1,0 +1,538 @@
+// K2 for several problems of one shape with M <= 128 whose column tiles do not fill the GPU evenly: the W4A16 GEMM on tcgen05 with the
+// dequantised weights as the tensor-memory operand (as w4a16_umma_ts_kernel in w4a16_umma.cu, which see), tiles cut between CTAs.
+//
+// No counterpart kernel exists in the reference (its INT4 support stops at the stand-alone dequantisation kernels,
+// src/t0/quant_kernels.rs:53-171).  y[m,n] = sum_k a[m,k] * w[k,n],  w = RNE_bf16((q - z) * s),  fp32 accumulate.
+//
+// The work is a list of chunks, 256 columns x 64 k, problem by problem, tile by tile, k last; every CTA (one per SM) takes an
+// equal contiguous range of it.  Per chunk:
+//   * one warp's lane fetches the packed words (8 rows x 256 columns), scales and zero points with three TMA boxes each into a ring of
+//     raw stages of two chunks, another warp's the activations (rows up to M rounded to 16; rows beyond M are zero-filled);
+//   * sixteen warps turn the words into bf16 (one LOP3 per nibble pair: 0x4300 | q is the bf16 128+q, minus 128+z, times s -
+//     bit-identical to the oracle because (q-z)*s is rounded once) and put them straight into tensor memory (tcgen05.st): the
+//     weights are the 128-row A operand, two halves of 128 columns of y;
+//   * one thread issues 2 x 4 tcgen05.mma (128 x M' x 16, M' = M rounded to 16) with the activations as the B operand in shared
+//     memory.  The accumulator is y transposed: lane = column of y, tensor-memory column = row of y.
+// A tile that lies wholly in one range is stored from tensor memory.  A tile cut by range boundaries is finished by the warps that
+// reach it last: see the epilogue.
+//
+// Whole tiles per CTA leave SMs idle where the tiles are few or just over a multiple of them: two problems of N = 11008 are 86 tiles on 148
+// SMs.  M = 128, K = 4096: 43.8 us with whole tiles, 40.4 cut; M = 107, N = 7936, K = 4352: 45.3 and 34.4; M = 81, N = 2560, K = 7424, four
+// problems: 72.0 and 37.3.  What bounds it is the chain of waits around a chunk (0.67 us; arithmetic alone would take about 0.15) and, per
+// launch, about 10 us for handing in and adding the parts of cut tiles; `w4a16_umma_cut_pays` weighs the two.
+#include "w4a16_common.cuh"
+
+using namespace t0;
+using namespace t0::w4;
+
+namespace {
+
+constexpr uint32_t kUmDqWarps = 16;
+// + the warps that fetch weights and activations and the one that issues the UMMAs.  Each is one lane working through a serial chain
+// of instructions per chunk, at several cycles an instruction, so the chains are kept short (running counters, no divisions, descriptors
+// stepped by addition) and apart: two lanes of one warp would take turns.
+constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;
+constexpr uint32_t kUmThreads = (kUmDqWarps + 3) * 32;
+constexpr uint32_t kUmBN = 256;                             // columns of y per tile
+constexpr uint32_t kUmBK = 64;                              // k per chunk: one 128-byte swizzle atom of bf16
+constexpr uint32_t kUmRawBytes = 8 * kUmBN * 4 + kUmBN * 2 + (kUmBN / 8) * 4;      // 8832: words, scales, zero points
+constexpr uint32_t kUmRawStride = 9216;                     // keeps every stage 1024-byte aligned
+constexpr uint32_t kUmXBytes = 128 * kUmBK * 2;             // 16 KiB: activations of a chunk at M = 128
+// Tensor memory (512 columns): accumulators 2 x 128 columns, then four A stages of 2 halves x 4 k-steps x 8 columns.
+constexpr uint32_t kUmTmemCols = 512;
+constexpr uint32_t kUmABase = 256;                          // first column of the A stages
+constexpr uint32_t kUmAStageCols = 64;
+constexpr uint32_t kUmAStages = 4;
+constexpr uint32_t kUmXStages = 4;                          // activation stages
+constexpr uint32_t kUmRawStages = 7;                        // raw weight stages of two chunks: 124 KB in flight per SM
+// (more than half an SM's shared memory: the kernel takes all 512 tensor-memory columns, so two of its CTAs must never share an SM)
+constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmXStages * kUmXBytes + 512 + 1024;
+constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long: below it the finish costs more than the range
+constexpr size_t kUmCounterBytes = 16 * 1024;               // one word per CTA and dequantisation warp (up to 256 CTAs)
+
+struct UmParams {
+    int* status;
+    uint32_t* counters;      // [grid][16]: arrivals at the tile that CTA begins and does not complete; zero between launches
+    float* pieces;           // [grid][2][rows][256]: partial sums of the cut tiles (slot 0 = the CTA's first piece)
+    uint64_t wait_limit_ns;
+    uint32_t M, N;
+    uint32_t rows;           // M rounded up to 16: width of the UMMAs and height of the activation boxes
+    uint32_t group;          // k per scale / zero-point row (a multiple of 64)
+    uint32_t n_tiles, n_chunks;
+    uint32_t total;          // chunks of the launch, shared out evenly (less than 2^24)
+};
+
+__device__ __forceinline__ uint32_t um_lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t um_lds16(uint32_t addr) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// First chunk of a CTA's range, and the CTA whose range holds a chunk: in 32 bits (at most 256 CTAs and 2^24 chunks), since a warp that
+// finishes a cut tile needs a few of these and a 64-bit division takes hundreds of cycles.
+__device__ __forceinline__ uint32_t um_begin(uint32_t cta, const UmParams& p) { return cta * p.total / gridDim.x; }
+__device__ __forceinline__ uint32_t um_owner(uint32_t chunk, const UmParams& p) { return ((chunk + 1) * gridDim.x - 1) / p.total; }
+
+template <bool kTiled>    // weights in the tile-major layout (3-D maps: column in tile, row, tile), else the row layout
+__global__ void __launch_bounds__(kUmThreads, 1)
+w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t raw_ring = smem;
+    const uint32_t x_ring = smem + kUmRawStages * 2 * kUmRawStride;           // activations: [rows][64 k] bf16, 128-byte swizzle, per stage
+    const uint32_t bars = x_ring + kUmXStages * kUmXBytes;
+    const uint32_t raw_full = bars, raw_empty = bars + 8 * kUmRawStages;
+    const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * kUmAStages;
+    const uint32_t x_full = a_empty + 8 * kUmAStages, x_empty = x_full + 8 * kUmXStages;
+    const uint32_t acc_full = x_empty + 8 * kUmXStages, acc_empty = acc_full + 8;
+    __shared__ uint32_t tmem_holder;
+    __shared__ int s_abort;
+    volatile int* abort_flag = &s_abort;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t n_chunks = p.n_chunks;
+    const uint32_t u0 = um_begin(blockIdx.x, p), u1 = um_begin(blockIdx.x + 1, p);
+
+    if (tid == 0) {
+        for (uint32_t s = 0; s < kUmRawStages; ++s) {
+            ptx::mbar_init(raw_full + 8 * s, 1);
+            ptx::mbar_init(raw_empty + 8 * s, kUmDqWarps);
+        }
+        for (uint32_t s = 0; s < kUmAStages; ++s) {
+            ptx::mbar_init(a_full + 8 * s, kUmDqWarps / 2);       // the eight warps that dequantise the chunk
+            ptx::mbar_init(a_empty + 8 * s, 1);
+        }
+        for (uint32_t s = 0; s < kUmXStages; ++s) {
+            ptx::mbar_init(x_full + 8 * s, 1);
+            ptx::mbar_init(x_empty + 8 * s, 1);
+        }
+        ptx::mbar_init(acc_full, 1);
+        ptx::mbar_init(acc_empty, kUmDqWarps);
+        s_abort = 0;
+        ptx::fence_barrier_init();
+        ptx::fence_proxy_async_smem();
+        for (uint32_t i = 0; i < 4; ++i) ptx::tma_prefetch_desc(&group.maps[4 * (u0 / (n_chunks * p.n_tiles)) + i]);
+    }
+    if (warp == kUmIssueWarp) {
+        ptx::tmem_alloc(ptx::smem_u32(&tmem_holder), kUmTmemCols);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    ptx::tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_holder;
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+
+    if (warp == kUmRawWarp) {
+        if (lane == 0) {
+            // ---------------------------------------------------------- raw weights, scales, zero points: three TMA boxes per chunk
+            uint32_t stage = 0, phase = 0;
+            const uint32_t item = u0 / n_chunks, per_group = p.group / kUmBK;
+            uint32_t c = u0 - item * n_chunks, tile = item;
+            uint32_t grp = c / per_group, in_group = c - grp * per_group;
+            const uint32_t prob = item / p.n_tiles;
+            tile = item - prob * p.n_tiles;
+            const CUtensorMap* mw = &group.maps[4 * prob];
+            const CUtensorMap* ms = mw + 1;
+            const CUtensorMap* mz = mw + 2;
+            for (uint32_t u = u0; u < u1;) {
+                if (!ptx::mbar_wait_relaxed(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns, 64)) {
+                    atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(c & 0xFFFFFF));
+                    break;
+                }
+                ptx::fence_proxy_async_smem();           // the stage was read through the generic proxy, the copies write it through the async proxy
+                const uint32_t fb = raw_full + 8 * stage;
+                uint32_t dst = raw_ring + stage * (2 * kUmRawStride);
+                const uint32_t u_stop = min(u1, u + 2);
+                ptx::mbar_arrive_expect_tx(fb, (u_stop - u) * kUmRawBytes);
+                for (; u < u_stop; ++u, dst += kUmRawStride) {
+                    if constexpr (kTiled) {
+                        // tile-major layout: the chunk's 8 KB of words are contiguous, as are its scales and zero points
+                        ptx::tma_load_3d(dst, mw, fb, 0, (int32_t)(c * (kUmBK / 8)), (int32_t)tile);
+                        ptx::tma_load_3d(dst + 8 * kUmBN * 4, ms, fb, 0, (int32_t)grp, (int32_t)tile);
+                        ptx::tma_load_3d(dst + 8 * kUmBN * 4 + kUmBN * 2, mz, fb, 0, (int32_t)grp, (int32_t)tile);
+                    } else {
+                        ptx::tma_load_2d(dst, mw, fb, (int32_t)(tile * kUmBN), (int32_t)(c * (kUmBK / 8)));
+                        ptx::tma_load_2d(dst + 8 * kUmBN * 4, ms, fb, (int32_t)(tile * kUmBN), (int32_t)grp);
+                        ptx::tma_load_2d(dst + 8 * kUmBN * 4 + kUmBN * 2, mz, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)grp);
+                    }
+                    if (++in_group == per_group) { in_group = 0; ++grp; }
+                    if (++c == n_chunks) {
+                        c = grp = in_group = 0;
+                        if (++tile == p.n_tiles) {
+                            tile = 0;
+                            mw += 4; ms += 4; mz += 4;
+                        }
+                    }
+                }
+                if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
+            }
+        }
+    } else if (warp == kUmXWarp) {
+        if (lane == 0) {
+            // ---------------------------------------------------------- activations: one box per chunk (rows beyond M are zero)
+            uint32_t xs = 0, xphase = 0;
+            const uint32_t item = u0 / n_chunks;
+            uint32_t c = u0 - item * n_chunks, tile = item;
+            const uint32_t prob = item / p.n_tiles;
+            tile = item - prob * p.n_tiles;
+            const CUtensorMap* ma = &group.maps[4 * prob + 3];
+            for (uint32_t u = u0; u < u1; ++u) {
+                if (!ptx::mbar_wait_relaxed(x_empty + 8 * xs, xphase ^ 1, abort_flag, p.wait_limit_ns, 64)) {
+                    atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
+                    break;
+                }
+                ptx::mbar_arrive_expect_tx(x_full + 8 * xs, p.rows * kUmBK * 2);
+                ptx::tma_load_3d(x_ring + xs * kUmXBytes, ma, x_full + 8 * xs, (int32_t)(c * kUmBK), 0, 0);
+                if (++xs == kUmXStages) { xs = 0; xphase ^= 1; }
+                if (++c == n_chunks) {
+                    c = 0;
+                    if (++tile == p.n_tiles) {
+                        tile = 0;
+                        ma += 4;
+                    }
+                }
+            }
+        }
+    } else if (warp == kUmIssueWarp) {
+        // -------------------------------------------------------------- UMMA issuer: per chunk 2 halves x 4 k-steps of M 128 x N rows x K 16
+        if (lane == 0) {
+            const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u);
+            uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0;
+            const uint64_t x_desc = ptx::make_smem_desc(x_ring, 16, 1024);      // (addresses enter a descriptor in 16-byte units: stages are added)
+            bool ok = true;
+            for (uint32_t u = u0; ok && u < u1; ++piece) {
+                const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks);
+                if (piece > 0 && !ptx::mbar_wait(acc_empty, (piece - 1) & 1, abort_flag, p.wait_limit_ns)) {
+                    atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
+                    break;
+                }
+                ptx::tc_fence_after_sync();
+                for (uint32_t first = 1; u < u_end; ++u, first = 0) {
+                    if (!ptx::mbar_wait(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
+                        !ptx::mbar_wait(a_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
+                        atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after_sync();
+                    const uint64_t x_stage = x_desc + xs * (kUmXBytes / 16);
+                    const uint32_t a_cols = tmem_base + kUmABase + as * kUmAStageCols;
+#pragma unroll
+                    for (uint32_t k4 = 0; k4 < kUmBK / 16; ++k4) {
+#pragma unroll
+                        for (uint32_t t = 0; t < 2; ++t)
+                            ptx::umma_bf16_ts(tmem_base + t * 128, a_cols + t * 32 + k4 * 8, x_stage + k4 * 2, idesc, (first && k4 == 0) ? 0u : 1u);
+                    }
+                    ptx::umma_commit(a_empty + 8 * as);
+                    ptx::umma_commit(x_empty + 8 * xs);
+                    if (++as == kUmAStages) { as = 0; aphase ^= 1; }
+                    if (++xs == kUmXStages) { xs = 0; xphase ^= 1; }
+                }
+                if (ok) ptx::umma_commit(acc_full);
+            }
+        }
+    } else {
+        // -------------------------------------------------------------- sixteen warps: dequantise into tensor memory, then the epilogue
+        // Warps 0..7 take the even chunks of the range, 8..15 the odd ones: a thread has one column and all eight words of its chunk, so that
+        // what stands around the arithmetic (two waits, two arrivals, the store and its wait) is paid once per eight words.  (All sixteen
+        // warps on every chunk, four words each: 3 % slower.)
+        const uint32_t q = warp & 3, t = (warp >> 2) & 1, h = warp >> 3;   // lane quadrant, 128-column half of the tile, chunk parity (and half of the rows in the epilogue)
+        const uint32_t n = t * 128 + q * 32 + lane;                          // this thread's column of the tile
+        const uint32_t lane_base = (q * 32) << 16;
+        const uint32_t m_begin = h * (p.rows / 2), m_end = min(p.M, m_begin + p.rows / 2);   // the rows of y this warp stores
+        uint32_t mask, magic;
+        asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
+        asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
+        uint32_t rs = 0, rphase = 0, as = h, aphase = 0, piece = 0;
+        bool ok = true;
+
+        // 16 columns of the accumulator (rows m0.. of y) for this warp's columns of y
+        auto load_rows = [&](uint32_t m0, float (&v)[16]) {
+            uint32_t r[16];
+            ptx::tmem_ld_32x32b_x16(tmem_base + lane_base + t * 128 + m0, r);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+        };
+        // partial sums of a cut tile: each warp's own block of a piece, four rows of a column per float4
+        const uint32_t row4s = p.rows / 8;                                   // float4s a lane holds
+        const size_t piece_f4 = (size_t)p.rows * (kUmBN / 4);
+        float4* const my_block = (float4*)p.pieces + (size_t)warp * row4s * 32 + lane;
+
+        for (uint32_t u = u0; u < u1; ++piece) {
+            const uint32_t item = u / n_chunks, tile_u0 = item * n_chunks, tile_u1 = tile_u0 + n_chunks;
+            const uint32_t u_end = min(u1, tile_u1);
+            const bool whole = u == tile_u0 && u_end == tile_u1;
+            for (uint32_t v = u + (((u - u0) & 1) != h ? 1 : 0); ok && v < u_end; v += 2) {
+                if (!ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(v & 0x3FFFFF));
+                    ok = false;
+                    break;
+                }
+                const uint32_t raw = raw_ring + rs * (2 * kUmRawStride) + h * kUmRawStride;
+                uint32_t words[8];
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) words[i] = um_lds32(raw + i * (kUmBN * 4) + n * 4);
+                const uint32_t sbits = um_lds16(raw + 8 * kUmBN * 4 + n * 2);
+                const uint32_t zword = um_lds32(raw + 8 * kUmBN * 4 + kUmBN * 2 + (n >> 3) * 4);
+                const uint32_t zz = ((zword >> ((n & 7) * 4)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
+                const uint32_t ss = sbits * 0x00010001u;                                               // (s, s)
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(raw_empty + 8 * rs);
+                if (++rs == kUmRawStages) { rs = 0; rphase ^= 1; }
+                uint32_t r[32];                                // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const uint32_t wd = words[i];
+                    const uint32_t v0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), zz), ss);            // k 0, 4
+                    const uint32_t v1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), zz), ss);       // k 1, 5
+                    const uint32_t v2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), zz), ss);       // k 2, 6
+                    const uint32_t v3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), zz), ss);      // k 3, 7
+                    if constexpr (kTiled) {                    // tile-major words are stored so that the pairs come out in k order
+                        r[4 * i] = v0; r[4 * i + 1] = v1; r[4 * i + 2] = v2; r[4 * i + 3] = v3;
+                    } else {                                   // row layout: pairs (0,4) (1,5) (2,6) (3,7)
+                        r[4 * i] = __byte_perm(v0, v1, 0x5410);
+                        r[4 * i + 1] = __byte_perm(v2, v3, 0x5410);
+                        r[4 * i + 2] = __byte_perm(v0, v1, 0x7632);
+                        r[4 * i + 3] = __byte_perm(v2, v3, 0x7632);
+                    }
+                }
+                // the A stage is free once the UMMAs of four chunks ago have read it
+                if (!ptx::mbar_wait(a_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(v & 0x3FFFFF));
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after_sync();
+                ptx::tmem_st_32x32b_x32(tmem_base + lane_base + kUmABase + as * kUmAStageCols + t * 32, r);
+                ptx::tmem_st_wait();
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(a_full + 8 * as);
+                as += 2;
+                if (as >= kUmAStages) { as -= kUmAStages; aphase ^= 1; }
+            }
+            u = u_end;
+            // A tile cut by range boundaries: each of its CTAs holds a partial sum over a part of K.  The 32 columns x rows a warp
+            // owns are finished by the same warp of whichever CTA gets to it last, so no warp ever waits for another of its CTA.  A
+            // warp first takes a ticket (low half of the tile's counter); all but the last then store their part and count it as
+            // written (high half).  The last one waits for those counts: the warps it waits for hold a ticket, so they are running,
+            // and the tiles before in their range can only wait for CTAs further down.  It adds the parts in k order whoever it is:
+            // repeated calls agree bit for bit.
+            uint32_t c_first = 0, first_slot = 0, n_parts = 1, ticket = 0;
+            uint32_t* counter = nullptr;
+            if (ok && !whole && m_begin < m_end) {
+                c_first = um_owner(tile_u0, p);
+                n_parts = um_owner(tile_u1 - 1, p) - c_first + 1;
+                first_slot = um_begin(c_first, p) < tile_u0 ? 1u : 0u;           // its range began in the tile before: this is not its first piece
+                counter = p.counters + c_first * kUmDqWarps + warp;
+                if (lane == 0) ticket = atomicAdd(counter, 1u) & 0xFFFFu;        // (its round trip passes under the last UMMAs)
+            }
+            // ---- epilogue: y[m][n0 + n] = D[lane n][column m]; a warp stores 32 consecutive columns of one row per instruction
+            if (ok && !ptx::mbar_wait(acc_full, piece & 1, abort_flag, p.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xC00000);
+                ok = false;
+            }
+            if (!ok) break;
+            ptx::tc_fence_after_sync();
+            ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
+            if (ticket + 1 != n_parts) {
+                float4* mine = my_block + ((size_t)blockIdx.x * 2 + (piece == 0 ? 0 : 1)) * piece_f4;
+#pragma unroll 1
+                for (uint32_t i = 0; i < row4s; i += 4) {
+                    float v[16];
+                    load_rows(m_begin + 4 * i, v);
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j)
+                        if (i + j < row4s) __stcg(mine + (i + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+                }
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    ptx::mbar_arrive(acc_empty);
+                    __threadfence();                       // the warp's part is visible before it is counted
+                    atomicAdd(counter, 0x10000u);
+                }
+                continue;
+            }
+            if (n_parts > 1) {
+                uint32_t good = 1;
+                if (lane == 0) {
+                    uint64_t t_start = 0;
+                    for (uint32_t spin = 1; (um_ld_acquire(counter) >> 16) + 1 != n_parts; ++spin) {
+                        if ((spin & 0x3F) == 0) {
+                            const uint64_t now = ptx::globaltimer_ns();
+                            if (t_start == 0) t_start = now;
+                            if (*abort_flag || now - t_start > p.wait_limit_ns) { *abort_flag = 1; good = 0; break; }
+                        }
+                    }
+                    if (good) *counter = 0;                // ready for the next launch
+                    else atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xE00000);
+                    __threadfence();
+                }
+                good = __shfl_sync(0xFFFFFFFFu, good, 0);
+                if (!good) { ok = false; break; }
+            }
+            const uint32_t prob = item / p.n_tiles;
+            float* const y_out = group.y[prob];
+            const uint32_t col = (item - prob * p.n_tiles) * kUmBN + n;
+#pragma unroll 1
+            for (uint32_t i = 0; i < row4s; i += 4) {
+                const uint32_t m0 = m_begin + 4 * i;
+                float sum[16];
+                if (n_parts == 1) load_rows(m0, sum);
+                if (n_parts > 1) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; ++j) sum[j] = 0.0f;
+#pragma unroll 1
+                    for (uint32_t part = 0; part < n_parts; part += 2) {
+                        // the loads of two parts are under way together
+                        float f[2][16];
+#pragma unroll
+                        for (uint32_t k = 0; k < 2; ++k) {
+                            const uint32_t cta = c_first + part + k;
+                            if (cta == blockIdx.x) {
+                                load_rows(m0, f[k]);
+                            } else if (part + k < n_parts) {
+                                const float4* theirs = my_block + ((size_t)cta * 2 + (part + k == 0 ? first_slot : 0u)) * piece_f4;
+#pragma unroll
+                                for (uint32_t j = 0; j < 4; ++j) {
+                                    const float4 x = i + j < row4s ? __ldcg(theirs + (i + j) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                                    f[k][4 * j] = x.x; f[k][4 * j + 1] = x.y; f[k][4 * j + 2] = x.z; f[k][4 * j + 3] = x.w;
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (uint32_t k = 0; k < 2; ++k) {
+                            if (part + k >= n_parts) break;
+#pragma unroll
+                            for (uint32_t j = 0; j < 16; ++j) sum[j] += f[k][j];
+                        }
+                    }
+                }
+                if (col < p.N) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; ++j)
+                        if (m0 + j < m_end) y_out[(size_t)(m0 + j) * p.N + col] = sum[j];
+                }
+            }
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(acc_empty);
+        }
+    }
+
+    __syncwarp();
+    if (*abort_flag) {
+        // give copies and UMMAs already in flight time to land before shared and tensor memory go away
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kUmIssueWarp) {
+        ptx::tc_fence_after_sync();
+        ptx::tmem_dealloc(tmem_base, kUmTmemCols);
+    }
+}
+
+}  // namespace
+
+namespace t0 {
+
+size_t w4a16_umma_scratch_bytes(uint32_t ctas, uint32_t rows) { return kUmCounterBytes + (size_t)ctas * 2 * rows * kUmBN * sizeof(float); }
+
+// Room for the counters and partial sums of `ctas` CTAs; the counters start at zero.
+int w4a16_umma_reserve(t0_runtime* rt, uint32_t ctas, uint32_t rows) {
+    const size_t need = w4a16_umma_scratch_bytes(ctas, rows);
+    if (need <= rt->scratch_um.size) return T0_OK;
+    int rc = ensure_scratch(rt, rt->scratch_um, need);
+    if (rc != T0_OK) return rc;
+    T0_CUDA(cudaMemsetAsync(rt->scratch_um.ptr, 0, kUmCounterBytes, rt->stream));
+    return T0_OK;
+}
+
+static uint32_t cut_grid(const t0_runtime* rt, uint64_t items, uint32_t n_chunks) {
+    const uint32_t ctas = std::min<uint32_t>((uint32_t)rt->sm_count, kUmCounterBytes / (kUmDqWarps * sizeof(uint32_t)));
+    uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, items * n_chunks / kUmMinChunks), ctas);
+    if (items * 2 <= ctas) {
+        // Few tiles: whole parts of a tile per CTA, at most four, where that leaves few CTAs idle - a CTA then has one piece to hand in, and
+        // a tile is not cut into more parts than pay.
+        const uint32_t parts = std::max<uint32_t>(1, std::min<uint32_t>({4u, ctas / (uint32_t)items, n_chunks / kUmMinChunks}));
+        if (parts == 4 || parts * kUmMinChunks * 2 > n_chunks || items * parts * 5 >= ctas * 4ull) grid = (uint32_t)items * parts;
+    }
+    return grid;
+}
+
+// Whether cutting the tiles of `count` problems beats whole tiles per CTA, in microseconds fitted at M = 128 and 32, K = 1152 ... 7424, 32 to 516
+// tiles: a chunk takes about 0.65 us either way, a launch with cut tiles about 10 us more.  Cut tiles need scratch: not while the
+// stream is being captured and the scratch does not exist yet.
+bool w4a16_umma_cut_pays(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count) {
+    const uint64_t items = (uint64_t)ceil_div(N, kUmBN) * count;
+    const uint32_t n_chunks = K / kUmBK, grid = cut_grid(rt, items, n_chunks);
+    if (items % grid == 0 || items * n_chunks >= (1u << 24)) return false;
+    const double whole = (double)((items + rt->sm_count - 1) / rt->sm_count) * n_chunks * 0.63 + 4.0;
+    const double cut = (double)items * n_chunks / grid * 0.67 + 14.4;
+    if (cut > 0.97 * whole) return false;
+    if (w4a16_umma_scratch_bytes(grid, 128) > rt->scratch_um.size) {
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+    }
+    return true;
+}
+
+uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }
+
+// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count) {
+    auto kern = tiled ? w4a16_umma_cut_kernel<true> : w4a16_umma_cut_kernel<false>;
+    static bool attr_set[2][64] = {};
+    if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
+    if (!attr_set[tiled][rt->device]) {
+        T0_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmSmem));
+        attr_set[tiled][rt->device] = true;
+    }
+    UmParams p;
+    memset(&p, 0, sizeof p);
+    p.status = rt->d_status;
+    const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
+    p.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
+    p.M = M; p.N = N; p.group = group_size;
+    p.rows = w4a16_umma_cut_rows(M);
+    p.n_tiles = ceil_div(N, kUmBN);
+    p.n_chunks = K / kUmBK;
+    const uint64_t items = (uint64_t)p.n_tiles * count;
+    const uint32_t grid = cut_grid(rt, items, p.n_chunks);
+    p.total = (uint32_t)(items * p.n_chunks);
+    int rc = w4a16_umma_reserve(rt, (uint32_t)rt->sm_count, 128);
+    if (rc != T0_OK) return rc;
+    p.counters = (uint32_t*)rt->scratch_um.ptr;
+    p.pieces = (float*)((uint8_t*)rt->scratch_um.ptr + kUmCounterBytes);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(kUmThreads, 1, 1);
+    cfg.dynamicSmemBytes = kUmSmem;
+    cfg.stream = rt->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    static const bool use_pdl = getenv("T0_NO_PDL") == nullptr;
+    cfg.numAttrs = use_pdl ? 1 : 0;
+    cudaError_t le = cudaLaunchKernelEx(&cfg, kern, p, group);
+    if (le != cudaSuccess) return fail(T0_ERR_CUDA, "W4A16 kernel launch failed: %s", cudaGetErrorString(le));
+    rt->launches.fetch_add(1);
+    return T0_OK;
+}
+
+}  // namespace t0

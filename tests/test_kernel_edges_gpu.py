@@ -104,6 +104,48 @@ def test_operands_at_any_element_address(t0, rt, layout, m, n, k, x_skip, b_skip
     assert np.array_equal(got, x @ b.T)
 
 
+@pytest.mark.parametrize("entry", ["tiled", "row"])
+@pytest.mark.parametrize("M,K,N,count", [(17, 8192, 512, 2), (33, 4096, 768, 1), (128, 4096, 2560, 2), (107, 4352, 7936, 2), (40, 4096, 11008, 2), (1, 4096, 2592, 3)])
+def test_w4a16_tiles_cut_between_ctas(t0, oracle, rt, entry, M, K, N, count):
+    # tiles that do not fill the GPU evenly: they are cut into the ranges of two or more CTAs, whose parts are added in k order whoever finishes: repeated
+    # calls agree bit for bit.  Bound: f32 sums of K exact products in another order, K * 2^-24 of the sum of their magnitudes at most
+    if entry == "row" and M <= 16:
+        pytest.skip("the row layout runs another kernel for M <= 16")
+    G = 128
+    calls, bufs, ys, refs = [], [], [], []
+    for i in range(count):
+        packed, scales, zeros = oracle.fill_u32((K // 8) * N, 10 + i), oracle.fill_range_bf16((K // G) * N, 20 + i, 0.001, 0.02), oracle.fill_u32((K // G) * (N // 8), 30 + i)
+        a = oracle.fill_normal_bf16(M * K, 40 + i)
+        ref = oracle.w4a16_gemm(a, packed, scales, zeros, M, N, K, G).astype(np.float64)
+        w = np.abs(oracle.bf16_to_f32(oracle.dequant_w4_b200(packed, scales, zeros, K, N, G)).reshape(K, N))
+        refs.append((ref, np.abs(oracle.bf16_to_f32(a).reshape(M, K)).astype(np.float64) @ w * (K * 2.0 ** -24)))
+        xp, xs, xz, xa, y = rt.upload(packed), rt.upload(scales), rt.upload(zeros), rt.upload(a), rt.alloc(M * N * 4)
+        bufs += [xp, xs, xz, xa, y]
+        ys.append(y)
+        if entry == "tiled":
+            t = rt.w4_to_tiled(xp.gpu_addr(), xs.gpu_addr(), xz.gpu_addr(), K, N, G)
+            bufs.append(t)
+            calls.append(t0.W4A16Args(xa.gpu_addr(), t.gpu_addr(), 0, 0, y.gpu_addr(), M, N, K, G))
+        else:
+            calls.append(t0.W4A16Args(xa.gpu_addr(), xp.gpu_addr(), xs.gpu_addr(), xz.gpu_addr(), y.gpu_addr(), M, N, K, G))
+    run = rt.w4a16_gemm_tiled_grouped if entry == "tiled" else rt.w4a16_gemm_grouped
+    first = None
+    for _ in range(4):
+        for y in ys:
+            y.write(np.full(M * N, np.nan, np.float32))
+        run(calls)
+        rt.synchronize()
+        got = [y.read(M * N * 4, np.float32).reshape(M, N) for y in ys]
+        if first is None:
+            first = got
+            for g, (ref, tol) in zip(got, refs):
+                assert np.all(np.abs(g - ref) <= tol)
+        for g, f in zip(got, first):
+            assert np.array_equal(g.view(np.uint32), f.view(np.uint32))
+    for b in bufs:
+        b.free()
+
+
 @pytest.mark.parametrize("layout", ["nt", "nn"])
 @pytest.mark.parametrize("tile_n,split_k", [(64, 2), (64, 8), (128, 2), (128, 4)])
 @pytest.mark.parametrize("m,n,k", [(40, 72, 512), (129, 200, 1024), (300, 640, 4096)])
