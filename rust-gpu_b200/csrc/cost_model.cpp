@@ -111,7 +111,7 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min
     static const uint32_t parts_tried[] = {1, 2, 3, 4, 6, 8};
     const uint32_t kb = ceil_div(k, 64);
     const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + 4.0 * (double)m * n) / 6.0e6;
-    GemmChoice best = {128, 1, false, min_split > 1};
+    GemmChoice best = {0, 0, false, false};
     double best_us = 1e30;
     auto consider = [&](double us, GemmChoice c) {
         us = std::max(us, 4.0 + bytes_us);

@@ -48,15 +48,18 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     // for the shape: tile, CTA pair or not, and into how many parts K is cut.
     if (q.tile_n == 0 && q.pair == 0 && q.split_k <= 1 && !q.planes && q.k >= 64) {
         t0_gemm_config c;
+        const bool known = t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK;
+        GemmChoice choice = {};
         if (!getenv("T0_FORCE_CFG")) {
-            const bool known = t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK;
             const uint32_t s = known && c.split_k > 1 && q.k % c.split_k == 0 ? c.split_k : 1;
-            const GemmChoice choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count);
+            choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count);
+        }
+        if (choice.parts) {
             q.tile_n = choice.tile_n;
             q.parts = choice.parts;
             q.halves = choice.halves;
             q.pair = choice.pair ? 1 : 2;
-        } else if (t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK) {
+        } else if (known) {
             const uint32_t s = c.split_k > 1 ? c.split_k : 1;
             const bool split_ok = s == 1 || (q.k % s == 0 && (q.k / s) % 8 == 0 && q.k % 8 == 0 && !(q.x & 15) && !(q.b & 15) && (!q.nn || q.n % 8 == 0));
             if (split_ok) {

@@ -164,7 +164,7 @@ def test_cluster_split_k_in_both_layouts(t0, rt, layout, tile_n, split_k, m, n, 
 
 @pytest.mark.parametrize("layout", ["nt", "nn"])
 @pytest.mark.parametrize("m,n,k", [(32, 752, 3984), (16, 2048, 2048), (100, 296, 8192), (512, 512, 2048), (1024, 512, 4096), (2048, 1024, 4096), (128, 4096, 1024),
-                                   (1, 8, 64), (64, 1024, 200), (130, 136, 72)])
+                                   (1, 8, 64), (64, 1024, 200), (130, 136, 72), (64, 5056, 6656), (16, 8, 10240)])
 def test_library_chosen_kernel(t0, rt, layout, m, n, k):
     # nothing fixed by the caller: parts of K that are not of one length, sums in two accumulators, pairs, and tiny products
     rng = np.random.default_rng(k)
