@@ -103,12 +103,14 @@ static std::vector<Candidate> schedule(uint32_t m, uint32_t n, uint32_t k) {
 
 // Microseconds of one launch among others, fitted to measurements of every kernel alone (2048 x 1024 x 4096 ... 256^3, both layouts, one
 // to four rounds of tiles): a launch's fixed part (prologue, first operands, last epilogue, exit), the k blocks of the longest CTA, and
-// per round what of its epilogue stays exposed.  The search above scores whole configurations for the public entry points; its
-// split-K entries stand for the two-launch and cluster forms.
-GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms) {
-    struct Fit { uint32_t tile_n; double fixed, kblock, round; };
-    static const Fit single[] = {{256, 5.5, 0.40, 1.0}, {128, 4.8, 0.31, 0.4}, {64, 4.4, 0.28, 0.2}, {32, 4.4, 0.26, 0.1}};
-    static const uint32_t parts_tried[] = {1, 2, 3, 4, 6, 8};
+// per round what of its epilogue stays exposed.  With K in parts there is one round, and instead the exchange in the clusters: longer with
+// the rows and columns of a tile, a little with every part, and a launch that leaves half of the SMs to the next one's prologue is
+// shorter (49 shapes of 16 to 1500 rows, both layouts: the choice is 1 % above the best one on average, 13 % at most).  The search above
+// scores whole configurations for the public entry points; its split-K entries stand for the two-launch and cluster forms.
+GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once) {
+    struct Fit { uint32_t tile_n; double fixed, kblock, round, exchange; };
+    static const Fit single[] = {{256, 5.5, 0.40, 1.0, 0.0}, {128, 4.8, 0.31, 0.4, 2.9}, {64, 4.4, 0.28, 0.2, 1.1}, {32, 4.4, 0.26, 0.1, 0.5}};
+    const double tile_rows = std::min(128u, ceil_div(m, 32) * 32) / 128.0;
     const uint32_t kb = ceil_div(k, 64);
     const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + 4.0 * (double)m * n) / 6.0e6;
     GemmChoice best = {0, 0, false, false};
@@ -128,13 +130,16 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min
         if (f.tile_n > 32 && n <= f.tile_n / 2) continue;           // more than half of the tile would be beyond N
         if (nn && f.tile_n < 64) continue;                          // B[K,N] boxes are 64 columns wide
         const uint64_t tiles = (uint64_t)ceil_div(m, 128) * ceil_div(n, f.tile_n);
-        for (uint32_t parts : parts_tried) {
-            if (parts > 1 && (tiles * parts > n_sms || kb < 2 * parts || f.tile_n == 256)) continue;      // parts pay while they find idle SMs
-            const bool halves = parts < min_split;                  // (two accumulators of up to 128 columns, double-buffered, fill tensor memory)
-            if (halves && (f.tile_n > 128 || 2 * parts < min_split)) continue;
-            const double rounds = std::ceil((double)(tiles * parts) / n_sms);
-            const double exchange = parts == 1 ? 0.0 : 1.6 + f.tile_n / 32.0 * (0.6 + 0.14 * parts);
-            consider(f.fixed + rounds * (ceil_div(kb, parts) * f.kblock + f.round) + exchange, {f.tile_n, parts, false, halves});
+        for (uint32_t parts = 1; parts <= kMaxClusterParts; ++parts) {
+            if (parts > 1 && (tiles > clusters_at_once[parts] || kb < 2 * parts || f.tile_n == 256)) continue;      // parts pay while they find idle SMs
+            if (parts < min_split && (f.tile_n > 128 || 2 * parts < min_split)) continue;
+            // Two accumulators (up to 128 columns, double-buffered, they fill tensor memory) where the sums have to be shorter, and wherever
+            // they cost a launch of one round under 1 %.
+            const bool halves = f.tile_n <= 128 && (parts < min_split || parts > 1 || (tiles <= n_sms && kb >= (2 * tiles <= n_sms ? 8u : 32u)));
+            const double us = parts == 1 ? f.fixed + std::ceil((double)tiles / n_sms) * (kb * f.kblock + f.round)
+                                         : 5.8 + ceil_div(kb, parts) * 0.293 + 0.16 * parts + tile_rows * f.exchange;
+            const double overlap = 2 * tiles * parts > n_sms ? 0.0 : parts == 1 ? 0.6 : 1.0;
+            consider(us - overlap, {f.tile_n, parts, false, halves});
         }
     }
     return best;

@@ -34,9 +34,7 @@ struct KParams {
     uint32_t tma_store;          // the output leaves through its tensor map
     uint32_t drop_load;          // self-test of the failure path: the producer of CTA 0 leaves out its first operand load
     uint32_t n_problems;         // split-K cluster kernel, grouped launch: problems of one shape in this launch (0 or 1 = a single problem)
-    float4* pieces;              // split-K with a complete result: the parts' partial sums, in the lanes' own order (see gemm_sm100.cu)
     uint32_t halves;             // tiles up to 128 wide: the second half of a part's k blocks goes to an accumulator of its own (see gemm_sm100.cu)
-    uint32_t* tickets;           // ... arrivals per tile and epilogue warp, zero between launches
     uint32_t n_peers;            // gathered output: every TMA-stored chunk also goes to this many other buffers (other GPUs' memory)
     const CUtensorMap* peer_maps; // their output tensor maps, in global memory (written by the host before the launch)
     float scale, clamp_min, clamp_max;
@@ -48,13 +46,6 @@ struct KParams {
 struct NoGroup { uint32_t unused; };
 
 struct WorkItem { uint32_t m_blk, n_blk, split; };
-
-// The k blocks of a part of K: a plane (split-K into planes, a third map dimension) or, for a complete result, a range of the whole K.
-struct KRange { uint32_t first, end, z; };
-__device__ __forceinline__ KRange k_range(uint32_t split, const KParams& p) {
-    if (!p.pieces) return {0, p.kb_per_split, split};
-    return {split * p.kb_per_split / p.split_k, (split + 1) * p.kb_per_split / p.split_k, 0};      // (kb_per_split is all of K here)
-}
 
 __device__ __forceinline__ WorkItem decode_work(uint32_t w, const KParams& p) {
     WorkItem it;
@@ -275,19 +266,29 @@ __device__ __forceinline__ void store_chunk(const KParams& p, const uint32_t (&r
 // Launch with programmatic stream serialisation so the prologue of this grid overlaps the tail of the
 // previous one (T0_NO_PDL=1 in the environment turns it off).
 template <typename Kernel, typename... Args>
-inline cudaError_t launch_pdl(Kernel kern, uint32_t grid, uint32_t block, uint32_t smem, cudaStream_t stream, const Args&... args) {
+inline cudaError_t launch_pdl_clusters(Kernel kern, uint32_t grid, uint32_t cluster, uint32_t block, uint32_t smem, cudaStream_t stream, const Args&... args) {
     static const bool use_pdl = getenv("T0_NO_PDL") == nullptr;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(block, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = use_pdl ? 1 : 0;
+    if (use_pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs++].val.clusterDim = {cluster, 1, 1};
+    }
     return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <typename Kernel, typename... Args>
+inline cudaError_t launch_pdl(Kernel kern, uint32_t grid, uint32_t block, uint32_t smem, cudaStream_t stream, const Args&... args) {
+    return launch_pdl_clusters(kern, grid, 1, block, smem, stream, args...);
 }
 
 // ------------------------------------------------------------------ tensor maps (host)

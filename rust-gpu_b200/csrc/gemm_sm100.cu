@@ -29,6 +29,14 @@ constexpr uint32_t kThreads = 192;
 
 __host__ __device__ constexpr uint32_t stages_for(uint32_t bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
 
+// The k blocks of a part of K: of a plane (a third map dimension), or, where the launch adds the parts itself, a range of the whole K.
+struct KRange { uint32_t first, end, z; };
+template <bool kCluster>
+__device__ __forceinline__ KRange k_range(uint32_t split, const KParams& p) {
+    if (!kCluster) return {0, p.kb_per_split, split};
+    return {split * p.kb_per_split / p.split_k, (split + 1) * p.kb_per_split / p.split_k, 0};      // (kb_per_split is all of K here)
+}
+
 // First k block of a part's second accumulator (the end of the part when it has only one).
 template <uint32_t kAccs>
 __device__ __forceinline__ uint32_t k_mid(const KRange& kr, const KParams& p) {
@@ -48,17 +56,82 @@ __device__ __forceinline__ void load_acc(uint32_t taddr, bool two_accs, uint32_t
     }
 }
 
-// Waits (bounded) until all parts but the caller's own are counted as written in the high half of the counter.
-__device__ __forceinline__ bool wait_for_parts(const uint32_t* counter, uint32_t n_parts, volatile int* abort_flag, uint64_t limit_ns) {
-    uint64_t t_start = 0;
-    for (uint32_t spin = 1;; ++spin) {
-        uint32_t v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-        if ((v >> 16) + 1 == n_parts) return true;
-        if ((spin & 0x3F) == 0) {
-            const uint64_t now = ptx::globaltimer_ns();
-            if (t_start == 0) t_start = now;
-            if (*abort_flag || now - t_start > limit_ns) { *abort_flag = 1; return false; }
+// Four columns of one row of the result.
+__device__ __forceinline__ void store4(const KParams& p, bool vec, uint32_t row, uint32_t col, const float (&o)[4]) {
+    if (row >= p.M) return;
+    const size_t off = (size_t)row * p.N + col;
+    if (vec) {
+        if (p.out_bf16) {
+            const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
+            *(uint2*)((__nv_bfloat16*)p.y + off) = *(const uint2*)h;
+        } else {
+            *(float4*)((float*)p.y + off) = make_float4(o[0], o[1], o[2], o[3]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (col + j >= p.N) break;
+        if (p.out_bf16) ((__nv_bfloat16*)p.y)[off + j] = __float2bfloat16_rn(o[j]);
+        else ((float*)p.y)[off + j] = o[j];
+    }
+}
+
+// The sums of a tile's parts as the CTAs of a cluster have parked them ([quarter][4 columns][32 rows] float4, the same layout in each):
+// items `first` .. `end` - 1 of `units` column units of the quarters that have rows, kItems of them and kParts parts under way at a time.
+// A lane reads its row.  Stored so, an instruction would touch 32 rows, 16 bytes of each; kItems lanes exchange their items first, so that it
+// writes 32 / kItems rows, kItems * 16 bytes of each.  688 x 1152 x 3136 in two parts, with bias: 20.1 us without this and with the epilogue
+// applied unit by unit, 16.7 so (18.2 when the parts went through L2 to the CTA that finished last).
+template <uint32_t BN, uint32_t kItems, uint32_t kParts>
+__device__ __forceinline__ void add_parked(const KParams& p, uint32_t park, uint32_t first, uint32_t end, uint32_t units, uint32_t row0, uint32_t col0, uint32_t lane) {
+    const bool vec = p.N % 4 == 0 && ((uintptr_t)p.y & 15) == 0;      // four columns of a row start on a 16-byte (bf16: 8-byte) boundary
+#pragma unroll 1
+    for (uint32_t i0 = first; i0 < end; i0 += kItems) {
+        float4 f[kItems][kParts];
+#pragma unroll
+        for (uint32_t e = 0; e < kItems; ++e) {
+            const uint32_t i = i0 + e < end ? i0 + e : i0, quarter = i / units, unit = i - quarter * units;
+#pragma unroll
+            for (uint32_t s = 0; s < kParts; ++s)
+                if (s < p.split_k) f[e][s] = ptx::ld_cluster_f4(ptx::mapa(park + quarter * (BM * BN) + unit * 512 + lane * 16, s));
+        }
+        float o[kItems][4];
+#pragma unroll
+        for (uint32_t e = 0; e < kItems; ++e) {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) o[e][j] = 0.0f;
+#pragma unroll
+            for (uint32_t s = 0; s < kParts; ++s)
+                if (s < p.split_k) { o[e][0] += f[e][s].x; o[e][1] += f[e][s].y; o[e][2] += f[e][s].z; o[e][3] += f[e][s].w; }
+        }
+        const uint32_t quarter = i0 / units, unit = i0 - quarter * units, row = row0 + quarter * 32;
+        if (i0 + kItems <= end && unit + kItems <= units) {            // (warp-uniform) all of one quarter
+            apply_epilogue(*(float (*)[kItems * 4])o, col0 + unit * 4, p);
+            // item e of lane l goes to item l % kItems of lane l - l % kItems + e, a bit at a time
+#pragma unroll
+            for (uint32_t bit = 1; bit < kItems; bit *= 2) {
+                const bool upper = lane & bit;
+#pragma unroll
+                for (uint32_t e = 0; e < kItems; ++e) {
+                    if (e & bit) continue;
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        const float got = __shfl_xor_sync(0xFFFFFFFFu, upper ? o[e][j] : o[e + bit][j], bit);
+                        if (upper) o[e][j] = got;
+                        else o[e + bit][j] = got;
+                    }
+                }
+            }
+#pragma unroll
+            for (uint32_t e = 0; e < kItems; ++e) store4(p, vec, row + lane / kItems * kItems + e, col0 + (unit + lane % kItems) * 4, o[e]);
+            continue;
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < kItems; ++e) {
+            const uint32_t i = i0 + e;
+            if (i >= end) break;
+            apply_epilogue(o[e], col0 + i % units * 4, p);
+            store4(p, vec, row0 + i / units * 32 + lane, col0 + i % units * 4, o[e]);
         }
     }
 }
@@ -72,7 +145,8 @@ struct GroupOperands3 {
 
 // B_MN = B is given as B[K,N] (N contiguous), A_MN = A is given as A[K,M] (M contiguous): boxes of 64(k) x 64 columns, read by the
 // UMMA through MN-major descriptors.
-template <uint32_t BN, bool B_MN, bool kGrouped = false, bool A_MN = false>
+// kCluster = the parts of a tile's K are the CTAs of a cluster, one tile each: they add their sums through distributed shared memory.
+template <uint32_t BN, bool B_MN, bool kGrouped = false, bool A_MN = false, bool kCluster = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_y, const KParams p,
@@ -97,7 +171,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint64_t* empty_bar = bars + kStages;            // [kStages] UMMAs finished reading the stage
     uint64_t* tmem_full_bar = bars + 2 * kStages;    // [2] accumulator complete
     uint64_t* tmem_empty_bar = bars + 2 * kStages + 2;  // [2] accumulator drained by the epilogue
-    uint32_t* tmem_holder = (uint32_t*)(bars + 2 * kStages + 4);
+    uint64_t* parked_bar = bars + 2 * kStages + 4;      // kCluster: every epilogue warp of the cluster has parked its rows
+    uint32_t* tmem_holder = (uint32_t*)(bars + 2 * kStages + 5);
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
 
     const uint32_t warp = threadIdx.x >> 5;
@@ -115,6 +190,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             ptx::mbar_init(ptx::smem_u32(&tmem_full_bar[b]), 1);
             ptx::mbar_init(ptx::smem_u32(&tmem_empty_bar[b]), 4);   // one arrival per epilogue warp
         }
+        if constexpr (kCluster) ptx::mbar_init(ptx::smem_u32(parked_bar), 4 * p.split_k);
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
@@ -128,6 +204,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     ptx::tc_fence_before_sync();
     __syncthreads();
+    if constexpr (kCluster) ptx::cluster_sync_all();          // every CTA's barriers exist before anyone signals across the cluster
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
     // everything above touched only shared and tensor memory; global memory comes after the previous grid is done
@@ -148,7 +225,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const CUtensorMap* ma = &map_a;
                 const CUtensorMap* mb = &map_b;
                 if constexpr (kGrouped) { ma = &group.maps[3 * prob]; mb = &group.maps[3 * prob + 1]; }
-                const KRange kr = k_range(wi.split, p);
+                const KRange kr = k_range<kCluster>(wi.split, p);
                 for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
                     if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
                         atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
@@ -194,7 +271,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const KRange kr = k_range(w % p.split_k, p);
+                const KRange kr = k_range<kCluster>(w % p.split_k, p);
                 const uint32_t kb_mid = k_mid<kAccs>(kr, p);
                 uint32_t tmem_d = tmem_base + buf * BN * kAccs;
                 for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
@@ -236,56 +313,51 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             if constexpr (kGrouped) { y_out = group.y[prob]; my = &group.maps[3 * prob + 2]; }
             const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
             const uint32_t row_base = wi.m_blk * BM + quarter * 32;
-            // Split-K with a complete result.  The parts of a tile are added by whichever CTA gets to it last, each epilogue warp its own 32
-            // rows: a warp takes a ticket (low half of the counter); all but the last store their partial sums in the order their lanes
-            // hold them and count them as written (high half); the last one waits for those counts and adds the parts in split order, so
-            // the result does not depend on who was last.  The warps it waits for hold a ticket: they are running and wait for nobody.
-            const bool in_parts = p.pieces != nullptr && row_base < p.M;
-            uint32_t ticket = 0;
-            uint32_t* const counter = p.tickets + (w / p.split_k) * 4 + quarter;
-            if (in_parts && lane == 0) ticket = atomicAdd(counter, 1u) & 0xFFFFu;      // (its round trip passes under the main loop)
+            if constexpr (kCluster) {
+                // the tile's bias into L1 under the main loop: the warps would wait for it once for every few columns they add
+                if (p.bias && lane * 32 < BN && wi.n_blk * BN + lane * 32 < p.N) ptx::prefetch_l1(p.bias + wi.n_blk * BN + lane * 32);
+            }
             if (!ptx::mbar_wait(ptx::smem_u32(&tmem_full_bar[buf]), acc_phase, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(w & 0xFFFFFF));
                 break;
             }
             ptx::tc_fence_after_sync();
-            const KRange kr = k_range(wi.split, p);
+            const KRange kr = k_range<kCluster>(wi.split, p);
             const bool two_accs = k_mid<kAccs>(kr, p) < kr.end;
             const uint32_t tmem_acc = tmem_base + ((quarter * 32) << 16) + buf * BN * kAccs;
-            constexpr uint32_t kPieceF4 = BM * BN / 4;                                 // of one part; BN / 32 chunks of 8 x 32 lanes per warp
-            float4* const piece0 = p.pieces + (size_t)(w - wi.split) * kPieceF4 + quarter * (kPieceF4 / 4) + lane;
-            if (in_parts) {
-                ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-                if (ticket + 1 != p.split_k) {
-                    float4* const mine = piece0 + (size_t)wi.split * kPieceF4;
+            if constexpr (kCluster) {
+                // Split-K with a complete result: the CTAs of the cluster hold the parts of one tile.  Every warp parks its rows' sums in its
+                // CTA's shared memory, over the ring that is idle by then, and tells every CTA.  The tile is then shared out evenly over all
+                // the warps of the cluster, whatever its rows and columns; the parts are added in split order, the same sums as the planes
+                // form.  Nothing but the operands and the result is in global memory, so launches may run beside one another, recorded or not.
+                // What bounds it is latency: park, signal, and one or two round trips of remote reads, about 3 us with the cluster's start.
+                // 16 x 2048 x 2048: 8.8 us, 10.9 with the parts added through L2 by the CTA that finishes last, 20.0 as clusters of
+                // eight that do not all run at once; 128 x 4096 x 4096 (32 clusters of four): 15.6 us, 16.9 with column slices read row by row.
+                const uint32_t park = ptx::smem_u32(smem);
 #pragma unroll 1
-                    for (uint32_t c = 0; c < BN / 32; ++c) {
-                        if (wi.n_blk * BN + c * 32 >= p.N) break;
-                        uint32_t r[32];
-                        load_acc<BN>(tmem_acc + c * 32, two_accs, r);
+                for (uint32_t c = 0; c < BN / 32 && row_base < p.M; ++c) {
+                    uint32_t r[32];
+                    load_acc<BN>(tmem_acc + c * 32, two_accs, r);
 #pragma unroll
-                        for (uint32_t j = 0; j < 8; ++j)
-                            __stcg(mine + (c * 8 + j) * 32, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
-                                                                        __uint_as_float(r[4 * j + 3])));
-                    }
-                    ptx::tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) {
-                        ptx::mbar_arrive(ptx::smem_u32(&tmem_empty_bar[buf]));
-                        __threadfence();                                               // the warp's part is visible before it is counted
-                        atomicAdd(counter, 0x10000u);
-                    }
-                    continue;
+                    for (uint32_t j = 0; j < 8; ++j)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(park + quarter * (BM * BN) + (c * 8 + j) * 512 + lane * 16), "r"(r[4 * j]),
+                                     "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3])
+                                     : "memory");
                 }
-                uint32_t good = 1;
-                if (lane == 0) {
-                    good = wait_for_parts(counter, p.split_k, abort_flag, p.wait_limit_ns) ? 1u : 0u;
-                    if (good) *counter = 0;                                            // ready for the next launch
-                    else atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(w & 0x7FFFFF));
-                    __threadfence();
+                __syncwarp();
+                if (lane == 0)
+                    for (uint32_t s = 0; s < p.split_k; ++s) ptx::mbar_arrive_cluster(ptx::mapa(ptx::smem_u32(parked_bar), s));
+                if (!ptx::mbar_wait_cluster(ptx::smem_u32(parked_bar), 0, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(w & 0x7FFFFF));
+                    break;
                 }
-                good = __shfl_sync(0xFFFFFFFFu, good, 0);
-                if (!good) break;
+                const uint32_t row0 = wi.m_blk * BM, col0 = wi.n_blk * BN;
+                const uint32_t units = (min(BN, p.N - col0) + 3) / 4;
+                const uint32_t items = (min(BM, p.M - row0) + 31) / 32 * units;
+                const uint32_t worker = wi.split * 4 + warp - 2, first = worker * items / (4 * p.split_k), end = (worker + 1) * items / (4 * p.split_k);
+                if (p.split_k <= 4) add_parked<BN, 4, 4>(p, park, first, end, units, row0, col0, lane);
+                else add_parked<BN, 2, 8>(p, park, first, end, units, row0, col0, lane);
+                break;                                   // a cluster has one tile
             }
 #pragma unroll 1
             for (uint32_t c = 0; c < BN / 32; ++c) {
@@ -293,35 +365,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 if (col0 >= p.N) break;   // warp-uniform
                 uint32_t r[32];
                 load_acc<BN>(tmem_acc + c * 32, two_accs, r);
-                if (in_parts) {
-                    float sum[32];
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) sum[j] = 0.0f;
-#pragma unroll 1
-                    for (uint32_t s0 = 0; s0 < p.split_k; s0 += 4) {
-                        // the loads of four parts are under way together: one round trip to L2 per chunk and four parts, not one per part
-                        float4 f[4][8];
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) {
-                            const float4* theirs = piece0 + (size_t)(s0 + i) * kPieceF4 + c * 8 * 32;
-                            const bool other = s0 + i < p.split_k && s0 + i != wi.split;
-#pragma unroll
-                            for (uint32_t j = 0; j < 8; ++j) {
-                                f[i][j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-                                if (other) f[i][j] = __ldcg(theirs + j * 32);
-                            }
-                        }
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; ++i) {
-                            if (s0 + i >= p.split_k) break;
-#pragma unroll
-                            for (uint32_t j = 0; j < 8; ++j) { sum[4 * j] += f[i][j].x; sum[4 * j + 1] += f[i][j].y; sum[4 * j + 2] += f[i][j].z; sum[4 * j + 3] += f[i][j].w; }
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[j]);
-                }
-                store_chunk(p, r, row_base, lane, c, col0, in_parts ? 0u : wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores,
+                store_chunk(p, r, row_base, lane, c, col0, wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores,
                             p.tma_store ? my : nullptr, y_out);
             }
             ptx::tc_fence_before_sync();
@@ -340,6 +384,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     ptx::tc_fence_before_sync();
     __syncthreads();
+    if constexpr (kCluster) ptx::cluster_sync_all();          // no CTA's shared memory goes away while a peer may still read it or signal its barrier
     if (warp == 1) {
         ptx::tc_fence_after_sync();
         ptx::tmem_dealloc(tmem_base, kTmemCols);
@@ -348,10 +393,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 // ------------------------------------------------------------------ host side
 
-template <uint32_t BN, bool B_MN, bool kGrouped = false, bool A_MN = false>
+template <uint32_t BN, bool B_MN, bool kGrouped = false, bool A_MN = false, bool kCluster = false>
 int launch_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const KParams& p, uint32_t grid, cudaStream_t stream,
                     const std::conditional_t<kGrouped, GroupOperands3, NoGroup>& group = {}) {
-    auto kern = gemm_bf16_tcgen05_kernel<BN, B_MN, kGrouped, A_MN>;
+    auto kern = gemm_bf16_tcgen05_kernel<BN, B_MN, kGrouped, A_MN, kCluster>;
     const uint32_t smem = gemm_smem_bytes(BN);
     static bool attr_set[64] = {};   // per instantiation, per device
     int dev = 0;
@@ -361,16 +406,44 @@ int launch_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensor
         if (e != cudaSuccess) return fail(T0_ERR_CUDA, "cudaFuncSetAttribute(smem=%u): %s", smem, cudaGetErrorString(e));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    cudaError_t e = launch_pdl(kern, grid, kThreads, smem, stream, ma, mb, my, p, group);
+    cudaError_t e = launch_pdl_clusters(kern, grid, kCluster ? p.split_k : 1, kThreads, smem, stream, ma, mb, my, p, group);
     if (e != cudaSuccess) return fail(T0_ERR_CUDA, "GEMM kernel launch failed: %s", cudaGetErrorString(e));
     return T0_OK;
 }
 
 }  // namespace
 
-size_t gemm_pieces_bytes(uint32_t m, uint32_t n, uint32_t tile_n, uint32_t split) {
-    const uint32_t bn = snap_tile_n(tile_n);
-    return (size_t)ceil_div(m, BM) * ceil_div(n, bn) * split * BM * bn * sizeof(float);
+// The SMs of a GPC hold whole clusters only, and GPCs differ in size: 148 SMs hold 15 clusters of eight, not 18.  Devices of one model may
+// differ a little, and a product is not to be cut otherwise on another of them, so the table keeps a margin below what a B200 reports
+// (74, 45, 33, 26, 22, 15, 15); the device's own figure counts only where it is lower still.
+const uint32_t* gemm_clusters_at_once() {
+    static uint32_t table[64][kMaxClusterParts + 1] = {};
+    static std::mutex mu;
+    static const uint32_t safe[kMaxClusterParts + 1] = {0, 148, 72, 40, 32, 24, 20, 14, 14};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return safe;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!table[dev][1]) {
+        auto kern = gemm_bf16_tcgen05_kernel<64, false, false, false, true>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes(64));
+        for (uint32_t size = 2; size <= kMaxClusterParts; ++size) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim = {size, 1, 1};
+            cfg.gridDim = dim3(size * 148, 1, 1);
+            cfg.blockDim = dim3(kThreads, 1, 1);
+            cfg.dynamicSmemBytes = gemm_smem_bytes(64);
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 1; }
+            table[dev][size] = std::min((uint32_t)n, safe[size]);
+        }
+        table[dev][1] = safe[1];
+    }
+    return table[dev];
 }
 
 uint32_t gemm_stage_count(uint32_t tile_n) { return stages_for(snap_tile_n(tile_n)); }
@@ -384,12 +457,12 @@ uint32_t gemm_smem_bytes(uint32_t tile_n) {
 int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     if (g.m == 0 || g.n == 0) return T0_OK;
     if (g.k == 0) return fail(T0_ERR_INVALID, "K must be positive");
-    // parts of K: planes of the output (and of the operand maps), or, with scratch for the partial sums, ranges of the whole K
-    const bool parts = g.pieces != nullptr && g.split_k > 1;
+    // parts of K: planes of the output (and of the operand maps), or, where the launch adds them itself, ranges of the whole K
+    const bool parts = g.cluster && g.split_k > 1;
     const uint32_t planes = parts || g.split_k == 0 ? 1 : g.split_k, split = parts ? g.split_k : planes;
     if (g.k % planes) return fail(T0_ERR_UNSUPPORTED, "K=%u not divisible by split_k=%u", g.k, split);
     const uint32_t kps = g.k / planes;
-    if (parts && (!g.tickets || split > ceil_div(g.k, BK) || ceil_div(g.m, BM) * (uint64_t)ceil_div(g.n, snap_tile_n(g.tile_n)) > kMaxTicketTiles))
+    if (parts && (split > kMaxClusterParts || split > ceil_div(g.k, BK)))
         return fail(T0_ERR_UNSUPPORTED, "split-K in one launch: %u parts of %u k blocks", split, ceil_div(g.k, BK));
     const uint32_t ldx = g.ldx ? g.ldx : (g.at ? g.m : g.k);
     const uint32_t ldb = g.ldb ? g.ldb : (g.nn ? g.n : g.k);
@@ -411,7 +484,6 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     p.out_bf16 = g.out_bf16 ? 1 : 0; p.epilogue = g.epilogue; p.n_ops = g.n_ops;
     p.scale = g.scale; p.clamp_min = g.clamp_min; p.clamp_max = g.clamp_max;
     memcpy(p.ops, g.ops, sizeof p.ops);
-    if (parts) { p.pieces = (float4*)g.pieces; p.tickets = g.tickets; }
     p.halves = g.halves ? 1 : 0;
 
     CUtensorMap ma, mb;
@@ -422,7 +494,7 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
 
     const uint64_t total = (uint64_t)p.tiles_m * p.tiles_n * split;
     if (total > 0x7FFFFFFFull) return fail(T0_ERR_UNSUPPORTED, "too many tiles");
-    const uint32_t grid = (uint32_t)std::min<uint64_t>(total, g.n_sms ? g.n_sms : 148);
+    const uint32_t grid = (uint32_t)(parts ? total : std::min<uint64_t>(total, g.n_sms ? g.n_sms : 148));
     CUtensorMap my = ma;   // a valid map either way; only read when p.tma_store is set
     if (tma_output_ok(g, planes, bn)) {
         rc = make_map_out(&my, g.y, g.m, g.n, planes, g.plane_stride, g.out_bf16);
@@ -432,6 +504,25 @@ int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream) {
     rc = stage_peer_maps(g, p, split, stream);
     if (rc != T0_OK) return rc;
 
+    if (parts) {
+        if (g.at && bn <= 128)
+            return bn == 64 ? launch_instance<64, true, false, true, true>(ma, mb, my, p, grid, stream)
+                            : launch_instance<128, true, false, true, true>(ma, mb, my, p, grid, stream);
+        if (g.at) return fail(T0_ERR_UNSUPPORTED, "no cluster form for a transposed first operand with 256-wide tiles");
+        if (g.nn) {
+            switch (bn) {
+                case 64: return launch_instance<64, true, false, false, true>(ma, mb, my, p, grid, stream);
+                case 128: return launch_instance<128, true, false, false, true>(ma, mb, my, p, grid, stream);
+                default: return launch_instance<256, true, false, false, true>(ma, mb, my, p, grid, stream);
+            }
+        }
+        switch (bn) {
+            case 32: return launch_instance<32, false, false, false, true>(ma, mb, my, p, grid, stream);
+            case 64: return launch_instance<64, false, false, false, true>(ma, mb, my, p, grid, stream);
+            case 128: return launch_instance<128, false, false, false, true>(ma, mb, my, p, grid, stream);
+            default: return launch_instance<256, false, false, false, true>(ma, mb, my, p, grid, stream);
+        }
+    }
     if (g.at) {
         switch (bn) {
             case 64: return launch_instance<64, true, false, true>(ma, mb, my, p, grid, stream);

@@ -42,31 +42,6 @@ __host__ __device__ constexpr uint32_t sk_bars_offset(uint32_t bn) {
 }
 constexpr uint32_t kSkMaxStages = 9;
 
-// wait with cluster-scope acquire: the arrivals come from other CTAs and order their shared-memory writes before our reads
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    uint64_t t_start = 0;
-    for (uint32_t spin = 1;; ++spin) {
-        if (mbar_try_wait_cluster(bar, parity)) return true;
-        if ((spin & 0xFF) == 0) {
-            if (*abort_flag) return false;
-            const uint64_t now = ptx::globaltimer_ns();
-            if (t_start == 0) t_start = now;
-            else if (now - t_start > limit_ns) { *abort_flag = 1; return false; }
-        }
-    }
-}
 __device__ __forceinline__ uint32_t cluster_id_x() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
@@ -77,12 +52,6 @@ __device__ __forceinline__ uint32_t n_clusters_x() {
     asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 // Grouped launch: the tensor maps and outputs of up to kMaxGroupedGemms problems of one shape ride in the kernel parameters
 // (8.4 KB; parameters may be 32 KB).  The single-problem kernel takes an empty record instead.
 struct GroupOperands {
@@ -245,7 +214,7 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
                 ok = false;
             }
             // the copy of the previous tile has been read by everyone before it is overwritten
-            if (ok && iter > 0 && !mbar_wait_cluster(readb, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) {
+            if (ok && iter > 0 && !ptx::mbar_wait_cluster(readb, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x400000 | (int)(w & 0x3FFFFF));
                 ok = false;
             }
@@ -273,7 +242,7 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
                 ptx::mbar_arrive(ptx::smem_u32(&tmem_empty_bar[buf]));                         // the issuer may reuse the accumulator
                 for (uint32_t s = 0; s < n_split; ++s) ptx::mbar_arrive_cluster(ptx::mapa(parked, s));   // tell every CTA (release, cluster scope)
             }
-            if (!mbar_wait_cluster(parked, iter & 1, abort_flag, p.wait_limit_ns)) {
+            if (!ptx::mbar_wait_cluster(parked, iter & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(w & 0x3FFFFF));
                 ok = false;
                 break;
@@ -296,7 +265,7 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
                         const bool live = r0 + u * rows_per_inst < quarter * 32 + 32;
 #pragma unroll
                         for (uint32_t s = 0; s < 8; ++s)
-                            part[u][s] = (live && s < n_split) ? ld_cluster_f4(ptx::mapa(park + (row_in * kPitch + col_in) * 4, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            part[u][s] = (live && s < n_split) ? ptx::ld_cluster_f4(ptx::mapa(park + (row_in * kPitch + col_in) * 4, s)) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
                     for (uint32_t u = 0; u < kU; ++u) {

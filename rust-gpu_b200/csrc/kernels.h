@@ -20,8 +20,7 @@ struct GemmLaunch {
     uint32_t ldx, ldb;    // row strides in elements (0 = dense)
     uint32_t tile_n;      // 32/64/128/256
     uint32_t split_k;     // >= 1
-    void* pieces;         // single-CTA kernel, split_k > 1: scratch of gemm_pieces_bytes; the result is then complete in y, in one launch
-    uint32_t* tickets;    // ... four words per output tile, zero before and after
+    bool cluster;         // single-CTA kernel, 1 < split_k <= kMaxClusterParts: the parts meet in clusters, the result is complete in y
     bool halves;          // single-CTA kernel, tile_n <= 128: sums of half the length, added in f32
     uint64_t plane_stride;  // elements between split planes
     bool nn, out_bf16, swap_grid;
@@ -50,8 +49,9 @@ constexpr uint32_t kMaxPeerY = 7;
 // K / split_k multiples of 8 elements, K % split_k == 0.  Returns a T0_* code.
 int launch_gemm_sm100(const GemmLaunch& g, cudaStream_t stream);
 
-size_t gemm_pieces_bytes(uint32_t m, uint32_t n, uint32_t tile_n, uint32_t split);
-constexpr uint32_t kMaxTicketTiles = 4096;
+constexpr uint32_t kMaxClusterParts = 8;       // the portable cluster size
+// How many clusters of 1 .. kMaxClusterParts CTAs (the index), one CTA per SM, run at once on the current device.
+const uint32_t* gemm_clusters_at_once();
 
 // The CTA-pair form (cta_group::2; 256 x 256 tiles, or 256 x 128 when tile_n <= 128); NT, and NN with 256-wide tiles.
 int launch_gemm_sm100_pair(const GemmLaunch& g, cudaStream_t stream);
@@ -70,7 +70,7 @@ int launch_gemm_sm100_splitk_grouped(const GemmLaunch* gs, uint32_t count, cudaS
 int launch_gemm_sm100_grouped(const GemmLaunch* gs, uint32_t count, cudaStream_t stream);
 
 // The kernel a product runs on when the caller fixes nothing: CTA pairs or single CTAs, the tile width, and into how many parts K is
-// cut (single CTAs; added in the same launch).
+// cut (single CTAs in clusters; added in the same launch).
 struct GemmChoice {
     uint32_t tile_n, parts;
     bool pair, halves;
@@ -78,7 +78,7 @@ struct GemmChoice {
 // No accumulation is longer than k / min_split: the tensor cores' error grows with the length of the sum (about 1e-9 of the result per
 // term), so a shape whose configuration (auto_select) cuts K keeps sums at least that short, in parts or in two accumulators.  parts = 0:
 // nothing here does that (many tiles and a deep cut); the configuration itself is to be taken.
-GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms);
+GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once);
 
 // y[i] = sum_s planes[s][i] in split order, then the epilogue; K4.
 int launch_splitk_reduce(const float* planes, void* y, const float* bias, uint32_t m, uint32_t n, uint32_t split_k,

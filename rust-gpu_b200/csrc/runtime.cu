@@ -52,7 +52,7 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
         GemmChoice choice = {};
         if (!getenv("T0_FORCE_CFG")) {
             const uint32_t s = known && c.split_k > 1 && q.k % c.split_k == 0 ? c.split_k : 1;
-            choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count);
+            choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count, gemm_clusters_at_once());
         }
         if (choice.parts) {
             q.tile_n = choice.tile_n;
@@ -138,30 +138,19 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
 
     bool fused_reduce = split > 1 && !q.planes;
     static const bool no_cluster = getenv("T0_NO_CLUSTER_SPLITK") != nullptr;
-    // Split-K in one launch, the parts added by the CTA that finishes last (gemm_sm100.cu).  A split the caller asked for runs this way
-    // where its parts are whole k blocks (the parts, and so the sums, are then those of the planes form) and the launch is about one wave.
+    // Split-K in one launch, the parts of a tile as the CTAs of a cluster (gemm_sm100.cu).  A split the caller asked for runs this way
+    // where its parts are whole k blocks (the parts, and so the sums, are then those of the planes form) and few clusters run one after the other.
     uint32_t parts = q.parts > 1 && !use_pair ? q.parts : 0;
-    if (fused_reduce && !use_pair && !no_cluster && q.k % (64u * split) == 0) parts = split;
-    if (parts) {
-        const uint64_t tiles = (uint64_t)ceil_div(q.m, 128) * ceil_div(q.n, g.tile_n);
-        const size_t bytes = gemm_pieces_bytes(q.m, q.n, g.tile_n, parts);
-        if (tiles > kMaxTicketTiles || tiles * parts > 4ull * (uint64_t)rt->sm_count) parts = 0;
-        // 128 x 128 tiles with most of their rows: 64 KB a part, which the CTAs of a cluster exchange faster (each adds a slice) than one of
-        // them reads the others' from L2: 16.7 against 17.8 us at 128 x 4096 x 4096 in four parts, but 17.9 against 16.8 at M = 64
-        if (parts && g.tile_n == 128 && q.m > 64 && !q.halves && !q.nn && !q.at && (parts == 2 || parts == 4) && q.k % (64u * parts) == 0 && !no_cluster) {
-            g.split_k = split = parts;
-            parts = 0;
-            fused_reduce = true;
-        }
-        if (parts && bytes > rt->scratch_planes.size) {
-            // nothing may be allocated while the stream is being captured: the forms without scratch then
-            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-            T0_CUDA(cudaStreamIsCapturing(rt->stream, &capturing));
-            if (capturing != cudaStreamCaptureStatusNone) parts = 0;
-            else if (int rc = ensure_scratch(rt, rt->scratch_planes, bytes)) return rc;
-        }
+    if (fused_reduce && !use_pair && !no_cluster && q.k % (64u * split) == 0 && split <= kMaxClusterParts) {
+        // (where several clusters would run one after the other: the persistent form of gemm_sm100_splitk.cu if it takes the
+        // request, and from about four waves on the planes)
+        const uint64_t tiles = (uint64_t)ceil_div(q.m, 128) * ceil_div(q.n, g.tile_n), at_once = gemm_clusters_at_once()[split];
+        if (tiles <= (gemm_splitk_cluster_supported(g) ? at_once : 4 * at_once)) parts = split;
     }
-    if (parts) { g.split_k = parts; g.pieces = rt->scratch_planes.ptr; g.tickets = rt->d_tickets; }
+    if (parts) {
+        g.split_k = parts;
+        g.cluster = true;
+    }
     if (fused_reduce && !use_pair && !parts) {
         // one launch: the CTAs that share a tile form a cluster and add their partial sums through distributed shared
         // memory (T0_NO_CLUSTER_SPLITK=1 keeps the two-launch form below for comparison)
@@ -377,8 +366,6 @@ int t0_rt_new(int device, t0_runtime** out) {
     T0_CUDA(cudaEventCreate(&rt->ev_stop));
     T0_CUDA(cudaMalloc(&rt->d_probe, (2 + 64) * sizeof(unsigned long long)));   // clock words + eight launches' trace stamps
     T0_CUDA(cudaMemset(rt->d_probe, 0, (2 + 64) * sizeof(unsigned long long)));
-    T0_CUDA(cudaMalloc(&rt->d_tickets, kMaxTicketTiles * 4 * sizeof(uint32_t)));
-    T0_CUDA(cudaMemset(rt->d_tickets, 0, kMaxTicketTiles * 4 * sizeof(uint32_t)));
     T0_CUDA(cudaHostAlloc(&rt->h_status, sizeof(int), cudaHostAllocMapped));
     *rt->h_status = 0;
     T0_CUDA(cudaHostGetDevicePointer(&rt->d_status, rt->h_status, 0));
@@ -395,7 +382,6 @@ void t0_rt_free(t0_runtime* rt) {
     for (Scratch* s : {&rt->scratch_a, &rt->scratch_b, &rt->scratch_planes, &rt->scratch_w4, &rt->scratch_um, &rt->scratch_w, &rt->scratch_cvt_a, &rt->scratch_cvt_b, &rt->scratch_cvt_c})
         if (s->ptr) cudaFree(s->ptr);
     if (rt->d_probe) cudaFree(rt->d_probe);
-    if (rt->d_tickets) cudaFree(rt->d_tickets);
     if (rt->d_peer_maps) cudaFree(rt->d_peer_maps);
     if (rt->h_status) cudaFreeHost(rt->h_status);
     if (rt->ev_start) cudaEventDestroy(rt->ev_start);

@@ -55,7 +55,6 @@ struct t0_runtime {
     void* d_peer_maps = nullptr;             // gathered output: device slot for the destinations' tensor maps (made on first use)
     std::vector<uint64_t> peer_maps_key;     // destinations and shape the slot currently describes
     Scratch scratch_a, scratch_b, scratch_planes;
-    uint32_t* d_tickets = nullptr;           // split-K in one launch: arrivals per output tile and epilogue warp, zero between launches
     Scratch scratch_w4;          // W4A16: slab arrival counters + straddling pieces
     Scratch scratch_um;          // tcgen05 W4A16, grouped: counters + partial sums of the cut tiles
     Scratch scratch_w;           // W4A16 general path: dequantised weights

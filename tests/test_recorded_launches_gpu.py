@@ -1,0 +1,223 @@
+"""GPU tests of launches recorded into a CUDA graph (stream capture of the runtime's stream) and replayed: later calls of the runtime may
+run larger products first, the replay may run on another stream beside the runtime's own, and nothing may be allocated while recording.
+"""
+import contextlib
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+class Driver:
+    """The few driver calls a program needs to record a stream and replay the graph (the library has no entry for it)."""
+
+    def __init__(self):
+        self.cu = C.CDLL("libcuda.so.1")
+        ctx = C.c_void_p()
+        self.call("cuDevicePrimaryCtxRetain", C.byref(ctx), 0)
+        self.call("cuCtxSetCurrent", ctx)
+
+    def call(self, name, *args):
+        rc = getattr(self.cu, name)(*args)
+        assert rc == 0, f"{name} returned {rc}"
+
+    @contextlib.contextmanager
+    def record(self, rt):
+        """Records what the block launches on the runtime's stream; the yielded list then holds the executable graph."""
+        out, graph, stream = [], C.c_void_p(), C.c_void_p(rt.stream())
+        self.call("cuStreamBeginCapture_v2", stream, 0)                      # 0 = global mode: an allocation would be refused
+        try:
+            yield out
+        finally:
+            rc = self.cu.cuStreamEndCapture(stream, C.byref(graph))
+        assert rc == 0, f"the capture was invalidated ({rc})"
+        ex = C.c_void_p()
+        self.call("cuGraphInstantiateWithFlags", C.byref(ex), graph, C.c_ulonglong(0))
+        self.call("cuGraphDestroy", graph)
+        out.append(ex)
+
+    def replay(self, ex, stream):
+        self.call("cuGraphLaunch", ex, C.c_void_p(stream))
+
+    def stream(self):
+        s = C.c_void_p()
+        self.call("cuStreamCreate", C.byref(s), 1)                           # 1 = does not synchronise with the default stream
+        return s.value
+
+    def sync(self, stream):
+        self.call("cuStreamSynchronize", C.c_void_p(stream))
+
+    def drop(self, ex=None, stream=None):
+        if ex is not None:
+            self.call("cuGraphExecDestroy", ex)
+        if stream is not None:
+            self.call("cuStreamDestroy_v2", C.c_void_p(stream))
+
+
+@pytest.fixture()
+def driver(rt):
+    return Driver()
+
+
+@pytest.fixture()
+def fresh(t0):
+    """A runtime of its own: no buffer has grown yet."""
+    r = t0.GpuRuntime(0)
+    yield r
+    r.close()
+
+
+def bf16_bits(v):
+    u = np.ascontiguousarray(v, np.float32).view(np.uint32).astype(np.uint64)
+    return ((u + 0x7FFF + ((u >> 16) & 1)) >> 16).astype(np.uint16)
+
+
+class Product:
+    """One bf16 product on the runtime: real-valued operands, so that another order of the sums would show in the bits."""
+
+    def __init__(self, t0, rt, m, n, k, seed, layout="nt", out_bf16=False, **kw):
+        rng = np.random.default_rng(seed)
+        self.rt, self.dims, self.words = rt, (m, n, k), m * n // (2 if out_bf16 else 1)
+        self.kw = dict(kw, out_bf16=out_bf16, transpose=t0.NN if layout == "nn" else t0.NT)
+        self.x, self.b = (rt.upload(bf16_bits(rng.uniform(-1, 1, c))) for c in (m * k, n * k))
+        self.ys = []
+
+    def out(self):
+        self.ys.append(self.rt.alloc(self.words * 4))
+        self.ys[-1].write(np.full(self.words, 0xFFFFFFFF, np.uint32))
+        return self.ys[-1]
+
+    def launch(self, y):
+        self.rt.gemm(self.x.gpu_addr(), self.b.gpu_addr(), y.gpu_addr(), *self.dims, **self.kw)
+
+    def eager(self):
+        y = self.out()
+        self.launch(y)
+        self.rt.synchronize()
+        return self.bits(y)
+
+    def bits(self, y):
+        return y.read(self.words * 4, np.uint32)
+
+    def free(self):
+        for buf in [self.x, self.b] + self.ys:
+            buf.free()
+
+
+# products whose K the library cuts: two to eight parts, tiles of 32, 64 and 128 columns, an odd number of k blocks, a ragged last chunk
+CUT = [(16, 2048, 2048), (64, 4096, 4096), (32, 752, 3984), (128, 4096, 2048), (128, 4096, 4096), (512, 512, 2048), (100, 296, 8192), (64, 512, 8192), (16, 40, 10240)]
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+@pytest.mark.parametrize("out_bf16", [False, True])
+def test_recorded_products_equal_eager_ones(t0, fresh, driver, layout, out_bf16):
+    # recorded on a fresh runtime (nothing reserved, nothing run), then larger products on the runtime, then the replay
+    cases = [Product(t0, fresh, m, n, k, seed=m + n, layout=layout, out_bf16=out_bf16) for m, n, k in CUT]
+    ys = [p.out() for p in cases]
+    with driver.record(fresh) as graphs:
+        for p, y in zip(cases, ys):
+            p.launch(y)
+    larger = [Product(t0, fresh, m, n, k, seed=1, layout=layout) for m, n, k in [(128, 4736, 8192), (256, 2048, 8192), (2048, 2048, 4096)]]
+    for p in larger:
+        p.eager()
+    want = [p.eager() for p in cases]
+    for _ in range(3):
+        for y, p in zip(ys, cases):
+            y.write(np.full(p.words, 0xFFFFFFFF, np.uint32))
+        driver.replay(graphs[0], fresh.stream())
+        fresh.synchronize()
+        for p, y, w in zip(cases, ys, want):
+            assert np.array_equal(p.bits(y), w), p.dims
+    driver.drop(graphs[0])
+    for p in cases + larger:
+        p.free()
+
+
+@pytest.mark.parametrize("layout,kw", [("nt", dict(tile_n=32, split_k=4)), ("nt", dict(tile_n=64, split_k=2)), ("nt", dict(tile_n=64, split_k=8)), ("nt", dict(tile_n=128, split_k=8)),
+                                       ("nt", dict(tile_n=256, split_k=4)), ("nn", dict(tile_n=64, split_k=4)), ("nn", dict(tile_n=128, split_k=2)),
+                                       ("nn", dict(tile_n=256, split_k=2)), ("nt", dict(tile_n=128, split_k=4))])
+@pytest.mark.parametrize("m,n,k", [(40, 328, 2048), (200, 520, 1024)])
+def test_recorded_splits_of_the_caller(t0, fresh, driver, layout, kw, m, n, k):
+    p = Product(t0, fresh, m, n, k, seed=3, layout=layout, pair_cta=2, **kw)
+    y = p.out()
+    with driver.record(fresh) as graphs:
+        p.launch(y)
+    want = p.eager()
+    driver.replay(graphs[0], fresh.stream())
+    fresh.synchronize()
+    assert np.array_equal(p.bits(y), want)
+    driver.drop(graphs[0])
+    p.free()
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+def test_replays_beside_the_runtime_s_own_stream(t0, fresh, driver, layout):
+    # two graphs of the same product on two streams, and the product itself on the runtime's stream, all under way together
+    m, n, k = 16, 1024, 4096
+    p = Product(t0, fresh, m, n, k, seed=9, layout=layout)
+    want = p.eager()
+    streams, execs, outs = [driver.stream() for _ in range(2)], [], []
+    for _ in range(2):
+        ys = [p.out() for _ in range(20)]
+        with driver.record(fresh) as graphs:
+            for y in ys:
+                p.launch(y)
+        execs.append(graphs[0])
+        outs.append(ys)
+    own = [p.out() for _ in range(20)]
+    for _ in range(5):
+        for ex, s in zip(execs, streams):
+            driver.replay(ex, s)
+        for y in own:
+            p.launch(y)
+    for s in streams:
+        driver.sync(s)
+    fresh.synchronize()
+    for y in outs[0] + outs[1] + own:
+        assert np.array_equal(p.bits(y), want)
+    for ex, s in zip(execs, streams):
+        driver.drop(ex, s)
+    p.free()
+
+
+def test_recorded_training_step(t0, fresh, driver):
+    # dW reads X as [K, M]; the eager step before the recording makes the conversion buffers
+    m, k, n = 2048, 128, 256
+    rng = np.random.default_rng(2)
+    x, w, dy = (fresh.upload(rng.uniform(-1, 1, s).astype(np.float32)) for s in ((m, k), (k, n), (m, n)))
+    sizes = (m * n, m * k, k * n)
+    eager, replayed = ([fresh.alloc(4 * c) for c in sizes] for _ in range(2))
+
+    def step(ys):
+        fresh.matmul_f32(x.gpu_addr(), w.gpu_addr(), ys[0].gpu_addr(), m, k, n)
+        fresh.matmul_f32_backward_data(dy.gpu_addr(), w.gpu_addr(), ys[1].gpu_addr(), m, k, n)
+        fresh.matmul_f32_backward_weight(x.gpu_addr(), dy.gpu_addr(), ys[2].gpu_addr(), m, k, n)
+
+    step(eager)
+    with driver.record(fresh) as graphs:
+        step(replayed)
+    driver.replay(graphs[0], fresh.stream())
+    fresh.synchronize()
+    for a, b, c in zip(eager, replayed, sizes):
+        assert np.array_equal(a.read(4 * c, np.uint32), b.read(4 * c, np.uint32))
+    driver.drop(graphs[0])
+    for buf in [x, w, dy] + eager + replayed:
+        buf.free()
+
+
+def test_recorded_part_that_never_arrives_ends_with_an_error(t0, fresh, driver):
+    # the first operand load of one part is left out: its cluster gives up after the wait limit, in every CTA, and the error is reported
+    p = Product(t0, fresh, 16, 2048, 2048, seed=4)
+    y = p.out()
+    fresh.set_wait_limit_ns(20_000_000)
+    fresh.selftest_drop_one_load()
+    with driver.record(fresh) as graphs:
+        p.launch(y)
+    driver.replay(graphs[0], fresh.stream())
+    with pytest.raises(t0.T0Error):
+        fresh.synchronize()
+    assert fresh.is_poisoned()
+    driver.drop(graphs[0])
+    p.free()
