@@ -189,7 +189,8 @@ int t0_rt_set_wait_limit_ns(t0_runtime* rt, uint64_t ns);
 int t0_rt_selftest_drop_one_load(t0_runtime* rt);
 /* Scratch buffers (no counterpart in the reference, whose dispatch paths allocate per call).  Some launch paths keep a
  * per-runtime device buffer that grows on first use at each larger size: growing drains the stream, frees and allocates,
- * so the first such call stalls a pipeline and is illegal inside a stream capture.  The paths and their buffers:
+ * so the first such call stalls a pipeline, and inside a stream capture it is refused (T0_ERR_UNSUPPORTED; the capture stays
+ * valid).  The paths and their buffers:
  *   t0_gemm_launch / t0_gemm_batch / t0_gemm_submit with a K that is not a multiple of 8 (or N in the NN layout) or an
  *     operand that is not 16-byte aligned: padded copies of the operands, T0_SCRATCH_OPERAND_A = M * roundup(K, 8) * 2 bytes, T0_SCRATCH_OPERAND_B = N * roundup(K, 8) * 2
  *     (NT) or K * roundup(N, 8) * 2 (NN);

@@ -92,9 +92,14 @@ inline int check_rt(const t0_runtime* rt) {
     return T0_OK;
 }
 
-// Grow-only scratch areas (staging copies, split-K planes). Growing waits for the stream first.
+// Grow-only scratch areas (staging copies, split-K planes). Growing waits for the stream first.  While the stream is being captured
+// that would invalidate the capture: the call is refused before anything is touched, and the capture goes on.
 inline int ensure_scratch(t0_runtime* rt, Scratch& s, size_t bytes) {
     if (bytes <= s.size) return T0_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    T0_CUDA(cudaStreamIsCapturing(rt->stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone)
+        return fail(T0_ERR_UNSUPPORTED, "the stream is being captured and this call needs %zu bytes of scratch (%zu there): t0_rt_reserve_scratch first", bytes, s.size);
     T0_CUDA(cudaStreamSynchronize(rt->stream));
     if (s.ptr) cudaFree(s.ptr);
     s.ptr = nullptr; s.size = 0;

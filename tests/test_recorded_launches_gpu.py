@@ -221,3 +221,35 @@ def test_recorded_part_that_never_arrives_ends_with_an_error(t0, fresh, driver):
     assert fresh.is_poisoned()
     driver.drop(graphs[0])
     p.free()
+
+
+def test_recording_without_room_is_refused_and_goes_on(t0, fresh, driver):
+    # a split into planes (no one-launch form: pair tiles) and a product with a padded operand need buffers: refused while recording, the capture
+    # and the runtime stay usable; reserved, they are recorded and replay like the eager calls
+    planes = Product(t0, fresh, 300, 512, 1024, seed=5, pair_cta=1, tile_n=256, split_k=2)
+    padded = Product(t0, fresh, 40, 72, 1001, seed=6)
+    plain = Product(t0, fresh, 64, 64, 512, seed=7)
+    outs = [p.out() for p in (planes, padded, plain)]
+    with driver.record(fresh) as graphs:
+        for p, y in ((planes, outs[0]), (padded, outs[1])):
+            with pytest.raises(t0.T0Error) as e:
+                p.launch(y)
+            assert e.value.code == 6
+        plain.launch(outs[2])
+    driver.replay(graphs[0], fresh.stream())
+    fresh.synchronize()
+    assert np.array_equal(plain.bits(outs[2]), plain.eager())
+    driver.drop(graphs[0])
+    fresh.reserve_scratch("splitk_planes", 300 * 512 * 2 * 4)
+    fresh.reserve_scratch("operand_a", 40 * 1008 * 2)
+    fresh.reserve_scratch("operand_b", 72 * 1008 * 2)
+    with driver.record(fresh) as graphs:
+        planes.launch(outs[0])
+        padded.launch(outs[1])
+    want = planes.eager(), padded.eager()
+    driver.replay(graphs[0], fresh.stream())
+    fresh.synchronize()
+    assert np.array_equal(planes.bits(outs[0]), want[0]) and np.array_equal(padded.bits(outs[1]), want[1])
+    driver.drop(graphs[0])
+    for p in (planes, padded, plain):
+        p.free()
