@@ -194,12 +194,13 @@ int t0_rt_selftest_drop_one_load(t0_runtime* rt);
  *   t0_gemm_launch / t0_gemm_batch / t0_gemm_submit with a K that is not a multiple of 8 (or N in the NN layout) or an
  *     operand that is not 16-byte aligned: padded copies of the operands, T0_SCRATCH_OPERAND_A = M * roundup(K, 8) * 2 bytes, T0_SCRATCH_OPERAND_B = N * roundup(K, 8) * 2
  *     (NT) or K * roundup(N, 8) * 2 (NN);
- *   split_k > 1 where no one-launch form applies (pair tiles; and, when K is not a multiple of 64 * split_k or the parts are more
- *     than about one wave of SMs, the NN layout, tile widths 32 and 256, more than 8 parts): T0_SCRATCH_SPLITK_PLANES = M * N * split_k * 4;
+ *   split_k > 1 where no one-launch form applies (pair tiles, more than 8 parts; the NN layout or tile widths 32 and 256 when K is not
+ *     a multiple of 64 * split_k or tiles * split_k exceeds about four per SM): T0_SCRATCH_SPLITK_PLANES = M * N * split_k * 4;
  *   t0_w4a16_gemm outside the fused shapes: T0_SCRATCH_W4_WEIGHTS = K * N * 2;
  *   every fused W4A16 call (row layout and streaming layout): T0_SCRATCH_W4_FUSED, t0_rt_w4_fused_scratch_bytes(rt) bytes,
- *     a fixed size per device, so only the first fused call of a runtime allocates (reserving it also makes room for the
- *     partial sums of the grouped calls with 16 < M <= 128, which go without them while the stream is being captured);
+ *     a fixed size per device, so only the first call of a runtime with M <= 16 and its first grouped call with 16 < M <= 128
+ *     or on tile-major weights allocate; reserving less (0 will do) makes room for the first kind alone.  The grouped calls run
+ *     without the buffer while the stream is being captured, or when there is no memory for it;
  *   t0_matmul_f32*, t0_blas_gemm_f32: bf16 copies of the operands, T0_SCRATCH_F32_A / _B = elements * 2 (an operand whose
  *     rows are not a multiple of 8 elements: T0_SCRATCH_OPERAND_A / _B = rows * roundup(columns, 8) * 2), and, for
  *     alpha/beta other than 1/0 or ldc != n, T0_SCRATCH_F32_C = m * n * 4;
@@ -209,7 +210,8 @@ int t0_rt_selftest_drop_one_load(t0_runtime* rt);
  * Recording: a launch recorded by stream capture keeps the addresses it was given.  One that uses a buffer of the list above needs
  * the buffer reserved first, for the largest shape the runtime will ever see, and its graph is replayed in order with the runtime's
  * other work (on t0_rt_stream, or behind an event).  The launches that use no buffer may be replayed on any stream, beside others;
- * products give the same bits recorded or not.  t0_gemm_launch_gather and the host-operand entries are not for recording.
+ * bf16 products give the same bits recorded or not, those W4A16 groups another order of the f32 sums.  t0_gemm_launch_gather and
+ * the host-operand entries are not for recording.
  * t0_rt_reserve_scratch grows one buffer to at least `bytes` ahead of time, so that later launches up to that size
  * neither allocate nor synchronise. */
 enum {

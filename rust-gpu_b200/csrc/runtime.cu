@@ -431,14 +431,16 @@ int t0_rt_reserve_scratch(t0_runtime* rt, int which, size_t bytes) {
         case T0_SCRATCH_F32_B: s = &rt->scratch_cvt_b; break;
         case T0_SCRATCH_F32_C: s = &rt->scratch_cvt_c; break;
         case T0_SCRATCH_W4_FUSED: {
-            // arrival counters (must start at zero) followed by two pieces per CTA; the size depends only on the device
-            const size_t need = std::max(bytes, t0_rt_w4_fused_scratch_bytes(rt));
+            // arrival counters (must start at zero) followed by two pieces per CTA; the size depends only on the device.  Less than
+            // the whole size makes room for M <= 16 alone.
+            const size_t all = t0_rt_w4_fused_scratch_bytes(rt), cut = w4a16_umma_scratch_bytes(rt);
+            const size_t need = std::max(bytes >= all ? bytes - cut : bytes, all - cut);
             if (need > rt->scratch_w4.size) {
                 rc = ensure_scratch(rt, rt->scratch_w4, need);
                 if (rc != T0_OK) return rc;
                 T0_CUDA(cudaMemsetAsync(rt->scratch_w4.ptr, 0, w4a16_counter_region_bytes(), rt->stream));
             }
-            return w4a16_umma_reserve(rt, (uint32_t)rt->sm_count, 128);
+            return bytes >= all ? w4a16_umma_reserve(rt) : T0_OK;
         }
         default: return fail(T0_ERR_INVALID, "unknown scratch kind %d", which);
     }
@@ -446,7 +448,7 @@ int t0_rt_reserve_scratch(t0_runtime* rt, int which, size_t bytes) {
 }
 
 size_t t0_rt_w4_fused_scratch_bytes(const t0_runtime* rt) {
-    return rt ? w4a16_fixed_scratch_bytes((uint32_t)rt->sm_count) : 0;
+    return rt ? w4a16_fixed_scratch_bytes((uint32_t)rt->sm_count) + w4a16_umma_scratch_bytes(rt) : 0;
 }
 
 void* t0_rt_stream(const t0_runtime* rt) { return rt ? (void*)rt->stream : nullptr; }

@@ -65,7 +65,8 @@ struct t0_runtime {
 namespace t0 {
 
 void host_pipe_free(t0_runtime* rt);   // host_pipeline.cu
-int w4a16_umma_reserve(t0_runtime* rt, uint32_t ctas, uint32_t rows);   // w4a16_umma_cut.cu
+size_t w4a16_umma_scratch_bytes(const t0_runtime* rt);   // w4a16_umma_cut.cu
+int w4a16_umma_reserve(t0_runtime* rt);
 // runtime.cu: one bf16 product of operands with row strides, everything else chosen by the library
 int gemm_strided(t0_runtime* rt, uint64_t a, uint32_t lda, bool at, uint64_t b, uint32_t ldb, bool nn, uint64_t y, uint32_t m, uint32_t n, uint32_t k);
 

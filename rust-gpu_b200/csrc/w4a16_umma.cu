@@ -817,7 +817,7 @@ __global__ void w4_to_tiled_kernel(const uint32_t* __restrict__ packed, const ui
 
 namespace t0 {
 
-bool w4a16_umma_cut_pays(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count);     // w4a16_umma_cut.cu
+bool w4a16_umma_cut_applies(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count);     // w4a16_umma_cut.cu
 uint32_t w4a16_umma_cut_rows(uint32_t M);
 int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count);
 
@@ -939,7 +939,7 @@ int launch_w4a16_umma_tiled_grouped(t0_runtime* rt, const t0_w4a16_args* args, u
     static UmGroup grp;
     static std::mutex grp_mu;
     std::lock_guard<std::mutex> lock(grp_mu);
-    const bool cut = w4a16_umma_cut_pays(rt, a0.n, a0.k, count);
+    const bool cut = w4a16_umma_cut_applies(rt, a0.n, a0.k, count);
     for (uint32_t i = 0; i < count; ++i) {
         const t0_w4a16_args& a = args[i];
         if (a.m != a0.m || a.n != a0.n || a.k != a0.k || a.group != a0.group) return fail(T0_ERR_INVALID, "grouped launch: problem %u differs from problem 0 in shape", i);
@@ -984,7 +984,7 @@ int launch_w4a16_umma_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_
     static UmGroup grp;                  // 16.6 KB: kept off the stack, filled under the lock, copied by the launch
     static std::mutex grp_mu;
     std::lock_guard<std::mutex> lock(grp_mu);
-    const bool cut = w4a16_umma_cut_pays(rt, a0.n, a0.k, count);
+    const bool cut = w4a16_umma_cut_applies(rt, a0.n, a0.k, count);
     for (uint32_t i = 0; i < count; ++i) {
         const t0_w4a16_args& a = args[i];
         if (a.m != a0.m || a.n != a0.n || a.k != a0.k || a.group != a0.group) return fail(T0_ERR_INVALID, "grouped launch: problem %u differs from problem 0 in shape", i);

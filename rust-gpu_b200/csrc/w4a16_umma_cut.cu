@@ -19,7 +19,7 @@
 // Whole tiles per CTA leave SMs idle where the tiles are few or just over a multiple of them: two problems of N = 11008 are 86 tiles on 148
 // SMs.  M = 128, K = 4096: 43.8 us with whole tiles, 40.4 cut; M = 107, N = 7936, K = 4352: 45.3 and 34.4; M = 81, N = 2560, K = 7424, four
 // problems: 72.0 and 37.3.  What bounds it is the chain of waits around a chunk (0.67 us; arithmetic alone would take about 0.15) and, per
-// launch, about 10 us for handing in and adding the parts of cut tiles; `w4a16_umma_cut_pays` weighs the two.
+// launch, about 10 us for handing in and adding the parts of cut tiles; `w4a16_umma_cut_applies` weighs the two.
 #include "w4a16_common.cuh"
 
 using namespace t0;
@@ -450,11 +450,12 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
 
 namespace t0 {
 
-size_t w4a16_umma_scratch_bytes(uint32_t ctas, uint32_t rows) { return kUmCounterBytes + (size_t)ctas * 2 * rows * kUmBN * sizeof(float); }
+// Counters and partial sums of a launch of one CTA per SM at M = 128: what any launch needs at most.
+size_t w4a16_umma_scratch_bytes(const t0_runtime* rt) { return kUmCounterBytes + (size_t)rt->sm_count * 2 * 128 * kUmBN * sizeof(float); }
 
-// Room for the counters and partial sums of `ctas` CTAs; the counters start at zero.
-int w4a16_umma_reserve(t0_runtime* rt, uint32_t ctas, uint32_t rows) {
-    const size_t need = w4a16_umma_scratch_bytes(ctas, rows);
+// Makes room for them; the counters start at zero.
+int w4a16_umma_reserve(t0_runtime* rt) {
+    const size_t need = w4a16_umma_scratch_bytes(rt);
     if (need <= rt->scratch_um.size) return T0_OK;
     int rc = ensure_scratch(rt, rt->scratch_um, need);
     if (rc != T0_OK) return rc;
@@ -474,26 +475,28 @@ static uint32_t cut_grid(const t0_runtime* rt, uint64_t items, uint32_t n_chunks
     return grid;
 }
 
-// Whether cutting the tiles of `count` problems beats whole tiles per CTA, in microseconds fitted at M = 128 and 32, K = 1152 ... 7424, 32 to 516
-// tiles: a chunk takes about 0.65 us either way, a launch with cut tiles about 10 us more.  Cut tiles need scratch: not while the
-// stream is being captured and the scratch does not exist yet.
-bool w4a16_umma_cut_pays(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count) {
+// Whether the tiles of `count` problems are to be cut: where that beats whole tiles per CTA, in microseconds fitted at M = 128 and 32,
+// K = 1152 ... 7424, 32 to 516 tiles (a chunk takes about 0.65 us either way, a launch with cut tiles about 10 us more); where there is room for
+// their parts; and only in launches of the runtime's own stream, whose launches run one after the other: a recorded launch may be replayed
+// beside others, which would share its counters and parts.
+bool w4a16_umma_cut_applies(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count) {
     const uint64_t items = (uint64_t)ceil_div(N, kUmBN) * count;
     const uint32_t n_chunks = K / kUmBK, grid = cut_grid(rt, items, n_chunks);
     if (items % grid == 0 || items * n_chunks >= (1u << 24)) return false;
     const double whole = (double)((items + rt->sm_count - 1) / rt->sm_count) * n_chunks * 0.63 + 4.0;
     const double cut = (double)items * n_chunks / grid * 0.67 + 14.4;
     if (cut > 0.97 * whole) return false;
-    if (w4a16_umma_scratch_bytes(grid, 128) > rt->scratch_um.size) {
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
-    }
-    return true;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+    if (w4a16_umma_reserve(rt) == T0_OK) return true;
+    cudaGetLastError();                    // (no memory for the parts: whole tiles need none)
+    return false;
 }
 
 uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }
 
-// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.
+// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape, for which
+// w4a16_umma_cut_applies.
 int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count) {
     auto kern = tiled ? w4a16_umma_cut_kernel<true> : w4a16_umma_cut_kernel<false>;
     static bool attr_set[2][64] = {};
@@ -514,8 +517,6 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint
     const uint64_t items = (uint64_t)p.n_tiles * count;
     const uint32_t grid = cut_grid(rt, items, p.n_chunks);
     p.total = (uint32_t)(items * p.n_chunks);
-    int rc = w4a16_umma_reserve(rt, (uint32_t)rt->sm_count, 128);
-    if (rc != T0_OK) return rc;
     p.counters = (uint32_t*)rt->scratch_um.ptr;
     p.pieces = (float*)((uint8_t*)rt->scratch_um.ptr + kUmCounterBytes);
     cudaLaunchConfig_t cfg = {};

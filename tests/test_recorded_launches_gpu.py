@@ -253,3 +253,103 @@ def test_recording_without_room_is_refused_and_goes_on(t0, fresh, driver):
     driver.drop(graphs[0])
     for p in (planes, padded, plain):
         p.free()
+
+
+class Group:
+    """W4A16 problems of one shape whose column tiles are cut between CTAs in an eager call; `bound` = f32 sums in any order."""
+
+    def __init__(self, t0, oracle, rt, M, K, N, count, G=128):
+        self.rt, self.M, self.N, self.K, self.bufs, self.args, self.refs = rt, M, N, K, [], [], []
+        for i in range(count):
+            packed, scales, zeros = oracle.fill_u32((K // 8) * N, 10 + i), oracle.fill_range_bf16((K // G) * N, 20 + i, 0.001, 0.02), oracle.fill_u32((K // G) * (N // 8), 30 + i)
+            a = oracle.fill_normal_bf16(M * K, 40 + i)
+            w = np.abs(oracle.bf16_to_f32(oracle.dequant_w4_b200(packed, scales, zeros, K, N, G)).reshape(K, N))
+            bound = np.abs(oracle.bf16_to_f32(a).reshape(M, K)).astype(np.float64) @ w * (K * 2.0 ** -24)
+            self.refs.append((oracle.w4a16_gemm(a, packed, scales, zeros, M, N, K, G).astype(np.float64), bound))
+            p, s, z, x = rt.upload(packed), rt.upload(scales), rt.upload(zeros), rt.upload(a)
+            t = rt.w4_to_tiled(p.gpu_addr(), s.gpu_addr(), z.gpu_addr(), K, N, G)
+            self.bufs += [p, s, z, x, t]
+            self.rows = p, s, z, x
+            self.args.append(lambda y, x=x, t=t: t0.W4A16Args(x.gpu_addr(), t.gpu_addr(), 0, 0, y.gpu_addr(), M, N, K, G))
+
+    def outs(self):
+        ys = [self.rt.alloc(self.M * self.N * 4) for _ in self.args]
+        for y in ys:
+            y.write(np.full(self.M * self.N, np.nan, np.float32))
+        self.bufs += ys
+        return ys
+
+    def launch(self, ys):
+        self.rt.w4a16_gemm_tiled_grouped([a(y) for a, y in zip(self.args, ys)])
+
+    def launch_row_layout(self, y):
+        p, s, z, x = self.rows
+        self.rt.w4a16_gemm(x.gpu_addr(), p.gpu_addr(), s.gpu_addr(), z.gpu_addr(), y.gpu_addr(), self.M, self.N, self.K, 128)
+
+    def check(self, ys):
+        for y, (ref, bound) in zip(ys, self.refs):
+            assert np.all(np.abs(y.read(self.M * self.N * 4, np.float32).reshape(self.M, self.N) - ref) <= bound)
+
+    def free(self):
+        for b in self.bufs:
+            b.free()
+
+
+def test_recorded_w4a16_group_beside_eager_ones(t0, oracle, fresh, driver):
+    # recorded before the runtime has a buffer for cut tiles, and again after: the replays run on another stream beside eager calls
+    g = Group(t0, oracle, fresh, 40, 4096, 2560, 2)
+    stream, execs, outs = driver.stream(), [], []
+    for _ in range(2):
+        ys = g.outs()
+        with driver.record(fresh) as graphs:
+            for _ in range(5):
+                g.launch(ys)
+        execs.append(graphs[0])
+        outs.append(ys)
+        outs.append(g.outs())
+        g.launch(outs[-1])                                                    # eager
+    for _ in range(10):
+        for ex in execs:
+            driver.replay(ex, stream)
+        g.launch(outs[-1])
+    driver.sync(stream)
+    fresh.synchronize()
+    for ys in outs:
+        g.check(ys)
+    driver.drop(execs[0])
+    driver.drop(execs[1], stream)
+    g.free()
+
+
+def test_reserved_w4a16_calls_allocate_nothing(t0, oracle, rt, driver):
+    # what t0_rt_w4_fused_scratch_bytes names covers every fused call of a runtime; a smaller reservation the calls with M <= 16
+    def free_bytes():
+        rt.synchronize()
+        f, t = C.c_size_t(), C.c_size_t()
+        driver.call("cuMemGetInfo_v2", C.byref(f), C.byref(t))
+        return f.value
+
+    one, many = Group(t0, oracle, rt, 4, 4096, 2560, 1), Group(t0, oracle, rt, 128, 4096, 2560, 2)
+    ys = [g.outs() for g in (one, many)]
+    one.launch_row_layout(ys[0][0]), many.launch(ys[1])                       # (the kernels are loaded)
+    rt.synchronize()
+    r = t0.GpuRuntime(0)
+    whole, before = r.w4_fused_scratch_bytes(), free_bytes()
+    r.reserve_scratch("w4_fused", 0)
+    small = before - free_bytes()
+    assert small < whole // 4                                                 # nothing for cut tiles yet
+    one.rt = many.rt = r
+    at = free_bytes()
+    one.launch_row_layout(ys[0][0])
+    r.synchronize()
+    assert free_bytes() == at
+    r.reserve_scratch("w4_fused", whole)
+    at = free_bytes()
+    assert before - at <= whole + (8 << 20)                                   # (buffers are whole megabytes)
+    one.launch_row_layout(ys[0][0]), many.launch(ys[1])
+    r.synchronize()
+    assert free_bytes() == at
+    one.check(ys[0]), many.check(ys[1])
+    r.close()
+    one.rt = many.rt = rt
+    one.free(), many.free()
