@@ -382,6 +382,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
                     __threadfence();
                 }
                 good = __shfl_sync(0xFFFFFFFFu, good, 0);
+                __syncwarp();                              // orders the other lanes' loads of the parts after lane 0's acquire (a shuffle does not)
                 if (!good) { ok = false; break; }
             }
             const uint32_t prob = item / p.n_tiles;
