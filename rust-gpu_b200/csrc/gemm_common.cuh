@@ -67,11 +67,10 @@ __device__ __forceinline__ WorkItem decode_work(uint32_t w, const KParams& p) {
 
 __device__ __forceinline__ float sigmoid_seq(float x) {
     // tile_ir.rs:3448-3477: negate, scale by log2(e), exp2, add one, reciprocal.
-    // The reciprocal of d = 1 + e is the hardware's approximation and one Newton step (r + r (1 - d r), both fused), within a hair of half
-    // a unit in the last place.  It runs on d / 4, so that neither d nor the result leaves the normal range before d overflows; from
-    // there on the result is zero.  With __frcp_rn, which cares for every special input in a branch of its own, a value of the
-    // epilogue took about 110 cycles: 35.7 us for a 2048^3 product with SiLU, 24.0 with this and the flushing exponential.
-    // (The exponential may flush to zero: below 2^-126 it does not change 1 + e.)
+    // The reciprocal of d = 1 + e: the hardware's approximation and one step of Newton's method for 1/d (r + r (1 - d r), both fused), at most
+    // one unit in the last place from the correctly rounded quotient.  It runs on d / 4, so that neither d nor the result leaves the
+    // normal range before d overflows; from there on the result is zero.  (The exponential may flush to zero: below 2^-126 it does not
+    // change 1 + e.)  A 2048^3 product with SiLU: 35.7 us with __frcp_rn and exp2f, 24.0 so.
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((-x) * 1.44269504088896340736f));
     const float d = __fmaf_rn(e, 0.25f, 0.25f);

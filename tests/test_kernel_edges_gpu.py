@@ -184,3 +184,34 @@ def test_parts_added_in_order_whoever_is_last(t0, rt):
     first = run_gemm(t0, rt, x, b, m, n, k)
     for _ in range(5):
         assert np.array_equal(run_gemm(t0, rt, x, b, m, n, k), first)
+
+
+@pytest.mark.parametrize("op,factor", [("silu", 1.0), ("gelu", 1.702)])
+def test_sigmoid_over_its_whole_range(t0, rt, op, factor):
+    # v arrives exactly, as the bias of a product of zeros: small and large arguments, beyond the exponential's range on both sides (from v = -88.7 on
+    # 1 + e overflows), infinities, NaN
+    import torch
+    rng = np.random.default_rng(8)
+    edges = np.array([0.0, -0.0, 87.2, 87.4, 88.0, 88.72, 88.73, 89.0, 103.0, 104.0, 1e4, 3e38, np.inf, 1e-30, 1e-40], np.float32) / np.float32(factor)
+    v = np.concatenate([edges, -edges, [np.nan], rng.uniform(-110, 110, 6000), rng.uniform(-90, -86, 1000) / factor,
+                        np.exp(rng.uniform(-80, 6, 1000)) * rng.choice([-1, 1], 1000)]).astype(np.float32)
+    n = v.size + -v.size % 8
+    v = np.pad(v, (0, n - v.size))
+    got = run_gemm(t0, rt, np.zeros((1, 64), np.float32), np.zeros((n, 64), np.float32), 1, n, 64, bias=v, tile_epilogue=["bias", op])[0]
+    # CUDA's exp2 and its correctly rounded quotient: the reciprocal is one unit off at most, the product rounds once more
+    x = torch.from_numpy(v).cuda()
+    z = x * factor if factor != 1.0 else x
+    s = 1.0 / (torch.exp2(-z * 1.4426950408889634) + 1.0)
+    want, s = (x * s).cpu().numpy(), s.cpu().numpy()
+    with np.errstate(invalid="ignore", over="ignore", under="ignore"):
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        fin = np.isfinite(want)
+        assert np.array_equal(got[~fin & ~np.isnan(want)], want[~fin & ~np.isnan(want)])
+        gap = np.abs(v[fin]).astype(np.float64) * np.spacing(s[fin]) + np.spacing(np.abs(want[fin]))
+        assert np.all(np.abs(got[fin].astype(np.float64) - want[fin]) <= gap)
+        # and 64 bits: the exponential's argument carries |z| roundings of 2^-24 (its factor another quarter, GELU's product another whole one), its value
+        # 2 units, the sum, the reciprocal and the product one each; where 1 + e overflows (z < -88.7) a sigmoid below 2^-127.9 becomes zero
+        x64, z64 = v[fin].astype(np.float64), v[fin].astype(np.float64) * factor
+        exact = x64 / (1.0 + np.exp(-np.clip(z64, -700, 700)))
+        assert np.all(np.abs(got[fin] - exact) <= np.abs(exact) * (1.25 * np.abs(z64) + 4) * 2.0 ** -23
+                      + np.where(z64 < -88.7, np.abs(x64) * 2.0 ** -127.9, (np.abs(x64) + 1) * 2.0 ** -149))
