@@ -215,3 +215,18 @@ def test_sigmoid_over_its_whole_range(t0, rt, op, factor):
         exact = x64 / (1.0 + np.exp(-np.clip(z64, -700, 700)))
         assert np.all(np.abs(got[fin] - exact) <= np.abs(exact) * (1.25 * np.abs(z64) + 4) * 2.0 ** -23
                       + np.where(z64 < -88.7, np.abs(x64) * 2.0 ** -127.9, (np.abs(x64) + 1) * 2.0 ** -149))
+
+
+@pytest.mark.parametrize("tile_n,split_k", [(64, 2), (64, 4), (64, 8), (128, 2), (128, 8)])
+@pytest.mark.parametrize("m,n,k", [(40, 72, 1088), (150, 330, 1088), (1500, 1300, 512)])
+@pytest.mark.parametrize("out_bf16", [False, True])
+def test_split_k_with_several_tiles_per_cluster(t0, rt, tile_n, split_k, m, n, k, out_bf16):
+    # the form in which a cluster walks a list of tiles: parts that are not whole 64-deep blocks of K (1088 / split), and more clusters than run at
+    # once (64- and 128-wide tiles of 1500 x 1300)
+    rng = np.random.default_rng(n)
+    x, b, bias = ints(rng, m, k), ints(rng, n, k), ints(rng, n, lim=100)
+    before = rt.launch_count()
+    got = run_gemm(t0, rt, x, b, m, n, k, out_bf16, bias, tile_n=tile_n, split_k=split_k, pair_cta=2, epilogue=t0.EPI_BIAS_ADD_STORE_F32)
+    assert rt.launch_count() - before == 1
+    want = x @ b.T + bias
+    assert np.array_equal(got, from_bf16(bf16_bits(want)) if out_bf16 else want)
