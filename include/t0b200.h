@@ -195,7 +195,7 @@ int t0_rt_selftest_drop_one_load(t0_runtime* rt);
  *     operand that is not 16-byte aligned: padded copies of the operands, T0_SCRATCH_OPERAND_A = M * roundup(K, 8) * 2 bytes, T0_SCRATCH_OPERAND_B = N * roundup(K, 8) * 2
  *     (NT) or K * roundup(N, 8) * 2 (NN);
  *   split_k > 1 where no one-launch form applies (pair tiles, more than 8 parts; the NN layout or tile widths 32 and 256 when K is not
- *     a multiple of 64 * split_k or tiles * split_k exceeds about four per SM): T0_SCRATCH_SPLITK_PLANES = M * N * split_k * 4;
+ *     a multiple of 64 * split_k or the tiles times split_k are more than about one wave of SMs): T0_SCRATCH_SPLITK_PLANES = M * N * split_k * 4;
  *   t0_w4a16_gemm outside the fused shapes: T0_SCRATCH_W4_WEIGHTS = K * N * 2;
  *   every fused W4A16 call (row layout and streaming layout): T0_SCRATCH_W4_FUSED, t0_rt_w4_fused_scratch_bytes(rt) bytes,
  *     a fixed size per device, so only the first call of a runtime with M <= 16 and its first grouped call with 16 < M <= 128

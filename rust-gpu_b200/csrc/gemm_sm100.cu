@@ -413,13 +413,14 @@ int launch_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensor
 
 }  // namespace
 
-// The SMs of a GPC hold whole clusters only, and GPCs differ in size: 148 SMs hold 15 clusters of eight, not 18.  Devices of one model may
-// differ a little, and a product is not to be cut otherwise on another of them, so the table keeps a margin below what a B200 reports
-// (74, 45, 33, 26, 22, 15, 15); the device's own figure counts only where it is lower still.
+// The SMs of a GPC hold whole clusters only, and GPCs differ in size: 148 SMs hold 15 clusters of eight, not 18 (a B200 reports 74, 45, 33,
+// 26, 22, 15, 15 for two to eight).  Behind a kernel whose blocks leave one by one, clusters of odd size do not pack as well (44 clusters of
+// three: 12.2 us behind one of their own, 17.6 behind a conversion; 40: no difference), so the table stays below that for them.  Where
+// the device's own figure is lower, it counts.
 const uint32_t* gemm_clusters_at_once() {
     static uint32_t table[64][kMaxClusterParts + 1] = {};
     static std::mutex mu;
-    static const uint32_t safe[kMaxClusterParts + 1] = {0, 148, 72, 40, 32, 24, 20, 14, 14};
+    static const uint32_t safe[kMaxClusterParts + 1] = {0, 148, 74, 40, 33, 24, 20, 14, 15};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return safe;

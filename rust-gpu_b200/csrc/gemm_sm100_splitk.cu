@@ -4,8 +4,9 @@
 // Replaces, for results that are wanted complete (not as planes), the two-launch form "GEMM into split_k planes, then a
 // reduction pass": the reference leaves the planes to the host to add (src/t0/gemm_gen.rs:447-448,
 // examples/test_gemm_correctness.rs:203-207); here the sum is the same fp32 sum of the per-split partial sums in split
-// order, so results are bit-identical to that form and from run to run.  The skinny, HBM-bound shapes this serves
-// (128 x 4096 x 4096, 64 x 4096 x 16384) spend a third of their time in the second launch and the gap before it.
+// order, so results are bit-identical to that form and from run to run.  A product whose clusters all run at once takes the form
+// in gemm_sm100.cu, which has one tile per cluster; this one serves what has more tiles than clusters: grouped launches, and splits of
+// the caller's.
 //
 // Roles per CTA as in gemm_sm100.cu (TMA producer, UMMA issuer, four epilogue warps, accumulators double-buffered in
 // tensor memory).  Differences:

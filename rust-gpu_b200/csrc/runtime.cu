@@ -139,13 +139,16 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     bool fused_reduce = split > 1 && !q.planes;
     static const bool no_cluster = getenv("T0_NO_CLUSTER_SPLITK") != nullptr;
     // Split-K in one launch, the parts of a tile as the CTAs of a cluster (gemm_sm100.cu).  A split the caller asked for runs this way
-    // where its parts are whole k blocks (the parts, and so the sums, are then those of the planes form) and few clusters run one after the other.
+    // where its parts are whole k blocks (the parts, and so the sums, are then those of the planes form) and all clusters run at once, if
+    // need be with wider tiles: two rounds of clusters cost more than either (16 x 2048 x 2048, B[K,N], 64-wide tiles, 8 parts: 23.4 us in
+    // two rounds, 10.3 as planes, 9.5 with 256-wide tiles).
     uint32_t parts = q.parts > 1 && !use_pair ? q.parts : 0;
     if (fused_reduce && !use_pair && !no_cluster && q.k % (64u * split) == 0 && split <= kMaxClusterParts) {
-        // (where several clusters would run one after the other: the persistent form of gemm_sm100_splitk.cu if it takes the
-        // request, and from about four waves on the planes)
-        const uint64_t tiles = (uint64_t)ceil_div(q.m, 128) * ceil_div(q.n, g.tile_n), at_once = gemm_clusters_at_once()[split];
-        if (tiles <= (gemm_splitk_cluster_supported(g) ? at_once : 4 * at_once)) parts = split;
+        for (uint32_t tile_n = g.tile_n; tile_n <= 256 && !parts; tile_n *= 2) {
+            if ((uint64_t)ceil_div(q.m, 128) * ceil_div(q.n, tile_n) > gemm_clusters_at_once()[split]) continue;
+            g.tile_n = tile_n;
+            parts = split;
+        }
     }
     if (parts) {
         g.split_k = parts;

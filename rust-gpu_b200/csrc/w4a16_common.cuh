@@ -76,6 +76,41 @@ __device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t mask, uint32_t m
     return r;
 }
 
+// The tcgen05 kernels (w4a16_umma.cu, w4a16_umma_cut.cu): a chunk of the raw weights is 8 packed rows x 256 columns, their scales and
+// zero points.
+constexpr uint32_t kUmBN = 256;                             // columns of y per tile
+constexpr uint32_t kUmBK = 64;                              // k per chunk: one 128-byte swizzle atom of bf16
+constexpr uint32_t kUmRawBytes = 8 * kUmBN * 4 + kUmBN * 2 + (kUmBN / 8) * 4;      // 8832: words, scales, zero points
+constexpr uint32_t kUmRawStride = 9216;                     // keeps every stage 1024-byte aligned
+
+__device__ __forceinline__ uint32_t um_lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t um_lds16(uint32_t addr) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// The eight codes of a packed word as bf16x2 pairs in k order, (0,1) (2,3) (4,5) (6,7): (code | 0x4300) is the bf16 128 + code, so minus (128 + z),
+// times s, is (q - z) * s rounded once.  zz = (128 + z) and ss = s, both halves alike.
+__device__ __forceinline__ void um_dequant_word(uint32_t wd, uint32_t mask, uint32_t magic, uint32_t zz, uint32_t ss, bool tiled, uint32_t (&o)[4]) {
+    const uint32_t v0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), zz), ss);            // row layout: k 0, 4
+    const uint32_t v1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), zz), ss);       // k 1, 5
+    const uint32_t v2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), zz), ss);       // k 2, 6
+    const uint32_t v3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), zz), ss);      // k 3, 7
+    if (tiled) {                           // tile-major words are stored so that the pairs come out in k order
+        o[0] = v0; o[1] = v1; o[2] = v2; o[3] = v3;
+    } else {
+        o[0] = __byte_perm(v0, v1, 0x5410);
+        o[1] = __byte_perm(v2, v3, 0x5410);
+        o[2] = __byte_perm(v0, v1, 0x7632);
+        o[3] = __byte_perm(v2, v3, 0x7632);
+    }
+}
+
 // Grouped launch of the tcgen05 kernels: the four tensor maps (weights, scales, zero points, activations) and the output of up to 32
 // problems of one shape in the kernel parameters (16.6 KB).
 constexpr uint32_t kUmMaxGroup = 32;

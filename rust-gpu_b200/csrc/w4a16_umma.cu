@@ -26,11 +26,7 @@ namespace {
 
 constexpr uint32_t kUmDqWarps = 16;
 constexpr uint32_t kUmThreads = (kUmDqWarps + 2) * 32;      // + producer warp + issuer warp
-constexpr uint32_t kUmBN = 256;                             // columns of y per tile
-constexpr uint32_t kUmBK = 64;                              // k per chunk: one 128-byte swizzle atom of bf16
 constexpr uint32_t kUmRawStages = 6;
-constexpr uint32_t kUmRawBytes = 8 * kUmBN * 4 + kUmBN * 2 + (kUmBN / 8) * 4;      // 8832: words, scales, zero points
-constexpr uint32_t kUmRawStride = 9216;                     // keeps every stage 1024-byte aligned
 constexpr uint32_t kUmAbStages = 3;
 constexpr uint32_t kUmBBytes = kUmBN * kUmBK * 2;           // 32 KiB
 constexpr uint32_t kUmABytes = 128 * kUmBK * 2;             // 16 KiB
@@ -56,30 +52,6 @@ struct UmParams {
     uint32_t n_problems;     // grouped launch: problems of one shape in this launch (their maps and outputs ride in the group record)
 };
 
-__device__ __forceinline__ bool um_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool um_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
-    if (um_try_wait_cluster(bar, parity)) return true;
-    uint64_t t_start = 0;
-    for (uint32_t spin = 1;; ++spin) {
-        if (um_try_wait_cluster(bar, parity)) return true;
-        if ((spin & 0xFF) == 0) {
-            if (*abort_flag) return false;
-            const uint64_t now = ptx::globaltimer_ns();
-            if (t_start == 0) t_start = now;
-            else if (now - t_start > limit_ns) { *abort_flag = 1; return false; }
-        }
-    }
-}
 __device__ __forceinline__ uint32_t um_cluster_id() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
@@ -90,25 +62,9 @@ __device__ __forceinline__ uint32_t um_n_clusters() {
     asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ uint32_t um_lds32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ uint32_t um_lds16(uint32_t addr) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ void um_sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
-__device__ __forceinline__ float4 um_ld_cluster_f4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 template <bool kGrouped>
 __global__ void __launch_bounds__(kUmThreads, 1)
 w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
@@ -180,7 +136,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 if constexpr (kGrouped) { prob = item / p.n_tiles; tile = item - prob * p.n_tiles; }
                 (void)prob; (void)tile;
                 // the rings double as the parking area: the previous tile's copy must have been read by the whole cluster
-                if (iter > 0 && !um_wait_cluster(read_bar, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) {
+                if (iter > 0 && !ptx::mbar_wait_cluster(read_bar, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) {
                     atomicCAS(p.status, 0, kStatusProducerTimeout | 0x800000);
                     break;
                 }
@@ -220,7 +176,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 uint32_t prob = 0, tile = item;
                 if constexpr (kGrouped) { prob = item / p.n_tiles; tile = item - prob * p.n_tiles; }
                 (void)prob; (void)tile;
-                if (iter > 0 && !um_wait_cluster(read_bar, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) break;
+                if (iter > 0 && !ptx::mbar_wait_cluster(read_bar, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) break;
                 for (uint32_t c = c_begin; c < c_end; ++c) {
                     if (!ptx::mbar_wait_relaxed(ab_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns, 64)) {
                         atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
@@ -288,7 +244,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             if constexpr (kGrouped) { prob = item / p.n_tiles; tile = item - prob * p.n_tiles; }
             (void)prob;
             const uint32_t n0 = tile * kUmBN;
-            if (ok && iter > 0 && !um_wait_cluster(read_bar, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) {
+            if (ok && iter > 0 && !ptx::mbar_wait_cluster(read_bar, (iter - 1) & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x400000);
                 ok = false;
             }
@@ -318,18 +274,9 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                 for (uint32_t j = 0; j < 8; ++j) {
                     const uint32_t wd = words[j];
-                    const uint32_t v0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), zz), ss);            // k 0, 4
-                    const uint32_t v1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), zz), ss);       // k 1, 5
-                    const uint32_t v2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), zz), ss);       // k 2, 6
-                    const uint32_t v3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), zz), ss);      // k 3, 7
-                    if (p.tiled) {
-                        // tile-major words hold their codes so that the four pairs come out as (0,1) (2,3) (4,5) (6,7)
-                        um_sts128(b_stage + ((j ^ (n & 7)) << 4), v0, v1, v2, v3);
-                    } else {
-                        // row layout: pairs (0,4) (1,5) (2,6) (3,7); back into k order
-                        um_sts128(b_stage + ((j ^ (n & 7)) << 4), __byte_perm(v0, v1, 0x5410), __byte_perm(v2, v3, 0x5410),
-                                  __byte_perm(v0, v1, 0x7632), __byte_perm(v2, v3, 0x7632));
-                    }
+                    uint32_t v[4];
+                    um_dequant_word(wd, mask, magic, zz, ss, p.tiled, v);
+                    um_sts128(b_stage + ((j ^ (n & 7)) << 4), v[0], v[1], v[2], v[3]);
                 }
                 // The UMMAs read these bytes through the async proxy.  The warp's writes are ordered before lane 0 by the warp
                 // barrier; lane 0's proxy fence and release-arrive then publish them (one fence per warp instead of 32:
@@ -398,7 +345,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 ptx::mbar_arrive(acc_empty);
                 for (uint32_t s = 0; s < p.split; ++s) ptx::mbar_arrive_cluster(ptx::mapa(parked_bar, s));
             }
-            if (!um_wait_cluster(parked_bar, iter & 1, abort_flag, p.wait_limit_ns)) {
+            if (!ptx::mbar_wait_cluster(parked_bar, iter & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xD00000);
                 ok = false;
                 break;
@@ -419,7 +366,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                         const uint32_t row = i / f4_per_row, c4 = i - row * f4_per_row;
 #pragma unroll
                         for (uint32_t s = 0; s < 4; ++s)
-                            part[u][s] = (i < items && s < p.split) ? um_ld_cluster_f4(ptx::mapa(park + (row * kUmPitch + s_begin + c4 * 4) * 4, s))
+                            part[u][s] = (i < items && s < p.split) ? ptx::ld_cluster_f4(ptx::mapa(park + (row * kUmPitch + s_begin + c4 * 4) * 4, s))
                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
 #pragma unroll
@@ -687,19 +634,10 @@ w4a16_umma_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
                     for (uint32_t half = 0; half < 2; ++half) {
                         const uint32_t wd = words[2 * jj + half];
-                        const uint32_t v0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), zz), ss);            // k 0, 4
-                        const uint32_t v1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), zz), ss);       // k 1, 5
-                        const uint32_t v2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), zz), ss);       // k 2, 6
-                        const uint32_t v3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), zz), ss);      // k 3, 7
-                        // k order: (0,1) (2,3) (4,5) (6,7), two consecutive k per tensor-memory column
-                        if (p.tiled) {                     // tile-major words are stored so that the pairs come out in that order
-                            r8[half * 4 + 0] = v0; r8[half * 4 + 1] = v1; r8[half * 4 + 2] = v2; r8[half * 4 + 3] = v3;
-                        } else {                           // row layout: pairs (0,4) (1,5) (2,6) (3,7)
-                            r8[half * 4 + 0] = __byte_perm(v0, v1, 0x5410);
-                            r8[half * 4 + 1] = __byte_perm(v2, v3, 0x5410);
-                            r8[half * 4 + 2] = __byte_perm(v0, v1, 0x7632);
-                            r8[half * 4 + 3] = __byte_perm(v2, v3, 0x7632);
-                        }
+                        uint32_t v[4];
+                        um_dequant_word(wd, mask, magic, zz, ss, p.tiled, v);
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; ++e) r8[half * 4 + e] = v[e];
                     }
                     ptx::tmem_st_32x32b_x8(a_cols + jj * 8, r8);
                 }

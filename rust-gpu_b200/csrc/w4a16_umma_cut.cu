@@ -33,10 +33,6 @@ constexpr uint32_t kUmDqWarps = 16;
 // stepped by addition) and apart: two lanes of one warp would take turns.
 constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;
 constexpr uint32_t kUmThreads = (kUmDqWarps + 3) * 32;
-constexpr uint32_t kUmBN = 256;                             // columns of y per tile
-constexpr uint32_t kUmBK = 64;                              // k per chunk: one 128-byte swizzle atom of bf16
-constexpr uint32_t kUmRawBytes = 8 * kUmBN * 4 + kUmBN * 2 + (kUmBN / 8) * 4;      // 8832: words, scales, zero points
-constexpr uint32_t kUmRawStride = 9216;                     // keeps every stage 1024-byte aligned
 constexpr uint32_t kUmXBytes = 128 * kUmBK * 2;             // 16 KiB: activations of a chunk at M = 128
 // Tensor memory (512 columns): accumulators 2 x 128 columns, then four A stages of 2 halves x 4 k-steps x 8 columns.
 constexpr uint32_t kUmTmemCols = 512;
@@ -62,16 +58,6 @@ struct UmParams {
     uint32_t total;          // chunks of the launch, shared out evenly (less than 2^24)
 };
 
-__device__ __forceinline__ uint32_t um_lds32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ uint32_t um_lds16(uint32_t addr) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -294,19 +280,10 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
                 uint32_t r[32];                                // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
 #pragma unroll
                 for (uint32_t i = 0; i < 8; ++i) {
-                    const uint32_t wd = words[i];
-                    const uint32_t v0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), zz), ss);            // k 0, 4
-                    const uint32_t v1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), zz), ss);       // k 1, 5
-                    const uint32_t v2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), zz), ss);       // k 2, 6
-                    const uint32_t v3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), zz), ss);      // k 3, 7
-                    if constexpr (kTiled) {                    // tile-major words are stored so that the pairs come out in k order
-                        r[4 * i] = v0; r[4 * i + 1] = v1; r[4 * i + 2] = v2; r[4 * i + 3] = v3;
-                    } else {                                   // row layout: pairs (0,4) (1,5) (2,6) (3,7)
-                        r[4 * i] = __byte_perm(v0, v1, 0x5410);
-                        r[4 * i + 1] = __byte_perm(v2, v3, 0x5410);
-                        r[4 * i + 2] = __byte_perm(v0, v1, 0x7632);
-                        r[4 * i + 3] = __byte_perm(v2, v3, 0x7632);
-                    }
+                    uint32_t v[4];
+                    um_dequant_word(words[i], mask, magic, zz, ss, kTiled, v);
+#pragma unroll
+                    for (uint32_t e = 0; e < 4; ++e) r[4 * i + e] = v[e];
                 }
                 // the A stage is free once the UMMAs of four chunks ago have read it
                 if (!ptx::mbar_wait(a_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
