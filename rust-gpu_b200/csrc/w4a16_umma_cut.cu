@@ -356,10 +356,9 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
                     }
                     if (good) *counter = 0;                // ready for the next launch
                     else atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xE00000);
-                    __threadfence();
                 }
-                good = __shfl_sync(0xFFFFFFFFu, good, 0);
                 __syncwarp();                              // orders the other lanes' loads of the parts after lane 0's acquire (a shuffle does not)
+                good = __shfl_sync(0xFFFFFFFFu, good, 0);
                 if (!good) { ok = false; break; }
             }
             const uint32_t prob = item / p.n_tiles;
