@@ -324,9 +324,12 @@ int t0_auto_select_backward_weight(uint32_t m, uint32_t n_orig, uint32_t k_orig,
     return t0_auto_select(n_orig, m, k_orig, out);   // gemm_gen.rs:545-549
 }
 
-int t0_cached_auto_select(uint32_t m, uint32_t k, uint32_t n, t0_gemm_config* out) {
-    if (!out) return fail(T0_ERR_INVALID, "null output");
-    { const int fr = forced_config(out); if (fr >= 0) return fr; }   // a forced config is never cached
+}  // extern "C"
+
+int t0::cached_config(uint32_t m, uint32_t k, uint32_t n, t0_gemm_config* out, bool* forced) {
+    const int fr = forced_config(out);      // (reading the environment costs as much as all the rest: once a call)
+    *forced = fr >= 0;
+    if (*forced) return fr;                 // a forced config is never cached
     auto key = std::make_tuple(m, k, n);
     {
         std::lock_guard<std::mutex> g(g_cache_mu);
@@ -338,6 +341,14 @@ int t0_cached_auto_select(uint32_t m, uint32_t k, uint32_t n, t0_gemm_config* ou
     std::lock_guard<std::mutex> g(g_cache_mu);
     g_cache[key] = *out;
     return T0_OK;
+}
+
+extern "C" {
+
+int t0_cached_auto_select(uint32_t m, uint32_t k, uint32_t n, t0_gemm_config* out) {
+    if (!out) return fail(T0_ERR_INVALID, "null output");
+    bool forced;
+    return t0::cached_config(m, k, n, out, &forced);
 }
 
 int t0_cached_auto_select_backward_data(uint32_t m, uint32_t n_orig, uint32_t k_orig, t0_gemm_config* out) {

@@ -80,6 +80,9 @@ struct GemmChoice {
 // nothing here does that (many tiles and a deep cut); the configuration itself is to be taken.
 GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once);
 
+// t0_cached_auto_select, saying whether the environment forces the configuration (T0_FORCE_CFG).
+int cached_config(uint32_t m, uint32_t k, uint32_t n, t0_gemm_config* out, bool* forced);
+
 // y[i] = sum_s planes[s][i] in split order, then the epilogue; K4.
 int launch_splitk_reduce(const float* planes, void* y, const float* bias, uint32_t m, uint32_t n, uint32_t split_k,
                          bool out_bf16, uint8_t epilogue, uint8_t n_ops, const uint8_t* ops, float scale, float clamp_min,

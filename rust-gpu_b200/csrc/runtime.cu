@@ -48,9 +48,10 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     // for the shape: tile, CTA pair or not, and into how many parts K is cut.
     if (q.tile_n == 0 && q.pair == 0 && q.split_k <= 1 && !q.planes && q.k >= 64) {
         t0_gemm_config c;
-        const bool known = t0_cached_auto_select(q.m, q.k, q.n, &c) == T0_OK;
+        bool forced;
+        const bool known = cached_config(q.m, q.k, q.n, &c, &forced) == T0_OK;
         GemmChoice choice = {};
-        if (!getenv("T0_FORCE_CFG")) {
+        if (!forced) {
             const uint32_t s = known && c.split_k > 1 && q.k % c.split_k == 0 ? c.split_k : 1;
             choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count, gemm_clusters_at_once());
         }
