@@ -23,7 +23,7 @@
 //     What bounds this loop is the instructions around the arithmetic as much as the arithmetic (15 per packed word of 8 codes, 8 words
 //     per warp and step) and, with two row groups, the rate of mma.sync (leaving the dequantisation out changes nothing at M = 16).  A
 //     warp that owned 16 columns and the whole k of a step read all the activation fragments of the step for half the columns, and 21
-//     warps left 80 registers a thread: 12 problems of M = 1, N = 11008, K = 4096 took 80.4 us, 70.5 so; two of them 19.3 and 18.7.
+//     warps left 80 registers a thread: 12 problems of M = 1, N = 11008, K = 4096 took 80.2 us, 73.8 so; two of them 19.3 and 18.6.
 //   * a band that lies wholly inside a range is stored directly; a band shared by several CTAs is finished by whichever
 //     CTA arrives last (per-band arrival counter, partial pieces in scratch, added in k order: deterministic, repeated
 //     calls agree bit for bit); no CTA ever waits for another.  A spare lane of the producer warp counts a range's leading

@@ -17,8 +17,8 @@
 // reach it last: see the epilogue.
 //
 // Whole tiles per CTA leave SMs idle where the tiles are few or just over a multiple of them: two problems of N = 11008 are 86 tiles on 148
-// SMs.  M = 128, K = 4096: 43.8 us with whole tiles, 40.4 cut; M = 107, N = 7936, K = 4352: 45.3 and 34.4; M = 81, N = 2560, K = 7424, four
-// problems: 72.0 and 37.3.  What bounds it is the chain of waits around a chunk (0.67 us; arithmetic alone would take about 0.15) and, per
+// SMs.  M = 128, K = 4096: 43.7 us with whole tiles, 40.6 cut; M = 107, N = 7936, K = 4352: 45.0 and 33.5; M = 81, N = 2560, K = 7424, four
+// problems: 71.5 and 36.3.  What bounds it is the chain of waits around a chunk (0.67 us; arithmetic alone would take about 0.15) and, per
 // launch, about 10 us for handing in and adding the parts of cut tiles; `w4a16_umma_cut_applies` weighs the two.
 #include "w4a16_common.cuh"
 
