@@ -74,6 +74,7 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     const bool needs_bias = q.n_ops ? std::find(q.ops, q.ops + q.n_ops, (uint8_t)T0_TEPI_BIAS_ADD) != q.ops + q.n_ops
                                     : q.epilogue != T0_EPI_STORE_F32;
     if (needs_bias && !q.bias) return fail(T0_ERR_INVALID, "epilogue needs a bias vector but bias is null");
+    if (!needs_bias) q.bias = 0;                   // given but not asked for: no kernel touches it
     uint32_t split = q.split_k > 1 ? q.split_k : 1;
     if (q.n_peer_y && (split > 1 || q.k == 0 || q.out_bf16 || q.planes))
         return fail(T0_ERR_UNSUPPORTED, "a gathered output takes a plain f32 product: no split-K, no bf16 output, K > 0");
