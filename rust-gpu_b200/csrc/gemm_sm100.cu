@@ -214,8 +214,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     probe.begin(p);
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // ------------------------------------------------------------ TMA producer: the whole warp walks, one lane issues
+        {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < total_work; w += gridDim.x) {
@@ -227,47 +227,50 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 if constexpr (kGrouped) { ma = &group.maps[3 * prob]; mb = &group.maps[3 * prob + 1]; }
                 const KRange kr = k_range<kCluster>(wi.split, p);
                 for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
+                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                        if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
                         ok = false;
                         break;
                     }
                     const uint32_t fb = ptx::smem_u32(&full_bar[stage]);
                     // self-test of the failure path: this stage is never filled, so the issuer's bounded wait must run out
                     if (p.drop_load && blockIdx.x == 0 && w == 0 && kb == 0) { if (++stage == kStages) { stage = 0; phase ^= 1; } continue; }
-                    ptx::mbar_arrive_expect_tx(fb, kStageBytes);
-                    if constexpr (!A_MN) {
-                        ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
-                                         (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)kr.z);
-                    } else {
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(fb, kStageBytes);
+                        if constexpr (!A_MN) {
+                            ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
+                                             (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)kr.z);
+                        } else {
 #pragma unroll
-                        for (uint32_t j = 0; j < BM / 64; ++j)
-                            ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), ma, fb,
-                                             (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
-                    }
-                    if constexpr (!B_MN) {
-                        ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
-                                         (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)kr.z);
-                    } else {
-                        // B[K,N]: one 64(k) x 64(n) box per 64 columns; each box is an [k][128 B] block
+                            for (uint32_t j = 0; j < BM / 64; ++j)
+                                ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), ma, fb,
+                                                 (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
+                        }
+                        if constexpr (!B_MN) {
+                            ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
+                                             (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)kr.z);
+                        } else {
+                            // B[K,N]: one 64(k) x 64(n) box per 64 columns; each box is an [k][128 B] block
 #pragma unroll
-                        for (uint32_t j = 0; j < BN / 64; ++j)
-                            ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes + j * (BK * 128)), mb, fb,
-                                             (int32_t)(wi.n_blk * BN + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
+                            for (uint32_t j = 0; j < BN / 64; ++j)
+                                ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes + j * (BK * 128)), mb, fb,
+                                                 (int32_t)(wi.n_blk * BN + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
+                        }
                     }
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ UMMA issuer
-        if (lane == 0) {
+        // ------------------------------------------------------------ UMMA issuer: the whole warp walks, one lane issues
+        {
             uint32_t stage = 0, phase = 0, iter = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < total_work; w += gridDim.x, ++iter) {
                 const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
-                if (!ptx::mbar_wait(ptx::smem_u32(&tmem_empty_bar[buf]), acc_phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                    atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w & 0xFFFFFF));
+                if (!ptx::mbar_wait_warp(ptx::smem_u32(&tmem_empty_bar[buf]), acc_phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w & 0xFFFFFF));
                     break;
                 }
                 ptx::tc_fence_after_sync();
@@ -275,29 +278,33 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const uint32_t kb_mid = k_mid<kAccs>(kr, p);
                 uint32_t tmem_d = tmem_base + buf * BN * kAccs;
                 for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
+                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
+                        if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after_sync();
                     if (kb == kb_mid) tmem_d += BN;
-                    const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
-                    const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
+                    if (ptx::elect_one()) {
+                        const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
+                        const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
 #pragma unroll
-                    for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
-                        // K-major, 128B swizzle: 8-row groups 1024 B apart; a 16-element K step is 32 B
-                        const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
-                                                 : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
-                        // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
-                        const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
-                                                 : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
-                        ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, ((kb != kr.first && kb != kb_mid) || k4 != 0) ? 1u : 0u);
+                        for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
+                            // K-major, 128B swizzle: 8-row groups 1024 B apart; a 16-element K step is 32 B
+                            const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
+                                                     : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
+                            // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
+                            const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
+                                                     : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
+                            ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, ((kb != kr.first && kb != kb_mid) || k4 != 0) ? 1u : 0u);
+                        }
+                        ptx::umma_commit(ptx::smem_u32(&empty_bar[stage]));
                     }
-                    ptx::umma_commit(ptx::smem_u32(&empty_bar[stage]));
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
-                if (ok) ptx::umma_commit(ptx::smem_u32(&tmem_full_bar[buf]));
+                if (ok && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(&tmem_full_bar[buf]));
+                __syncwarp();
             }
         }
     } else {

@@ -104,8 +104,8 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
     probe.begin(p);
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
+        // ------------------------------------------------------------ TMA producer (both CTAs): the whole warp walks, one lane issues
+        {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (uint32_t w = pair_id; ok && w < total_work; w += n_pairs) {
@@ -113,87 +113,94 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                 const uint32_t half = tail ? ((w - tail_start) & 1u) : 0u;
                 const WorkItem wi = decode_work(tail ? tail_start + ((w - tail_start) >> 1) : w, p);
                 for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
+                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                        if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
                         ok = false;
                         break;
                     }
                     const uint32_t fb_local = ptx::smem_u32(&full_bar[stage]);
                     // self-test of the failure path: neither CTA of pair 0 fills this stage, so the issuer's bounded wait must run out
                     if (p.drop_load && pair_id == 0 && w == 0 && kb == 0) { if (++stage == kStages) { stage = 0; phase ^= 1; } continue; }
-                    if (cta_rank == 0) ptx::mbar_arrive_expect_tx(fb_local, 2 * (kAStageBytes + (tail ? kBHalfStageBytes : kBStageBytes)));   // bytes of both CTAs
-                    const uint32_t fb = ptx::mapa(fb_local, 0);   // the even CTA's barrier, from either CTA
-                    if constexpr (!A_MN) {
-                        ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes), &map_a, fb,
-                                              (int32_t)(kb * BK), (int32_t)(wi.m_blk * kPairM + cta_rank * BM), (int32_t)wi.split);
-                    } else {
+                    if (ptx::elect_one()) {
+                        if (cta_rank == 0) ptx::mbar_arrive_expect_tx(fb_local, 2 * (kAStageBytes + (tail ? kBHalfStageBytes : kBStageBytes)));   // bytes of both CTAs
+                        const uint32_t fb = ptx::mapa(fb_local, 0);   // the even CTA's barrier, from either CTA
+                        if constexpr (!A_MN) {
+                            ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes), &map_a, fb,
+                                                  (int32_t)(kb * BK), (int32_t)(wi.m_blk * kPairM + cta_rank * BM), (int32_t)wi.split);
+                        } else {
 #pragma unroll
-                        for (uint32_t j = 0; j < BM / 64; ++j)
-                            ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), &map_a, fb,
-                                                  (int32_t)(wi.m_blk * kPairM + cta_rank * BM + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                            for (uint32_t j = 0; j < BM / 64; ++j)
+                                ptx::tma_load_3d_pair(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), &map_a, fb,
+                                                      (int32_t)(wi.m_blk * kPairM + cta_rank * BM + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                        }
+                        if constexpr (B_MN) {
+                            // this CTA's columns of B[K,N]: one 64(k) x 64(n) box (a [k][128 B] block) per 64 columns
+                            const uint32_t cols = tail ? kHalfN / 2 : kBHalfRows;
+                            const uint32_t n0 = wi.n_blk * kPairN + (tail ? half * kHalfN : 0) + cta_rank * cols;
+                            for (uint32_t j = 0; j < cols / 64; ++j)
+                                ptx::tma_load_3d_pair(ptx::smem_u32(b_tiles + stage * kBStageBytes + j * (BK * 128)), &map_b, fb,
+                                                      (int32_t)(n0 + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
+                        } else if (!tail) {
+                            ptx::tma_load_3d_pair(ptx::smem_u32(b_tiles + stage * kBStageBytes), &map_b, fb,
+                                                  (int32_t)(kb * BK), (int32_t)(wi.n_blk * kPairN + cta_rank * kBHalfRows), (int32_t)wi.split);
+                        } else {
+                            ptx::tma_load_3d_pair(ptx::smem_u32(b_tiles + stage * kBStageBytes), &map_b_half, fb,
+                                                  (int32_t)(kb * BK), (int32_t)(wi.n_blk * kPairN + half * kHalfN + cta_rank * (kHalfN / 2)), (int32_t)wi.split);
+                        }
                     }
-                    if constexpr (B_MN) {
-                        // this CTA's columns of B[K,N]: one 64(k) x 64(n) box (a [k][128 B] block) per 64 columns
-                        const uint32_t cols = tail ? kHalfN / 2 : kBHalfRows;
-                        const uint32_t n0 = wi.n_blk * kPairN + (tail ? half * kHalfN : 0) + cta_rank * cols;
-                        for (uint32_t j = 0; j < cols / 64; ++j)
-                            ptx::tma_load_3d_pair(ptx::smem_u32(b_tiles + stage * kBStageBytes + j * (BK * 128)), &map_b, fb,
-                                                  (int32_t)(n0 + j * 64), (int32_t)(kb * BK), (int32_t)wi.split);
-                    } else if (!tail) {
-                        ptx::tma_load_3d_pair(ptx::smem_u32(b_tiles + stage * kBStageBytes), &map_b, fb,
-                                              (int32_t)(kb * BK), (int32_t)(wi.n_blk * kPairN + cta_rank * kBHalfRows), (int32_t)wi.split);
-                    } else {
-                        ptx::tma_load_3d_pair(ptx::smem_u32(b_tiles + stage * kBStageBytes), &map_b_half, fb,
-                                              (int32_t)(kb * BK), (int32_t)(wi.n_blk * kPairN + half * kHalfN + cta_rank * (kHalfN / 2)), (int32_t)wi.split);
-                    }
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ UMMA issuer (even CTA only)
-        if (lane == 0 && cta_rank == 0) {
+        // ------------------------------------------------------------ UMMA issuer (even CTA only): the whole warp walks, one lane issues
+        if (cta_rank == 0) {
             uint32_t stage = 0, phase = 0, iter = 0;
             bool ok = true;
             for (uint32_t w = pair_id; ok && w < total_work; w += n_pairs, ++iter) {
                 const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
-                if (!ptx::mbar_wait(ptx::smem_u32(&tmem_empty_bar[buf]), acc_phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                    atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w & 0xFFFFFF));
+                if (!ptx::mbar_wait_warp(ptx::smem_u32(&tmem_empty_bar[buf]), acc_phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w & 0xFFFFFF));
                     break;
                 }
                 ptx::tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + buf * kPairN;
                 const uint32_t idesc = w >= tail_start ? kIdescHalf : kIdesc;
                 for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
+                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
+                        if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after_sync();
-                    if (kb == 0 && w == pair_id) trace_stamp(p, 3);
-                    const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
-                    const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
+                    if (ptx::elect_one()) {
+                        if (kb == 0 && w == pair_id) trace_stamp(p, 3);
+                        const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
+                        const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
 #pragma unroll
-                    for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
-                        const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
-                                                 : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
-                        // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
-                        const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
-                                                 : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
-                        ptx::umma_bf16_ss_pair(tmem_d, da, db, idesc, (kb | k4) != 0 ? 1u : 0u);
+                        for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
+                            const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
+                                                     : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
+                            // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
+                            const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
+                                                     : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
+                            ptx::umma_bf16_ss_pair(tmem_d, da, db, idesc, (kb | k4) != 0 ? 1u : 0u);
+                        }
+                        // the stage is free in both CTAs once these UMMAs have read it
+                        const uint32_t eb = ptx::smem_u32(&empty_bar[stage]);
+                        ptx::umma_commit_pair(eb);
+                        ptx::umma_commit_pair(ptx::mapa(eb, 1));
                     }
-                    // the stage is free in both CTAs once these UMMAs have read it
-                    const uint32_t eb = ptx::smem_u32(&empty_bar[stage]);
-                    ptx::umma_commit_pair(eb);
-                    ptx::umma_commit_pair(ptx::mapa(eb, 1));
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
-                if (ok) {
+                if (ok && ptx::elect_one()) {
                     const uint32_t tb = ptx::smem_u32(&tmem_full_bar[buf]);
                     ptx::umma_commit_pair(tb);
                     ptx::umma_commit_pair(ptx::mapa(tb, 1));
                 }
+                __syncwarp();
             }
         }
     } else {

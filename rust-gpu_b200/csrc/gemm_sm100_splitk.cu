@@ -129,8 +129,8 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
     probe.begin(p);
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // ------------------------------------------------------------ TMA producer: the whole warp walks, one lane issues
+        {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (uint32_t w = cluster_id_x(); ok && w < n_items; w += n_clusters_x()) {
@@ -141,54 +141,61 @@ gemm_bf16_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const
                 const CUtensorMap* mb = &map_b;
                 if constexpr (kGrouped) { ma = &group.maps[2 * prob]; mb = &group.maps[2 * prob + 1]; }
                 for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
+                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                        if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
                         ok = false;
                         break;
                     }
                     const uint32_t fb = ptx::smem_u32(&full_bar[stage]);
-                    ptx::mbar_arrive_expect_tx(fb, kStageBytes);
-                    ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
-                                     (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)split);
-                    ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
-                                     (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)split);
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(fb, kStageBytes);
+                        ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
+                                         (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)split);
+                        ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
+                                         (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)split);
+                    }
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ UMMA issuer
-        if (lane == 0) {
+        // ------------------------------------------------------------ UMMA issuer: the whole warp walks, one lane issues
+        {
             uint32_t stage = 0, phase = 0, iter = 0;
             bool ok = true;
             for (uint32_t w = cluster_id_x(); ok && w < n_items; w += n_clusters_x(), ++iter) {
                 const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
-                if (!ptx::mbar_wait(ptx::smem_u32(&tmem_empty_bar[buf]), acc_phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                    atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w & 0xFFFFFF));
+                if (!ptx::mbar_wait_warp(ptx::smem_u32(&tmem_empty_bar[buf]), acc_phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w & 0xFFFFFF));
                     break;
                 }
                 ptx::tc_fence_after_sync();
                 const uint32_t tmem_d = tmem_base + buf * BN;
                 for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
+                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
+                        if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after_sync();
-                    if (kb == 0 && iter == 0) trace_stamp(p, 3);
-                    const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
-                    const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
+                    if (ptx::elect_one()) {
+                        if (kb == 0 && iter == 0) trace_stamp(p, 3);
+                        const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
+                        const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
 #pragma unroll
-                    for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
-                        const uint64_t da = ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
-                        const uint64_t db = ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
-                        ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, (kb | k4) != 0 ? 1u : 0u);
+                        for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
+                            const uint64_t da = ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
+                            const uint64_t db = ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
+                            ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, (kb | k4) != 0 ? 1u : 0u);
+                        }
+                        ptx::umma_commit(ptx::smem_u32(&empty_bar[stage]));
                     }
-                    ptx::umma_commit(ptx::smem_u32(&empty_bar[stage]));
+                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }
-                if (ok) ptx::umma_commit(ptx::smem_u32(&tmem_full_bar[buf]));
+                if (ok && ptx::elect_one()) ptx::umma_commit(ptx::smem_u32(&tmem_full_bar[buf]));
+                __syncwarp();
             }
         }
     }

@@ -68,6 +68,36 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// The same wait by a whole converged warp; the result is the same in every lane, and the compiler knows it: what follows stays in
+// uniform registers, from which the tensor-core and TMA instructions take their operands.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    uint64_t t_start = 0;
+    for (uint32_t spin = 1;; ++spin) {
+        if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+        if ((spin & 0xFF) == 0) {
+            const uint64_t now = globaltimer_ns();
+            if (t_start == 0) t_start = now;
+            const bool expired = now - t_start > limit_ns;
+            if (expired) *abort_flag = 1;
+            if (__any_sync(0xFFFFFFFFu, expired || *abort_flag != 0)) return false;
+        }
+    }
+}
+// True in one lane of a converged warp, the same one every time.  A branch on it is one the compiler knows to be taken by a single thread,
+// so operands computed by the whole warp need no move per lane.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(is));
+    return is != 0;
+}
+
 // The same wait for a role that runs well ahead of the roles it waits on (a producer that fills a deep ring, a helper
 // that prepares later steps): between polls the thread sleeps, so that its polling takes no issue slots from the warps
 // that do the arithmetic.  In the W4A16 kernel five such lanes polling back to back executed a quarter of all instructions.

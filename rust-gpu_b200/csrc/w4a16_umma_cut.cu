@@ -192,28 +192,28 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
         }
     } else if (warp == kUmIssueWarp) {
         // -------------------------------------------------------------- UMMA issuer: per chunk 2 halves x 4 k-steps of M 128 x N rows x K 16
-        if (lane == 0) {
-            const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u);
-            uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0;
-            const uint64_t x_desc = ptx::make_smem_desc(x_ring, 16, 1024);      // (addresses enter a descriptor in 16-byte units: stages are added)
-            bool ok = true;
-            for (uint32_t u = u0; ok && u < u1; ++piece) {
-                const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks);
-                if (piece > 0 && !ptx::mbar_wait(acc_empty, (piece - 1) & 1, abort_flag, p.wait_limit_ns)) {
-                    atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
+        const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u);
+        uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0;
+        const uint64_t x_desc = ptx::make_smem_desc(x_ring, 16, 1024);      // (addresses enter a descriptor in 16-byte units: stages are added)
+        bool ok = true;
+        for (uint32_t u = u0; ok && u < u1; ++piece) {
+            const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks);
+            if (piece > 0 && !ptx::mbar_wait_warp(acc_empty, (piece - 1) & 1, abort_flag, p.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
+                break;
+            }
+            ptx::tc_fence_after_sync();
+            for (uint32_t first = 1; u < u_end; ++u, first = 0) {
+                if (!ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
+                    !ptx::mbar_wait_warp(a_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
+                    ok = false;
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                for (uint32_t first = 1; u < u_end; ++u, first = 0) {
-                    if (!ptx::mbar_wait(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
-                        !ptx::mbar_wait(a_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
-                        atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after_sync();
-                    const uint64_t x_stage = x_desc + xs * (kUmXBytes / 16);
-                    const uint32_t a_cols = tmem_base + kUmABase + as * kUmAStageCols;
+                const uint64_t x_stage = x_desc + xs * (kUmXBytes / 16);
+                const uint32_t a_cols = tmem_base + kUmABase + as * kUmAStageCols;
+                if (ptx::elect_one()) {
 #pragma unroll
                     for (uint32_t k4 = 0; k4 < kUmBK / 16; ++k4) {
 #pragma unroll
@@ -222,11 +222,13 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
                     }
                     ptx::umma_commit(a_empty + 8 * as);
                     ptx::umma_commit(x_empty + 8 * xs);
-                    if (++as == kUmAStages) { as = 0; aphase ^= 1; }
-                    if (++xs == kUmXStages) { xs = 0; xphase ^= 1; }
                 }
-                if (ok) ptx::umma_commit(acc_full);
+                __syncwarp();
+                if (++as == kUmAStages) { as = 0; aphase ^= 1; }
+                if (++xs == kUmXStages) { xs = 0; xphase ^= 1; }
             }
+            if (ok && ptx::elect_one()) ptx::umma_commit(acc_full);
+            __syncwarp();
         }
     } else {
         // -------------------------------------------------------------- sixteen warps: dequantise into tensor memory, then the epilogue
