@@ -28,9 +28,11 @@ using namespace t0::w4;
 namespace {
 
 constexpr uint32_t kUmDqWarps = 16;
-// + the warps that fetch weights and activations and the one that issues the UMMAs.  Each is one lane working through a serial chain
-// of instructions per chunk, at several cycles an instruction, so the chains are kept short (running counters, no divisions, descriptors
-// stepped by addition) and apart: two lanes of one warp would take turns.
+// + the warps that fetch weights and activations and the one that issues the UMMAs.  Each works through a serial chain of instructions per
+// chunk, at several cycles an instruction, so the chains are kept short (running counters, no divisions, descriptors stepped by addition,
+// one barrier for both operands of a chunk) and apart.  The issuer's chain took 1190 cycles a chunk as one diverged lane with a barrier per
+// operand, which the sixteen dequantising warps spent waiting: two problems of M = 128, N = 11008, K = 4096 39.7 us, 33.3 with the warp
+// converged, 31.7 with one barrier.
 constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;
 constexpr uint32_t kUmThreads = (kUmDqWarps + 3) * 32;
 constexpr uint32_t kUmXBytes = 128 * kUmBK * 2;             // 16 KiB: activations of a chunk at M = 128
@@ -38,11 +40,10 @@ constexpr uint32_t kUmXBytes = 128 * kUmBK * 2;             // 16 KiB: activatio
 constexpr uint32_t kUmTmemCols = 512;
 constexpr uint32_t kUmABase = 256;                          // first column of the A stages
 constexpr uint32_t kUmAStageCols = 64;
-constexpr uint32_t kUmAStages = 4;
-constexpr uint32_t kUmXStages = 4;                          // activation stages
+constexpr uint32_t kUmAStages = 4;                          // operand stages: weights in tensor memory, activations in shared memory
 constexpr uint32_t kUmRawStages = 7;                        // raw weight stages of two chunks: 124 KB in flight per SM
 // (more than half an SM's shared memory: the kernel takes all 512 tensor-memory columns, so two of its CTAs must never share an SM)
-constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmXStages * kUmXBytes + 512 + 1024;
+constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmAStages * kUmXBytes + 512 + 1024;
 constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long: below it the finish costs more than the range
 constexpr size_t kUmCounterBytes = 16 * 1024;               // one word per CTA and dequantisation warp (up to 256 CTAs)
 
@@ -76,11 +77,10 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
     const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t raw_ring = smem;
     const uint32_t x_ring = smem + kUmRawStages * 2 * kUmRawStride;           // activations: [rows][64 k] bf16, 128-byte swizzle, per stage
-    const uint32_t bars = x_ring + kUmXStages * kUmXBytes;
+    const uint32_t bars = x_ring + kUmAStages * kUmXBytes;
     const uint32_t raw_full = bars, raw_empty = bars + 8 * kUmRawStages;
     const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * kUmAStages;
-    const uint32_t x_full = a_empty + 8 * kUmAStages, x_empty = x_full + 8 * kUmXStages;
-    const uint32_t acc_full = x_empty + 8 * kUmXStages, acc_empty = acc_full + 8;
+    const uint32_t acc_full = a_empty + 8 * kUmAStages, acc_empty = acc_full + 8;
     __shared__ uint32_t tmem_holder;
     __shared__ int s_abort;
     volatile int* abort_flag = &s_abort;
@@ -94,12 +94,8 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
             ptx::mbar_init(raw_empty + 8 * s, kUmDqWarps);
         }
         for (uint32_t s = 0; s < kUmAStages; ++s) {
-            ptx::mbar_init(a_full + 8 * s, kUmDqWarps / 2);       // the eight warps that dequantise the chunk
+            ptx::mbar_init(a_full + 8 * s, kUmDqWarps / 2 + 1);   // the eight warps that dequantise the chunk, and the activations' bytes
             ptx::mbar_init(a_empty + 8 * s, 1);
-        }
-        for (uint32_t s = 0; s < kUmXStages; ++s) {
-            ptx::mbar_init(x_full + 8 * s, 1);
-            ptx::mbar_init(x_empty + 8 * s, 1);
         }
         ptx::mbar_init(acc_full, 1);
         ptx::mbar_init(acc_empty, kUmDqWarps);
@@ -119,81 +115,78 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
 
+    // The three serial roles walk with their whole warp and let one elected lane issue: see ptx::elect_one.
     if (warp == kUmRawWarp) {
-        if (lane == 0) {
-            // ---------------------------------------------------------- raw weights, scales, zero points: three TMA boxes per chunk
-            uint32_t stage = 0, phase = 0;
-            const uint32_t item = u0 / n_chunks, per_group = p.group / kUmBK;
-            uint32_t c = u0 - item * n_chunks, tile = item;
-            uint32_t grp = c / per_group, in_group = c - grp * per_group;
-            const uint32_t prob = item / p.n_tiles;
-            tile = item - prob * p.n_tiles;
-            const CUtensorMap* mw = &group.maps[4 * prob];
-            const CUtensorMap* ms = mw + 1;
-            const CUtensorMap* mz = mw + 2;
-            for (uint32_t u = u0; u < u1;) {
-                if (!ptx::mbar_wait_relaxed(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns, 64)) {
-                    atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(c & 0xFFFFFF));
-                    break;
-                }
-                ptx::fence_proxy_async_smem();           // the stage was read through the generic proxy, the copies write it through the async proxy
-                const uint32_t fb = raw_full + 8 * stage;
-                uint32_t dst = raw_ring + stage * (2 * kUmRawStride);
-                const uint32_t u_stop = min(u1, u + 2);
+        // -------------------------------------------------------------- raw weights, scales, zero points: three TMA boxes per chunk
+        uint32_t stage = 0, phase = 0;
+        const uint32_t item = u0 / n_chunks, per_group = p.group / kUmBK;
+        uint32_t c = u0 - item * n_chunks, tile = item;
+        uint32_t grp = c / per_group, in_group = c - grp * per_group;
+        uint32_t prob = item / p.n_tiles;
+        tile = item - prob * p.n_tiles;
+        for (uint32_t u = u0; u < u1;) {
+            if (!ptx::mbar_wait_warp(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(c & 0xFFFFFF));
+                break;
+            }
+            const uint32_t fb = raw_full + 8 * stage;
+            uint32_t dst = raw_ring + stage * (2 * kUmRawStride);
+            const uint32_t u_stop = min(u1, u + 2);
+            if (ptx::elect_one()) {
+                ptx::fence_proxy_async_smem();       // the stage was read through the generic proxy, the copies write it through the async proxy
                 ptx::mbar_arrive_expect_tx(fb, (u_stop - u) * kUmRawBytes);
-                for (; u < u_stop; ++u, dst += kUmRawStride) {
+            }
+            __syncwarp();
+            for (; u < u_stop; ++u, dst += kUmRawStride) {
+                if (ptx::elect_one()) {
+                    const CUtensorMap* const mw = &group.maps[4 * prob];
                     if constexpr (kTiled) {
                         // tile-major layout: the chunk's 8 KB of words are contiguous, as are its scales and zero points
                         ptx::tma_load_3d(dst, mw, fb, 0, (int32_t)(c * (kUmBK / 8)), (int32_t)tile);
-                        ptx::tma_load_3d(dst + 8 * kUmBN * 4, ms, fb, 0, (int32_t)grp, (int32_t)tile);
-                        ptx::tma_load_3d(dst + 8 * kUmBN * 4 + kUmBN * 2, mz, fb, 0, (int32_t)grp, (int32_t)tile);
+                        ptx::tma_load_3d(dst + 8 * kUmBN * 4, mw + 1, fb, 0, (int32_t)grp, (int32_t)tile);
+                        ptx::tma_load_3d(dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, 0, (int32_t)grp, (int32_t)tile);
                     } else {
                         ptx::tma_load_2d(dst, mw, fb, (int32_t)(tile * kUmBN), (int32_t)(c * (kUmBK / 8)));
-                        ptx::tma_load_2d(dst + 8 * kUmBN * 4, ms, fb, (int32_t)(tile * kUmBN), (int32_t)grp);
-                        ptx::tma_load_2d(dst + 8 * kUmBN * 4 + kUmBN * 2, mz, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)grp);
-                    }
-                    if (++in_group == per_group) { in_group = 0; ++grp; }
-                    if (++c == n_chunks) {
-                        c = grp = in_group = 0;
-                        if (++tile == p.n_tiles) {
-                            tile = 0;
-                            mw += 4; ms += 4; mz += 4;
-                        }
+                        ptx::tma_load_2d(dst + 8 * kUmBN * 4, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)grp);
+                        ptx::tma_load_2d(dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)grp);
                     }
                 }
-                if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
+                __syncwarp();
+                if (++in_group == per_group) { in_group = 0; ++grp; }
+                if (++c == n_chunks) {
+                    c = grp = in_group = 0;
+                    if (++tile == p.n_tiles) { tile = 0; ++prob; }
+                }
             }
+            if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
         }
     } else if (warp == kUmXWarp) {
-        if (lane == 0) {
-            // ---------------------------------------------------------- activations: one box per chunk (rows beyond M are zero)
-            uint32_t xs = 0, xphase = 0;
-            const uint32_t item = u0 / n_chunks;
-            uint32_t c = u0 - item * n_chunks, tile = item;
-            const uint32_t prob = item / p.n_tiles;
-            tile = item - prob * p.n_tiles;
-            const CUtensorMap* ma = &group.maps[4 * prob + 3];
-            for (uint32_t u = u0; u < u1; ++u) {
-                if (!ptx::mbar_wait_relaxed(x_empty + 8 * xs, xphase ^ 1, abort_flag, p.wait_limit_ns, 64)) {
-                    atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
-                    break;
-                }
-                ptx::mbar_arrive_expect_tx(x_full + 8 * xs, p.rows * kUmBK * 2);
-                ptx::tma_load_3d(x_ring + xs * kUmXBytes, ma, x_full + 8 * xs, (int32_t)(c * kUmBK), 0, 0);
-                if (++xs == kUmXStages) { xs = 0; xphase ^= 1; }
-                if (++c == n_chunks) {
-                    c = 0;
-                    if (++tile == p.n_tiles) {
-                        tile = 0;
-                        ma += 4;
-                    }
-                }
+        // -------------------------------------------------------------- activations: one box per chunk (rows beyond M are zero)
+        uint32_t as = 0, aphase = 0;
+        const uint32_t item = u0 / n_chunks;
+        uint32_t c = u0 - item * n_chunks, tile = item;
+        uint32_t prob = item / p.n_tiles;
+        tile = item - prob * p.n_tiles;
+        for (uint32_t u = u0; u < u1; ++u) {
+            if (!ptx::mbar_wait_warp(a_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
+                break;
+            }
+            if (ptx::elect_one()) {
+                ptx::mbar_arrive_expect_tx(a_full + 8 * as, p.rows * kUmBK * 2);
+                ptx::tma_load_3d(x_ring + as * kUmXBytes, &group.maps[4 * prob + 3], a_full + 8 * as, (int32_t)(c * kUmBK), 0, 0);
+            }
+            __syncwarp();
+            if (++as == kUmAStages) { as = 0; aphase ^= 1; }
+            if (++c == n_chunks) {
+                c = 0;
+                if (++tile == p.n_tiles) { tile = 0; ++prob; }
             }
         }
     } else if (warp == kUmIssueWarp) {
         // -------------------------------------------------------------- UMMA issuer: per chunk 2 halves x 4 k-steps of M 128 x N rows x K 16
         const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u);
-        uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0;
+        uint32_t as = 0, aphase = 0, piece = 0;
         const uint64_t x_desc = ptx::make_smem_desc(x_ring, 16, 1024);      // (addresses enter a descriptor in 16-byte units: stages are added)
         bool ok = true;
         for (uint32_t u = u0; ok && u < u1; ++piece) {
@@ -204,14 +197,13 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
             }
             ptx::tc_fence_after_sync();
             for (uint32_t first = 1; u < u_end; ++u, first = 0) {
-                if (!ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
-                    !ptx::mbar_wait_warp(a_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
+                if (!ptx::mbar_wait_warp(a_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
                     if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const uint64_t x_stage = x_desc + xs * (kUmXBytes / 16);
+                const uint64_t x_stage = x_desc + as * (kUmXBytes / 16);
                 const uint32_t a_cols = tmem_base + kUmABase + as * kUmAStageCols;
                 if (ptx::elect_one()) {
 #pragma unroll
@@ -221,11 +213,9 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
                             ptx::umma_bf16_ts(tmem_base + t * 128, a_cols + t * 32 + k4 * 8, x_stage + k4 * 2, idesc, (first && k4 == 0) ? 0u : 1u);
                     }
                     ptx::umma_commit(a_empty + 8 * as);
-                    ptx::umma_commit(x_empty + 8 * xs);
                 }
                 __syncwarp();
                 if (++as == kUmAStages) { as = 0; aphase ^= 1; }
-                if (++xs == kUmXStages) { xs = 0; xphase ^= 1; }
             }
             if (ok && ptx::elect_one()) ptx::umma_commit(acc_full);
             __syncwarp();
