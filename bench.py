@@ -221,13 +221,13 @@ def run_hbm_workload(args, name, rt=None, brief=False):
                 # 32 independent problems per launch (distinct weights and outputs): t0_w4a16_gemm_tiled_grouped
                 for i in range(0, len(cs), 32):
                     rt.w4a16_gemm_tiled_grouped(cs[i:i + 32])
-            kernel = "w4a16_umma_ts_kernel over the column tiles of 32 problems per launch (tile-major weights, dequantised into tensor memory in the main loop of a tcgen05 GEMM)"
+            kernel = "w4a16_umma_cut_kernel over the column tiles of 32 problems per launch (tile-major weights, dequantised into tensor memory in the main loop of a tcgen05 GEMM)"
         elif M > 16:
             def submit(cs):
                 # 32 independent problems per launch (distinct weights and outputs): t0_w4a16_gemm_grouped
                 for i in range(0, len(cs), 32):
                     rt.w4a16_gemm_grouped(cs[i:i + 32])
-            kernel = "w4a16_umma_kernel over the column tiles of 32 problems per launch (row-layout weights, dequantisation in the main loop of a tcgen05 GEMM)"
+            kernel = "w4a16_umma_cut_kernel over the column tiles of 32 problems per launch (row-layout weights, dequantised into tensor memory in the main loop of a tcgen05 GEMM)"
         else:
             submit = rt.w4a16_gemm_batch
             kernel = "w4a16_tc_kernel (row layout, tcgen05)"

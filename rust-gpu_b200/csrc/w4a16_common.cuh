@@ -119,6 +119,10 @@ struct UmGroup {
     float* y[kUmMaxGroup];
 };
 
+// How a launch shares out its tiles: the parts of a tile's K over the CTAs of a cluster (one problem); whole tiles per CTA; equal ranges of the
+// list of chunks, tiles cut where ranges end.
+enum { kUmClusters, kUmWhole, kUmCut };
+
 // Trace buffer of the T0_W4_TRACE debugging aid: freed on every path out of the entry point that made it.
 struct StampBuffer {
     unsigned long long* d = nullptr;

@@ -1,5 +1,5 @@
-// K2 for several problems of one shape with M <= 128 whose column tiles do not fill the GPU evenly: the W4A16 GEMM on tcgen05 with the
-// dequantised weights as the tensor-memory operand (as w4a16_umma_ts_kernel in w4a16_umma.cu, which see), tiles cut between CTAs.
+// K2 for lists of problems of one shape with M <= 128 (and most single ones): the W4A16 GEMM on tcgen05 with the dequantised weights as the
+// tensor-memory operand, tiles taken whole or cut between CTAs.
 //
 // No counterpart kernel exists in the reference (its INT4 support stops at the stand-alone dequantisation kernels,
 // src/t0/quant_kernels.rs:53-171).  y[m,n] = sum_k a[m,k] * w[k,n],  w = RNE_bf16((q - z) * s),  fp32 accumulate.
@@ -17,9 +17,9 @@
 // reach it last: see the epilogue.
 //
 // Whole tiles per CTA leave SMs idle where the tiles are few or just over a multiple of them: two problems of N = 11008 are 86 tiles on 148
-// SMs.  M = 128, K = 4096: 43.7 us with whole tiles, 40.6 cut; M = 107, N = 7936, K = 4352: 45.0 and 33.5; M = 81, N = 2560, K = 7424, four
-// problems: 71.5 and 36.3.  What bounds it is the chain of waits around a chunk (0.67 us; arithmetic alone would take about 0.15) and, per
-// launch, about 10 us for handing in and adding the parts of cut tiles; `w4a16_umma_cut_applies` weighs the two.
+// SMs.  A launch takes its tiles whole or cut, or leaves a single problem to the clusters of w4a16_umma.cu: `w4a16_umma_plan` weighs them.
+// What bounds it is the dequantising warps' instructions and the waits around them (0.4 us a chunk, 0.5 at M = 128; the UMMAs of a chunk take
+// 0.27 there), and per launch with cut tiles 2 to 10 us for handing in and adding their parts.
 #include "w4a16_common.cuh"
 
 using namespace t0;
@@ -57,6 +57,7 @@ struct UmParams {
     uint32_t group;          // k per scale / zero-point row (a multiple of 64)
     uint32_t n_tiles, n_chunks;
     uint32_t total;          // chunks of the launch, shared out evenly (less than 2^24)
+    uint32_t whole;          // shared out by tiles instead: no tile is cut
 };
 
 __device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
@@ -67,7 +68,9 @@ __device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
 
 // First chunk of a CTA's range, and the CTA whose range holds a chunk: in 32 bits (at most 256 CTAs and 2^24 chunks), since a warp that
 // finishes a cut tile needs a few of these and a 64-bit division takes hundreds of cycles.
-__device__ __forceinline__ uint32_t um_begin(uint32_t cta, const UmParams& p) { return cta * p.total / gridDim.x; }
+__device__ __forceinline__ uint32_t um_begin(uint32_t cta, const UmParams& p) {
+    return p.whole ? cta * (p.total / p.n_chunks) / gridDim.x * p.n_chunks : cta * p.total / gridDim.x;
+}
 __device__ __forceinline__ uint32_t um_owner(uint32_t chunk, const UmParams& p) { return ((chunk + 1) * gridDim.x - 1) / p.total; }
 
 template <bool kTiled>    // weights in the tile-major layout (3-D maps: column in tile, row, tile), else the row layout
@@ -444,29 +447,34 @@ static uint32_t cut_grid(const t0_runtime* rt, uint64_t items, uint32_t n_chunks
     return grid;
 }
 
-// Whether the tiles of `count` problems are to be cut: where that beats whole tiles per CTA, in microseconds fitted at M = 128 and 32,
-// K = 1152 ... 7424, 32 to 516 tiles (a chunk takes about 0.65 us either way, a launch with cut tiles about 10 us more); where there is room for
-// their parts; and only in launches of the runtime's own stream, whose launches run one after the other: a recorded launch may be replayed
-// beside others, which would share its counters and parts.
-bool w4a16_umma_cut_applies(t0_runtime* rt, uint32_t N, uint32_t K, uint32_t count) {
+// How to share out the tiles of `count` problems: the fastest form, by times in microseconds fitted to M = 17 ... 128, 4 ... 516 tiles and
+// K = 1024 ... 8192.  A chunk takes 0.42 us at small M and 0.52 at M = 128 in either form of this kernel; handing in and adding parts adds 2 to 10 us
+// with M.  Measured, whole tiles / cut: 2 x (128 x 11008 x 4096) 36.6 / 34.1, 12 of them 142 / 140, 4 x (64 x 1024 x 2048) 18.0 / 13.1; one problem
+// as clusters / cut: 128 x 11008 x 4096 21.8 / 22.7, 32 x 11008 x 4096 21.3 / 15.6, 100 x 1024 x 2048 14.1 / 16.5, 20 x 14336 x 2048 19.6 / 13.1.
+// `cluster_split` > 1 is what the cluster form would take (one problem; it sums no longer a part of K than cut tiles do).  Cut tiles need room
+// for their parts, and run only in launches of the runtime's own stream, whose launches run one after the other: a recorded launch may be
+// replayed beside others, which would share its counters and parts.
+int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split) {
     const uint64_t items = (uint64_t)ceil_div(N, kUmBN) * count;
-    const uint32_t n_chunks = K / kUmBK, grid = cut_grid(rt, items, n_chunks);
-    if (items % grid == 0 || items * n_chunks >= (1u << 24)) return false;
-    const double whole = (double)((items + rt->sm_count - 1) / rt->sm_count) * n_chunks * 0.63 + 4.0;
-    const double cut = (double)items * n_chunks / grid * 0.67 + 14.4;
-    if (cut > 0.97 * whole) return false;
+    const uint32_t n_chunks = K / kUmBK, grid = cut_grid(rt, items, n_chunks), sms = (uint32_t)rt->sm_count;
+    const int other = cluster_split > 1 ? kUmClusters : kUmWhole;
+    if (items % grid == 0 || items * n_chunks >= (1u << 24)) return other;
+    const double chunk = 0.42 + 0.0008 * M;
+    const double cut = (double)items * n_chunks / grid * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0);
+    const double without = other == kUmClusters ? (double)ceil_div(n_chunks, cluster_split) * 0.495 + 10.2 : (double)((items + sms - 1) / sms) * n_chunks * chunk + 4.2;
+    if (cut > 0.97 * without) return other;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
-    if (w4a16_umma_reserve(rt) == T0_OK) return true;
-    cudaGetLastError();                    // (no memory for the parts: whole tiles need none)
-    return false;
+    if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return other;
+    if (w4a16_umma_reserve(rt) == T0_OK) return kUmCut;
+    cudaGetLastError();                    // (no memory for the parts: the other forms need none)
+    return other;
 }
 
 uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }
 
-// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape, for which
-// w4a16_umma_cut_applies.
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count) {
+// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.  `cut`: w4a16_umma_plan has
+// made room for the parts of cut tiles; otherwise every CTA takes whole tiles.
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, bool cut) {
     auto kern = tiled ? w4a16_umma_cut_kernel<true> : w4a16_umma_cut_kernel<false>;
     static bool attr_set[2][64] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
@@ -484,10 +492,14 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint
     p.n_tiles = ceil_div(N, kUmBN);
     p.n_chunks = K / kUmBK;
     const uint64_t items = (uint64_t)p.n_tiles * count;
-    const uint32_t grid = cut_grid(rt, items, p.n_chunks);
+    if (items * p.n_chunks > 0x7FFFFFFFull || items > (1u << 23)) return fail(T0_ERR_UNSUPPORTED, "too many tiles");
+    const uint32_t grid = cut ? cut_grid(rt, items, p.n_chunks) : (uint32_t)std::min<uint64_t>(items, std::min(rt->sm_count, 256));
     p.total = (uint32_t)(items * p.n_chunks);
-    p.counters = (uint32_t*)rt->scratch_um.ptr;
-    p.pieces = (float*)((uint8_t*)rt->scratch_um.ptr + kUmCounterBytes);
+    p.whole = cut ? 0 : 1;
+    if (cut) {
+        p.counters = (uint32_t*)rt->scratch_um.ptr;
+        p.pieces = (float*)((uint8_t*)rt->scratch_um.ptr + kUmCounterBytes);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(kUmThreads, 1, 1);

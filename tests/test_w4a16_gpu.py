@@ -545,6 +545,13 @@ def test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, count):
         b.free()
 
 
+# what the plan of a launch makes of these: a single problem cut between CTAs, and as clusters; whole tiles (one chunk of K, more tiles than SMs);
+# several problems cut, the last tile ragged
+@pytest.mark.parametrize("M,K,N,G,count", [(20, 2048, 14344, 128, 1), (128, 2048, 2560, 128, 1), (16, 64, 38144, 64, 1), (33, 1024, 2312, 64, 3)])
+def test_tiled_forms_of_a_launch(t0, oracle, rt, M, K, N, G, count):
+    test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, count)
+
+
 def test_tiled_grouped_dequantises_bit_exactly(t0, oracle, rt):
     # one-hot activations through the grouped launch (weights as the tensor-memory operand): row m of y is row base + m of the
     # dequantised weights, exactly
