@@ -101,15 +101,17 @@ static std::vector<Candidate> schedule(uint32_t m, uint32_t n, uint32_t k) {
     return out;
 }
 
-// Microseconds of one launch among others, fitted to measurements of every kernel alone (2048 x 1024 x 4096 ... 256^3, both layouts, one
-// to four rounds of tiles): a launch's fixed part (prologue, first operands, last epilogue, exit), the k blocks of the longest CTA, and
+// Microseconds of one launch among others, fitted to measurements of every kernel alone (38 shapes of 128 ... 11008 a side, both layouts,
+// one to five rounds of tiles; 6 to 9 % off on average): a launch's fixed part (prologue, first operands, last epilogue, exit), the k blocks of the longest CTA, and
 // per round what of its epilogue stays exposed.  With K in parts there is one round, and instead the exchange in the clusters: longer with
 // the rows and columns of a tile, a little with every part, and a launch that leaves half of the SMs to the next one's prologue is
-// shorter (49 shapes of 16 to 1500 rows, both layouts: the choice is 1 % above the best one on average, 13 % at most).  The search above
+// shorter.  The pair's 256 x 128 tile takes in 24 KB a k block where the 128 x 128 tiles of two CTAs take 32: 2048 x 1024 x 4096 22.1 -> 20.3 us,
+// 1664 x 1056 x 3248 18.6 -> 17.4.  The search above
 // scores whole configurations for the public entry points; its split-K entries stand for the two-launch and cluster forms.
 GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once) {
     struct Fit { uint32_t tile_n; double fixed, kblock, round, exchange; };
-    static const Fit single[] = {{256, 5.5, 0.40, 1.0, 0.0}, {128, 4.8, 0.31, 0.4, 2.9}, {64, 4.4, 0.28, 0.2, 1.1}, {32, 4.4, 0.26, 0.1, 0.5}};
+    static const Fit single[] = {{256, 3.0, 0.383, 3.8, 0.0}, {128, 3.2, 0.269, 1.9, 2.9}, {64, 3.3, 0.247, 0.8, 1.1}, {32, 3.3, 0.240, 0.5, 0.5}};
+    static const Fit pair[] = {{256, 3.5, 0.334, 3.8, 0.0}, {128, 3.3, 0.220, 2.5, 0.0}};
     const double tile_rows = std::min(128u, ceil_div(m, 32) * 32) / 128.0;
     const uint32_t kb = ceil_div(k, 64);
     const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + 4.0 * (double)m * n) / 6.0e6;
@@ -119,12 +121,15 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min
         us = std::max(us, 4.0 + bytes_us);
         if (us < best_us) { best_us = us; best = c; }
     };
-    if (m > 128 && n > 128 && min_split <= 1) {
-        // 256 x 256 per pair; the tiles of a last wave that at most half fills the GPU are cut in two
+    for (const Fit& f : pair) {
+        // 256 x 256 or 256 x 128 per pair; the tiles of a last wave that at most half fills the GPU are cut in two (not 128 wide over B[K,N])
+        if (m <= 128 || n <= 128 || min_split > 256 / f.tile_n) continue;
         const uint32_t pairs = n_sms / 2;
-        const uint64_t tiles = (uint64_t)ceil_div(m, 256) * ceil_div(n, 256), rest = tiles % pairs;
-        const double rounds = (double)(tiles / pairs) + (rest == 0 ? 0.0 : (2 * rest <= pairs && tiles > pairs) ? 0.55 : 1.0);
-        consider(6.7 + rounds * (kb * 0.36 + 0.8), {256, 1, true, false});
+        const uint64_t tiles = (uint64_t)ceil_div(m, 256) * ceil_div(n, f.tile_n), rest = tiles % pairs;
+        const bool cut = 2 * rest <= pairs && tiles > pairs && !(nn && f.tile_n == 128);
+        const double rounds = (double)(tiles / pairs) + (rest == 0 ? 0.0 : cut ? 0.55 : 1.0);
+        const bool halves = f.tile_n == 128 && (min_split > 1 || (tiles <= pairs && kb >= 32));
+        consider(f.fixed + rounds * (kb * f.kblock + f.round), {f.tile_n, 1, true, halves});
     }
     for (const Fit& f : single) {
         if (f.tile_n > 32 && n <= f.tile_n / 2) continue;           // more than half of the tile would be beyond N
@@ -137,8 +142,8 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min
             // they cost a launch of one round under 1 %.
             const bool halves = f.tile_n <= 128 && (parts < min_split || parts > 1 || (tiles <= n_sms && kb >= (2 * tiles <= n_sms ? 8u : 32u)));
             const double us = parts == 1 ? f.fixed + std::ceil((double)tiles / n_sms) * (kb * f.kblock + f.round)
-                                         : 5.8 + ceil_div(kb, parts) * 0.293 + 0.16 * parts + tile_rows * f.exchange;
-            const double overlap = 2 * tiles * parts > n_sms ? 0.0 : parts == 1 ? 0.6 : 1.0;
+                                         : 5.8 + ceil_div(kb, parts) * 0.270 + 0.16 * parts + tile_rows * f.exchange;
+            const double overlap = 2 * tiles * parts > n_sms ? 0.0 : parts == 1 ? 0.3 : 1.0;
             consider(us - overlap, {f.tile_n, parts, false, halves});
         }
     }

@@ -260,6 +260,20 @@ __device__ __forceinline__ void store_chunk(const KParams& p, const uint32_t (&r
     __syncwarp();
 }
 
+// 32 columns of a warp's rows of the accumulator, of both where there are two.
+template <uint32_t BN>
+__device__ __forceinline__ void load_acc(uint32_t taddr, bool two_accs, uint32_t (&r)[32]) {
+    ptx::tmem_ld_32x32b_x32(taddr, r);
+    ptx::tmem_ld_wait();
+    if (two_accs) {                                    // warp-uniform
+        uint32_t r2[32];
+        ptx::tmem_ld_32x32b_x32(taddr + BN, r2);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+    }
+}
+
 // ------------------------------------------------------------------ launch (host)
 
 // Launch with programmatic stream serialisation so the prologue of this grid overlaps the tail of the

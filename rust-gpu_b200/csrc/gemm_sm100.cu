@@ -42,20 +42,6 @@ template <uint32_t kAccs>
 __device__ __forceinline__ uint32_t k_mid(const KRange& kr, const KParams& p) {
     return kAccs == 2 && p.halves ? kr.first + (kr.end - kr.first + 1) / 2 : kr.end;
 }
-// 32 columns of a warp's rows of the accumulator, of both where there are two.
-template <uint32_t BN>
-__device__ __forceinline__ void load_acc(uint32_t taddr, bool two_accs, uint32_t (&r)[32]) {
-    ptx::tmem_ld_32x32b_x32(taddr, r);
-    ptx::tmem_ld_wait();
-    if (two_accs) {                                    // warp-uniform
-        uint32_t r2[32];
-        ptx::tmem_ld_32x32b_x32(taddr + BN, r2);
-        ptx::tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
-    }
-}
-
 // Four columns of one row of the result.
 __device__ __forceinline__ void store4(const KParams& p, bool vec, uint32_t row, uint32_t col, const float (&o)[4]) {
     if (row >= p.M) return;

@@ -38,7 +38,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
     constexpr uint32_t kBStageBytes = kBHalfRows * BK * 2;
     constexpr uint32_t kStageBytes = kAStageBytes + kBStageBytes;  // per CTA
     constexpr uint32_t kStages = pair_stages(kPairN);
-    constexpr uint32_t kTmemCols = 2 * kPairN;                     // two accumulator buffers
+    // Two accumulator buffers; 128 columns wide a buffer holds two accumulators: with p.halves the first and second half of the k blocks are
+    // summed apart and added in f32 by the epilogue, as in gemm_sm100.cu.
+    constexpr uint32_t kAccs = kPairN == 128 ? 2 : 1;
+    constexpr uint32_t kTmemCols = 2 * kPairN * kAccs;
     constexpr uint32_t kIdesc = ptx::make_idesc_bf16_f32(kPairM, kPairN, B_MN ? 1u : 0u, A_MN ? 1u : 0u);
     // Tail of the tile list: when the last wave would leave more than half of the pairs idle, its tiles are cut into two
     // half-width tiles (work items >= p.tail_start; item tail_start + 2i + h is half h of tile tail_start + i), so the wave
@@ -68,6 +71,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
     const uint32_t n_tiles = p.tiles_m * p.tiles_n * p.split_k;
     const uint32_t tail_start = min(p.tail_start, n_tiles);
     const uint32_t total_work = tail_start + 2 * (n_tiles - tail_start);
+    const uint32_t kb_mid = kAccs == 2 && p.halves ? (p.kb_per_split + 1) / 2 : p.kb_per_split;     // first k block of the second accumulator
 
     if (threadIdx.x == 0) {
         trace_stamp(p, 0);
@@ -165,7 +169,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const uint32_t tmem_d = tmem_base + buf * kPairN;
+                uint32_t tmem_d = tmem_base + buf * kPairN * kAccs;
                 const uint32_t idesc = w >= tail_start ? kIdescHalf : kIdesc;
                 for (uint32_t kb = 0; kb < p.kb_per_split; ++kb) {
                     if (!ptx::mbar_wait_warp(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
@@ -174,6 +178,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                         break;
                     }
                     ptx::tc_fence_after_sync();
+                    if (kb == kb_mid) tmem_d += kPairN;
                     if (ptx::elect_one()) {
                         if (kb == 0 && w == pair_id) trace_stamp(p, 3);
                         const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
@@ -185,7 +190,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                             // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
                             const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
                                                      : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
-                            ptx::umma_bf16_ss_pair(tmem_d, da, db, idesc, (kb | k4) != 0 ? 1u : 0u);
+                            ptx::umma_bf16_ss_pair(tmem_d, da, db, idesc, ((kb != 0 && kb != kb_mid) || k4 != 0) ? 1u : 0u);
                         }
                         // the stage is free in both CTAs once these UMMAs have read it
                         const uint32_t eb = ptx::smem_u32(&empty_bar[stage]);
@@ -225,8 +230,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const _
                 const uint32_t col0 = wi.n_blk * kPairN + half * kHalfN + c * 32;
                 if (col0 >= p.N) break;
                 uint32_t r[32];
-                ptx::tmem_ld_32x32b_x32(tmem_base + ((quarter * 32) << 16) + buf * kPairN + c * 32, r);
-                ptx::tmem_ld_wait();
+                load_acc<kPairN>(tmem_base + ((quarter * 32) << 16) + buf * kPairN * kAccs + c * 32, kb_mid < p.kb_per_split, r);
                 store_chunk(p, r, row_base, lane, c, col0, wi.split, epi_stage + quarter * 2 * kEpiStageBytes, n_stores, p.tma_store ? &map_y : nullptr);
             }
             ptx::tc_fence_before_sync();
@@ -331,6 +335,7 @@ int launch_gemm_sm100_pair(const GemmLaunch& g, cudaStream_t stream) {
     p.M = g.m; p.N = g.n; p.K = g.k;
     p.tiles_m = ceil_div(g.m, kPairM); p.tiles_n = ceil_div(g.n, pair_n); p.split_k = split;
     p.kb_per_split = ceil_div(kps, BK);
+    p.halves = g.halves ? 1 : 0;
     p.swap_grid = g.swap_grid ? 1 : 0; p.raster_group = 8;
     p.out_bf16 = g.out_bf16 ? 1 : 0; p.epilogue = g.epilogue; p.n_ops = g.n_ops;
     p.scale = g.scale; p.clamp_min = g.clamp_min; p.clamp_max = g.clamp_max;

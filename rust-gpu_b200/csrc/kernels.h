@@ -21,7 +21,7 @@ struct GemmLaunch {
     uint32_t tile_n;      // 32/64/128/256
     uint32_t split_k;     // >= 1
     bool cluster;         // single-CTA kernel, 1 < split_k <= kMaxClusterParts: the parts meet in clusters, the result is complete in y
-    bool halves;          // single-CTA kernel, tile_n <= 128: sums of half the length, added in f32
+    bool halves;          // tile_n <= 128: sums of half the length, added in f32
     uint64_t plane_stride;  // elements between split planes
     bool nn, out_bf16, swap_grid;
     bool at;              // x is given transposed, [K,M] with M contiguous (row stride ldx, 0 = M); only together with nn
