@@ -238,13 +238,13 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
         uint32_t rs = 0, rphase = 0, as = h, aphase = 0, piece = 0;
         bool ok = true;
 
-        // 16 columns of the accumulator (rows m0.. of y) for this warp's columns of y
-        auto load_rows = [&](uint32_t m0, float (&v)[16]) {
-            uint32_t r[16];
-            ptx::tmem_ld_32x32b_x16(tmem_base + lane_base + t * 128 + m0, r);
+        // 32 columns of the accumulator (rows m0.. of y) for this warp's columns of y; a narrow tile's columns beyond its rows are not used
+        auto load_rows = [&](uint32_t m0, float (&v)[32]) {
+            uint32_t r[32];
+            ptx::tmem_ld_32x32b_x32(tmem_base + lane_base + t * 128 + m0, r);
             ptx::tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
         };
         // partial sums of a cut tile: each warp's own block of a piece, four rows of a column per float4
         const uint32_t row4s = p.rows / 8;                                   // float4s a lane holds
@@ -322,11 +322,11 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
             if (ticket + 1 != n_parts) {
                 float4* mine = my_block + ((size_t)blockIdx.x * 2 + (piece == 0 ? 0 : 1)) * piece_f4;
 #pragma unroll 1
-                for (uint32_t i = 0; i < row4s; i += 4) {
-                    float v[16];
+                for (uint32_t i = 0; i < row4s; i += 8) {
+                    float v[32];
                     load_rows(m_begin + 4 * i, v);
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j)
+                    for (uint32_t j = 0; j < 8; ++j)
                         if (i + j < row4s) __stcg(mine + (i + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
                 }
                 ptx::tc_fence_before_sync();
@@ -359,43 +359,39 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
             const uint32_t prob = item / p.n_tiles;
             float* const y_out = group.y[prob];
             const uint32_t col = (item - prob * p.n_tiles) * kUmBN + n;
+            // Thirty-two rows at a time, part after part in k order.  What this costs is the round trips of the parts' loads, so eight of a lane's
+            // 16-byte loads are under way together: two problems of M = 128, N = 11008 31.7 us with sixteen rows of two parts at a time, 29.7 so;
+            // M = 40, N = 2560 16.2 and 15.2; M = 64, N = 14336, three problems 40.8 and 39.0.  (Where a warp has eight to sixteen rows the former is
+            // faster, 9.1 against 9.5 us at M = 17, N = 1024; both side by side make the loop above slower than either gains.)
 #pragma unroll 1
-            for (uint32_t i = 0; i < row4s; i += 4) {
+            for (uint32_t i = 0; i < row4s; i += 8) {
                 const uint32_t m0 = m_begin + 4 * i;
-                float sum[16];
+                float sum[32];
                 if (n_parts == 1) load_rows(m0, sum);
                 if (n_parts > 1) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 16; ++j) sum[j] = 0.0f;
+                    for (uint32_t j = 0; j < 32; ++j) sum[j] = 0.0f;
 #pragma unroll 1
-                    for (uint32_t part = 0; part < n_parts; part += 2) {
-                        // the loads of two parts are under way together
-                        float f[2][16];
+                    for (uint32_t part = 0; part < n_parts; ++part) {
+                        float f[32];
+                        const uint32_t cta = c_first + part;
+                        if (cta == blockIdx.x) {
+                            load_rows(m0, f);
+                        } else {
+                            const float4* theirs = my_block + ((size_t)cta * 2 + (part == 0 ? first_slot : 0u)) * piece_f4;
 #pragma unroll
-                        for (uint32_t k = 0; k < 2; ++k) {
-                            const uint32_t cta = c_first + part + k;
-                            if (cta == blockIdx.x) {
-                                load_rows(m0, f[k]);
-                            } else if (part + k < n_parts) {
-                                const float4* theirs = my_block + ((size_t)cta * 2 + (part + k == 0 ? first_slot : 0u)) * piece_f4;
-#pragma unroll
-                                for (uint32_t j = 0; j < 4; ++j) {
-                                    const float4 x = i + j < row4s ? __ldcg(theirs + (i + j) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-                                    f[k][4 * j] = x.x; f[k][4 * j + 1] = x.y; f[k][4 * j + 2] = x.z; f[k][4 * j + 3] = x.w;
-                                }
+                            for (uint32_t j = 0; j < 8; ++j) {
+                                const float4 x = i + j < row4s ? __ldcg(theirs + (i + j) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                                f[4 * j] = x.x; f[4 * j + 1] = x.y; f[4 * j + 2] = x.z; f[4 * j + 3] = x.w;
                             }
                         }
 #pragma unroll
-                        for (uint32_t k = 0; k < 2; ++k) {
-                            if (part + k >= n_parts) break;
-#pragma unroll
-                            for (uint32_t j = 0; j < 16; ++j) sum[j] += f[k][j];
-                        }
+                        for (uint32_t j = 0; j < 32; ++j) sum[j] += f[j];
                     }
                 }
                 if (col < p.N) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 16; ++j)
+                    for (uint32_t j = 0; j < 32; ++j)
                         if (m0 + j < m_end) y_out[(size_t)(m0 + j) * p.N + col] = sum[j];
                 }
             }
