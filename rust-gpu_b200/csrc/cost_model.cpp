@@ -108,13 +108,16 @@ static std::vector<Candidate> schedule(uint32_t m, uint32_t n, uint32_t k) {
 // shorter.  The pair's 256 x 128 tile takes in 24 KB a k block where the 128 x 128 tiles of two CTAs take 32: 2048 x 1024 x 4096 22.1 -> 20.3 us,
 // 1664 x 1056 x 3248 18.6 -> 17.4.  The search above
 // scores whole configurations for the public entry points; its split-K entries stand for the two-launch and cluster forms.
-GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once) {
+GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf16, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once) {
     struct Fit { uint32_t tile_n; double fixed, kblock, round, exchange; };
     static const Fit single[] = {{256, 3.0, 0.383, 3.8, 0.0}, {128, 3.2, 0.269, 1.9, 2.9}, {64, 3.3, 0.247, 0.8, 1.1}, {32, 3.3, 0.240, 0.5, 0.5}};
     static const Fit pair[] = {{256, 3.5, 0.334, 3.8, 0.0}, {128, 3.3, 0.220, 2.5, 0.0}};
     const double tile_rows = std::min(128u, ceil_div(m, 32) * 32) / 128.0;
     const uint32_t kb = ceil_div(k, 64);
-    const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + 4.0 * (double)m * n) / 6.0e6;
+    // A bf16 result is half as much to write, and a good part of what a round leaves exposed is that, more so of the narrow single tiles
+    // (3048 x 1664 x 192 in bf16: single 128 9.0 us, pair 256 10.0, pair 128 10.5; 1024 x 4096 x 512: 9.6, 10.1, 10.3).
+    auto round_share = [&](uint32_t tile_n, bool pair) { return !out_bf16 ? 1.0 : pair || tile_n == 256 ? 0.8 : 0.65; };
+    const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + (out_bf16 ? 2.0 : 4.0) * (double)m * n) / 6.0e6;
     GemmChoice best = {0, 0, false, false};
     double best_us = 1e30;
     auto consider = [&](double us, GemmChoice c) {
@@ -129,7 +132,7 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min
         const bool cut = 2 * rest <= pairs && tiles > pairs && !(nn && f.tile_n == 128);
         const double rounds = (double)(tiles / pairs) + (rest == 0 ? 0.0 : cut ? 0.55 : 1.0);
         const bool halves = f.tile_n == 128 && (min_split > 1 || (tiles <= pairs && kb >= 32));
-        consider(f.fixed + rounds * (kb * f.kblock + f.round), {f.tile_n, 1, true, halves});
+        consider(f.fixed + rounds * (kb * f.kblock + f.round * round_share(f.tile_n, true)), {f.tile_n, 1, true, halves});
     }
     for (const Fit& f : single) {
         if (f.tile_n > 32 && n <= f.tile_n / 2) continue;           // more than half of the tile would be beyond N
@@ -141,7 +144,7 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, uint32_t min
             // Two accumulators (up to 128 columns, double-buffered, they fill tensor memory) where the sums have to be shorter, and wherever
             // they cost a launch of one round under 1 %.
             const bool halves = f.tile_n <= 128 && (parts < min_split || parts > 1 || (tiles <= n_sms && kb >= (2 * tiles <= n_sms ? 8u : 32u)));
-            const double us = parts == 1 ? f.fixed + std::ceil((double)tiles / n_sms) * (kb * f.kblock + f.round)
+            const double us = parts == 1 ? f.fixed + std::ceil((double)tiles / n_sms) * (kb * f.kblock + f.round * round_share(f.tile_n, false))
                                          : 5.8 + ceil_div(kb, parts) * 0.270 + 0.16 * parts + tile_rows * f.exchange;
             const double overlap = 2 * tiles * parts > n_sms ? 0.0 : parts == 1 ? 0.3 : 1.0;
             consider(us - overlap, {f.tile_n, parts, false, halves});

@@ -53,7 +53,7 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
         GemmChoice choice = {};
         if (!forced) {
             const uint32_t s = known && c.split_k > 1 && q.k % c.split_k == 0 ? c.split_k : 1;
-            choice = choose_gemm(q.m, q.n, q.k, q.nn, s, (uint32_t)rt->sm_count, gemm_clusters_at_once());
+            choice = choose_gemm(q.m, q.n, q.k, q.nn, q.out_bf16, s, (uint32_t)rt->sm_count, gemm_clusters_at_once());
         }
         if (choice.parts) {
             q.tile_n = choice.tile_n;
