@@ -307,7 +307,7 @@ w4a16_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 const uint32_t s_begin = split * slice_w, s_end = min(kUmBN, s_begin + slice_w);
                 const uint32_t f4_per_row = s_end > s_begin ? (s_end - s_begin) / 4 : 0;
                 const uint32_t items = 128 * f4_per_row;
-                const bool vec = ((uintptr_t)p.y & 15) == 0;         // (N % 32 == 0 is a condition of this kernel)
+                const bool vec = ((uintptr_t)p.y & 15) == 0 && p.N % 4 == 0;   // (any N with tile-major weights)
                 constexpr uint32_t kU = 2;
                 for (uint32_t i0 = tid; i0 < items; i0 += kU * kUmDqWarps * 32) {
                     float4 part[kU][4];

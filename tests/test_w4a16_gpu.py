@@ -552,6 +552,13 @@ def test_tiled_forms_of_a_launch(t0, oracle, rt, M, K, N, G, count):
     test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, count)
 
 
+# Tile-major weights take any N.  One problem as clusters: rows of y start 4 and 8 bytes off a 16-byte boundary; the last tile ragged, N below a tile, below
+# eight columns; K too short for more than one part.
+@pytest.mark.parametrize("M,K,N,G", [(128, 1024, 1030, 128), (100, 1024, 1001, 128), (33, 512, 255, 64), (128, 1024, 7, 128), (17, 64, 1030, 64)])
+def test_tiled_weights_any_n(t0, oracle, rt, M, K, N, G):
+    test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, 1)
+
+
 def test_tiled_grouped_dequantises_bit_exactly(t0, oracle, rt):
     # one-hot activations through the grouped launch (weights as the tensor-memory operand): row m of y is row base + m of the
     # dequantised weights, exactly
