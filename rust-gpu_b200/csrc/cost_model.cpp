@@ -108,23 +108,50 @@ static std::vector<Candidate> schedule(uint32_t m, uint32_t n, uint32_t k) {
 // shorter.  The pair's 256 x 128 tile takes in 24 KB a k block where the 128 x 128 tiles of two CTAs take 32: 2048 x 1024 x 4096 22.1 -> 20.3 us,
 // 1664 x 1056 x 3248 18.6 -> 17.4.  The search above
 // scores whole configurations for the public entry points; its split-K entries stand for the two-launch and cluster forms.
-GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf16, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once) {
-    struct Fit { uint32_t tile_n; double fixed, kblock, round, exchange; };
-    static const Fit single[] = {{256, 3.0, 0.383, 3.8, 0.0}, {128, 3.2, 0.269, 1.9, 2.9}, {64, 3.3, 0.247, 0.8, 1.1}, {32, 3.3, 0.240, 0.5, 0.5}};
-    static const Fit pair[] = {{256, 3.5, 0.334, 3.8, 0.0}, {128, 3.3, 0.220, 2.5, 0.0}};
-    const double tile_rows = std::min(128u, ceil_div(m, 32) * 32) / 128.0;
-    const uint32_t kb = ceil_div(k, 64);
+struct Fit { uint32_t tile_n; double fixed, kblock, round, exchange; };
+struct ChoiceFit {
+    Fit pair[2], single[4];
+    double part_kblock, overlap;       // a k block of a part; what the next launch's prologue saves an uncut launch on half of the SMs
     // A bf16 result is half as much to write, and a good part of what a round leaves exposed is that, more so of the narrow single tiles
     // (3048 x 1664 x 192 in bf16: single 128 9.0 us, pair 256 10.0, pair 128 10.5; 1024 x 4096 x 512: 9.6, 10.1, 10.3).
-    auto round_share = [&](uint32_t tile_n, bool pair) { return !out_bf16 ? 1.0 : pair || tile_n == 256 ? 0.8 : 0.65; };
+    double bf16_wide, bf16_narrow;
+};
+static constexpr ChoiceFit kTimes = {{{256, 3.5, 0.334, 3.8, 0.0}, {128, 3.3, 0.220, 2.5, 0.0}},
+                                     {{256, 3.0, 0.383, 3.8, 0.0}, {128, 3.2, 0.269, 1.9, 2.9}, {64, 3.3, 0.247, 0.8, 1.1}, {32, 3.3, 0.240, 0.5, 0.5}},
+                                     0.270, 0.3, 0.8, 0.65};
+// How long a sum may be is not for the times to decide.  The tensor cores' error grows with the length of an accumulation, so a shape whose K is cut,
+// or summed in two accumulators, does not lose that to a kernel that is somewhat faster.  By the times alone 1352 x 248 x 1672 would run as one sum of 27 k
+// blocks where it had 5: 10.4 us instead of 12.4, and 1.5e-6 off the exact result instead of 2.2e-7; 64 x 4992 x 1096, B[K,N], 10.3 instead of 10.0 us
+// and 9.3e-7 instead of 1.5e-7.  This fit, of the kernels before their serial roles walked converged, sets the length and is kept for that
+// alone: it does not follow the times.
+static constexpr ChoiceFit kSums = {{{256, 6.7, 0.36, 0.8, 0.0}, {128, 1e30, 0.0, 0.0, 0.0}},
+                                    {{256, 5.5, 0.40, 1.0, 0.0}, {128, 4.8, 0.31, 0.4, 2.9}, {64, 4.4, 0.28, 0.2, 1.1}, {32, 4.4, 0.26, 0.1, 0.5}},
+                                    0.293, 0.6, 1.0, 1.0};
+
+// k blocks of the longest accumulation of a choice.
+static uint32_t sum_blocks(const GemmChoice& c, uint32_t kb) {
+    const uint32_t part = ceil_div(kb, c.parts);
+    return c.halves ? (part + 1) / 2 : part;
+}
+
+// The fastest choice by `fit` none of whose sums is longer than `longest` k blocks.
+static GemmChoice search_choice(const ChoiceFit& fit, uint32_t longest, uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf16, uint32_t min_split, uint32_t n_sms,
+                                const uint32_t* clusters_at_once) {
+    const double tile_rows = std::min(128u, ceil_div(m, 32) * 32) / 128.0;
+    const uint32_t kb = ceil_div(k, 64);
+    auto round_share = [&](uint32_t tile_n, bool pair) { return !out_bf16 ? 1.0 : pair || tile_n == 256 ? fit.bf16_wide : fit.bf16_narrow; };
     const double bytes_us = (2.0 * m * k + 2.0 * (double)n * k + (out_bf16 ? 2.0 : 4.0) * (double)m * n) / 6.0e6;
     GemmChoice best = {0, 0, false, false};
     double best_us = 1e30;
     auto consider = [&](double us, GemmChoice c) {
+        if (sum_blocks(c, kb) > longest) {
+            c.halves = c.tile_n <= 128;
+            if (sum_blocks(c, kb) > longest) return;
+        }
         us = std::max(us, 4.0 + bytes_us);
         if (us < best_us) { best_us = us; best = c; }
     };
-    for (const Fit& f : pair) {
+    for (const Fit& f : fit.pair) {
         // 256 x 256 or 256 x 128 per pair; the tiles of a last wave that at most half fills the GPU are cut in two (not 128 wide over B[K,N])
         if (m <= 128 || n <= 128 || min_split > 256 / f.tile_n) continue;
         const uint32_t pairs = n_sms / 2;
@@ -134,7 +161,7 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf1
         const bool halves = f.tile_n == 128 && (min_split > 1 || (tiles <= pairs && kb >= 32));
         consider(f.fixed + rounds * (kb * f.kblock + f.round * round_share(f.tile_n, true)), {f.tile_n, 1, true, halves});
     }
-    for (const Fit& f : single) {
+    for (const Fit& f : fit.single) {
         if (f.tile_n > 32 && n <= f.tile_n / 2) continue;           // more than half of the tile would be beyond N
         if (nn && f.tile_n < 64) continue;                          // B[K,N] boxes are 64 columns wide
         const uint64_t tiles = (uint64_t)ceil_div(m, 128) * ceil_div(n, f.tile_n);
@@ -145,12 +172,18 @@ GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf1
             // they cost a launch of one round under 1 %.
             const bool halves = f.tile_n <= 128 && (parts < min_split || parts > 1 || (tiles <= n_sms && kb >= (2 * tiles <= n_sms ? 8u : 32u)));
             const double us = parts == 1 ? f.fixed + std::ceil((double)tiles / n_sms) * (kb * f.kblock + f.round * round_share(f.tile_n, false))
-                                         : 5.8 + ceil_div(kb, parts) * 0.270 + 0.16 * parts + tile_rows * f.exchange;
-            const double overlap = 2 * tiles * parts > n_sms ? 0.0 : parts == 1 ? 0.3 : 1.0;
+                                         : 5.8 + ceil_div(kb, parts) * fit.part_kblock + 0.16 * parts + tile_rows * f.exchange;
+            const double overlap = 2 * tiles * parts > n_sms ? 0.0 : parts == 1 ? fit.overlap : 1.0;
             consider(us - overlap, {f.tile_n, parts, false, halves});
         }
     }
     return best;
+}
+
+GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf16, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once) {
+    const uint32_t kb = ceil_div(k, 64);
+    const GemmChoice sums = search_choice(kSums, kb, m, n, k, nn, false, min_split, n_sms, clusters_at_once);
+    return search_choice(kTimes, sums.parts ? sum_blocks(sums, kb) : kb, m, n, k, nn, out_bf16, min_split, n_sms, clusters_at_once);
 }
 
 static t0_gemm_config legacy(uint32_t m, uint32_t k, uint32_t n) {

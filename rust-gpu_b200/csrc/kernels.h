@@ -76,7 +76,8 @@ struct GemmChoice {
     bool pair, halves;
 };
 // No accumulation is longer than k / min_split: the tensor cores' error grows with the length of the sum (about 1e-9 of the result per
-// term), so a shape whose configuration (auto_select) cuts K keeps sums at least that short, in parts or in two accumulators.  parts = 0:
+// term), so a shape whose configuration (auto_select) cuts K keeps sums at least that short, in parts or in two accumulators.  Nor is one longer than
+// the library has made it for the shape before (kSums in cost_model.cpp).  parts = 0:
 // nothing here does that (many tiles and a deep cut); the configuration itself is to be taken.
 GemmChoice choose_gemm(uint32_t m, uint32_t n, uint32_t k, bool nn, bool out_bf16, uint32_t min_split, uint32_t n_sms, const uint32_t* clusters_at_once);
 
