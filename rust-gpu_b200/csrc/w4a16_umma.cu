@@ -422,9 +422,9 @@ __global__ void w4_to_tiled_kernel(const uint32_t* __restrict__ packed, const ui
 namespace t0 {
 
 // w4a16_umma_cut.cu
-int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split);
+int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas);
 uint32_t w4a16_umma_cut_rows(uint32_t M);
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, bool cut);
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas);
 
 static t0_w4a16_args um_args(uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t y, uint32_t M, uint32_t N, uint32_t K, uint32_t group) {
     t0_w4a16_args q;
@@ -519,7 +519,7 @@ static UmParams um_params(t0_runtime* rt, uint64_t a, uint64_t y, uint32_t M, ui
 
 // Problems of one shape on the kernel that takes whole tiles or cuts them (w4a16_umma_cut.cu); `count` problems in one launch, which run
 // concurrently.  Tile-major weights, or the row layout.
-static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count, bool tiled, int plan) {
+static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count, bool tiled, uint32_t cut_ctas) {
     const t0_w4a16_args& a0 = args[0];
     static UmGroup grp;                  // 16.9 KB: kept off the stack, filled under the lock, copied by the launch
     static std::mutex grp_mu;
@@ -532,15 +532,16 @@ static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t co
         if (rc != T0_OK) return rc;
         grp.y[i] = (float*)a.y;
     }
-    return launch_w4a16_umma_cut(rt, grp, tiled, a0.m, a0.n, a0.k, a0.group, count, plan == kUmCut);
+    return launch_w4a16_umma_cut(rt, grp, tiled, a0.m, a0.n, a0.k, a0.group, count, cut_ctas);
 }
 
 static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
     // as many parts of K as fill the machine (the parts of a tile form a cluster of at most four CTAs)
     const uint32_t n_tiles = ceil_div(a.n, kUmBN);
     const uint32_t split = std::min(std::max<uint32_t>(1, std::min<uint32_t>(4, (uint32_t)rt->sm_count / std::max<uint32_t>(1, n_tiles))), a.k / kUmBK);
-    const int plan = w4a16_umma_plan(rt, a.m, a.n, a.k, 1, split);
-    if (plan != kUmClusters) return um_launch_list(rt, &a, 1, tiled, plan);
+    uint32_t ctas;
+    const int plan = w4a16_umma_plan(rt, a.m, a.n, a.k, 1, split, &ctas);
+    if (plan != kUmClusters) return um_launch_list(rt, &a, 1, tiled, plan == kUmCut ? ctas : 0);
     UmParams p = um_params(rt, a.a, a.y, a.m, a.n, a.k, a.group);
     p.tiled = tiled ? 1 : 0;
     CUtensorMap m4[4];
@@ -570,7 +571,9 @@ static int um_launch_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_t
         if (!(tiled ? um_tiled_supported(a.a, a.packed, a.y, a.m, a.n, a.k, a.group) : w4a16_umma_supported(a.a, a.packed, a.scales, a.zeros, a.y, a.m, a.n, a.k, a.group)))
             return fail(T0_ERR_UNSUPPORTED, "grouped launch: problem %u is not a shape of the fused tcgen05 kernel", i);
     }
-    return um_launch_list(rt, args, count, tiled, w4a16_umma_plan(rt, a0.m, a0.n, a0.k, count, 1));
+    uint32_t ctas;
+    const int plan = w4a16_umma_plan(rt, a0.m, a0.n, a0.k, count, 0, &ctas);
+    return um_launch_list(rt, args, count, tiled, plan == kUmCut ? ctas : 0);
 }
 
 int launch_w4a16_umma_tiled_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count) { return um_launch_grouped(rt, args, count, true); }

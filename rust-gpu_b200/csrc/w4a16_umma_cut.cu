@@ -44,7 +44,7 @@ constexpr uint32_t kUmAStages = 4;                          // operand stages: w
 constexpr uint32_t kUmRawStages = 7;                        // raw weight stages of two chunks: 124 KB in flight per SM
 // (more than half an SM's shared memory: the kernel takes all 512 tensor-memory columns, so two of its CTAs must never share an SM)
 constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmAStages * kUmXBytes + 512 + 1024;
-constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long: below it the finish costs more than the range
+constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long where sums may be: below it the finish costs more than the range
 constexpr size_t kUmCounterBytes = 16 * 1024;               // one word per CTA and dequantisation warp (up to 256 CTAs)
 
 struct UmParams {
@@ -431,8 +431,8 @@ int w4a16_umma_reserve(t0_runtime* rt) {
     return T0_OK;
 }
 
-static uint32_t cut_grid(const t0_runtime* rt, uint64_t items, uint32_t n_chunks) {
-    const uint32_t ctas = std::min<uint32_t>((uint32_t)rt->sm_count, kUmCounterBytes / (kUmDqWarps * sizeof(uint32_t)));
+static uint32_t cut_grid(uint32_t sms, uint64_t items, uint32_t n_chunks) {
+    const uint32_t ctas = std::min<uint32_t>(sms, kUmCounterBytes / (kUmDqWarps * sizeof(uint32_t)));
     uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1, items * n_chunks / kUmMinChunks), ctas);
     if (items * 2 <= ctas) {
         // Few tiles: whole parts of a tile per CTA, at most four, where that leaves few CTAs idle - a CTA then has one piece to hand in, and
@@ -447,18 +447,35 @@ static uint32_t cut_grid(const t0_runtime* rt, uint64_t items, uint32_t n_chunks
 // K = 1024 ... 8192.  A chunk takes 0.42 us at small M and 0.52 at M = 128 in either form of this kernel; handing in and adding parts adds 2 to 10 us
 // with M.  Measured, whole tiles / cut: 2 x (128 x 11008 x 4096) 36.6 / 34.1, 12 of them 142 / 140, 4 x (64 x 1024 x 2048) 18.0 / 13.1; one problem
 // as clusters / cut: 128 x 11008 x 4096 21.8 / 22.7, 32 x 11008 x 4096 21.3 / 15.6, 100 x 1024 x 2048 14.1 / 16.5, 20 x 14336 x 2048 19.6 / 13.1.
-// `cluster_split` > 1 is what the cluster form would take (one problem; it sums no longer a part of K than cut tiles do).  Cut tiles need room
-// for their parts, and run only in launches of the runtime's own stream, whose launches run one after the other: a recorded launch may be
-// replayed beside others, which would share its counters and parts.
-int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split) {
+// `cluster_split`: into how many parts the cluster form would cut K (1: one problem that has tiles enough; 0: a list).
+//
+// The times choose only among forms whose sums are no longer than the library has made them for the problem, since the tensor cores' error grows with
+// the length of an accumulation.  One problem: its pieces are no longer than the parts of the clusters (K = 768: four of 3 chunks, where the grid
+// above would make three of 4; 39 x 3264 x 768 12.4 us as clusters, 9.2 so).  Lists: whole tiles, all of K in a sum, only where the kernels of before their roles walked converged were no faster
+// cut; that fit (0.63 us a chunk whole, 0.67 cut, 14.4 us for the parts) is kept for this alone.  2 x (114 x 4680 x 1664): 26 chunks in one sum whole, 7 cut.
+// Gives the form, and for cut tiles the number of CTAs in *ctas.
+int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas) {
     const uint64_t items = (uint64_t)ceil_div(N, kUmBN) * count;
-    const uint32_t n_chunks = K / kUmBK, grid = cut_grid(rt, items, n_chunks), sms = (uint32_t)rt->sm_count;
+    const uint32_t n_chunks = K / kUmBK;
     const int other = cluster_split > 1 ? kUmClusters : kUmWhole;
+    uint32_t grid = cut_grid(sms, items, n_chunks);
+    if (other == kUmClusters && (items * n_chunks + grid - 1) / grid > ceil_div(n_chunks, cluster_split)) grid = (uint32_t)items * cluster_split;
+    *ctas = grid;
     if (items % grid == 0 || items * n_chunks >= (1u << 24)) return other;
+    const double per_cta = (double)items * n_chunks / grid;
+    const double rounds = (double)((items + sms - 1) / sms);
+    if (cluster_split == 0 && per_cta * 0.67 + 14.4 <= 0.97 * (rounds * n_chunks * 0.63 + 4.0)) return kUmCut;
     const double chunk = 0.42 + 0.0008 * M;
-    const double cut = (double)items * n_chunks / grid * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0);
-    const double without = other == kUmClusters ? (double)ceil_div(n_chunks, cluster_split) * 0.495 + 10.2 : (double)((items + sms - 1) / sms) * n_chunks * chunk + 4.2;
-    if (cut > 0.97 * without) return other;
+    const double cut = per_cta * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0);
+    const double without = other == kUmClusters ? (double)ceil_div(n_chunks, cluster_split) * 0.495 + 10.2 : rounds * n_chunks * chunk + 4.2;
+    return cut > 0.97 * without ? other : kUmCut;
+}
+
+// The form of a launch.  Cut tiles need room for their parts, and run only in launches of the runtime's own stream, whose launches run one after the
+// other: a recorded launch may be replayed beside others, which would share its counters and parts.
+int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas) {
+    const int other = cluster_split > 1 ? kUmClusters : kUmWhole;
+    if (w4a16_umma_form((uint32_t)rt->sm_count, M, N, K, count, cluster_split, ctas) != kUmCut) return other;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return other;
     if (w4a16_umma_reserve(rt) == T0_OK) return kUmCut;
@@ -468,9 +485,9 @@ int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t
 
 uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }
 
-// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.  `cut`: w4a16_umma_plan has
-// made room for the parts of cut tiles; otherwise every CTA takes whole tiles.
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, bool cut) {
+// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.  `cut_ctas`: tiles cut between so
+// many CTAs, w4a16_umma_plan has made room for their parts; 0: every CTA takes whole tiles.
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas) {
     auto kern = tiled ? w4a16_umma_cut_kernel<true> : w4a16_umma_cut_kernel<false>;
     static bool attr_set[2][64] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
@@ -489,10 +506,10 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint
     p.n_chunks = K / kUmBK;
     const uint64_t items = (uint64_t)p.n_tiles * count;
     if (items * p.n_chunks > 0x7FFFFFFFull || items > (1u << 23)) return fail(T0_ERR_UNSUPPORTED, "too many tiles");
-    const uint32_t grid = cut ? cut_grid(rt, items, p.n_chunks) : (uint32_t)std::min<uint64_t>(items, std::min(rt->sm_count, 256));
+    const uint32_t grid = cut_ctas ? cut_ctas : (uint32_t)std::min<uint64_t>(items, std::min(rt->sm_count, 256));
     p.total = (uint32_t)(items * p.n_chunks);
-    p.whole = cut ? 0 : 1;
-    if (cut) {
+    p.whole = cut_ctas ? 0 : 1;
+    if (cut_ctas) {
         p.counters = (uint32_t*)rt->scratch_um.ptr;
         p.pieces = (float*)((uint8_t*)rt->scratch_um.ptr + kUmCounterBytes);
     }

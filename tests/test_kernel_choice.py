@@ -9,12 +9,20 @@ PROGRAM = r"""
 #include <cstdio>
 #include <cstring>
 #include "kernels.h"
+namespace t0 { int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas); }     // w4a16_umma_cut.cu
 using namespace t0;
 int main() {
     static const uint32_t clusters[kMaxClusterParts + 1] = {0, 148, 74, 40, 33, 24, 20, 14, 15};
     char what[16];
     while (scanf("%15s", what) == 1) {
         unsigned m, n, k, nn, bf16;
+        if (!strcmp(what, "w4a16")) {
+            unsigned count, split, ctas;
+            if (scanf("%u %u %u %u %u", &m, &n, &k, &count, &split) != 5) return 1;
+            const int form = w4a16_umma_form(148, m, n, k, count, split, &ctas);
+            printf("%d %u\n", form, ctas);
+            continue;
+        }
         if (scanf("%u %u %u %u %u", &m, &n, &k, &nn, &bf16) != 5) return 1;
         t0_gemm_config c;
         bool forced;
@@ -64,3 +72,31 @@ LONGEST = [((1352, 248, 1672, 0, 0), 5), ((56, 7952, 1984, 0, 0), 8), ((1016, 27
 def test_sums_are_no_longer_than_they_have_been(ask):
     for ((m, n, k, nn, bf16), longest), (choice, blocks) in zip(LONGEST, gemm_choices(ask, [s for s, _ in LONGEST])):
         assert blocks <= longest, (m, n, k, nn, bf16, choice, blocks, longest)
+
+
+CLUSTERS, WHOLE, CUT = 0, 1, 2
+
+
+def w4a16_form(ask, m, n, k, count):
+    """How `count` problems (0: one that is not given as a list, whose K clusters would cut into at most four parts) are shared out, and the 64-deep chunks of
+    the longest accumulation."""
+    tiles, chunks = -(-n // 256) * (count or 1), k // 64
+    split = 0 if count else min(max(1, min(4, 148 // tiles)), chunks)
+    form, ctas = ask([("w4a16", m, n, k, count or 1, split)])[0]
+    if form != CUT:
+        return form, -(-chunks // max(split, 1))
+    ends = [c * tiles * chunks // ctas for c in range(ctas + 1)] + [t * chunks for t in range(tiles)]      # of the CTAs' ranges, and of the tiles
+    ends = sorted(set(ends))
+    return form, max(b - a for a, b in zip(ends, ends[1:]))
+
+
+# lists whose tiles have been cut, and single problems, with the chunks of the longest accumulation the library has given them
+W4A16_LONGEST = [((113, 4456, 1920, 3), 11), ((125, 9800, 2944, 2), 25), ((114, 4680, 1664, 2), 7), ((128, 1632, 2240, 8), 14), ((121, 5144, 3008, 4), 27),
+                 ((58, 592, 960, 0), 4), ((50, 4840, 576, 0), 3), ((36, 304, 576, 0), 3), ((20, 3200, 768, 0), 3), ((50, 7736, 832, 0), 4), ((128, 256, 64, 0), 1),
+                 ((17, 1024, 256, 0), 1), ((52, 8968, 576, 0), 3), ((128, 11008, 4096, 0), 22), ((20, 14336, 2048, 0), 16), ((100, 28672, 1024, 0), 16)]
+
+
+def test_w4a16_sums_are_no_longer_than_they_have_been(ask):
+    for (m, n, k, count), longest in W4A16_LONGEST:
+        form, chunks = w4a16_form(ask, m, n, k, count)
+        assert chunks <= longest, (m, n, k, count, form, chunks)
