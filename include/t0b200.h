@@ -198,9 +198,9 @@ int t0_rt_selftest_drop_one_load(t0_runtime* rt);
  *     a multiple of 64 * split_k or the tiles times split_k are more than about one wave of SMs): T0_SCRATCH_SPLITK_PLANES = M * N * split_k * 4;
  *   t0_w4a16_gemm outside the fused shapes: T0_SCRATCH_W4_WEIGHTS = K * N * 2;
  *   every fused W4A16 call (row layout and streaming layout): T0_SCRATCH_W4_FUSED, t0_rt_w4_fused_scratch_bytes(rt) bytes,
- *     a fixed size per device, so only the first call of a runtime with M <= 16 and its first grouped call with 16 < M <= 128
- *     or on tile-major weights allocate; reserving less (0 will do) makes room for the first kind alone.  The grouped calls run
- *     without the buffer while the stream is being captured, or when there is no memory for it;
+ *     a fixed size per device.  The part for 16 < M <= 128 and for tile-major weights (39 MB) is made with the runtime, so only the first
+ *     call with M <= 16 allocates; reserving less than the whole (0 will do) makes room for that call alone.  Where there was no memory for the
+ *     first part the calls run without it, until a reservation of the whole finds some; calls being recorded always do;
  *   t0_matmul_f32*, t0_blas_gemm_f32: bf16 copies of the operands, T0_SCRATCH_F32_A / _B = elements * 2 (an operand whose
  *     rows are not a multiple of 8 elements: T0_SCRATCH_OPERAND_A / _B = rows * roundup(columns, 8) * 2), and, for
  *     alpha/beta other than 1/0 or ldc != n, T0_SCRATCH_F32_C = m * n * 4;
@@ -210,7 +210,8 @@ int t0_rt_selftest_drop_one_load(t0_runtime* rt);
  * Recording: a launch recorded by stream capture keeps the addresses it was given.  One that uses a buffer of the list above needs
  * the buffer reserved first, for the largest shape the runtime will ever see, and its graph is replayed in order with the runtime's
  * other work (on t0_rt_stream, or behind an event).  The launches that use no buffer may be replayed on any stream, beside others;
- * bf16 products give the same bits recorded or not, those W4A16 groups another order of the f32 sums.  t0_gemm_launch_gather and
+ * bf16 products give the same bits recorded or not; W4A16 calls of 16 < M <= 128 or on tile-major weights, single or grouped, may add their f32 sums
+ * in another order (what is recorded cuts no column tile between CTAs).  t0_gemm_launch_gather and
  * the host-operand entries are not for recording.
  * t0_rt_reserve_scratch grows one buffer to at least `bytes` ahead of time, so that later launches up to that size
  * neither allocate nor synchronise. */

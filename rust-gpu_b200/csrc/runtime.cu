@@ -372,6 +372,7 @@ int t0_rt_new(int device, t0_runtime** out) {
     T0_CUDA(cudaHostAlloc(&rt->h_status, sizeof(int), cudaHostAllocMapped));
     *rt->h_status = 0;
     T0_CUDA(cudaHostGetDevicePointer(&rt->d_status, rt->h_status, 0));
+    if (w4a16_umma_reserve(rt.get()) != T0_OK) cudaGetLastError();     // (without room the W4A16 calls take forms that need none)
     *out = rt.release();
     return T0_OK;
 }

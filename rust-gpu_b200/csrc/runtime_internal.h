@@ -56,7 +56,7 @@ struct t0_runtime {
     std::vector<uint64_t> peer_maps_key;     // destinations and shape the slot currently describes
     Scratch scratch_a, scratch_b, scratch_planes;
     Scratch scratch_w4;          // W4A16: slab arrival counters + straddling pieces
-    Scratch scratch_um;          // tcgen05 W4A16, grouped: counters + partial sums of the cut tiles
+    Scratch scratch_um;          // tcgen05 W4A16: counters + partial sums of the cut tiles (made with the runtime)
     Scratch scratch_w;           // W4A16 general path: dequantised weights
     Scratch scratch_cvt_a, scratch_cvt_b, scratch_cvt_c;   // f32 entries: bf16 copies of the operands, f32 product before alpha/beta
     void* host_pipe = nullptr;   // host-operand GEMM pipeline (streams, events, staging sets), made on first use

@@ -421,7 +421,7 @@ namespace t0 {
 // Counters and partial sums of a launch of one CTA per SM at M = 128: what any launch needs at most.
 size_t w4a16_umma_scratch_bytes(const t0_runtime* rt) { return kUmCounterBytes + (size_t)rt->sm_count * 2 * 128 * kUmBN * sizeof(float); }
 
-// Makes room for them; the counters start at zero.
+// Makes room for them, once, when the runtime is made: no call allocates, and none stalls the stream for it.  The counters start at zero.
 int w4a16_umma_reserve(t0_runtime* rt) {
     const size_t need = w4a16_umma_scratch_bytes(rt);
     if (need <= rt->scratch_um.size) return T0_OK;
@@ -478,9 +478,7 @@ int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t
     if (w4a16_umma_form((uint32_t)rt->sm_count, M, N, K, count, cluster_split, ctas) != kUmCut) return other;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return other;
-    if (w4a16_umma_reserve(rt) == T0_OK) return kUmCut;
-    cudaGetLastError();                    // (no memory for the parts: the other forms need none)
-    return other;
+    return rt->scratch_um.ptr ? kUmCut : other;      // (a runtime made while there was no memory for the parts: the other forms need none)
 }
 
 uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }

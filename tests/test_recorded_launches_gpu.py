@@ -353,3 +353,32 @@ def test_reserved_w4a16_calls_allocate_nothing(t0, oracle, rt, driver):
     r.close()
     one.rt = many.rt = rt
     one.free(), many.free()
+
+
+@pytest.mark.parametrize("M,K,N", [(20, 2048, 2560), (128, 4096, 11008)])
+def test_single_w4a16_calls_allocate_nothing(t0, oracle, rt, driver, M, K, N):
+    # one problem of 16 < M <= 128, cut between CTAs or as clusters: the first call of a new runtime takes no memory, and further calls give the same bits
+    def free_bytes():
+        rt.synchronize()
+        f, t = C.c_size_t(), C.c_size_t()
+        driver.call("cuMemGetInfo_v2", C.byref(f), C.byref(t))
+        return f.value
+
+    g = Group(t0, oracle, rt, M, K, N, 1)
+    ys = [g.outs() for _ in range(4)]
+    g.launch(ys[0]), g.launch_row_layout(ys[0][0])                            # (the kernels are loaded)
+    r = t0.GpuRuntime(0)
+    g.rt = r
+    at = free_bytes()
+    for y in ys[:2]:
+        g.launch(y)
+    for y in ys[2:]:
+        g.launch_row_layout(y[0])
+    r.synchronize()
+    assert free_bytes() == at
+    for y in ys:
+        g.check(y)
+        assert np.array_equal(y[0].read(M * N * 4, np.uint32), ys[0][0].read(M * N * 4, np.uint32))
+    r.close()
+    g.rt = rt
+    g.free()
