@@ -104,7 +104,11 @@ int run_gemm(t0_runtime* rt, const GemmRequest& q_in) {
     if (q.nn && g.tile_n < 64) g.tile_n = 64;
     // the CTA-pair kernel (256 x 256 tiles) pays off once there are enough tiles to fill the machine
     const bool pair_fits = (uint64_t)ceil_div(q.m, 256) * ceil_div(q.n, 256) * split >= (uint64_t)rt->sm_count / 2;
-    const bool use_pair = (q.pair == 1 || (q.pair == 0 && pair_fits && (q.tile_n == 0 || q.tile_n >= 256)));
+    // A caller's 128-wide pair over B[K,N] runs as single CTAs of the width asked for: with split_k the parts then meet in clusters (one launch, no buffer,
+    // may be recorded), and without it the pair is no sure gain (us, pair / single: 129 x 512 x 512 with tile_n 64 7.3 / 5.8, 64 x 8192 x 1024 with 128
+    // 9.6 / 9.3, 2048 x 4096 x 1024 22.8 / 23.8).  The library's own choice takes the pair where its times say so.
+    const bool pair_ok = !q.nn || q.tile_n == 0 || q.tile_n >= 256 || q.parts != 0;
+    const bool use_pair = pair_ok && (q.pair == 1 || (q.pair == 0 && pair_fits && (q.tile_n == 0 || q.tile_n >= 256)));
     if (use_pair) g.tile_n = q.tile_n;   // 0/256 -> 256-wide pair tiles, <= 128 -> 128-wide
     auto launch = [&](const GemmLaunch& gl) { return use_pair ? launch_gemm_sm100_pair(gl, rt->stream) : launch_gemm_sm100(gl, rt->stream); };
 

@@ -232,8 +232,8 @@ def test_split_k_with_several_tiles_per_cluster(t0, rt, tile_n, split_k, m, n, k
     assert np.array_equal(got, from_bf16(bf16_bits(want)) if out_bf16 else want)
 
 
-# Pair tiles of 128 columns: over B[K,N] as asked for, and as the library's own choice, which sums K in two accumulators (odd numbers of k blocks, one
-# ragged; more tiles than pairs, the last wave cut).  Integer operands: exact whatever the order.
+# Pair tiles of 128 columns: as asked for (B[N,K]; over B[K,N] single CTAs run in their place), and as the library's own choice in either layout, which sums K
+# in two accumulators (odd numbers of k blocks, one ragged; more tiles than pairs, the last wave cut).  Integer operands: exact whatever the order.
 @pytest.mark.parametrize("layout", ["nt", "nn"])
 @pytest.mark.parametrize("m,n,k,fixed", [(300, 264, 64, True), (257, 1000, 200, True), (1500, 2056, 136, True), (2048, 1024, 4096, False), (1664, 1056, 3248, False)])
 def test_pair_tiles_128_wide(t0, rt, layout, m, n, k, fixed):

@@ -152,6 +152,23 @@ def test_recorded_splits_of_the_caller(t0, fresh, driver, layout, kw, m, n, k):
     p.free()
 
 
+@pytest.mark.parametrize("kw", [dict(tile_n=64, split_k=2), dict(tile_n=128, split_k=4), dict(tile_n=128, split_k=8)])
+def test_recorded_splits_of_narrow_pairs_over_kn(t0, fresh, driver, kw):
+    # pair tiles of 128 columns or less asked for over B[K,N], K cut: one launch that needs no buffer, so it is recorded on a runtime that has none
+    p = Product(t0, fresh, 300, 520, 1024, seed=13, layout="nn", pair_cta=1, **kw)
+    y = p.out()
+    before = fresh.launch_count()
+    with driver.record(fresh) as graphs:
+        p.launch(y)
+    assert fresh.launch_count() - before == 1
+    want = p.eager()
+    driver.replay(graphs[0], fresh.stream())
+    fresh.synchronize()
+    assert np.array_equal(p.bits(y), want)
+    driver.drop(graphs[0])
+    p.free()
+
+
 @pytest.mark.parametrize("layout", ["nt", "nn"])
 def test_replays_beside_the_runtime_s_own_stream(t0, fresh, driver, layout):
     # two graphs of the same product on two streams, and the product itself on the runtime's stream, all under way together
