@@ -422,7 +422,7 @@ __global__ void w4_to_tiled_kernel(const uint32_t* __restrict__ packed, const ui
 namespace t0 {
 
 // w4a16_umma_cut.cu
-int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas);
+int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas);
 uint32_t w4a16_umma_cut_rows(uint32_t M);
 int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas);
 
@@ -466,19 +466,38 @@ static bool um_tiled_supported(uint64_t a, uint64_t tiled, uint64_t y, uint32_t 
     return ((a | tiled) & 15) == 0 && (y & 3) == 0;
 }
 
-static int um_launch(t0_runtime* rt, const CUtensorMap* m4, UmParams p, uint32_t split) {
-    auto kern = w4a16_umma_kernel;
-    constexpr uint32_t kSmemBytes = kUmSmem;
+// How many clusters of `split` CTAs the device holds at once.  Makes the kernel ready for a launch.
+static int um_clusters_at_once(t0_runtime* rt, uint32_t split, uint32_t* clusters) {
     static bool attr_set[64] = {};
     static int max_clusters[64][5] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
     if (!attr_set[rt->device]) {
-        T0_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        T0_CUDA(cudaFuncSetAttribute(w4a16_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmSmem));
         attr_set[rt->device] = true;
     }
+    if (!max_clusters[rt->device][split]) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = split; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(split * ((uint32_t)rt->sm_count / split), 1, 1);
+        cfg.blockDim = dim3(kUmThreads, 1, 1);
+        cfg.dynamicSmemBytes = kUmSmem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, w4a16_umma_kernel, &cfg);
+        if (e != cudaSuccess || n <= 0) { cudaGetLastError(); n = (int)((uint32_t)rt->sm_count / split) * 3 / 4; }
+        max_clusters[rt->device][split] = std::max(n, 1);
+    }
+    *clusters = (uint32_t)max_clusters[rt->device][split];
+    return T0_OK;
+}
+
+static int um_launch(t0_runtime* rt, const CUtensorMap* m4, UmParams p, uint32_t split, uint32_t clusters_at_once) {
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kUmThreads, 1, 1);
-    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.dynamicSmemBytes = kUmSmem;
     cfg.stream = rt->stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -486,20 +505,12 @@ static int um_launch(t0_runtime* rt, const CUtensorMap* m4, UmParams p, uint32_t
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    if (!max_clusters[rt->device][split]) {
-        cfg.gridDim = dim3(split * ((uint32_t)rt->sm_count / split), 1, 1);
-        cfg.numAttrs = 1;
-        int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
-        if (e != cudaSuccess || n <= 0) { cudaGetLastError(); n = (int)((uint32_t)rt->sm_count / split) * 3 / 4; }
-        max_clusters[rt->device][split] = std::max(n, 1);
-    }
     p.split = split;
     static const bool use_pdl = getenv("T0_NO_PDL") == nullptr;
-    const uint32_t clusters = std::min<uint32_t>(p.n_tiles, (uint32_t)max_clusters[rt->device][split]);
+    const uint32_t clusters = std::min(p.n_tiles, clusters_at_once);
     cfg.gridDim = dim3(clusters * split, 1, 1);
     cfg.numAttrs = use_pdl ? 2 : 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, kern, m4[0], m4[1], m4[2], m4[3], p);
+    cudaError_t le = cudaLaunchKernelEx(&cfg, w4a16_umma_kernel, m4[0], m4[1], m4[2], m4[3], p);
     if (le != cudaSuccess) return fail(T0_ERR_CUDA, "W4A16 kernel launch failed: %s", cudaGetErrorString(le));
     rt->launches.fetch_add(1);
     return T0_OK;
@@ -539,15 +550,17 @@ static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
     // as many parts of K as fill the machine (the parts of a tile form a cluster of at most four CTAs)
     const uint32_t n_tiles = ceil_div(a.n, kUmBN);
     const uint32_t split = std::min(std::max<uint32_t>(1, std::min<uint32_t>(4, (uint32_t)rt->sm_count / std::max<uint32_t>(1, n_tiles))), a.k / kUmBK);
-    uint32_t ctas;
-    const int plan = w4a16_umma_plan(rt, a.m, a.n, a.k, 1, split, &ctas);
+    uint32_t ctas, clusters = 1;
+    int rc = split > 1 ? um_clusters_at_once(rt, split, &clusters) : T0_OK;
+    if (rc != T0_OK) return rc;
+    const int plan = w4a16_umma_plan(rt, a.m, a.n, a.k, 1, split, ceil_div(n_tiles, clusters), &ctas);
     if (plan != kUmClusters) return um_launch_list(rt, &a, 1, tiled, plan == kUmCut ? ctas : 0);
     UmParams p = um_params(rt, a.a, a.y, a.m, a.n, a.k, a.group);
     p.tiled = tiled ? 1 : 0;
     CUtensorMap m4[4];
-    int rc = tiled ? um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, m4) : um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, m4);
+    rc = tiled ? um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, m4) : um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, m4);
     if (rc != T0_OK) return rc;
-    return um_launch(rt, m4, p, split);
+    return um_launch(rt, m4, p, split, clusters);
 }
 
 int launch_w4a16_umma(t0_runtime* rt, uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t y, uint32_t M, uint32_t N, uint32_t K,
@@ -572,7 +585,7 @@ static int um_launch_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_t
             return fail(T0_ERR_UNSUPPORTED, "grouped launch: problem %u is not a shape of the fused tcgen05 kernel", i);
     }
     uint32_t ctas;
-    const int plan = w4a16_umma_plan(rt, a0.m, a0.n, a0.k, count, 0, &ctas);
+    const int plan = w4a16_umma_plan(rt, a0.m, a0.n, a0.k, count, 0, 0, &ctas);
     return um_launch_list(rt, args, count, tiled, plan == kUmCut ? ctas : 0);
 }
 

@@ -447,14 +447,15 @@ static uint32_t cut_grid(uint32_t sms, uint64_t items, uint32_t n_chunks) {
 // K = 1024 ... 8192.  A chunk takes 0.42 us at small M and 0.52 at M = 128 in either form of this kernel; handing in and adding parts adds 2 to 10 us
 // with M.  Measured, whole tiles / cut: 2 x (128 x 11008 x 4096) 36.6 / 34.1, 12 of them 142 / 140, 4 x (64 x 1024 x 2048) 18.0 / 13.1; one problem
 // as clusters / cut: 128 x 11008 x 4096 21.8 / 22.7, 32 x 11008 x 4096 21.3 / 15.6, 100 x 1024 x 2048 14.1 / 16.5, 20 x 14336 x 2048 19.6 / 13.1.
-// `cluster_split`: into how many parts the cluster form would cut K (1: one problem that has tiles enough; 0: a list).
+// `cluster_split`: into how many parts the cluster form would cut K (1: one problem that has tiles enough; 0: a list); `cluster_rounds`: in how many rounds
+// its clusters fit on the GPU (the GPCs hold 33 of four CTAs, not 37: 128 x 9472 x 4096 36.4 us in two rounds of clusters, 20.7 cut).
 //
 // The times choose only among forms whose sums are no longer than the library has made them for the problem, since the tensor cores' error grows with
 // the length of an accumulation.  One problem: its pieces are no longer than the parts of the clusters (K = 768: four of 3 chunks, where the grid
 // above would make three of 4; 39 x 3264 x 768 12.4 us as clusters, 9.2 so).  Lists: whole tiles, all of K in a sum, only where the kernels of before their roles walked converged were no faster
 // cut; that fit (0.63 us a chunk whole, 0.67 cut, 14.4 us for the parts) is kept for this alone.  2 x (114 x 4680 x 1664): 26 chunks in one sum whole, 7 cut.
 // Gives the form, and for cut tiles the number of CTAs in *ctas.
-int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas) {
+int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas) {
     const uint64_t items = (uint64_t)ceil_div(N, kUmBN) * count;
     const uint32_t n_chunks = K / kUmBK;
     const int other = cluster_split > 1 ? kUmClusters : kUmWhole;
@@ -467,15 +468,15 @@ int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t c
     if (cluster_split == 0 && per_cta * 0.67 + 14.4 <= 0.97 * (rounds * n_chunks * 0.63 + 4.0)) return kUmCut;
     const double chunk = 0.42 + 0.0008 * M;
     const double cut = per_cta * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0);
-    const double without = other == kUmClusters ? (double)ceil_div(n_chunks, cluster_split) * 0.495 + 10.2 : rounds * n_chunks * chunk + 4.2;
+    const double without = other == kUmClusters ? cluster_rounds * (ceil_div(n_chunks, cluster_split) * 0.495 + 8.2) + 2.0 : rounds * n_chunks * chunk + 4.2;
     return cut > 0.97 * without ? other : kUmCut;
 }
 
 // The form of a launch.  Cut tiles need room for their parts, and run only in launches of the runtime's own stream, whose launches run one after the
 // other: a recorded launch may be replayed beside others, which would share its counters and parts.
-int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas) {
+int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas) {
     const int other = cluster_split > 1 ? kUmClusters : kUmWhole;
-    if (w4a16_umma_form((uint32_t)rt->sm_count, M, N, K, count, cluster_split, ctas) != kUmCut) return other;
+    if (w4a16_umma_form((uint32_t)rt->sm_count, M, N, K, count, cluster_split, cluster_rounds, ctas) != kUmCut) return other;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(rt->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return other;
     return rt->scratch_um.ptr ? kUmCut : other;      // (a runtime made while there was no memory for the parts: the other forms need none)

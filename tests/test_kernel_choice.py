@@ -9,7 +9,7 @@ PROGRAM = r"""
 #include <cstdio>
 #include <cstring>
 #include "kernels.h"
-namespace t0 { int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t* ctas); }     // w4a16_umma_cut.cu
+namespace t0 { int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas); }     // w4a16_umma_cut.cu
 using namespace t0;
 int main() {
     static const uint32_t clusters[kMaxClusterParts + 1] = {0, 148, 74, 40, 33, 24, 20, 14, 15};
@@ -17,9 +17,9 @@ int main() {
     while (scanf("%15s", what) == 1) {
         unsigned m, n, k, nn, bf16;
         if (!strcmp(what, "w4a16")) {
-            unsigned count, split, ctas;
-            if (scanf("%u %u %u %u %u", &m, &n, &k, &count, &split) != 5) return 1;
-            const int form = w4a16_umma_form(148, m, n, k, count, split, &ctas);
+            unsigned count, split, rounds, ctas;
+            if (scanf("%u %u %u %u %u %u", &m, &n, &k, &count, &split, &rounds) != 6) return 1;
+            const int form = w4a16_umma_form(148, m, n, k, count, split, rounds, &ctas);
             printf("%d %u\n", form, ctas);
             continue;
         }
@@ -82,7 +82,8 @@ def w4a16_form(ask, m, n, k, count):
     the longest accumulation."""
     tiles, chunks = -(-n // 256) * (count or 1), k // 64
     split = 0 if count else min(max(1, min(4, 148 // tiles)), chunks)
-    form, ctas = ask([("w4a16", m, n, k, count or 1, split)])[0]
+    at_once = {0: tiles, 1: tiles, 2: 74, 3: 48, 4: 33}[split]                                                # clusters of `split` CTAs that fit at once
+    form, ctas = ask([("w4a16", m, n, k, count or 1, split, -(-tiles // at_once))])[0]
     if form != CUT:
         return form, -(-chunks // max(split, 1))
     ends = [c * tiles * chunks // ctas for c in range(ctas + 1)] + [t * chunks for t in range(tiles)]      # of the CTAs' ranges, and of the tiles
@@ -100,3 +101,10 @@ def test_w4a16_sums_are_no_longer_than_they_have_been(ask):
     for (m, n, k, count), longest in W4A16_LONGEST:
         form, chunks = w4a16_form(ask, m, n, k, count)
         assert chunks <= longest, (m, n, k, count, form, chunks)
+
+
+def test_w4a16_clusters_in_two_rounds_are_weighed_as_such(ask):
+    # 33 clusters of four CTAs fit at once: 33 tiles take one round, 34 take two and are cut in their place
+    assert w4a16_form(ask, 128, 33 * 256, 4096, 0)[0] == CLUSTERS
+    for tiles in (34, 37):
+        assert w4a16_form(ask, 128, tiles * 256, 4096, 0)[0] == CUT

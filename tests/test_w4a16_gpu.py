@@ -559,8 +559,9 @@ def test_tiled_weights_any_n(t0, oracle, rt, M, K, N, G):
     test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, 1)
 
 
-# One problem of few chunks, cut between CTAs: pieces of one chunk (half of the dequantising warps have none) and of two or three, one tile and several
-@pytest.mark.parametrize("M,K,N,G", [(17, 128, 200, 64), (20, 256, 1030, 64), (64, 256, 8960, 128), (40, 576, 9000, 64), (39, 768, 3264, 128)])
+# One problem of few chunks, cut between CTAs: pieces of one chunk (half of the dequantising warps have none) and of two or three, one tile and
+# several; 37 tiles, whose clusters of four would not all run at once
+@pytest.mark.parametrize("M,K,N,G", [(17, 128, 200, 64), (20, 256, 1030, 64), (64, 256, 8960, 128), (40, 576, 9000, 64), (39, 768, 3264, 128), (128, 1024, 9300, 128)])
 def test_tiled_weights_short_pieces(t0, oracle, rt, M, K, N, G):
     test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, 1)
 
