@@ -424,7 +424,8 @@ namespace t0 {
 // w4a16_umma_cut.cu
 int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas);
 uint32_t w4a16_umma_cut_rows(uint32_t M);
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas);
+template <uint32_t kProblems>
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems>& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas);
 
 static t0_w4a16_args um_args(uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t y, uint32_t M, uint32_t N, uint32_t K, uint32_t group) {
     t0_w4a16_args q;
@@ -528,22 +529,25 @@ static UmParams um_params(t0_runtime* rt, uint64_t a, uint64_t y, uint32_t M, ui
     return p;
 }
 
-// Problems of one shape on the kernel that takes whole tiles or cuts them (w4a16_umma_cut.cu); `count` problems in one launch, which run
-// concurrently.  Tile-major weights, or the row layout.
+// The maps and output of problem i of a launch on the kernel that takes whole tiles or cuts them (w4a16_umma_cut.cu).  Tile-major weights, or the row layout.
+template <uint32_t kProblems>
+static int um_group_entry(UmGroup<kProblems>& grp, uint32_t i, const t0_w4a16_args& a, bool tiled) {
+    const uint32_t rows = w4a16_umma_cut_rows(a.m);
+    grp.y[i] = (float*)a.y;
+    return tiled ? um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows)
+                 : um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows);
+}
+
+// `count` problems of one shape in one launch, which run concurrently.
 static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count, bool tiled, uint32_t cut_ctas) {
-    const t0_w4a16_args& a0 = args[0];
-    static UmGroup grp;                  // 16.9 KB: kept off the stack, filled under the lock, copied by the launch
+    static UmGroup<kUmMaxGroup> grp;     // 16.6 KB: kept off the stack, filled under the lock, copied by the launch
     static std::mutex grp_mu;
     std::lock_guard<std::mutex> lock(grp_mu);
-    const uint32_t rows = w4a16_umma_cut_rows(a0.m);
     for (uint32_t i = 0; i < count; ++i) {
-        const t0_w4a16_args& a = args[i];
-        int rc = tiled ? um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows)
-                       : um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows);
+        int rc = um_group_entry(grp, i, args[i], tiled);
         if (rc != T0_OK) return rc;
-        grp.y[i] = (float*)a.y;
     }
-    return launch_w4a16_umma_cut(rt, grp, tiled, a0.m, a0.n, a0.k, a0.group, count, cut_ctas);
+    return launch_w4a16_umma_cut(rt, grp, tiled, args[0].m, args[0].n, args[0].k, args[0].group, count, cut_ctas);
 }
 
 static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
@@ -554,7 +558,11 @@ static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
     int rc = split > 1 ? um_clusters_at_once(rt, split, &clusters) : T0_OK;
     if (rc != T0_OK) return rc;
     const int plan = w4a16_umma_plan(rt, a.m, a.n, a.k, 1, split, ceil_div(n_tiles, clusters), &ctas);
-    if (plan != kUmClusters) return um_launch_list(rt, &a, 1, tiled, plan == kUmCut ? ctas : 0);
+    if (plan != kUmClusters) {
+        UmGroup<1> one;
+        rc = um_group_entry(one, 0, a, tiled);
+        return rc != T0_OK ? rc : launch_w4a16_umma_cut(rt, one, tiled, a.m, a.n, a.k, a.group, 1, plan == kUmCut ? ctas : 0);
+    }
     UmParams p = um_params(rt, a.a, a.y, a.m, a.n, a.k, a.group);
     p.tiled = tiled ? 1 : 0;
     CUtensorMap m4[4];

@@ -73,9 +73,10 @@ __device__ __forceinline__ uint32_t um_begin(uint32_t cta, const UmParams& p) {
 }
 __device__ __forceinline__ uint32_t um_owner(uint32_t chunk, const UmParams& p) { return ((chunk + 1) * gridDim.x - 1) / p.total; }
 
-template <bool kTiled>    // weights in the tile-major layout (3-D maps: column in tile, row, tile), else the row layout
+// kTiled: weights in the tile-major layout (3-D maps: column in tile, row, tile), else the row layout; kProblems: room for so many problems
+template <bool kTiled, uint32_t kProblems>
 __global__ void __launch_bounds__(kUmThreads, 1)
-w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup group) {
+w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblems> group) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t raw_ring = smem;
@@ -486,8 +487,9 @@ uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }
 
 // `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.  `cut_ctas`: tiles cut between so
 // many CTAs, w4a16_umma_plan has made room for their parts; 0: every CTA takes whole tiles.
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas) {
-    auto kern = tiled ? w4a16_umma_cut_kernel<true> : w4a16_umma_cut_kernel<false>;
+template <uint32_t kProblems>
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems>& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas) {
+    auto kern = tiled ? w4a16_umma_cut_kernel<true, kProblems> : w4a16_umma_cut_kernel<false, kProblems>;
     static bool attr_set[2][64] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
     if (!attr_set[tiled][rt->device]) {
@@ -528,5 +530,8 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup& group, bool tiled, uint
     rt->launches.fetch_add(1);
     return T0_OK;
 }
+
+template int launch_w4a16_umma_cut<1>(t0_runtime*, const UmGroup<1>&, bool, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t);
+template int launch_w4a16_umma_cut<kUmMaxGroup>(t0_runtime*, const UmGroup<kUmMaxGroup>&, bool, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t);
 
 }  // namespace t0
