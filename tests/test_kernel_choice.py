@@ -108,3 +108,25 @@ def test_w4a16_clusters_in_two_rounds_are_weighed_as_such(ask):
     assert w4a16_form(ask, 128, 33 * 256, 4096, 0)[0] == CLUSTERS
     for tiles in (34, 37):
         assert w4a16_form(ask, 128, tiles * 256, 4096, 0)[0] == CUT
+
+
+# The shapes by which the GPU tests mean to reach a kernel: a refit that moved one would leave the kernel untested.
+PAIR_128_HALVES = [(2048, 1024, 4096, 0, 0), (2048, 1024, 4096, 1, 0), (1664, 1056, 3248, 0, 0), (1664, 1056, 3248, 1, 0), (280, 3339, 2036, 0, 1), (280, 3339, 2040, 1, 1),
+                   (263, 3318, 2218, 0, 1), (263, 3320, 2218, 1, 0), (768, 2048, 4096, 1, 1), (645, 7493, 4864, 0, 0)]
+
+
+def test_shapes_of_the_gpu_tests_reach_pair_tiles_128_wide(ask):
+    for shape, (choice, _) in zip(PAIR_128_HALVES, gemm_choices(ask, PAIR_128_HALVES)):
+        assert choice == (128, 1, True, True), (shape, choice)
+    tiles = -(-645 // 256) * -(-7493 // 128)                                     # more than the 74 pairs, and the last wave at most half full
+    assert tiles > 74 and 0 < 2 * (tiles % 74) <= 74
+
+
+@pytest.mark.parametrize("form,problems", [
+    (CUT, [(20, 14344, 2048, 0), (33, 2312, 1024, 3), (17, 200, 128, 0), (20, 1030, 256, 0), (64, 8960, 256, 0), (40, 9000, 576, 0), (39, 3264, 768, 0), (128, 9300, 1024, 0),
+           (33, 255, 512, 0), (20, 2560, 2048, 0), (40, 2560, 4096, 2)]),
+    (CLUSTERS, [(128, 2560, 2048, 0), (128, 1030, 1024, 0), (100, 1001, 1024, 0), (128, 7, 1024, 0), (128, 11008, 4096, 0)]),
+    (WHOLE, [(16, 38144, 64, 0), (17, 1030, 64, 0)])])
+def test_shapes_of_the_gpu_tests_reach_every_w4a16_form(ask, form, problems):
+    for m, n, k, count in problems:
+        assert w4a16_form(ask, m, n, k, count)[0] == form, (m, n, k, count)

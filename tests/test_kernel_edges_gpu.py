@@ -242,3 +242,27 @@ def test_pair_tiles_128_wide(t0, rt, layout, m, n, k, fixed):
     kw = {"tile_n": 128, "pair_cta": 1} if fixed else {}
     got = run_gemm(t0, rt, x, b, m, n, k, transpose=t0.NN if layout == "nn" else t0.NT, **kw)
     assert np.array_equal(got, x @ (b if layout == "nn" else b.T))
+
+
+# The library's own choice of those tiles with two accumulators (test_kernel_choice.py asserts it for these shapes): a bias and ReLU on the sum of both, bf16
+# results, odd N, a ragged last k block; more tiles than pairs, the tiles of the last wave cut in two.
+@pytest.mark.parametrize("layout,m,n,k,out_bf16", [("nt", 280, 3339, 2036, True), ("nn", 280, 3339, 2040, True), ("nt", 263, 3318, 2218, True), ("nn", 263, 3320, 2218, False),
+                                                   ("nn", 768, 2048, 4096, True), ("nt", 645, 7493, 4864, False)])
+def test_pair_tiles_128_wide_with_two_accumulators(t0, rt, layout, m, n, k, out_bf16):
+    rng = np.random.default_rng(m + n)
+    x, b, bias = ints(rng, m, k), ints(rng, *((k, n) if layout == "nn" else (n, k))), ints(rng, n, lim=100)
+    got = run_gemm(t0, rt, x, b, m, n, k, out_bf16, bias, transpose=t0.NN if layout == "nn" else t0.NT, epilogue=t0.EPI_BIAS_ADD_RELU_STORE_F32)
+    want = np.maximum(x @ (b if layout == "nn" else b.T) + bias, 0)
+    assert np.array_equal(got, from_bf16(bf16_bits(want)) if out_bf16 else want)
+
+
+# The same tiles over a first operand that is read transposed: dW = X^T dY, [k, n] summed over m.
+@pytest.mark.parametrize("m,k,n", [(4096, 2048, 1024), (2218, 263, 3320)])
+def test_transposed_operand_on_pair_tiles_128_wide(t0, rt, m, k, n):
+    rng = np.random.default_rng(m)
+    x, dy = ints(rng, m, k), ints(rng, m, n)
+    xd, yd, dw = rt.upload(x), rt.upload(dy), rt.alloc(k * n * 4)
+    rt.matmul_f32_backward_weight(xd.gpu_addr(), yd.gpu_addr(), dw.gpu_addr(), m, k, n)
+    assert np.array_equal(rt.read_f32(dw, k * n).reshape(k, n), x.T @ dy)
+    for buf in (xd, yd, dw):
+        buf.free()

@@ -313,7 +313,7 @@ class Group:
 
 
 def test_recorded_w4a16_group_beside_eager_ones(t0, oracle, fresh, driver):
-    # recorded before the runtime has a buffer for cut tiles, and again after: the replays run on another stream beside eager calls
+    # recorded before the runtime has cut a tile, and again after: the replays run on another stream beside eager calls
     g = Group(t0, oracle, fresh, 40, 4096, 2560, 2)
     stream, execs, outs = driver.stream(), [], []
     for _ in range(2):
@@ -338,6 +338,26 @@ def test_recorded_w4a16_group_beside_eager_ones(t0, oracle, fresh, driver):
     g.free()
 
 
+@pytest.mark.parametrize("row_layout", [False, True])
+def test_recorded_single_w4a16_problem_beside_eager_ones(t0, oracle, fresh, driver, row_layout):
+    # one problem that an eager call cuts between CTAs: recorded it runs as clusters, without the buffer, so its replays may run beside eager calls
+    g = Group(t0, oracle, fresh, 20, 2048, 2560, 1)
+    launch = (lambda ys: g.launch_row_layout(ys[0])) if row_layout else g.launch
+    stream, recorded, eager = driver.stream(), g.outs(), g.outs()
+    with driver.record(fresh) as graphs:
+        for _ in range(5):
+            launch(recorded)
+    for _ in range(10):
+        driver.replay(graphs[0], stream)
+        for _ in range(5):
+            launch(eager)
+    driver.sync(stream)
+    fresh.synchronize()
+    g.check(recorded), g.check(eager)
+    driver.drop(graphs[0], stream)
+    g.free()
+
+
 def test_reserved_w4a16_calls_allocate_nothing(t0, oracle, rt, driver):
     # what t0_rt_w4_fused_scratch_bytes names covers every fused call of a runtime; a smaller reservation the calls with M <= 16
     def free_bytes():
@@ -354,7 +374,7 @@ def test_reserved_w4a16_calls_allocate_nothing(t0, oracle, rt, driver):
     whole, before = r.w4_fused_scratch_bytes(), free_bytes()
     r.reserve_scratch("w4_fused", 0)
     small = before - free_bytes()
-    assert small < whole // 4                                                 # nothing for cut tiles yet
+    assert small < whole // 4                                                 # (the room for cut tiles was made with the runtime)
     one.rt = many.rt = r
     at = free_bytes()
     one.launch_row_layout(ys[0][0])

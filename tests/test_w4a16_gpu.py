@@ -545,15 +545,15 @@ def test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, count):
         b.free()
 
 
-# what the plan of a launch makes of these: a single problem cut between CTAs, and as clusters; whole tiles (one chunk of K, more tiles than SMs);
-# several problems cut, the last tile ragged
+# What the plan of a launch makes of these (test_kernel_choice.py asserts it): a single problem cut between CTAs, and as clusters; whole tiles (one chunk of K,
+# more tiles than SMs); several problems cut, the last tile ragged.
 @pytest.mark.parametrize("M,K,N,G,count", [(20, 2048, 14344, 128, 1), (128, 2048, 2560, 128, 1), (16, 64, 38144, 64, 1), (33, 1024, 2312, 64, 3)])
 def test_tiled_forms_of_a_launch(t0, oracle, rt, M, K, N, G, count):
     test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, count)
 
 
-# Tile-major weights take any N.  One problem as clusters: rows of y start 4 and 8 bytes off a 16-byte boundary; the last tile ragged, N below a tile, below
-# eight columns; K too short for more than one part.
+# Tile-major weights take any N.  One problem as clusters: rows of y start 4 and 8 bytes off a 16-byte boundary, the last tile ragged, N below eight
+# columns; cut, N below a tile; whole tiles, K too short for more than one part.
 @pytest.mark.parametrize("M,K,N,G", [(128, 1024, 1030, 128), (100, 1024, 1001, 128), (33, 512, 255, 64), (128, 1024, 7, 128), (17, 64, 1030, 64)])
 def test_tiled_weights_any_n(t0, oracle, rt, M, K, N, G):
     test_tiled_weights_single_and_grouped(t0, oracle, rt, M, K, N, G, 1)
