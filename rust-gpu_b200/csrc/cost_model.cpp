@@ -32,10 +32,11 @@ struct Candidate {
     double pred_tflops;
 };
 
-// Measured main-loop cost per 64-deep k-block on B200 (SM cycles, from the in-kernel cycle probe at 2048^3..8192^3):
-// the tensor pipe needs tn/2 cycles per UMMA and four UMMAs per k-block, but narrow tiles are bound by the
-// shared-memory operand feed (A is re-read for every UMMA) and the single-CTA 128x256 tile by L2->SM latency with
-// only four stages in flight.  The CTA pair (256x256 over two SMs) comes closest to the pipe's 512 cycles.
+// Main-loop cost per 64-deep k-block on B200 in SM cycles, from the in-kernel cycle probe at 2048^3..8192^3, of the kernels before their serial roles
+// walked converged (the roles' instructions, not the tensor pipe, then set the pace of all tiles under 256 x 256).  Converged the same blocks take
+// 330 to 343 ns as a pair, 390 / 255 / 242 / 234 ns at 256 / 128 / 64 / 32 columns (kTimes below, by which products that fix nothing are
+// launched).  These figures stay: they rank the configurations that auto_select and the tuner hand out, which callers store, and the parts of K in those
+// bound the lengths of the sums.
 static double kblock_cycles(uint32_t tn, bool pair) {
     if (pair) return 590.0;
     switch (tn) {

@@ -7,9 +7,8 @@
 // math), the tensor cores read the other half of B from the partner's shared memory.  A third less
 // L2->SM traffic and a deeper ring (6 stages) for the same shared-memory budget.
 //
-// The serial roles walk with their whole warp and one elected lane issues: a diverged lane's operands go from per-lane into uniform registers
-// before every tcgen05 and TMA instruction (85 to 102 cycles each, 35 so), which made a k block 590 cycles where the UMMAs take 512: 4096^3
-// 123.8 -> 112.2 us, 8192^3 872 -> 811.
+// The serial roles walk with their whole warp and one elected lane issues (see ptx::mbar_wait_warp): as one diverged lane a tcgen05 or TMA instruction took
+// 85 to 102 cycles, 35 so, which made a k block 590 cycles where the UMMAs take 512: 4096^3 125.8 -> 115.0 us, 8192^3 883 -> 832.
 //
 // Roles per CTA are those of the single-CTA kernel.  Differences:
 //   * both CTAs' TMA loads credit the EVEN CTA's `full` barrier (it expects the bytes of both);

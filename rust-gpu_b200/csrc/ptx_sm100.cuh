@@ -68,8 +68,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
-// The same wait by a whole converged warp; the result is the same in every lane, and the compiler knows it: what follows stays in
-// uniform registers, from which the tensor-core and TMA instructions take their operands.
+// The same wait by a whole converged warp, with the same result in every lane.  A role that waits so and lets one elected lane issue (below) spends 35
+// cycles on a tcgen05 or TMA instruction by the clock, where a role written as one diverged lane (if (lane == 0)) spent 85 to 102: those
+// instructions take warp-uniform operands, which a diverged lane's are not.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
     if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
     uint64_t t_start = 0;
@@ -84,8 +85,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
         }
     }
 }
-// True in one lane of a converged warp, the same one every time.  A branch on it is one the compiler knows to be taken by a single thread,
-// so operands computed by the whole warp need no move per lane.
+// True in one lane of a converged warp, the same one every time: what the whole warp has computed is issued once.
 __device__ __forceinline__ bool elect_one() {
     uint32_t is;
     asm volatile(
@@ -196,15 +196,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// 32 lanes x 16 consecutive 32-bit columns
-__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
 // 32 lanes x 8 consecutive 32-bit columns (load / store); thread t of the warp owns lane (taddr.lane + t).
 __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

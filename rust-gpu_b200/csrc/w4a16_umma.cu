@@ -14,7 +14,7 @@
 //     operand: 256 rows (n) x 64 k, K-major, 128-byte swizzle.  A packed word holds eight consecutive k of one column
 //     and the nibble pairs come out as (k, k+4); four byte permutes put them back into k order, so that the activations
 //     (the 128-row A operand) can come straight from global memory through TMA (rows beyond M are zero-filled);
-//   * one thread issues four tcgen05.mma (128 x 256 x 16) per chunk into a 128 x 256 fp32 accumulator in tensor memory.
+//   * a third serial warp issues four tcgen05.mma (128 x 256 x 16) per chunk into a 128 x 256 fp32 accumulator in tensor memory.
 // At the end the sixteen warps read the accumulator, park it in shared memory (over the rings, idle by then), exchange
 // across the cluster and store.  Every wait is bounded.
 #include "w4a16_common.cuh"
@@ -26,7 +26,7 @@ namespace {
 
 constexpr uint32_t kUmDqWarps = 16;
 // + the warps that fetch weights and activations and the one that issues the UMMAs; each walks whole and lets one elected lane issue
-// (ptx::elect_one), which shortens the serial chain that sets a chunk's pace.
+// (ptx::mbar_wait_warp), which shortens the serial chain that sets a chunk's pace.
 constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;
 constexpr uint32_t kUmThreads = (kUmDqWarps + 3) * 32;
 constexpr uint32_t kUmRawStages = 6;
@@ -41,11 +41,10 @@ constexpr uint32_t kUmSmem = kUmRingBytes + 512 + 1024;
 constexpr uint32_t kUmTmemCols = 256;
 
 struct UmParams {
-    const uint16_t* a;
     float* y;
     int* status;
     uint64_t wait_limit_ns;
-    uint32_t M, N, K;
+    uint32_t M, N;
     uint32_t group;          // k per scale / zero-point row (a multiple of 64)
     uint32_t n_tiles, n_chunks, split;
     uint32_t tiled;          // the weights are in the tile-major layout (3-D maps: column in tile, row, tile) instead of the row layout
@@ -517,13 +516,13 @@ static int um_launch(t0_runtime* rt, const CUtensorMap* m4, UmParams p, uint32_t
     return T0_OK;
 }
 
-static UmParams um_params(t0_runtime* rt, uint64_t a, uint64_t y, uint32_t M, uint32_t N, uint32_t K, uint32_t group) {
+static UmParams um_params(t0_runtime* rt, uint64_t y, uint32_t M, uint32_t N, uint32_t K, uint32_t group) {
     UmParams p;
     memset(&p, 0, sizeof p);
-    p.a = (const uint16_t*)a; p.y = (float*)y; p.status = rt->d_status;
+    p.y = (float*)y; p.status = rt->d_status;
     const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
     p.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
-    p.M = M; p.N = N; p.K = K; p.group = group;
+    p.M = M; p.N = N; p.group = group;
     p.n_tiles = ceil_div(N, kUmBN);
     p.n_chunks = K / kUmBK;
     return p;
@@ -563,7 +562,7 @@ static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
         rc = um_group_entry(one, 0, a, tiled);
         return rc != T0_OK ? rc : launch_w4a16_umma_cut(rt, one, tiled, a.m, a.n, a.k, a.group, 1, plan == kUmCut ? ctas : 0);
     }
-    UmParams p = um_params(rt, a.a, a.y, a.m, a.n, a.k, a.group);
+    UmParams p = um_params(rt, a.y, a.m, a.n, a.k, a.group);
     p.tiled = tiled ? 1 : 0;
     CUtensorMap m4[4];
     rc = tiled ? um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, m4) : um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, m4);

@@ -6,12 +6,12 @@
 //
 // The work is a list of chunks, 256 columns x 64 k, problem by problem, tile by tile, k last; every CTA (one per SM) takes an
 // equal contiguous range of it.  Per chunk:
-//   * one warp's lane fetches the packed words (8 rows x 256 columns), scales and zero points with three TMA boxes each into a ring of
+//   * one warp fetches the packed words (8 rows x 256 columns), scales and zero points with three TMA boxes each into a ring of
 //     raw stages of two chunks, another warp's the activations (rows up to M rounded to 16; rows beyond M are zero-filled);
 //   * sixteen warps turn the words into bf16 (one LOP3 per nibble pair: 0x4300 | q is the bf16 128+q, minus 128+z, times s -
 //     bit-identical to the oracle because (q-z)*s is rounded once) and put them straight into tensor memory (tcgen05.st): the
 //     weights are the 128-row A operand, two halves of 128 columns of y;
-//   * one thread issues 2 x 4 tcgen05.mma (128 x M' x 16, M' = M rounded to 16) with the activations as the B operand in shared
+//   * a third serial warp issues 2 x 4 tcgen05.mma (128 x M' x 16, M' = M rounded to 16) with the activations as the B operand in shared
 //     memory.  The accumulator is y transposed: lane = column of y, tensor-memory column = row of y.
 // A tile that lies wholly in one range is stored from tensor memory.  A tile cut by range boundaries is finished by the warps that
 // reach it last: see the epilogue.
@@ -32,7 +32,8 @@ constexpr uint32_t kUmDqWarps = 16;
 // chunk, at several cycles an instruction, so the chains are kept short (running counters, no divisions, descriptors stepped by addition,
 // one barrier for both operands of a chunk) and apart.  The issuer's chain took 1190 cycles a chunk as one diverged lane with a barrier per
 // operand, which the sixteen dequantising warps spent waiting: two problems of M = 128, N = 11008, K = 4096 39.7 us, 33.3 with the warp
-// converged, 31.7 with one barrier.
+// converged, 31.7 with one barrier
+// (device time of queued launches, as below; the same call takes 34 us by the host's clock in blocks of calls).
 constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;
 constexpr uint32_t kUmThreads = (kUmDqWarps + 3) * 32;
 constexpr uint32_t kUmXBytes = 128 * kUmBK * 2;             // 16 KiB: activations of a chunk at M = 128
@@ -119,7 +120,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
 
-    // The three serial roles walk with their whole warp and let one elected lane issue: see ptx::elect_one.
+    // The three serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
     if (warp == kUmRawWarp) {
         // -------------------------------------------------------------- raw weights, scales, zero points: three TMA boxes per chunk
         uint32_t stage = 0, phase = 0;
