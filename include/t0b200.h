@@ -466,8 +466,10 @@ int t0_w4_dequant(t0_runtime* rt, uint64_t packed, uint64_t scales, uint64_t zer
  *   M <= 16 (N % 32 == 0, K % 128 == 0, group % 128 == 0): one fused kernel on this row layout.  The row layout puts the 16 KiB
  *     a CTA needs per step in sixteen pieces 4N bytes apart, so this entry is the slower of the two M <= 16 entries;
  *     the fast one is t0_w4a16_gemm_prepacked below, on weights rewritten once by t0_w4_prepack;
- *   16 < M <= 128 (N % 32 == 0, K % 64 == 0, group % 64 == 0, 16-byte aligned pointers): one fused tcgen05 kernel, weights
- *     dequantised into the shared-memory operand inside the main loop, split along K across a thread-block cluster;
+ *   16 < M <= 128 (N % 32 == 0, K % 64 == 0, group % 64 == 0, 16-byte aligned pointers): one fused tcgen05 kernel, weights dequantised inside
+ *     the main loop.  By shape the column tiles are taken whole, cut along K between CTAs (the parts meet in the runtime's buffer, in k order) or
+ *     split along K over a thread-block cluster; a call being recorded is never cut between CTAs.  Repeated calls agree bit for bit, a recorded
+ *     and an eager one to rounding;
  *   anything else: dequantise once into runtime scratch (allocated on first use, K*N*2 bytes), then the bf16 GEMM. */
 int t0_w4a16_gemm(t0_runtime* rt, uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t y, uint32_t M, uint32_t N,
                   uint32_t K, uint32_t group);
@@ -480,9 +482,9 @@ typedef struct t0_w4a16_args {
 int t0_w4a16_gemm_batch(t0_runtime* rt, const t0_w4a16_args* args, size_t count);
 /* `count` INDEPENDENT problems (no y is the a or the y of another: checked, T0_ERR_INVALID).  Where they share one shape with
  * 16 < M <= 128 that the fused tcgen05 kernel takes, up to 32 of them run in ONE launch whose CTAs walk the column tiles of all
- * the problems: K is then not split, so launch, prologue and the exchange between the parts of K are paid once per launch
- * instead of once per GEMM (the projections of a decode or small-batch prefill step that read the same input).  The fp32
- * sums run along K in one piece, so y agrees with t0_w4a16_gemm to rounding, not bit for bit.  Anything else is submitted
+ * the problems, so launch and prologue are paid once per launch instead of once per GEMM (the projections of a decode or small-batch prefill step that
+ * read the same input).  Tiles are taken whole, all of K in one sum, or cut along K where whole ones would leave SMs idle (not
+ * while recording), so y agrees with t0_w4a16_gemm to rounding, not bit for bit.  Anything else is submitted
  * back to back as by t0_w4a16_gemm_batch. */
 int t0_w4a16_gemm_grouped(t0_runtime* rt, const t0_w4a16_args* args, size_t count);
 /* Streaming weight layout for the fused kernel (no counterpart in the reference).  The row layout above puts the 16 KiB
@@ -514,7 +516,7 @@ int t0_w4a16_gemm_prepacked_batch(t0_runtime* rt, const t0_w4a16_args* args, siz
  * which the kernels' pairwise extraction yields consecutive k.  K % 64 == 0, group % 64 == 0, group | K; any N.
  * t0_w4a16_gemm_tiled computes the same product as t0_w4a16_gemm from that buffer (M <= 128; y f32 [M,N]);
  * t0_w4a16_gemm_tiled_grouped takes INDEPENDENT problems (checked) whose .packed is the tile-major buffer (.scales / .zeros are
- * ignored) and runs consecutive problems of one shape up to 32 per launch: K is then not split, and the dequantised weights
+ * ignored) and runs consecutive problems of one shape up to 32 per launch, tiles whole or cut as by t0_w4a16_gemm_grouped; the dequantised weights
  * are the tensor-memory operand of the UMMAs (they never pass through shared memory). */
 size_t t0_w4_tiled_bytes(uint32_t K, uint32_t N, uint32_t group);
 int t0_w4_to_tiled(t0_runtime* rt, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t out, uint32_t K, uint32_t N, uint32_t group);
