@@ -429,7 +429,12 @@ int w4a16_umma_reserve(t0_runtime* rt) {
     if (need <= rt->scratch_um.size) return T0_OK;
     int rc = ensure_scratch(rt, rt->scratch_um, need);
     if (rc != T0_OK) return rc;
-    T0_CUDA(cudaMemsetAsync(rt->scratch_um.ptr, 0, kUmCounterBytes, rt->stream));
+    const cudaError_t e = cudaMemsetAsync(rt->scratch_um.ptr, 0, kUmCounterBytes, rt->stream);
+    if (e != cudaSuccess) {                // counters that may hold anything: no buffer then
+        cudaFree(rt->scratch_um.ptr);
+        rt->scratch_um = Scratch();
+        return fail(T0_ERR_CUDA, "clearing the counters of cut tiles: %s", cudaGetErrorString(e));
+    }
     return T0_OK;
 }
 
