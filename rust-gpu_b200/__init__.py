@@ -770,7 +770,7 @@ class GpuRuntime:
         """``t0_w4_to_tiled``: the weights rewritten into the tile-major layout (a new buffer)."""
         n = int(lib().t0_w4_tiled_bytes(K, N, group))
         if n == 0:
-            raise T0Error(f"the tile-major layout does not take K={K} group={group}")
+            raise T0Error(6, f"the tile-major layout does not take K={K} group={group}")
         out = self.alloc(n)
         _check(lib().t0_w4_to_tiled(self._h, packed, scales, zeros, out.gpu_addr(), K, N, group))
         return out

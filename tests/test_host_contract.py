@@ -253,6 +253,14 @@ def test_no_gpu_means_loud_failure(t0):
     assert "no CPU fallback" in str(e.value)
 
 
+def test_layouts_that_do_not_take_a_shape_say_so(t0):
+    # refused before the runtime is touched: K or the group is no multiple of what the layout stores
+    for convert, k in ((t0.GpuRuntime.w4_to_tiled, 100), (t0.GpuRuntime.w4_prepack, 192)):
+        with pytest.raises(t0.T0Error) as e:
+            convert(None, 0, 0, 0, k, 256, 64)
+        assert e.value.code == 6
+
+
 def test_warp_layout_planners(t0):
     # the reference's own known answers: src/t0/tile_ir.rs:8552-8618
     l = t0.WarpLayout.row_dominant(4, 128, 64)
