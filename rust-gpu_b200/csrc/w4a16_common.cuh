@@ -94,6 +94,12 @@ __device__ __forceinline__ uint32_t um_lds16(uint32_t addr) {
     return v;
 }
 
+__device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // The eight codes of a packed word as bf16x2 pairs in k order, (0,1) (2,3) (4,5) (6,7): (code | 0x4300) is the bf16 128 + code, so minus (128 + z),
 // times s, is (q - z) * s rounded once.  zz = (128 + z) and ss = s, both halves alike.
 __device__ __forceinline__ void um_dequant_word(uint32_t wd, uint32_t mask, uint32_t magic, uint32_t zz, uint32_t ss, bool tiled, uint32_t (&o)[4]) {

@@ -8,26 +8,26 @@
 // y[m,n] = sum_k a[m,k] * w[k,n],  w = RNE_bf16((q - z) * s),  fp32 accumulate.  The int4 weights are ~97 % of the bytes,
 // so the kernel is organised around streaming them exactly once at HBM rate:
 //   * weights come in the layout of t0_w4_prepack: per (256-column band, 128-deep k step) one contiguous 16 KiB tile whose
-//     words are already in mma.sync fragment order; a "unit" is one such tile.  The units of ALL problems of a launch form
+//     words are in 16 x 16 fragment order; a "unit" is one such tile.  The units of ALL problems of a launch form
 //     one list, cut into equal contiguous ranges, one per CTA (one CTA per SM), so that launch, pipeline fill and the band
 //     fix-up at the end of a range are paid once per launch instead of once per problem;
-//   * warp 16 (one lane) streams the tiles of the range into a ring of stages with one 16 KiB bulk copy each;
-//   * warps 17..19 prepare, one step each in turn and a few steps ahead of the consumers, what else a step needs in the
-//     same stage: the activations of the step as mma.sync B fragments, and per column pair the words {128+z, s} the
-//     dequantisation uses, so that a consumer gets them with one 16-byte load and no decoding;
-//   * warps 0..15 (consumers): warps 2i and 2i + 1 own columns 32i .. 32i + 31 of the band, each one k half of every step: two
-//     LDS.128 fetch a lane's eight packed words; nibble pairs become bf16x2 with one LOP3 (0x4300 | q is the bf16 128+q), minus
-//     (128+z), times s - bit-identical to the oracle because (q-z)*s is rounded once - and every dequantised word IS the
-//     16 x 16 A fragment of one mma.sync.m16n8k16 whose 8-column B operand is the activations.  The two halves meet in shared
-//     memory when a band ends.
-//     What bounds this loop is the instructions around the arithmetic as much as the arithmetic (15 per packed word of 8 codes, 8 words
-//     per warp and step) and, with two row groups, the rate of mma.sync (leaving the dequantisation out changes nothing at M = 16).  A
-//     warp that owned 16 columns and the whole k of a step read all the activation fragments of the step for half the columns, and 21
-//     warps left 80 registers a thread: 12 problems of M = 1, N = 11008, K = 4096 took 80.2 us, 73.8 so; two of them 19.3 and 18.6.
-//   * a band that lies wholly inside a range is stored directly; a band shared by several CTAs is finished by whichever
-//     CTA arrives last (per-band arrival counter, partial pieces in scratch, added in k order: deterministic, repeated
-//     calls agree bit for bit); no CTA ever waits for another.  A spare lane of the producer warp counts a range's leading
-//     partial band in while the consumers go on.
+//   * one warp streams the range into a ring of stages: per step the 16 KiB tile, its scales and zero points (three bulk copies) and
+//     the step's activations (two TMA boxes of 16 rows x 64 k, 128-byte swizzle, rows beyond M read as zero);
+//   * sixteen warps dequantise, eight of them (32 columns each) per step in turn: nibble pairs become bf16x2 with one LOP3 (0x4300 | q is the
+//     bf16 128+q), minus (128+z), times s - bit-identical to the oracle because (q-z)*s is rounded once - and every word IS the 16 x 16
+//     fragment that tcgen05.st.16x128b puts into tensor memory, where the weights are the 128-row A operand;
+//   * two warps, one per half of the band's columns, issue tcgen05.mma 128 x 16 x 16, the activations being the B operand in shared memory as TMA
+//     delivers them.  The accumulator is y transposed (lane = column of y).  Four accumulators, by k step modulo four, keep the sums as short as
+//     they were on mma.sync (two warps with two accumulators each);
+//   * four warps empty the accumulators: a band that lies wholly inside a range is stored directly; a band shared by several CTAs is finished by
+//     whichever CTA arrives last (per-band arrival counter, partial pieces in scratch, added in k order: deterministic, repeated calls agree bit
+//     for bit); no CTA ever waits for another.  A spare warp counts a range's leading partial band in meanwhile.
+// What bounds the loop is the pipes of the dequantisation (15 instructions per packed word, on two pipes that take one per two cycles; a step is 512 cycles
+// of theirs at the least and takes about 940), then HBM (710).  Everything else was taken off the dequantising warps' schedulers: with mma.sync the
+// products and the activation fragments were theirs as well.  Two problems of M = 1, N = 11008, K = 4096: 18.6 us with mma.sync, 17.2 so; four of M = 16,
+// N = 14336: 53.2 and 35.6.  On the way there: one issuing warp, its instructions behind a branch and not predicated, a division per step in
+// the producer, waits between the arithmetic and its stores: 38.3 at M = 16.  Tried and taken back: three groups of eight dequantising warps (35.8),
+// a warp that prepares scales and zero points for them (35.9), barriers tested a step ahead (36.7).
 // Every barrier wait is bounded; a wait that runs out raises the CTA's abort flag, the roles unwind, the status word is
 // written and the host reports T0_ERR_TIMEOUT.
 #include "w4a16_common.cuh"
@@ -37,48 +37,70 @@ using namespace t0::w4;
 
 namespace {
 
-constexpr int kStConsumers = 16;                      // consumer warps: warp w owns columns 32 (w / 2) .. + 31 of the band, k half w % 2 of every step
-constexpr int kStHelpers = 3;                         // warps that prepare activations and scale / zero-point words
-constexpr int kStProducerWarp = kStConsumers;
-constexpr int kStHelperWarp0 = kStConsumers + 1;
-constexpr int kStThreads = (kStHelperWarp0 + kStHelpers) * 32;    // 640: five warps per scheduler, which leaves 96 registers a thread
-constexpr int kStSzBytes = 2048;                      // per stage: [16 warps][8 g] uint4 {128+z(col), s(col), 128+z(col+8), s(col+8)} as bf16x2 pairs
-constexpr int kStAFragBytes = 2048;                   // per stage and group of eight rows: [2 j][2 pr][32 lanes] uint4 B fragments
-constexpr int kStMaxProblems = 32;                    // problems per launch (the table travels as a kernel parameter)
-
-__host__ __device__ constexpr int st_stage_bytes(int m_groups) { return kWeightBytes + kStSzBytes + m_groups * kStAFragBytes; }
-__host__ __device__ constexpr int st_stages(int m_groups) { return m_groups == 1 ? 10 : 9; }
-__host__ __device__ constexpr int st_exchange_bytes(int m_groups) { return kStConsumers * m_groups * 512; }     // one accumulator fragment per warp and row group
-__host__ __device__ constexpr size_t st_smem_bytes(int m_groups) {
-    return 128 + (size_t)st_stages(m_groups) * st_stage_bytes(m_groups) + 256 + st_exchange_bytes(m_groups);
-}
+constexpr int kStDqWarps = 16;                        // dequantising warps: warp w owns columns 32 (w % 8) .. + 31 of the band in every second step, w / 8 saying which
+constexpr int kStEpWarps = 4;                         // empty the accumulators (one per tensor-memory lane quadrant)
+constexpr int kStProducerWarp = 0, kStIssueWarp0 = 1; // two warps issue the UMMAs, one per 128-column half of the band
+constexpr int kStHeadWarp = 3;                        // counts in the first piece of a range
+constexpr int kStEpWarp0 = 4, kStDqWarp0 = 8;
+constexpr int kStThreads = (kStDqWarp0 + kStDqWarps) * 32;
+constexpr int kStMRows = 16;                          // rows of the activations the UMMAs take
+constexpr int kStSzOff = kWeightBytes;                // in a stage: the tile, scales and zero points, activations
+constexpr int kStXOff = kWeightBytes + 1024;
+constexpr int kStXChunk = kStMRows * 128;             // 64 k of the activations
+constexpr int kStStageBytes = kStXOff + 2 * kStXChunk;
+constexpr int kStStages = 10;
+constexpr int kStTxBytes = kWeightBytes + kScaleBytes + kZeroBytes + 2 * kStXChunk;
+// Tensor memory (512 columns): the accumulators [half of the band][k step % 4] x 16, then three A stages, a step each: [half][k step] x 8 columns.
+constexpr uint32_t kStTmemCols = 512;
+constexpr uint32_t kStAccCols = 128;
+constexpr uint32_t kStAStages = 3;
+constexpr uint32_t kStAStageCols = 128;
+constexpr uint32_t kStBars = 2 * kStStages + 4 * kStAStages + 4;
+constexpr size_t kStSmem = 1024 + (size_t)kStStages * kStStageBytes + kStBars * 8;      // (more than half an SM's: two CTAs must never share its tensor memory)
 
 struct StProblem {
-    const uint16_t* a;         // [M][K] bf16
     float* y;                  // [M][N] f32
     const uint8_t* tiles;      // [band][kstep][16][256] u32
     const uint8_t* scales_t;   // [band][K/G][256] bf16
     const uint8_t* zeros_t;    // [band][K/G][32] u32
-    uint32_t M, N, K;
+    uint32_t M, N;
     uint32_t ksteps, groups, units_per_group, n_bands;
     uint32_t unit_begin;       // first unit of this problem in the launch's list
     uint32_t band_begin;       // first arrival counter of this problem
-    uint32_t _pad;
 };
 
+template <uint32_t kProblems>
 struct StParams {
-    StProblem prob[kStMaxProblems];
+    CUtensorMap x[kProblems];  // activations, boxes of 16 rows x 64 k
+    StProblem prob[kProblems];
     float* partials;           // [grid][2][16*256]
     int* counters;             // one per band of the launch, zero between launches
     int* status;               // error word of the runtime (bounded waits)
     unsigned long long* stamps;   // optional trace: 4 nanosecond stamps per CTA (entry, first step landed, loop done, exit)
     uint64_t wait_limit_ns;
     uint32_t n_problems, total_units;
+    uint32_t per_cta, rest;    // total_units = grid * per_cta + rest
+    float cta_per_unit;        // grid / total_units
 };
+constexpr uint32_t kStMaxProblems = 32;               // problems per launch (the table travels as a kernel parameter) ...
+constexpr uint32_t kStFewProblems = 4;                // ... or as a parameter of a seventh of the size
+
+// First unit of a CTA's range, floor(cta * total / grid), and the CTA whose range holds a unit: without the 64-bit divisions, which take hundreds of cycles
+// where a band is finished.
+template <class Params>
+__device__ __forceinline__ uint32_t st_begin(const Params& P, uint32_t cta) { return cta * P.per_cta + cta * P.rest / gridDim.x; }
+template <class Params>
+__device__ __forceinline__ uint32_t st_owner(const Params& P, uint32_t unit) {
+    uint32_t c = (uint32_t)((float)unit * P.cta_per_unit);     // off by a CTA at most
+    if (st_begin(P, c) > unit) --c;
+    if (c + 1 < gridDim.x && st_begin(P, c + 1) <= unit) ++c;
+    return c;
+}
 
 struct Cursor { uint32_t p, band, ks; };
 
-__device__ __forceinline__ Cursor locate(const StParams& P, uint32_t unit) {
+template <class Params>
+__device__ __forceinline__ Cursor locate(const Params& P, uint32_t unit) {
     Cursor c;
     c.p = 0;
     while (c.p + 1 < P.n_problems && P.prob[c.p + 1].unit_begin <= unit) ++c.p;
@@ -87,16 +109,14 @@ __device__ __forceinline__ Cursor locate(const StParams& P, uint32_t unit) {
     c.ks = r - c.band * ks;
     return c;
 }
-__device__ __forceinline__ void advance(const StParams& P, Cursor& c) {
-    if (++c.ks == P.prob[c.p].ksteps) {
-        c.ks = 0;
-        if (++c.band == P.prob[c.p].n_bands) { c.band = 0; ++c.p; }
-    }
-}
 
-// the two warps of a column pair (barriers 2..9; 1 is the consumers')
-__device__ __forceinline__ void st_pair_sync(uint32_t pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 2) : "memory"); }
-__device__ __forceinline__ void st_consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStConsumers * 32) : "memory"); }
+constexpr uint32_t kStFinishers = kStDqWarps * 32;    // threads that finish a cut band ...
+constexpr uint32_t kStInFlight = 8;                   // ... each with so many 16-byte loads of contributors' pieces under way together
+
+// barriers 1: the epilogue warps, 2: these and the dequantising warps, 3: the dequantising warps
+__device__ __forceinline__ void st_epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStEpWarps * 32) : "memory"); }
+__device__ __forceinline__ void st_tail_sync() { asm volatile("bar.sync 2, %0;" ::"n"((kStDqWarps + kStEpWarps) * 32) : "memory"); }
+__device__ __forceinline__ void st_finishers_sync() { asm volatile("bar.sync 3, %0;" ::"n"(kStFinishers) : "memory"); }
 // explicit shared-space accesses: the ring's address went through an integer for alignment, so plain pointers would make
 // the compiler use generic loads and 64-bit address arithmetic
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
@@ -104,386 +124,466 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
+
 __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+// Item i of a band's outputs: four columns of a row.
+__device__ __forceinline__ void st_store4(const StProblem& pr, uint32_t band, uint32_t i, const float4& v) {
+    const uint32_t row = i / (kBandCols / 4), col = band * kBandCols + (i % (kBandCols / 4)) * 4;
+    const float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+        if (col + j < pr.N) pr.y[(size_t)row * pr.N + col + j] = o[j];
+}
 
-template <int kMGroups>    // 1: every M <= 8, 2: M <= 16
+// The CTAs that share a cut band.  Only the first can hold the band in slot 1 of its two pieces (its range began in the band before).
+struct StShare { uint32_t first, last, first_slot; };
+template <class Params>
+__device__ __forceinline__ StShare st_share(const Params& P, uint32_t first_unit, uint32_t ksteps) {
+    StShare h;
+    h.first = st_owner(P, first_unit);
+    h.last = st_owner(P, first_unit + ksteps - 1);
+    h.first_slot = st_begin(P, h.first) < first_unit ? 1u : 0u;
+    return h;
+}
+template <class Params>
+__device__ __forceinline__ const float* st_piece(const Params& P, const StShare& h, uint32_t cta) {
+    return P.partials + ((size_t)cta * 2 + (cta == h.first ? h.first_slot : 0u)) * kPieceFloats;
+}
+
+// The CTA that contributes last to a band adds the pieces and stores; nobody waits for anybody.  By its dequantising warps: a thread has four columns of a row,
+// and where that leaves threads over, up to eight of them make a sum, which add parts of the list of contributors and then, through shared memory, each
+// other's: always in the same order, whoever does it.  (A band of N = 1024, K = 4096 has 32 contributors, whose pieces one thread fetches in eight round trips
+// of 0.7 us.)  The shares are worked out before it is known who finishes, since a division takes longer than such a warp has then.
+struct StFinish {
+    StShare h;
+    uint32_t p, band, items, groups, g, i, begin, end;
+};
+template <class Params>
+__device__ __forceinline__ StFinish st_finish(const Params& P, uint32_t p, uint32_t band, uint32_t t) {
+    StFinish f;
+    const StProblem& pr = P.prob[p];
+    f.h = st_share(P, pr.unit_begin + band * pr.ksteps, pr.ksteps);
+    f.p = p; f.band = band;
+    f.items = pr.M * (kBandCols / 4);
+    const uint32_t count = f.h.last - f.h.first + 1;
+    f.groups = max(1u, min(min(8u, kStFinishers / f.items), (count + kStInFlight - 1) / kStInFlight));
+    f.g = f.groups > 1 ? t / f.items : 0;
+    f.i = t - f.g * f.items;
+    const uint32_t per = (count + f.groups - 1) / f.groups;
+    f.begin = f.h.first + f.g * per;
+    f.end = f.g < f.groups ? min(f.begin + per, f.h.last + 1) : 0;
+    return f;
+}
+// The sums of kItems items of a thread over its contributors, in CTA order, one contributor after the other.
+template <uint32_t kItems, class Params>
+__device__ __forceinline__ void st_add_pieces(const Params& P, const StFinish& f, float4 (&sum)[kItems]) {
+    constexpr uint32_t kCo = kStInFlight / kItems;
+    const float4* piece = (const float4*)st_piece(P, f.h, f.begin);
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t c = f.begin; c < f.end; c += kCo) {
+        float4 v[kCo][kItems];
+#pragma unroll
+        for (uint32_t b = 0; b < kCo; ++b) {
+            const float4* src = (c + b == f.begin ? piece : (const float4*)(P.partials + (size_t)(c + b) * 2 * kPieceFloats)) + f.i;
+#pragma unroll
+            for (uint32_t j = 0; j < kItems; ++j) {
+                v[b][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c + b < f.end && f.i + j * kStFinishers < f.items) v[b][j] = __ldcg(src + j * kStFinishers);
+            }
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < kCo; ++b)
+#pragma unroll
+            for (uint32_t j = 0; j < kItems; ++j) {
+                sum[j].x += v[b][j].x; sum[j].y += v[b][j].y; sum[j].z += v[b][j].z; sum[j].w += v[b][j].w;
+            }
+    }
+}
+template <class Params>
+__device__ __forceinline__ void st_reduce_band(const Params& P, const StFinish& f, uint32_t t, uint32_t exchange) {
+    const StProblem& pr = P.prob[f.p];
+    if (f.items > kStFinishers) {                     // M > 8: two items a thread (16 * 64 at most)
+        float4 sum[2];
+        st_add_pieces<2>(P, f, sum);
+        st_store4(pr, f.band, f.i, sum[0]);
+        if (f.i + kStFinishers < f.items) st_store4(pr, f.band, f.i + kStFinishers, sum[1]);
+    } else {
+        float4 sum[1];
+        if (f.g < f.groups && f.i < f.items) {
+            st_add_pieces<1>(P, f, sum);
+            if (f.groups == 1) st_store4(pr, f.band, f.i, sum[0]);
+            else sts128(exchange + (f.g * f.items + f.i) * 16, make_uint4(__float_as_uint(sum[0].x), __float_as_uint(sum[0].y), __float_as_uint(sum[0].z), __float_as_uint(sum[0].w)));
+        }
+        if (f.groups > 1) {
+            st_finishers_sync();
+            if (t < f.items) {
+                sum[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (uint32_t j = 0; j < f.groups; ++j) {
+                    const uint4 v = lds128(exchange + (j * f.items + t) * 16);
+                    sum[0].x += __uint_as_float(v.x); sum[0].y += __uint_as_float(v.y); sum[0].z += __uint_as_float(v.z); sum[0].w += __uint_as_float(v.w);
+                }
+                st_store4(pr, f.band, t, sum[0]);
+            }
+            st_finishers_sync();                      // (the exchange is free again)
+        }
+    }
+    if (t == 0) P.counters[pr.band_begin + f.band] = 0;   // ready for the next launch
+}
+
+template <uint32_t kProblems>
 __global__ void __launch_bounds__(kStThreads, 1)
-w4a16_stream_kernel(const __grid_constant__ StParams P) {
-    constexpr int kSt = st_stages(kMGroups);
-    constexpr int kSB = st_stage_bytes(kMGroups);
+w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
     extern __shared__ uint8_t smem_raw[];
-    const uint32_t ring = (ptx::smem_u32(smem_raw) + 127u) & ~127u;      // kSt x {16 KiB tile, 2 KiB scale/zero words, kMGroups x 2 KiB B fragments}
-    const uint32_t full_bar = ring + kSt * kSB;                          // [kSt] x 8 bytes
-    const uint32_t empty_bar = full_bar + kSt * 8;
-    const uint32_t head_written_bar = empty_bar + kSt * 8;               // all 16 consumer warps have stored their part of the head piece
-    const uint32_t head_counted_bar = head_written_bar + 8;              // the head piece is counted in and s_head_last is valid
-    const uint32_t exchange = full_bar + 256;                            // [16 warps][kMGroups][32 lanes] float4
-    __shared__ int s_flags[4];
-    volatile int* abort_flag = &s_flags[0];
-    int* s_last = &s_flags[1];
-    int* s_head_last = &s_flags[2];                                      // 1 when this CTA turned out to be the last contributor of its head band
+    const uint32_t ring = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t full_bar = ring + kStStages * kStStageBytes;          // the stage's bytes have landed
+    const uint32_t empty_bar = full_bar + kStStages * 8;                 // read by eight dequantising warps and the UMMAs
+    const uint32_t a_full = empty_bar + kStStages * 8;                   // A stages, [half][stage]: four warps have written their step
+    const uint32_t a_empty = a_full + 2 * kStAStages * 8;
+    const uint32_t acc_full = a_empty + 2 * kStAStages * 8;              // accumulators
+    const uint32_t acc_empty = acc_full + 8;
+    const uint32_t head_written = acc_empty + 8;                         // the epilogue warps have stored the head piece
+    const uint32_t head_counted = head_written + 8;                      // it is counted in and s_head_last is valid
+    __shared__ uint32_t tmem_holder;
+    __shared__ int s_abort, s_last, s_all, s_head_last, s_head_go;
+    volatile int* abort_flag = &s_abort;
 
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t U0 = range_begin(blockIdx.x, gridDim.x, P.total_units);
-    const uint32_t U1 = range_begin(blockIdx.x + 1, gridDim.x, P.total_units);
-    if (U0 >= U1) return;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;     // (the shuffle tells the compiler that a role is the whole warp's)
+    const uint32_t U0 = st_begin(P, blockIdx.x);
+    const uint32_t U1 = st_begin(P, blockIdx.x + 1);
     auto stamp = [&](int i) {
         if (P.stamps) P.stamps[blockIdx.x * 4 + i] = ptx::globaltimer_ns();
     };
     if (tid == 0) {
-        for (int s = 0; s < kSt; ++s) {
-            ptx::mbar_init(full_bar + s * 8, 2);                 // the tile's bytes (producer) + the prepared words (a helper warp)
-            ptx::mbar_init(empty_bar + s * 8, kStConsumers);
+        for (int s = 0; s < kStStages; ++s) {
+            ptx::mbar_init(full_bar + s * 8, 1);
+            ptx::mbar_init(empty_bar + s * 8, kStDqWarps / 2);
         }
-        ptx::mbar_init(head_written_bar, kStConsumers);
-        ptx::mbar_init(head_counted_bar, 1);
-        *abort_flag = 0;
-        *s_head_last = 0;
+        for (uint32_t s = 0; s < 2 * kStAStages; ++s) {
+            ptx::mbar_init(a_full + s * 8, kStDqWarps / 4);
+            ptx::mbar_init(a_empty + s * 8, 1);
+        }
+        ptx::mbar_init(acc_full, 2);
+        ptx::mbar_init(acc_empty, kStEpWarps);
+        ptx::mbar_init(head_written, kStEpWarps);
+        ptx::mbar_init(head_counted, 1);
+        s_abort = 0;
+        s_last = s_all = s_head_last = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
     }
+    if (warp == kStIssueWarp0) {
+        ptx::tmem_alloc(ptx::smem_u32(&tmem_holder), kStTmemCols);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before_sync();
     __syncthreads();
+    ptx::tc_fence_after_sync();
+    constexpr uint32_t tmem_base = 0;    // all columns are allocated: tensor-memory addresses are constants
     ptx::grid_launch_dependents();
     const Cursor c0 = locate(P, U0);
-    const uint32_t n_units = U1 - U0;
+    Cursor c = c0;
+    if (warp == kStProducerWarp && lane == 0) ptx::tma_prefetch_desc(&P.x[c.p]);
     ptx::grid_dependency_wait();      // global memory is read and written only after the previous grid in the stream is done
     if (tid == 0) stamp(0);
-    // A head piece: the range starts inside a band and goes on into the next one.  Counting it in (fence, atomic round
-    // trip) is the head warp's job, so no consumer warp falls behind the others while the range goes on.
-    const uint32_t head_end = U0 - c0.ks + P.prob[c0.p].ksteps;    // one past the last unit of the first band
-    const bool has_head = c0.ks != 0 && head_end < U1;
-
-    if (warp == kStProducerWarp) {
-        if (lane == 1 && has_head) {
-            // ------------------------------------------------------------ lane 1 counts the head piece in (while lane 0 streams)
+    // the last piece of the range (the steps of one band this CTA owns) goes on in the next CTA, or began in the one before
+    const Cursor c_end = locate(P, U1 - 1);
+    const uint32_t end_first = P.prob[c_end.p].unit_begin + c_end.band * P.prob[c_end.p].ksteps;
+    const bool tail_cut = end_first < U0 || end_first + P.prob[c_end.p].ksteps > U1;
+    // A head piece: the range starts inside a band and goes on into the next one.  Counting it in (fence, atomic round trip) is a spare warp's job, so
+    // that the epilogue warps are there for the last piece, which may come soon.
+    const uint32_t head_first = U0 - c0.ks, head_ksteps = P.prob[c0.p].ksteps;
+    const bool has_head = c0.ks != 0 && head_first + head_ksteps < U1;
+    // The serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
+    if (warp == kStHeadWarp) {
+        if (lane == 0 && has_head) {
             int last = 0;
-            if (ptx::mbar_wait_relaxed(head_written_bar, 0, abort_flag, P.wait_limit_ns, 1000)) {
-                const uint32_t first_unit = head_end - P.prob[c0.p].ksteps;
-                const uint32_t c_first = owner_of(first_unit, gridDim.x, P.total_units);
-                const uint32_t c_last = owner_of(head_end - 1, gridDim.x, P.total_units);
-                __threadfence();                   // the piece is visible before this CTA is counted
-                last = atomicAdd(&P.counters[P.prob[c0.p].band_begin + c0.band], 1) == (int)(c_last - c_first);
+            if (ptx::mbar_wait(head_written, 0, abort_flag, P.wait_limit_ns)) {
+                const StShare h = st_share(P, head_first, head_ksteps);
+                __threadfence();                       // the piece is visible before this CTA is counted
+                last = atomicAdd(&P.counters[P.prob[c0.p].band_begin + c0.band], 1) == (int)(h.last - h.first);
                 if (last) __threadfence();
             } else {
                 atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xD00000);
             }
-            *s_head_last = last;                   // looked at when the range is done
-            ptx::mbar_arrive(head_counted_bar);
+            s_head_last = last;
+            ptx::mbar_arrive(head_counted);
         }
-        // ------------------------------------------------------------ lane 0, producer: one 16 KiB bulk copy per step
-        if (lane == 0) {
-            Cursor c = c0;
-            uint32_t stage = 0, phase = 0;
-            const uint8_t* src = P.prob[c.p].tiles + ((size_t)c.band * P.prob[c.p].ksteps + c.ks) * kWeightBytes;
-            for (uint32_t u = U0; u < U1; ++u) {
-                if (!ptx::mbar_wait_relaxed(empty_bar + stage * 8, phase ^ 1, abort_flag, P.wait_limit_ns, 100)) {
-                    atomicCAS(P.status, 0, kStatusProducerTimeout | (int)(u & 0xFFFFFF));
+    } else if (warp == kStProducerWarp) {
+        // (A problem's tiles lie one behind the other in the order of its units, its rows of scales and zero points likewise: running addresses.  The chain of
+        // this warp is kept short: with a division per step it took 800 cycles a step from the four dequantising warps it shares a scheduler with.)
+        uint32_t stage = 0, phase = 0;
+        for (uint32_t u = U0; u < U1; ++c.p) {
+            const StProblem& pr = P.prob[c.p];
+            const uint32_t at = u - pr.unit_begin, row = at / pr.units_per_group, u_stop = min(U1, pr.unit_begin + pr.ksteps * pr.n_bands);
+            const uint8_t* tile = pr.tiles + (size_t)at * kWeightBytes;
+            const uint8_t* scales = pr.scales_t + (size_t)row * kScaleBytes;
+            const uint8_t* zeros = pr.zeros_t + (size_t)row * kZeroBytes;
+            uint32_t in_row = at - row * pr.units_per_group, k = (at % pr.ksteps) * kUnitK;
+            bool ok = true;
+            for (; u < u_stop; ++u) {
+                ok = ptx::mbar_wait_warp(empty_bar + stage * 8, phase ^ 1, abort_flag, P.wait_limit_ns);
+                if (!ok) break;
+                const uint32_t dst = ring + stage * kStStageBytes, fb = full_bar + stage * 8;
+                if (ptx::elect_one()) {
+                    ptx::fence_proxy_async_smem();       // the stage was read through the generic proxy, the copies write it through the async proxy
+                    ptx::mbar_arrive_expect_tx(fb, kStTxBytes);
+                    ptx::bulk_load(dst, tile, kWeightBytes, fb);
+                    ptx::bulk_load(dst + kStSzOff, scales, kScaleBytes, fb);
+                    ptx::bulk_load(dst + kStSzOff + kScaleBytes, zeros, kZeroBytes, fb);
+                    ptx::tma_load_3d(dst + kStXOff, &P.x[c.p], fb, (int32_t)k, 0, 0);
+                    ptx::tma_load_3d(dst + kStXOff + kStXChunk, &P.x[c.p], fb, (int32_t)k + 64, 0, 0);
+                }
+                __syncwarp();
+                if (++stage == kStStages) { stage = 0; phase ^= 1; }
+                tile += kWeightBytes;
+                if (++in_row == pr.units_per_group) { in_row = 0; scales += kScaleBytes; zeros += kZeroBytes; }
+                k += kUnitK;
+                if (k == pr.ksteps * kUnitK) k = 0;
+            }
+            if (!ok) {
+                if (lane == 0) atomicCAS(P.status, 0, kStatusProducerTimeout | (int)(u & 0xFFFFFF));
+                break;
+            }
+        }
+    } else if (warp < kStHeadWarp) {
+        // -------------------------------------------------------------- UMMA issuers: per 64 k four k steps of M 128 x N 16 x K 16
+        constexpr uint32_t idesc = ptx::make_idesc_bf16_f32(128, kStMRows, 0u);
+        const uint32_t t = warp - kStIssueWarp0;
+        const uint32_t my_full = a_full + t * kStAStages * 8, my_empty = a_empty + t * kStAStages * 8;
+        const uint32_t x0 = ((ring + kStXOff) & 0x3FFFFu) >> 4;      // addresses enter a descriptor in 16-byte units
+        uint32_t x = x0, aphase = 0, piece = 0, as = 0;
+        const uint32_t acc = t * 64;
+        bool ok = true;
+        for (uint32_t u = U0; ok && u < U1; ++piece) {
+            const uint32_t u_end = min(U1, u + P.prob[c.p].ksteps - c.ks);
+            if (piece > 0 && !ptx::mbar_wait_warp(acc_empty, (piece & 1) ^ 1, abort_flag, P.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(P.status, 0, kStatusMmaTimeout | 0x800000);
+                break;
+            }
+            for (uint32_t first = 1; u < u_end; ++u, first = 0) {
+                // (what the dequantising warps waited for before they signal includes the activations of the step)
+                if (!ptx::mbar_wait_warp(my_full + as * 8, aphase, abort_flag, P.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(P.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
+                    ok = false;
                     break;
                 }
-                // The consumers read the stage through the generic proxy (their reads are ordered before this point by
-                // their release-arrive and the acquire-wait above); the copy overwrites it through the async proxy, and
-                // this fence orders the two.  Without a proxy fence, launches with cold TLBs consumed sectors of the
-                // step loaded into the same stage a ring later.
-                ptx::fence_proxy_async_smem();
-                const uint32_t fb = full_bar + stage * 8;
-                ptx::mbar_arrive_expect_tx(fb, kWeightBytes);
-                ptx::bulk_load(ring + stage * kSB, src, kWeightBytes, fb);
-                if (++stage == kSt) { stage = 0; phase ^= 1; }
-                // the tiles of one problem are consecutive in memory in the order the range walks them
-                src += kWeightBytes;
-                if (++c.ks == P.prob[c.p].ksteps) {
-                    c.ks = 0;
-                    if (++c.band == P.prob[c.p].n_bands) { c.band = 0; ++c.p; if (u + 1 < U1) src = P.prob[c.p].tiles; }
-                }
-            }
-        }
-        return;
-    }
-    if (warp >= kStHelperWarp0) {
-        // ------------------------------------------------------------ helpers: step i of the range is prepared by helper i % kStHelpers
-        const uint32_t h = warp - kStHelperWarp0;
-        if (h >= n_units) return;
-        Cursor c = c0;
-        for (uint32_t k = 0; k < h; ++k) advance(P, c);
-        const uint32_t g = lane >> 2, t = lane & 3;
-        const uint32_t w2 = lane >> 1, hh = lane & 1;          // scale / zero-point words: this lane makes entries 8 w2 + 4 hh + 0..3
-        uint32_t cur_p = 0xFFFFFFFFu, ksteps = 1, n_bands = 1, upg = 1, groups = 1, M = 0;
-        const uint16_t* arow[kMGroups];                        // this lane's row of the activations per group of eight rows, at k = 2t
-        const uint8_t* sbase = nullptr; const uint8_t* zbase = nullptr;
-        for (uint32_t i = h;;) {
-            if (c.p != cur_p) {
-                const StProblem& pr = P.prob[c.p];
-                cur_p = c.p; ksteps = pr.ksteps; n_bands = pr.n_bands; upg = pr.units_per_group; groups = pr.groups; M = pr.M;
+                ptx::tc_fence_after_sync();
+                const uint32_t issue = ptx::elect_one(), a_cols = kStAccCols + t * 64 + as * kStAStageCols;
+                if (first) {
 #pragma unroll
-                for (int mg = 0; mg < kMGroups; ++mg) arow[mg] = pr.a + (size_t)(mg * 8 + g) * pr.K + 2 * t;
-                sbase = pr.scales_t + w2 * 32 + hh * 8;
-                zbase = pr.zeros_t + w2 * 8;
-            }
-            const uint32_t stage = i % kSt, round = i / kSt;
-            // loads first (they do not touch the stage), then the wait for the stage, then the stores
-            // -- scale / zero-point words: entry e = 8w + g serves consumer warp w, lanes g: columns 16w + g and 16w + g + 8
-            const size_t sz_row = (size_t)c.band * groups + c.ks / upg;
-            const uint2 sa = __ldg((const uint2*)(sbase + sz_row * kScaleBytes));            // scales of columns 16 w2 + 4 hh + 0..3
-            const uint2 sb = __ldg((const uint2*)(sbase + sz_row * kScaleBytes + 16));       // ... of columns 16 w2 + 8 + 4 hh + 0..3
-            const uint2 zz = __ldg((const uint2*)(zbase + sz_row * kZeroBytes));             // zero points of columns 16 w2 + 0..7, 16 w2 + 8..15
-            // -- activations of the step as B fragments: for row group mg, half j, pair pr2, lane (g, t) one uint4
-            // {b0(s), b1(s), b0(s+1), b1(s+1)}, s = 4j + 2 pr2, b0(s) = a[m][k0 + 16s + 2t .. +1], b1(s) = a[m][k0 + 16s + 2t + 8 .. +9], m = 8 mg + g
-            uint4 av[kMGroups * 4];
+                    for (uint32_t k4 = 0; k4 < 4; ++k4) ptx::umma_bf16_ts_if<false>(issue, acc + k4 * kStMRows, a_cols + k4 * 8, x + k4 * 2, idesc);
+                } else {
 #pragma unroll
-            for (int mg = 0; mg < kMGroups; ++mg) {
-                const uint32_t* row = (const uint32_t*)(arow[mg] + c.ks * kUnitK);   // 4-byte aligned
-                const bool in = (uint32_t)(mg * 8) + g < M;
-#pragma unroll
-                for (int f = 0; f < 4; ++f) {       // f = 2j + pr2: the step's k range in quarters of 32
-                    av[mg * 4 + f] = make_uint4(0, 0, 0, 0);
-                    if (in) {
-                        av[mg * 4 + f].x = __ldg(row + f * 16); av[mg * 4 + f].y = __ldg(row + f * 16 + 4);
-                        av[mg * 4 + f].z = __ldg(row + f * 16 + 8); av[mg * 4 + f].w = __ldg(row + f * 16 + 12);
-                    }
-                }
-            }
-            uint32_t okw = 1;
-            if (lane == 0 && !ptx::mbar_wait_relaxed(empty_bar + stage * 8, (round & 1) ^ 1, abort_flag, P.wait_limit_ns, 400)) {
-                atomicCAS(P.status, 0, kStatusProducerTimeout | 0x800000 | (int)((U0 + i) & 0x7FFFFF));
-                okw = 0;
-            }
-            okw = __shfl_sync(0xFFFFFFFFu, okw, 0);
-            if (!okw) break;
-            const uint32_t st = ring + stage * kSB + kWeightBytes;
-            {
-                const uint32_t sc0[4] = {sa.x & 0xFFFFu, sa.x >> 16, sa.y & 0xFFFFu, sa.y >> 16};
-                const uint32_t sc1[4] = {sb.x & 0xFFFFu, sb.x >> 16, sb.y & 0xFFFFu, sb.y >> 16};
-                const uint32_t z0 = zz.x >> (16 * hh), z1 = zz.y >> (16 * hh);      // the lane's four columns' zero points in the low 16 bits
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {
-                    uint4 o;
-                    o.x = ((z0 >> (4 * q)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
-                    o.y = sc0[q] * 0x00010001u;                                     // (s, s)
-                    o.z = ((z1 >> (4 * q)) & 0xFu) * 0x00010001u + 0x43004300u;
-                    o.w = sc1[q] * 0x00010001u;
-                    sts128(st + (lane * 4 + q) * 16, o);
-                }
-            }
-#pragma unroll
-            for (uint32_t f = 0; f < kMGroups * 4; ++f)
-                if ((f >> 2) * 8 + g < M) sts128(st + kStSzBytes + f * 512 + lane * 16, av[f]);      // (rows that do not exist are left as they are: their products are never stored)
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(full_bar + stage * 8);
-            i += kStHelpers;
-            if (i >= n_units) break;
-            c.ks += kStHelpers;
-            while (c.ks >= ksteps) {
-                c.ks -= ksteps;
-                if (++c.band == n_bands) {
-                    c.band = 0; ++c.p;
-                    ksteps = P.prob[c.p].ksteps; n_bands = P.prob[c.p].n_bands;     // (the other fields follow at the top of the loop)
-                }
-            }
-        }
-        return;
-    }
-
-    // ---------------------------------------------------------------- consumers (16 warps)
-    const uint32_t g = lane >> 2, t = lane & 3;
-    const uint32_t pair = warp >> 1, khalf = warp & 1;        // columns 32 pair .. + 31, k half of every step
-    // per row group and column group two accumulator sets, taken in turn: consecutive MMAs must not wait for each other's result
-    float acc[kMGroups][2][2][4];
-#pragma unroll
-    for (int mg = 0; mg < kMGroups; ++mg)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[mg][a >> 1][a & 1][j] = 0.0f;
-    uint32_t mask, magic;
-    asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
-    asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
-    Cursor c = c0;
-    bool ok = true;    // false after a wait expired: the warps keep walking (barriers stay matched) but do no work
-    const uint32_t col0 = warp * 16 + g;                      // the lane's two columns within the band once the k halves are added: col0 and col0 + 8
-    // a lane's place in a stage's words ([16 column groups][2 k halves][32 lanes] uint4), scale / zero words and B fragments
-    const uint32_t lane_w = ring + pair * 2048 + khalf * 512 + lane * 16;
-    const uint32_t lane_sz = ring + kWeightBytes + (pair * 16 + g) * 16;
-    const uint32_t lane_af = ring + kWeightBytes + kStSzBytes + khalf * 1024 + lane * 16;
-    uint32_t stage = 0, phase = 0;
-
-    // The CTA that contributes last to a band adds the pieces in k order (CTA order) and stores; nobody waits for anybody.
-    // Only the first contributor can hold the band in slot 1 (its range began in the band before).
-    auto reduce_band = [&](uint32_t rp, uint32_t rb) {
-        const StProblem& pr = P.prob[rp];
-        const uint32_t first_unit = pr.unit_begin + rb * pr.ksteps;
-        const uint32_t c_first = owner_of(first_unit, gridDim.x, P.total_units);
-        const uint32_t c_last = owner_of(first_unit + pr.ksteps - 1, gridDim.x, P.total_units);
-        const uint32_t first_slot = range_begin(c_first, gridDim.x, P.total_units) < first_unit ? 1u : 0u;
-        constexpr int kPer = kMGroups * 8 * kBandCols / (kStConsumers * 32);   // outputs per thread: 4 for M <= 8, 8 for M <= 16
-        constexpr int kCo = 4;                                                  // contributors whose pieces are in flight together
-        float total[kPer];
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) total[j] = 0.0f;
-        for (uint32_t cc0 = c_first; cc0 <= c_last; cc0 += kCo) {
-            float v[kCo][kPer];
-#pragma unroll
-            for (int b = 0; b < kCo; ++b) {
-                const uint32_t cc = cc0 + b;
-                const float* src = P.partials + ((size_t)cc * 2 + (cc == c_first ? first_slot : 0u)) * kPieceFloats;
-#pragma unroll
-                for (int j = 0; j < kPer; ++j) {
-                    const uint32_t idx = tid + j * (kStConsumers * 32);
-                    v[b][j] = (cc <= c_last && idx < pr.M * kBandCols) ? __ldcg(src + idx) : 0.0f;
-                }
-            }
-#pragma unroll
-            for (int b = 0; b < kCo; ++b)       // still added in CTA order, one contributor after the other
-#pragma unroll
-                for (int j = 0; j < kPer; ++j) total[j] += v[b][j];
-        }
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            const uint32_t idx = tid + j * (kStConsumers * 32);
-            if (idx < pr.M * kBandCols) {
-                const uint32_t row = idx / kBandCols, col = idx - row * kBandCols;
-                const uint32_t nc = rb * kBandCols + col;
-                if (nc < pr.N) pr.y[(size_t)row * pr.N + nc] = total[j];
-            }
-        }
-        if (tid == 0) P.counters[pr.band_begin + rb] = 0;   // ready for the next launch
-    };
-
-    // The end of a piece (the steps of one band this CTA owns; `u_next` is the unit after it): a band that lies wholly in
-    // the range is stored, a partial one goes to scratch and is counted in.
-    auto flush_piece = [&](uint32_t u_next) {
-        const StProblem& pr = P.prob[c.p];
-        const uint32_t first_unit = pr.unit_begin + c.band * pr.ksteps, last_unit = first_unit + pr.ksteps;   // [first, last)
-        const bool whole = first_unit >= U0 && last_unit <= U1;
-        const uint32_t c_first = owner_of(first_unit, gridDim.x, P.total_units);
-        const uint32_t c_last = owner_of(last_unit - 1, gridDim.x, P.total_units);
-        const uint32_t slot = (first_unit <= U0) ? 0u : 1u;   // the piece of the band holding this CTA's first unit is slot 0
-        float* piece = P.partials + ((size_t)blockIdx.x * 2 + slot) * kPieceFloats;
-        // The two k halves meet: a warp gives the other's column group away and keeps its own (column group khalf of the pair).
-#pragma unroll
-        for (int mg = 0; mg < kMGroups; ++mg) {
-            float give[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) give[j] = khalf ? acc[mg][0][0][j] + acc[mg][0][1][j] : acc[mg][1][0][j] + acc[mg][1][1][j];
-            sts128(exchange + ((warp ^ 1) * kMGroups + mg) * 512 + lane * 16,
-                   make_uint4(__float_as_uint(give[0]), __float_as_uint(give[1]), __float_as_uint(give[2]), __float_as_uint(give[3])));
-        }
-        st_pair_sync(pair);
-        // accumulator fragment: c0,c1 = (column col0, rows 2t, 2t+1), c2,c3 = (column col0 + 8, same rows)
-#pragma unroll
-        for (int mg = 0; mg < kMGroups; ++mg) {
-            const uint4 got4 = lds128(exchange + (warp * kMGroups + mg) * 512 + lane * 16);
-            const uint32_t got[4] = {got4.x, got4.y, got4.z, got4.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t m = mg * 8 + 2 * t + (j & 1), col = col0 + (j >> 1) * 8;
-                const uint32_t ncol = c.band * kBandCols + col;
-                const float own = khalf ? acc[mg][1][0][j] + acc[mg][1][1][j] : acc[mg][0][0][j] + acc[mg][0][1][j];
-                const float v = khalf ? __uint_as_float(got[j]) + own : own + __uint_as_float(got[j]);      // lower k half first
-                if (m < pr.M) {
-                    if (!whole) piece[m * kBandCols + col] = v;
-                    else if (ncol < pr.N) pr.y[(size_t)m * pr.N + ncol] = v;
+                    for (uint32_t k4 = 0; k4 < 4; ++k4) ptx::umma_bf16_ts_if<true>(issue, acc + k4 * kStMRows, a_cols + k4 * 8, x + k4 * 2, idesc);
                 }
 #pragma unroll
-                for (int a = 0; a < 4; ++a) acc[mg][a >> 1][a & 1][j] = 0.0f;
-            }
-        }
-        st_pair_sync(pair);                                    // both have read before either writes again
-        if (!whole) {
-            if (u_next < U1) {
-                // head piece, more steps follow: hand it to the counting lane and go on
+                for (uint32_t k4 = 0; k4 < 4; ++k4) ptx::umma_bf16_ts_if<true>(issue, acc + k4 * kStMRows, a_cols + 32 + k4 * 8, x + kStXChunk / 16 + k4 * 2, idesc);
+                ptx::umma_commit_if(issue, my_empty + as * 8);
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(head_written_bar);
-            } else {
-                st_consumer_sync();                    // every thread's part of the piece is written ...
-                if (tid == 0) {
-                    __threadfence();                   // ... and made visible before this CTA is counted
-                    *s_last = atomicAdd(&P.counters[pr.band_begin + c.band], 1) == (int)(c_last - c_first);
-                    if (*s_last) __threadfence();
+                if (++as == kStAStages) { as = 0; aphase ^= 1; }
+                x = x == x0 + (kStStages - 1) * (kStStageBytes / 16) ? x0 : x + kStStageBytes / 16;
+            }
+            if (!ok) break;
+            if (ptx::elect_one()) ptx::umma_commit(acc_full);
+            __syncwarp();
+            c.ks = 0;
+            if (++c.band == P.prob[c.p].n_bands) { c.band = 0; ++c.p; }
+        }
+    } else if (warp >= kStDqWarp0) {
+        // -------------------------------------------------------------- sixteen warps: dequantise into tensor memory
+        const uint32_t set = (warp - kStDqWarp0) >> 3, pair = warp & 7, g = lane >> 2;      // every second step; columns 32 pair .. + 31; a lane has columns g + 8 i of these
+        const uint32_t a_lane = (((pair & 3) * 32) << 16) + kStAccCols + (pair >> 2) * 64;
+        const uint32_t my_full = a_full + (pair >> 2) * kStAStages * 8, my_empty = a_empty + (pair >> 2) * kStAStages * 8;
+        uint32_t mask, magic;
+        asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
+        asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
+        uint32_t stage = set, phase = 0, as = set, aphase = 0;
+        const uint32_t lane_w = ring + pair * 2048 + lane * 16;              // [16 column groups][2 k halves][32 lanes] uint4
+        const uint32_t lane_s = ring + kStSzOff + (pair * 32 + g) * 2;
+        const uint32_t lane_z = ring + kStSzOff + kScaleBytes + pair * 16;
+        for (uint32_t u = U0 + set; u < U1; u += 2) {
+            if (!ptx::mbar_wait(full_bar + stage * 8, phase, abort_flag, P.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | (int)(u & 0x3FFFFF));
+                break;
+            }
+            if (tid == kStDqWarp0 * 32 && u == U0) stamp(1);
+            const uint32_t off = stage * kStStageBytes;
+            uint4 q[2][2];                            // [k half][column group]
+#pragma unroll
+            for (int kh = 0; kh < 2; ++kh)
+#pragma unroll
+                for (int cg = 0; cg < 2; ++cg) q[kh][cg] = lds128(lane_w + off + cg * 1024 + kh * 512);
+            const uint4 z4 = lds128(lane_z + off);
+            uint32_t zz[4], ss[4];                    // columns g + 8 i: bf16x2 (128+z, 128+z) and (s, s)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ss[i] = um_lds16(lane_s + off + i * 16);
+            // The A stage is free once the UMMAs of three steps ago have read it.  (Waited for here and not before the stores: values that live across
+            // a wait are moved once more to where the store takes them, 64 moves a step.)
+            if (!ptx::mbar_wait(my_empty + as * 8, aphase ^ 1, abort_flag, P.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(u & 0x3FFFFF));
+                break;
+            }
+            ptx::tc_fence_after_sync();
+            // So the step of three ago is done with its ring stage: dequantised, and its activations read.
+            ptx::mbar_arrive_if(empty_bar + (stage < 3 ? stage + kStStages - 3 : stage - 3) * 8, lane == 0 && u >= U0 + 3);
+            {
+                const uint32_t z[4] = {z4.x, z4.y, z4.z, z4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    zz[i] = ((z[i] >> (4 * g)) & 0xFu) * 0x00010001u + 0x43004300u;
+                    ss[i] *= 0x00010001u;
                 }
-                st_consumer_sync();
-                if (*s_last) reduce_band(c.p, c.band);
             }
-        }
-        c.ks = 0;          // a further piece starts a new band
-        if (++c.band == pr.n_bands) { c.band = 0; ++c.p; }
-    };
-
-    // Every warp walks the ring at its own pace: it waits for the stage, reads it, and tells the producer when it is done.  The words of
-    // the next step are fetched before the arithmetic of this one when they are there already, so that a warp does not begin each
-    // step with an empty pipeline.
-    uint32_t ksteps_cur = P.prob[c.p].ksteps;
-    uint4 q[2];
-    auto wait_stage = [&](uint32_t u, uint32_t s, uint32_t ph) {
-        if (ok && !ptx::mbar_wait(full_bar + s * 8, ph, abort_flag, P.wait_limit_ns)) {
-            if (lane == 0) atomicCAS(P.status, 0, kStatusMmaTimeout | (int)(u & 0xFFFFFF));
-            ok = false;
-        }
-    };
-    wait_stage(U0, 0, 0);
-    if (tid == 0) stamp(1);
-    q[0] = lds128(lane_w);
-    q[1] = lds128(lane_w + 1024);
-    for (uint32_t u = U0; u < U1; ++u) {
-        const uint32_t off = stage * kSB;
-        uint32_t next = stage + 1, next_phase = phase;
-        if (next == kSt) { next = 0; next_phase ^= 1; }
-        bool ready = false;
-        if (ok) {
-            uint4 sz[2], bf[kMGroups][2];
-            sz[0] = lds128(lane_sz + off);               // {128+z, s} of columns g, then g + 8, of the first column group
-            sz[1] = lds128(lane_sz + off + 128);         // ... of the second
+            const uint32_t dst = a_lane + as * kStAStageCols;
 #pragma unroll
-            for (int mg = 0; mg < kMGroups; ++mg)        // (rows that do not exist: stale bytes, whose products are never stored)
-#pragma unroll
-                for (int p2 = 0; p2 < 2; ++p2) bf[mg][p2] = lds128(lane_af + off + mg * kStAFragBytes + p2 * 512);
-            ready = u + 1 < U1 && ptx::mbar_try_wait(full_bar + next * 8, next_phase);
-            uint4 n0 = q[0], n1 = q[1];
-            if (ready) {
-                n0 = lds128(lane_w + next * kSB);
-                n1 = lds128(lane_w + next * kSB + 1024);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {                // k step 4 khalf + e: one word per column group
+            for (int kh = 0; kh < 2; ++kh) {
 #pragma unroll
                 for (int cg = 0; cg < 2; ++cg) {
-                    const uint32_t wd = e == 0 ? q[cg].x : e == 1 ? q[cg].y : e == 2 ? q[cg].z : q[cg].w;
-                    const uint32_t a0 = bf16x2_mul(bf16x2_sub(and_or(wd, mask, magic), sz[cg].x), sz[cg].y);
-                    const uint32_t a1 = bf16x2_mul(bf16x2_sub(and_or(wd >> 4, mask, magic), sz[cg].z), sz[cg].w);
-                    const uint32_t a2 = bf16x2_mul(bf16x2_sub(and_or(wd >> 8, mask, magic), sz[cg].x), sz[cg].y);
-                    const uint32_t a3 = bf16x2_mul(bf16x2_sub(and_or(wd >> 12, mask, magic), sz[cg].z), sz[cg].w);
+                    const uint32_t w[4] = {q[kh][cg].x, q[kh][cg].y, q[kh][cg].z, q[kh][cg].w};
+                    uint32_t r[16];
 #pragma unroll
-                    for (int mg = 0; mg < kMGroups; ++mg) {
-                        const uint4& b = bf[mg][e >> 1];
-                        mma_bf16_16816(acc[mg][cg][e & 1], a0, a1, a2, a3, e & 1 ? b.z : b.x, e & 1 ? b.w : b.y);
+                    for (int e = 0; e < 4; ++e) {     // one word per k step: fragment registers (columns g, g + 8) x (k 2t, 2t + 8)
+                        r[4 * e + 0] = bf16x2_mul(bf16x2_sub(and_or(w[e], mask, magic), zz[2 * cg]), ss[2 * cg]);
+                        r[4 * e + 1] = bf16x2_mul(bf16x2_sub(and_or(w[e] >> 4, mask, magic), zz[2 * cg + 1]), ss[2 * cg + 1]);
+                        r[4 * e + 2] = bf16x2_mul(bf16x2_sub(and_or(w[e] >> 8, mask, magic), zz[2 * cg]), ss[2 * cg]);
+                        r[4 * e + 3] = bf16x2_mul(bf16x2_sub(and_or(w[e] >> 12, mask, magic), zz[2 * cg + 1]), ss[2 * cg + 1]);
                     }
+                    ptx::tmem_st_16x128b_x8(dst + kh * 32 + ((cg * 16u) << 16), r);
                 }
             }
-            q[0] = n0; q[1] = n1;
+            ptx::tmem_st_wait();
+            ptx::tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(empty_bar + stage * 8);          // this warp has read the stage
+            ptx::mbar_arrive_if(my_full + as * 8, lane == 0);
+            as += 2;
+            if (as >= kStAStages) { as -= kStAStages; aphase ^= 1; }
+            stage += 2;
+            if (stage >= kStStages) { stage -= kStStages; phase ^= 1; }
         }
-        stage = next; phase = next_phase;
-        if (++c.ks == ksteps_cur || u + 1 == U1) {
-            if (u + 1 == U1 && tid == 0) stamp(2);
-            flush_piece(u + 1);
-            if (u + 1 < U1) ksteps_cur = P.prob[c.p].ksteps;
+        if (tid == kStDqWarp0 * 32) stamp(2);
+        // Finish the bands of the last and the first piece, where this CTA turned out to be the last to contribute to them.  (The last step is done with by
+        // then, so the ring is free.)
+        const uint32_t ft = tid - kStDqWarp0 * 32;
+        if (tail_cut) {
+            const StFinish f = st_finish(P, c_end.p, c_end.band, ft);
+            st_tail_sync();
+            if (s_last) st_reduce_band(P, f, ft, ring);
         }
-        if (u + 1 < U1 && !ready) {
-            wait_stage(u + 1, stage, phase);
-            q[0] = lds128(lane_w + stage * kSB);
-            q[1] = lds128(lane_w + stage * kSB + 1024);
+        if (has_head) {
+            const StFinish f = st_finish(P, c0.p, c0.band, ft);
+            if (ft == 0) s_head_go = ptx::mbar_wait(head_counted, 0, abort_flag, P.wait_limit_ns) && s_head_last;
+            if (tail_cut) st_finishers_sync();
+            else st_tail_sync();
+            if (s_head_go) st_reduce_band(P, f, ft, ring);
         }
+    } else {
+        // -------------------------------------------------------------- four warps: accumulators to y, or to a piece
+        const uint32_t quad = warp - kStEpWarp0, et = tid - kStEpWarp0 * 32;
+        bool ok = true;
+        uint32_t piece = 0;
+        for (uint32_t u = U0; u < U1; ++piece) {
+            const StProblem& pr = P.prob[c.p];
+            const uint32_t first_unit = pr.unit_begin + c.band * pr.ksteps, last_unit = first_unit + pr.ksteps;   // [first, last)
+            const bool whole = first_unit >= U0 && last_unit <= U1, tail = last_unit >= U1;
+            const StShare h = st_share(P, first_unit, pr.ksteps);
+            int* const counter = P.counters + pr.band_begin + c.band;
+            float* const part = P.partials + ((size_t)blockIdx.x * 2 + (first_unit <= U0 ? 0u : 1u)) * kPieceFloats;   // slot 0: the piece with this CTA's first unit
+            // The last piece is on the way of everything behind the launch.  Where its band has one more part, that lies as a rule in a range that began with it,
+            // and is long there: looked for as the last step's bytes land, it is fetched and added to the accumulators at once, with no hand-in, fence and atomic.
+            bool rest_there = false;
+            float other[2][16];
+            if (!whole && tail && h.last - h.first == 1) {      // (barriers are met whether or not a wait has run out)
+                const uint32_t i = U1 - 1 - U0, cta = h.first == blockIdx.x ? h.last : h.first;
+                ok = ok && ptx::mbar_wait(full_bar + (i % kStStages) * 8, (i / kStStages) & 1, abort_flag, P.wait_limit_ns);
+                if (et == 0) s_all = ok && um_ld_acquire((const uint32_t*)counter) != 0;
+                st_epilogue_sync();
+                rest_there = s_all != 0;
+                if (rest_there) {
+#pragma unroll
+                    for (uint32_t t = 0; t < 2; ++t)
+#pragma unroll
+                        for (uint32_t m = 0; m < 16; ++m) other[t][m] = m < pr.M ? __ldcg(st_piece(P, h, cta) + m * kBandCols + t * 128 + quad * 32 + lane) : 0.0f;
+                }
+            }
+            if (ok && !ptx::mbar_wait(acc_full, piece & 1, abort_flag, P.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xC00000);
+                ok = false;
+            }
+            if (ok) {
+                ptx::tc_fence_after_sync();
+#pragma unroll
+                for (uint32_t t = 0; t < 2; ++t) {
+                    const uint32_t col = t * 128 + quad * 32 + lane, n = c.band * kBandCols + col;
+#pragma unroll
+                    for (uint32_t m0 = 0; m0 < 16; m0 += 8) {
+                        if (m0 >= pr.M) break;
+                        uint32_t d[4][8];
+                        float v[8];
+#pragma unroll
+                        for (uint32_t k4 = 0; k4 < 4; ++k4) ptx::tmem_ld_32x32b_x8(tmem_base + ((quad * 32) << 16) + t * 64 + k4 * kStMRows + m0, d[k4]);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j)
+                            v[j] = (__uint_as_float(d[0][j]) + __uint_as_float(d[1][j])) + (__uint_as_float(d[2][j]) + __uint_as_float(d[3][j]));
+                        if (whole || rest_there) {
+                            // (of two parts the order does not matter; the zero gives a sum of negative zeros the sign it has where the pieces are added)
+                            if (rest_there) {
+#pragma unroll
+                                for (uint32_t j = 0; j < 8; ++j) v[j] = (0.0f + v[j]) + other[t][m0 + j];
+                            }
+                            if (n < pr.N) {
+#pragma unroll
+                                for (uint32_t j = 0; j < 8; ++j)
+                                    if (m0 + j < pr.M) pr.y[(size_t)(m0 + j) * pr.N + n] = v[j];
+                            }
+                        } else {
+#pragma unroll
+                            for (uint32_t j = 0; j < 8; ++j)
+                                if (m0 + j < pr.M) part[(m0 + j) * kBandCols + col] = v[j];
+                        }
+                    }
+                }
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(acc_empty);
+            }
+            if (!whole && !tail) {
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(head_written);
+            } else if (!whole) {
+                st_epilogue_sync();                    // every thread's part of the piece is written ...
+                if (et == 0) {
+                    int last = 0;
+                    if (rest_there) {
+                        *counter = 0;                  // ready for the next launch
+                    } else if (ok) {
+                        __threadfence();               // ... and made visible before this CTA is counted
+                        last = atomicAdd(counter, 1) == (int)(h.last - h.first);
+                        if (last) __threadfence();
+                    }
+                    s_last = last;
+                }
+            }
+            u = min(U1, last_unit);
+            c.ks = 0;
+            if (++c.band == pr.n_bands) { c.band = 0; ++c.p; }
+        }
+        if (tail_cut || has_head) st_tail_sync();
     }
-    if (has_head) {
-        if (!ptx::mbar_wait(head_counted_bar, 0, abort_flag, P.wait_limit_ns) && lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xE00000);
-        st_consumer_sync();
-        if (*s_head_last) reduce_band(c0.p, c0.band);
-    }
+
+    __syncwarp();
     if (*abort_flag) {
-        // give bulk copies already in flight time to land before shared memory goes away
+        // give copies and UMMAs already in flight time to land before shared and tensor memory go away
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    }
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kStIssueWarp0) {
+        ptx::tc_fence_after_sync();
+        ptx::tmem_dealloc(tmem_base, kStTmemCols);
     }
     if (tid == 0) stamp(3);
 }
@@ -562,27 +662,27 @@ uint32_t prepack_grid_for(uint64_t n, uint32_t block) {
     return (uint32_t)(gsz < 1 ? 1 : (gsz > cap ? cap : gsz));
 }
 
-// One launch for up to kStMaxProblems problems (already validated).
+// One launch for up to kProblems problems (already validated).
+template <uint32_t kProblems>
 int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count) {
-    StParams P;
+    StParams<kProblems> P;
     memset(&P, 0, sizeof P);
     uint64_t total = 0, bands = 0;
-    uint32_t max_m = 0;
     for (size_t i = 0; i < count; ++i) {
         const t0_w4a16_args& a = args[i];
         const PrepackLayout L = prepack_layout(a.k, a.n, a.group);
+        int rc = gemm::make_map_kmajor(&P.x[i], (const void*)a.a, a.m, a.k, a.k, 1, kStMRows);
+        if (rc != T0_OK) return rc;
         StProblem& q = P.prob[i];
-        q.a = (const uint16_t*)a.a;
         q.y = (float*)a.y;
         q.tiles = (const uint8_t*)a.packed + L.off_tiles;
         q.scales_t = (const uint8_t*)a.packed + L.off_scales;
         q.zeros_t = (const uint8_t*)a.packed + L.off_zeros;
-        q.M = a.m; q.N = a.n; q.K = a.k;
+        q.M = a.m; q.N = a.n;
         q.ksteps = L.ksteps; q.groups = L.groups; q.units_per_group = a.group / kUnitK; q.n_bands = L.bands;
         q.unit_begin = (uint32_t)total; q.band_begin = (uint32_t)bands;
         total += (uint64_t)L.bands * L.ksteps;
         bands += L.bands;
-        max_m = std::max(max_m, a.m);
     }
     if (total == 0) return T0_OK;
     if (total > 0x7FFFFFFFull || bands * sizeof(int) > kCounterRegion) return fail(T0_ERR_UNSUPPORTED, "batch too large: %llu steps, %llu bands", (unsigned long long)total, (unsigned long long)bands);
@@ -599,11 +699,11 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
     const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
     P.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
     P.n_problems = (uint32_t)count; P.total_units = (uint32_t)total;
-    const int m_groups = max_m <= 8 ? 1 : 2;
+    P.per_cta = (uint32_t)total / grid; P.rest = (uint32_t)total % grid; P.cta_per_unit = (float)grid / (float)total;
     static bool attr_set[64] = {};
-    if (rt->device < 64 && !attr_set[rt->device]) {
-        T0_CUDA(cudaFuncSetAttribute(w4a16_stream_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st_smem_bytes(1)));
-        T0_CUDA(cudaFuncSetAttribute(w4a16_stream_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st_smem_bytes(2)));
+    if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
+    if (!attr_set[rt->device]) {
+        T0_CUDA(cudaFuncSetAttribute(w4a16_stream_kernel<kProblems>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStSmem));
         attr_set[rt->device] = true;
     }
     // T0_W4_TRACE=1: per-CTA stamps, summarised on stderr after a blocking wait (a debugging aid, off by default)
@@ -618,14 +718,14 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(kStThreads, 1, 1);
-    cfg.dynamicSmemBytes = st_smem_bytes(m_groups);
+    cfg.dynamicSmemBytes = kStSmem;
     cfg.stream = rt->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    cudaError_t le = m_groups == 1 ? cudaLaunchKernelEx(&cfg, w4a16_stream_kernel<1>, P) : cudaLaunchKernelEx(&cfg, w4a16_stream_kernel<2>, P);
+    cudaError_t le = cudaLaunchKernelEx(&cfg, w4a16_stream_kernel<kProblems>, P);
     if (le != cudaSuccess) return fail(T0_ERR_CUDA, "W4A16 kernel launch failed: %s", cudaGetErrorString(le));
     rt->launches.fetch_add(1);
     if (trace) {
@@ -710,7 +810,7 @@ int t0_w4a16_gemm_prepacked_batch(t0_runtime* rt, const t0_w4a16_args* args, siz
             bands += L.bands; units += (uint64_t)L.bands * L.ksteps;
             ++n;
         }
-        rc = launch_stream_chunk(rt, live.data() + i, n);
+        rc = n <= kStFewProblems ? launch_stream_chunk<kStFewProblems>(rt, live.data() + i, n) : launch_stream_chunk<kStMaxProblems>(rt, live.data() + i, n);
         if (rc != T0_OK) return rc;
         i += n;
     }

@@ -61,12 +61,6 @@ struct UmParams {
     uint32_t whole;          // shared out by tiles instead: no tile is cut
 };
 
-__device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
 // First chunk of a CTA's range, and the CTA whose range holds a chunk: in 32 bits (at most 256 CTAs and 2^24 chunks), since a warp that
 // finishes a cut tile needs a few of these and a 64-bit division takes hundreds of cycles.
 __device__ __forceinline__ uint32_t um_begin(uint32_t cta, const UmParams& p) {

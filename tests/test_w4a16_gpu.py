@@ -622,3 +622,27 @@ def test_tiled_grouped_random_shapes(t0, oracle, rt):
             assert np.all(got[M * N:] == -9999.0), ("wrote past the output", case, M, N, K, G)
         for b in [xp, xs, xz, tiled] + xas + ys:
             b.free()
+
+
+@pytest.mark.parametrize("shapes", [
+    [(1, 128, 8, 128)],                                                            # one step, one CTA
+    [(1, 14336, 40, 128)], [(2, 7168, 256, 1024)], [(16, 3584, 136, 3584)],        # one band, a CTA per step: contributors added in groups of threads (M = 1, 2) and by one (M = 16)
+    [(8, 4096, 18944, 128)], [(9, 4096, 18944, 128)],                              # 74 bands on 148 CTAs: two contributors each, the edge of eight rows
+    [(16, 1024, 33000, 128), (3, 1024, 4736, 256)],                                # whole bands, cut ones, and a range across two problems
+    [(m, 512, 1000, 512) for m in (1, 7, 16, 9)], [(m, 512, 1000, 512) for m in (1, 7, 16, 9, 8)],   # the two sizes of parameter block
+])
+def test_streaming_kernel_edges(t0, oracle, rt, shapes):
+    probs, bufs = _batch_problems(oracle, rt, shapes, 700)
+    calls = [t0.W4A16Args(p["xa"].gpu_addr(), p["pre"].gpu_addr(), 0, 0, p["y"].gpu_addr(), p["M"], p["N"], p["K"], p["G"]) for p in probs]
+    outs = []
+    for _ in range(6):                                                             # who finishes a band depends on timing, its sum does not
+        rt.w4a16_gemm_prepacked_batch(calls)
+        rt.synchronize()
+        outs.append([p["y"].read(p["M"] * p["N"] * 4, np.float32).reshape(p["M"], p["N"]) for p in probs])
+    for i, p in enumerate(probs):
+        assert np.all(p["y"].read_bytes(p["M"] * p["N"] * 4, 4096, np.float32) == -9999.0), "wrote past the output"
+        assert_close(outs[0][i], oracle.w4a16_gemm(p["a"], p["packed"], p["scales"], p["zeros"], p["M"], p["N"], p["K"], p["G"]), p["K"])
+        for again in outs[1:]:
+            assert np.array_equal(again[i], outs[0][i])
+    for b in bufs:
+        b.free()
