@@ -34,17 +34,18 @@ constexpr uint32_t kUmDqWarps = 16;
 // operand, which the sixteen dequantising warps spent waiting: two problems of M = 128, N = 11008, K = 4096 39.7 us, 33.3 with the warp
 // converged, 31.7 with one barrier
 // (device time of queued launches, as below; the same call takes 34 us by the host's clock in blocks of calls).
-constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;
-constexpr uint32_t kUmThreads = (kUmDqWarps + 3) * 32;
-constexpr uint32_t kUmXBytes = 128 * kUmBK * 2;             // 16 KiB: activations of a chunk at M = 128
+constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;     // (two issuing warps)
+constexpr uint32_t kUmThreads = (kUmDqWarps + 4) * 32;
+constexpr uint32_t kUmXBytes = 6 * 128 * kUmBK * 2;         // activations: six chunks at M = 128, as many more as fit at less, eight at most
+constexpr uint32_t kUmMaxXStages = 8;
 // Tensor memory (512 columns): accumulators 2 x 128 columns, then four A stages of 2 halves x 4 k-steps x 8 columns.
 constexpr uint32_t kUmTmemCols = 512;
 constexpr uint32_t kUmABase = 256;                          // first column of the A stages
 constexpr uint32_t kUmAStageCols = 64;
-constexpr uint32_t kUmAStages = 4;                          // operand stages: weights in tensor memory, activations in shared memory
-constexpr uint32_t kUmRawStages = 7;                        // raw weight stages of two chunks: 124 KB in flight per SM
+constexpr uint32_t kUmAStages = 4;
+constexpr uint32_t kUmRawStages = 6;                        // raw weight stages of two chunks: 106 KB in flight per SM (an even number: a set of warps has every second one)
 // (more than half an SM's shared memory: the kernel takes all 512 tensor-memory columns, so two of its CTAs must never share an SM)
-constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmAStages * kUmXBytes + 512 + 1024;
+constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmXBytes + 512 + 1024;
 constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long where sums may be: below it the finish costs more than the range
 constexpr size_t kUmCounterBytes = 16 * 1024;               // one word per CTA and dequantisation warp (up to 256 CTAs)
 
@@ -76,27 +77,33 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t raw_ring = smem;
     const uint32_t x_ring = smem + kUmRawStages * 2 * kUmRawStride;           // activations: [rows][64 k] bf16, 128-byte swizzle, per stage
-    const uint32_t bars = x_ring + kUmAStages * kUmXBytes;
+    const uint32_t bars = x_ring + kUmXBytes;
     const uint32_t raw_full = bars, raw_empty = bars + 8 * kUmRawStages;
-    const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * kUmAStages;
-    const uint32_t acc_full = a_empty + 8 * kUmAStages, acc_empty = acc_full + 8;
+    const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * 2 * kUmAStages;     // [128-column half][stage]
+    const uint32_t x_full = a_empty + 8 * 2 * kUmAStages, x_empty = x_full + 8 * kUmMaxXStages;
+    const uint32_t acc_full = x_empty + 8 * kUmMaxXStages, acc_empty = acc_full + 8;
+    const uint32_t x_bytes = p.rows * kUmBK * 2, x_stages = min(kUmMaxXStages, kUmXBytes / x_bytes);
     __shared__ uint32_t tmem_holder;
     __shared__ int s_abort;
     volatile int* abort_flag = &s_abort;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     const uint32_t n_chunks = p.n_chunks;
     const uint32_t u0 = um_begin(blockIdx.x, p), u1 = um_begin(blockIdx.x + 1, p);
 
     if (tid == 0) {
         for (uint32_t s = 0; s < kUmRawStages; ++s) {
             ptx::mbar_init(raw_full + 8 * s, 1);
-            ptx::mbar_init(raw_empty + 8 * s, kUmDqWarps);
+            ptx::mbar_init(raw_empty + 8 * s, kUmDqWarps / 2);
         }
-        for (uint32_t s = 0; s < kUmAStages; ++s) {
-            ptx::mbar_init(a_full + 8 * s, kUmDqWarps / 2 + 1);   // the eight warps that dequantise the chunk, and the activations' bytes
+        for (uint32_t s = 0; s < 2 * kUmAStages; ++s) {
+            ptx::mbar_init(a_full + 8 * s, kUmDqWarps / 4);       // the four warps that dequantise this half of the chunk
             ptx::mbar_init(a_empty + 8 * s, 1);
         }
-        ptx::mbar_init(acc_full, 1);
+        for (uint32_t s = 0; s < x_stages; ++s) {
+            ptx::mbar_init(x_full + 8 * s, 1);
+            ptx::mbar_init(x_empty + 8 * s, 2);
+        }
+        ptx::mbar_init(acc_full, 2);
         ptx::mbar_init(acc_empty, kUmDqWarps);
         s_abort = 0;
         ptx::fence_barrier_init();
@@ -110,7 +117,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     ptx::tc_fence_before_sync();
     __syncthreads();
     ptx::tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_holder;
+    constexpr uint32_t tmem_base = 0;    // all columns are allocated: tensor-memory addresses are constants
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
 
@@ -161,32 +168,34 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
         }
     } else if (warp == kUmXWarp) {
         // -------------------------------------------------------------- activations: one box per chunk (rows beyond M are zero)
-        uint32_t as = 0, aphase = 0;
+        uint32_t xs = 0, phase = 0;
         const uint32_t item = u0 / n_chunks;
         uint32_t c = u0 - item * n_chunks, tile = item;
         uint32_t prob = item / p.n_tiles;
         tile = item - prob * p.n_tiles;
         for (uint32_t u = u0; u < u1; ++u) {
-            if (!ptx::mbar_wait_warp(a_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
+            if (!ptx::mbar_wait_warp(x_empty + 8 * xs, phase ^ 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
                 break;
             }
             if (ptx::elect_one()) {
-                ptx::mbar_arrive_expect_tx(a_full + 8 * as, p.rows * kUmBK * 2);
-                ptx::tma_load_3d(x_ring + as * kUmXBytes, &group.maps[4 * prob + 3], a_full + 8 * as, (int32_t)(c * kUmBK), 0, 0);
+                ptx::fence_proxy_async_smem();
+                ptx::mbar_arrive_expect_tx(x_full + 8 * xs, x_bytes);
+                ptx::tma_load_3d(x_ring + xs * x_bytes, &group.maps[4 * prob + 3], x_full + 8 * xs, (int32_t)(c * kUmBK), 0, 0);
             }
             __syncwarp();
-            if (++as == kUmAStages) { as = 0; aphase ^= 1; }
+            if (++xs == x_stages) { xs = 0; phase ^= 1; }
             if (++c == n_chunks) {
                 c = 0;
                 if (++tile == p.n_tiles) { tile = 0; ++prob; }
             }
         }
-    } else if (warp == kUmIssueWarp) {
-        // -------------------------------------------------------------- UMMA issuer: per chunk 2 halves x 4 k-steps of M 128 x N rows x K 16
-        const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u);
-        uint32_t as = 0, aphase = 0, piece = 0;
-        const uint64_t x_desc = ptx::make_smem_desc(x_ring, 16, 1024);      // (addresses enter a descriptor in 16-byte units: stages are added)
+    } else if (warp >= kUmIssueWarp) {
+        // -------------------------------------------------------------- UMMA issuers, one per half of the columns: per chunk 4 k-steps of M 128 x N rows x K 16
+        const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u), t = warp - kUmIssueWarp;
+        const uint32_t my_full = a_full + 8 * kUmAStages * t, my_empty = a_empty + 8 * kUmAStages * t;
+        uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0;
+        const uint32_t x_desc = (x_ring & 0x3FFFFu) >> 4;                   // (addresses enter a descriptor in 16-byte units)
         bool ok = true;
         for (uint32_t u = u0; ok && u < u1; ++piece) {
             const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks);
@@ -194,44 +203,44 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
                 if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
                 break;
             }
-            ptx::tc_fence_after_sync();
             for (uint32_t first = 1; u < u_end; ++u, first = 0) {
-                if (!ptx::mbar_wait_warp(a_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
+                if (!ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
+                    !ptx::mbar_wait_warp(my_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
                     if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const uint64_t x_stage = x_desc + as * (kUmXBytes / 16);
-                const uint32_t a_cols = tmem_base + kUmABase + as * kUmAStageCols;
-                if (ptx::elect_one()) {
+                const uint32_t x = x_desc + xs * (x_bytes / 16), a_cols = kUmABase + as * kUmAStageCols + t * 32, issue = ptx::elect_one();
+                if (first)
+                    ptx::umma_bf16_ts_if<false>(issue, t * 128, a_cols, x, idesc);
+                else
+                    ptx::umma_bf16_ts_if<true>(issue, t * 128, a_cols, x, idesc);
 #pragma unroll
-                    for (uint32_t k4 = 0; k4 < kUmBK / 16; ++k4) {
-#pragma unroll
-                        for (uint32_t t = 0; t < 2; ++t)
-                            ptx::umma_bf16_ts(tmem_base + t * 128, a_cols + t * 32 + k4 * 8, x_stage + k4 * 2, idesc, (first && k4 == 0) ? 0u : 1u);
-                    }
-                    ptx::umma_commit(a_empty + 8 * as);
-                }
+                for (uint32_t k4 = 1; k4 < kUmBK / 16; ++k4) ptx::umma_bf16_ts_if<true>(issue, t * 128, a_cols + k4 * 8, x + k4 * 2, idesc);
+                ptx::umma_commit_if(issue, my_empty + 8 * as);
+                ptx::umma_commit_if(issue, x_empty + 8 * xs);
                 __syncwarp();
                 if (++as == kUmAStages) { as = 0; aphase ^= 1; }
+                if (++xs == x_stages) { xs = 0; xphase ^= 1; }
             }
-            if (ok && ptx::elect_one()) ptx::umma_commit(acc_full);
+            if (ok) ptx::umma_commit_if(ptx::elect_one(), acc_full);
             __syncwarp();
         }
     } else {
         // -------------------------------------------------------------- sixteen warps: dequantise into tensor memory, then the epilogue
-        // Warps 0..7 take the even chunks of the range, 8..15 the odd ones: a thread has one column and all eight words of its chunk, so that
-        // what stands around the arithmetic (two waits, two arrivals, the store and its wait) is paid once per eight words.  (All sixteen
-        // warps on every chunk, four words each: 3 % slower.)
-        const uint32_t q = warp & 3, t = (warp >> 2) & 1, h = warp >> 3;   // lane quadrant, 128-column half of the tile, chunk parity (and half of the rows in the epilogue)
+        // Eight warps take two chunks of the range, a raw stage, the other eight the next two: a thread has one column and all eight words of a chunk, so
+        // that what stands around the arithmetic is paid once per eight words.
+        const uint32_t q = warp & 3, t = (warp >> 2) & 1, h = warp >> 3;   // lane quadrant, 128-column half of the tile, which of the two sets (and half of the rows in the epilogue)
         const uint32_t n = t * 128 + q * 32 + lane;                          // this thread's column of the tile
         const uint32_t lane_base = (q * 32) << 16;
         const uint32_t m_begin = h * (p.rows / 2), m_end = min(p.M, m_begin + p.rows / 2);   // the rows of y this warp stores
         uint32_t mask, magic;
         asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
         asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
-        uint32_t rs = 0, rphase = 0, as = h, aphase = 0, piece = 0;
+        const uint32_t my_full = a_full + 8 * kUmAStages * t, my_empty = a_empty + 8 * kUmAStages * t;
+        uint32_t rs = h, rphase = 0, piece = 0;
+        uint32_t v = u0 + 2 * h;                                             // this warp's next chunk
         bool ok = true;
 
         // 32 columns of the accumulator (rows m0.. of y) for this warp's columns of y; a narrow tile's columns beyond its rows are not used
@@ -251,45 +260,49 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
             const uint32_t item = u / n_chunks, tile_u0 = item * n_chunks, tile_u1 = tile_u0 + n_chunks;
             const uint32_t u_end = min(u1, tile_u1);
             const bool whole = u == tile_u0 && u_end == tile_u1;
-            for (uint32_t v = u + (((u - u0) & 1) != h ? 1 : 0); ok && v < u_end; v += 2) {
-                if (!ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns)) {
+            while (ok && v < u_end) {
+                const uint32_t second = (v - u0) & 1, as = (v - u0) & 3, aphase = ((v - u0) >> 2) & 1;     // of the two chunks of a raw stage
+                if (!second && !ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns)) {
                     if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(v & 0x3FFFFF));
                     ok = false;
                     break;
                 }
-                const uint32_t raw = raw_ring + rs * (2 * kUmRawStride) + h * kUmRawStride;
+                const uint32_t raw = raw_ring + rs * (2 * kUmRawStride) + second * kUmRawStride;
                 uint32_t words[8];
 #pragma unroll
                 for (uint32_t i = 0; i < 8; ++i) words[i] = um_lds32(raw + i * (kUmBN * 4) + n * 4);
                 const uint32_t sbits = um_lds16(raw + 8 * kUmBN * 4 + n * 2);
                 const uint32_t zword = um_lds32(raw + 8 * kUmBN * 4 + kUmBN * 2 + (n >> 3) * 4);
-                const uint32_t zz = ((zword >> ((n & 7) * 4)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
-                const uint32_t ss = sbits * 0x00010001u;                                               // (s, s)
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(raw_empty + 8 * rs);
-                if (++rs == kUmRawStages) { rs = 0; rphase ^= 1; }
-                uint32_t r[32];                                // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
-#pragma unroll
-                for (uint32_t i = 0; i < 8; ++i) {
-                    uint32_t v[4];
-                    um_dequant_word(words[i], mask, magic, zz, ss, kTiled, v);
-#pragma unroll
-                    for (uint32_t e = 0; e < 4; ++e) r[4 * i + e] = v[e];
-                }
-                // the A stage is free once the UMMAs of four chunks ago have read it
-                if (!ptx::mbar_wait(a_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
+                // The A stage is free once the UMMAs of four chunks ago have read it.  (Waited for here and not before the store: values that live across a
+                // wait are moved once more to where the store takes them.)
+                if (!ptx::mbar_wait(my_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
                     if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(v & 0x3FFFFF));
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after_sync();
+                const uint32_t zz = ((zword >> ((n & 7) * 4)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
+                const uint32_t ss = sbits * 0x00010001u;                                               // (s, s)
+                __syncwarp();
+                ptx::mbar_arrive_if(raw_empty + 8 * rs, second && lane == 0);
+                uint32_t r[32];                                // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    uint32_t d[4];
+                    um_dequant_word(words[i], mask, magic, zz, ss, kTiled, d);
+#pragma unroll
+                    for (uint32_t e = 0; e < 4; ++e) r[4 * i + e] = d[e];
+                }
                 ptx::tmem_st_32x32b_x32(tmem_base + lane_base + kUmABase + as * kUmAStageCols + t * 32, r);
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(a_full + 8 * as);
-                as += 2;
-                if (as >= kUmAStages) { as -= kUmAStages; aphase ^= 1; }
+                ptx::mbar_arrive_if(my_full + 8 * as, lane == 0);
+                v += 1 + 2 * second;
+                if (second) {
+                    rs += 2;
+                    if (rs >= kUmRawStages) { rs -= kUmRawStages; rphase ^= 1; }
+                }
             }
             u = u_end;
             // A tile cut by range boundaries: each of its CTAs holds a partial sum over a part of K.  The 32 columns x rows a warp
