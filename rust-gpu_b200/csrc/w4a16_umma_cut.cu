@@ -34,10 +34,11 @@ constexpr uint32_t kUmDqWarps = 16;
 // operand, which the sixteen dequantising warps spent waiting: two problems of M = 128, N = 11008, K = 4096 39.7 us, 33.3 with the warp
 // converged, 31.7 with one barrier
 // (device time of queued launches, as below; the same call takes 34 us by the host's clock in blocks of calls).
-constexpr uint32_t kUmRawWarp = kUmDqWarps, kUmXWarp = kUmDqWarps + 1, kUmIssueWarp = kUmDqWarps + 2;     // (two issuing warps)
-constexpr uint32_t kUmThreads = (kUmDqWarps + 4) * 32;
-constexpr uint32_t kUmXBytes = 6 * 128 * kUmBK * 2;         // activations: six chunks at M = 128, as many more as fit at less, eight at most
-constexpr uint32_t kUmMaxXStages = 8;
+constexpr uint32_t kUmEpWarp0 = kUmDqWarps, kUmEpWarps = 4;  // empty the accumulators of all but the last tile of a range, one per tensor-memory lane quadrant
+constexpr uint32_t kUmIssueWarp = kUmEpWarp0 + kUmEpWarps, kUmLoadWarp = kUmIssueWarp + 2;     // (two issuing warps)
+constexpr uint32_t kUmThreads = (kUmLoadWarp + 1) * 32;
+constexpr uint32_t kUmXBytes = 6 * 128 * kUmBK * 2;         // activations, in stages of two chunks: three at M = 128, four at M <= 96
+constexpr uint32_t kUmMaxXStages = 4;
 // Tensor memory (512 columns): accumulators 2 x 128 columns, then four A stages of 2 halves x 4 k-steps x 8 columns.
 constexpr uint32_t kUmTmemCols = 512;
 constexpr uint32_t kUmABase = 256;                          // first column of the A stages
@@ -81,14 +82,15 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     const uint32_t raw_full = bars, raw_empty = bars + 8 * kUmRawStages;
     const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * 2 * kUmAStages;     // [128-column half][stage]
     const uint32_t x_full = a_empty + 8 * 2 * kUmAStages, x_empty = x_full + 8 * kUmMaxXStages;
-    const uint32_t acc_full = x_empty + 8 * kUmMaxXStages, acc_empty = acc_full + 8;
-    const uint32_t x_bytes = p.rows * kUmBK * 2, x_stages = min(kUmMaxXStages, kUmXBytes / x_bytes);
+    const uint32_t acc_full = x_empty + 8 * kUmMaxXStages, acc_empty = acc_full + 16;                // [accumulator set]
+    const uint32_t x_bytes = p.rows * kUmBK * 2, x_stages = min(kUmMaxXStages, kUmXBytes / (2 * x_bytes));
     __shared__ uint32_t tmem_holder;
     __shared__ int s_abort;
     volatile int* abort_flag = &s_abort;
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     const uint32_t n_chunks = p.n_chunks;
     const uint32_t u0 = um_begin(blockIdx.x, p), u1 = um_begin(blockIdx.x + 1, p);
+    const uint32_t acc_sets = p.rows <= 64 ? 2 : 1;          // accumulators of 128 columns a half: two sets, taken in turn, where a tile needs no more than half of them
 
     if (tid == 0) {
         for (uint32_t s = 0; s < kUmRawStages; ++s) {
@@ -103,8 +105,10 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
             ptx::mbar_init(x_full + 8 * s, 1);
             ptx::mbar_init(x_empty + 8 * s, 2);
         }
-        ptx::mbar_init(acc_full, 2);
-        ptx::mbar_init(acc_empty, kUmDqWarps);
+        for (uint32_t s = 0; s < 2; ++s) {
+            ptx::mbar_init(acc_full + 8 * s, 2);
+            ptx::mbar_init(acc_empty + 8 * s, kUmEpWarps);
+        }
         s_abort = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
@@ -121,43 +125,38 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
 
-    // The three serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
-    if (warp == kUmRawWarp) {
-        // -------------------------------------------------------------- raw weights, scales, zero points: three TMA boxes per chunk
-        uint32_t stage = 0, phase = 0;
+    // The serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
+    if (warp == kUmLoadWarp) {
+        // -------------------------------------------------------------- per two chunks: raw weights, scales, zero points (three TMA boxes a chunk), then activations (one)
+        uint32_t stage = 0, phase = 0, xs = 0, xphase = 0;
         const uint32_t item = u0 / n_chunks, per_group = p.group / kUmBK;
-        uint32_t c = u0 - item * n_chunks, tile = item;
+        uint32_t c = u0 - item * n_chunks;
         uint32_t grp = c / per_group, in_group = c - grp * per_group;
-        uint32_t prob = item / p.n_tiles;
-        tile = item - prob * p.n_tiles;
+        uint32_t prob = item / p.n_tiles, tile = item - prob * p.n_tiles;
         for (uint32_t u = u0; u < u1;) {
             if (!ptx::mbar_wait_warp(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(c & 0xFFFFFF));
                 break;
             }
-            const uint32_t fb = raw_full + 8 * stage;
-            uint32_t dst = raw_ring + stage * (2 * kUmRawStride);
-            const uint32_t u_stop = min(u1, u + 2);
-            if (ptx::elect_one()) {
-                ptx::fence_proxy_async_smem();       // the stage was read through the generic proxy, the copies write it through the async proxy
-                ptx::mbar_arrive_expect_tx(fb, (u_stop - u) * kUmRawBytes);
-            }
-            __syncwarp();
+            const uint32_t fb = raw_full + 8 * stage, u_stop = min(u1, u + 2), issue = ptx::elect_one();
+            const uint32_t c_x[2] = {c, c + 1 == n_chunks ? 0 : c + 1}, prob_x0 = prob;
+            uint32_t prob_x1 = prob, dst = raw_ring + stage * (2 * kUmRawStride);
+            const uint32_t two = u_stop - u == 2;
+            ptx::fence_proxy_async_smem();           // the stage was read through the generic proxy, the copies write it through the async proxy
+            ptx::mbar_arrive_expect_tx_if(issue, fb, (u_stop - u) * kUmRawBytes);
             for (; u < u_stop; ++u, dst += kUmRawStride) {
-                if (ptx::elect_one()) {
-                    const CUtensorMap* const mw = &group.maps[4 * prob];
-                    if constexpr (kTiled) {
-                        // tile-major layout: the chunk's 8 KB of words are contiguous, as are its scales and zero points
-                        ptx::tma_load_3d(dst, mw, fb, 0, (int32_t)(c * (kUmBK / 8)), (int32_t)tile);
-                        ptx::tma_load_3d(dst + 8 * kUmBN * 4, mw + 1, fb, 0, (int32_t)grp, (int32_t)tile);
-                        ptx::tma_load_3d(dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, 0, (int32_t)grp, (int32_t)tile);
-                    } else {
-                        ptx::tma_load_2d(dst, mw, fb, (int32_t)(tile * kUmBN), (int32_t)(c * (kUmBK / 8)));
-                        ptx::tma_load_2d(dst + 8 * kUmBN * 4, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)grp);
-                        ptx::tma_load_2d(dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)grp);
-                    }
+                const CUtensorMap* const mw = &group.maps[4 * prob];
+                prob_x1 = prob;
+                if constexpr (kTiled) {
+                    // tile-major layout: the chunk's 8 KB of words are contiguous, as are its scales and zero points
+                    ptx::tma_load_3d_if(issue, dst, mw, fb, 0, (int32_t)(c * (kUmBK / 8)), (int32_t)tile);
+                    ptx::tma_load_3d_if(issue, dst + 8 * kUmBN * 4, mw + 1, fb, 0, (int32_t)grp, (int32_t)tile);
+                    ptx::tma_load_3d_if(issue, dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, 0, (int32_t)grp, (int32_t)tile);
+                } else {
+                    ptx::tma_load_2d_if(issue, dst, mw, fb, (int32_t)(tile * kUmBN), (int32_t)(c * (kUmBK / 8)));
+                    ptx::tma_load_2d_if(issue, dst + 8 * kUmBN * 4, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)grp);
+                    ptx::tma_load_2d_if(issue, dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)grp);
                 }
-                __syncwarp();
                 if (++in_group == per_group) { in_group = 0; ++grp; }
                 if (++c == n_chunks) {
                     c = grp = in_group = 0;
@@ -165,248 +164,242 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
                 }
             }
             if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
-        }
-    } else if (warp == kUmXWarp) {
-        // -------------------------------------------------------------- activations: one box per chunk (rows beyond M are zero)
-        uint32_t xs = 0, phase = 0;
-        const uint32_t item = u0 / n_chunks;
-        uint32_t c = u0 - item * n_chunks, tile = item;
-        uint32_t prob = item / p.n_tiles;
-        tile = item - prob * p.n_tiles;
-        for (uint32_t u = u0; u < u1; ++u) {
-            if (!ptx::mbar_wait_warp(x_empty + 8 * xs, phase ^ 1, abort_flag, p.wait_limit_ns)) {
+            if (!ptx::mbar_wait_warp(x_empty + 8 * xs, xphase ^ 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
                 break;
             }
-            if (ptx::elect_one()) {
-                ptx::fence_proxy_async_smem();
-                ptx::mbar_arrive_expect_tx(x_full + 8 * xs, x_bytes);
-                ptx::tma_load_3d(x_ring + xs * x_bytes, &group.maps[4 * prob + 3], x_full + 8 * xs, (int32_t)(c * kUmBK), 0, 0);
-            }
+            const uint32_t xb = x_full + 8 * xs, xd = x_ring + xs * 2 * x_bytes;
+            ptx::mbar_arrive_expect_tx_if(issue, xb, (1 + two) * x_bytes);      // (rows beyond M are zero)
+            ptx::tma_load_3d_if(issue, xd, &group.maps[4 * prob_x0 + 3], xb, (int32_t)(c_x[0] * kUmBK), 0, 0);
+            ptx::tma_load_3d_if(issue & two, xd + x_bytes, &group.maps[4 * prob_x1 + 3], xb, (int32_t)(c_x[1] * kUmBK), 0, 0);
             __syncwarp();
-            if (++xs == x_stages) { xs = 0; phase ^= 1; }
-            if (++c == n_chunks) {
-                c = 0;
-                if (++tile == p.n_tiles) { tile = 0; ++prob; }
-            }
+            if (++xs == x_stages) { xs = 0; xphase ^= 1; }
         }
     } else if (warp >= kUmIssueWarp) {
         // -------------------------------------------------------------- UMMA issuers, one per half of the columns: per chunk 4 k-steps of M 128 x N rows x K 16
         const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u), t = warp - kUmIssueWarp;
         const uint32_t my_full = a_full + 8 * kUmAStages * t, my_empty = a_empty + 8 * kUmAStages * t;
-        uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0;
+        uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0, second = 0;
         const uint32_t x_desc = (x_ring & 0x3FFFFu) >> 4;                   // (addresses enter a descriptor in 16-byte units)
         bool ok = true;
         for (uint32_t u = u0; ok && u < u1; ++piece) {
-            const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks);
-            if (piece > 0 && !ptx::mbar_wait_warp(acc_empty, (piece - 1) & 1, abort_flag, p.wait_limit_ns)) {
+            const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks), set = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
+            const uint32_t acc = t * 128 + set * 64;
+            if (use > 0 && !ptx::mbar_wait_warp(acc_empty + 8 * set, (use - 1) & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
                 break;
             }
             for (uint32_t first = 1; u < u_end; ++u, first = 0) {
-                if (!ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
+                if ((!second && !ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns)) ||
                     !ptx::mbar_wait_warp(my_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
                     if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const uint32_t x = x_desc + xs * (x_bytes / 16), a_cols = kUmABase + as * kUmAStageCols + t * 32, issue = ptx::elect_one();
+                const uint32_t x = x_desc + (2 * xs + second) * (x_bytes / 16), a_cols = kUmABase + as * kUmAStageCols + t * 32, issue = ptx::elect_one();
                 if (first)
-                    ptx::umma_bf16_ts_if<false>(issue, t * 128, a_cols, x, idesc);
+                    ptx::umma_bf16_ts_if<false>(issue, acc, a_cols, x, idesc);
                 else
-                    ptx::umma_bf16_ts_if<true>(issue, t * 128, a_cols, x, idesc);
+                    ptx::umma_bf16_ts_if<true>(issue, acc, a_cols, x, idesc);
 #pragma unroll
-                for (uint32_t k4 = 1; k4 < kUmBK / 16; ++k4) ptx::umma_bf16_ts_if<true>(issue, t * 128, a_cols + k4 * 8, x + k4 * 2, idesc);
+                for (uint32_t k4 = 1; k4 < kUmBK / 16; ++k4) ptx::umma_bf16_ts_if<true>(issue, acc, a_cols + k4 * 8, x + k4 * 2, idesc);
                 ptx::umma_commit_if(issue, my_empty + 8 * as);
-                ptx::umma_commit_if(issue, x_empty + 8 * xs);
+                if (second) {
+                    ptx::umma_commit_if(issue, x_empty + 8 * xs);
+                    if (++xs == x_stages) { xs = 0; xphase ^= 1; }
+                }
                 __syncwarp();
+                second ^= 1;
                 if (++as == kUmAStages) { as = 0; aphase ^= 1; }
-                if (++xs == x_stages) { xs = 0; xphase ^= 1; }
             }
-            if (ok) ptx::umma_commit_if(ptx::elect_one(), acc_full);
+            if (ok) ptx::umma_commit_if(ptx::elect_one(), acc_full + 8 * set);
             __syncwarp();
         }
     } else {
-        // -------------------------------------------------------------- sixteen warps: dequantise into tensor memory, then the epilogue
-        // Eight warps take two chunks of the range, a raw stage, the other eight the next two: a thread has one column and all eight words of a chunk, so
-        // that what stands around the arithmetic is paid once per eight words.
-        const uint32_t q = warp & 3, t = (warp >> 2) & 1, h = warp >> 3;   // lane quadrant, 128-column half of the tile, which of the two sets (and half of the rows in the epilogue)
-        const uint32_t n = t * 128 + q * 32 + lane;                          // this thread's column of the tile
-        const uint32_t lane_base = (q * 32) << 16;
-        const uint32_t m_begin = h * (p.rows / 2), m_end = min(p.M, m_begin + p.rows / 2);   // the rows of y this warp stores
-        uint32_t mask, magic;
-        asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
-        asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
-        const uint32_t my_full = a_full + 8 * kUmAStages * t, my_empty = a_empty + 8 * kUmAStages * t;
-        uint32_t rs = h, rphase = 0, piece = 0;
-        uint32_t v = u0 + 2 * h;                                             // this warp's next chunk
+        const uint32_t q = warp & 3, lane_base = (q * 32) << 16;             // lane quadrant
+        const bool dq = warp < kUmDqWarps;
         bool ok = true;
-
-        // 32 columns of the accumulator (rows m0.. of y) for this warp's columns of y; a narrow tile's columns beyond its rows are not used
-        auto load_rows = [&](uint32_t m0, float (&v)[32]) {
-            uint32_t r[32];
-            ptx::tmem_ld_32x32b_x32(tmem_base + lane_base + t * 128 + m0, r);
-            ptx::tmem_ld_wait();
+        if (dq) {
+            // ---------------------------------------------------------- sixteen warps: dequantise into tensor memory
+            // Eight warps take two chunks of the range, a raw stage, the other eight the next two: a thread has one column and all eight words of a chunk, so
+            // that what stands around the arithmetic is paid once per eight words.  They go on over the ends of tiles.
+            const uint32_t t = (warp >> 2) & 1, h = warp >> 3;               // 128-column half of the tile, which of the two sets
+            const uint32_t n = t * 128 + q * 32 + lane;                      // this thread's column of the tile
+            uint32_t mask, magic;
+            asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
+            asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
+            const uint32_t my_full = a_full + 8 * (kUmAStages * t + 2 * h), my_empty = a_empty + 8 * (kUmAStages * t + 2 * h);
+            const uint32_t lane_w = raw_ring + n * 4, lane_s = raw_ring + 8 * kUmBN * 4 + n * 2, lane_z = raw_ring + 8 * kUmBN * 4 + kUmBN * 2 + (n >> 3) * 4;
+            const uint32_t a_col = tmem_base + lane_base + kUmABase + 2 * h * kUmAStageCols + t * 32;
+            uint32_t rs = h, rphase = 0, aphase = 0;
+            for (uint32_t v = u0 + 2 * h; v < u1; v += 4) {
+                ok = ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns);
+#pragma unroll 1
+                for (uint32_t i = 0; ok && i < min(2u, u1 - v); ++i) {
+                    const uint32_t off = rs * (2 * kUmRawStride) + i * kUmRawStride;
+                    uint32_t words[8];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        };
-        // partial sums of a cut tile: each warp's own block of a piece, four rows of a column per float4
-        const uint32_t row4s = p.rows / 8;                                   // float4s a lane holds
-        const size_t piece_f4 = (size_t)p.rows * (kUmBN / 4);
-        float4* const my_block = (float4*)p.pieces + (size_t)warp * row4s * 32 + lane;
-
-        for (uint32_t u = u0; u < u1; ++piece) {
-            const uint32_t item = u / n_chunks, tile_u0 = item * n_chunks, tile_u1 = tile_u0 + n_chunks;
-            const uint32_t u_end = min(u1, tile_u1);
-            const bool whole = u == tile_u0 && u_end == tile_u1;
-            while (ok && v < u_end) {
-                const uint32_t second = (v - u0) & 1, as = (v - u0) & 3, aphase = ((v - u0) >> 2) & 1;     // of the two chunks of a raw stage
-                if (!second && !ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns)) {
+                    for (uint32_t j = 0; j < 8; ++j) words[j] = um_lds32(lane_w + off + j * (kUmBN * 4));
+                    const uint32_t sbits = um_lds16(lane_s + off), zword = um_lds32(lane_z + off);
+                    // The A stage is free once the UMMAs of four chunks ago have read it.  (Waited for here and not before the store: values that live across
+                    // a wait are moved once more to where the store takes them.)
+                    ok = ptx::mbar_wait(my_empty + 8 * i, aphase ^ 1, abort_flag, p.wait_limit_ns);
+                    if (!ok) break;
+                    ptx::tc_fence_after_sync();
+                    const uint32_t zz = ((zword >> ((n & 7) * 4)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
+                    const uint32_t ss = sbits * 0x00010001u;                                               // (s, s)
+                    uint32_t r[32];                            // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j) {
+                        uint32_t d[4];
+                        um_dequant_word(words[j], mask, magic, zz, ss, kTiled, d);
+#pragma unroll
+                        for (uint32_t e = 0; e < 4; ++e) r[4 * j + e] = d[e];
+                    }
+                    ptx::tmem_st_32x32b_x32(a_col + i * kUmAStageCols, r);
+                    ptx::tmem_st_wait();
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    ptx::mbar_arrive_if(my_full + 8 * i, lane == 0);
+                }
+                if (!ok) {
                     if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(v & 0x3FFFFF));
-                    ok = false;
                     break;
                 }
-                const uint32_t raw = raw_ring + rs * (2 * kUmRawStride) + second * kUmRawStride;
-                uint32_t words[8];
-#pragma unroll
-                for (uint32_t i = 0; i < 8; ++i) words[i] = um_lds32(raw + i * (kUmBN * 4) + n * 4);
-                const uint32_t sbits = um_lds16(raw + 8 * kUmBN * 4 + n * 2);
-                const uint32_t zword = um_lds32(raw + 8 * kUmBN * 4 + kUmBN * 2 + (n >> 3) * 4);
-                // The A stage is free once the UMMAs of four chunks ago have read it.  (Waited for here and not before the store: values that live across a
-                // wait are moved once more to where the store takes them.)
-                if (!ptx::mbar_wait(my_empty + 8 * as, aphase ^ 1, abort_flag, p.wait_limit_ns)) {
-                    if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0x800000 | (int)(v & 0x3FFFFF));
-                    ok = false;
-                    break;
-                }
-                ptx::tc_fence_after_sync();
-                const uint32_t zz = ((zword >> ((n & 7) * 4)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
-                const uint32_t ss = sbits * 0x00010001u;                                               // (s, s)
-                __syncwarp();
-                ptx::mbar_arrive_if(raw_empty + 8 * rs, second && lane == 0);
-                uint32_t r[32];                                // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
-#pragma unroll
-                for (uint32_t i = 0; i < 8; ++i) {
-                    uint32_t d[4];
-                    um_dequant_word(words[i], mask, magic, zz, ss, kTiled, d);
-#pragma unroll
-                    for (uint32_t e = 0; e < 4; ++e) r[4 * i + e] = d[e];
-                }
-                ptx::tmem_st_32x32b_x32(tmem_base + lane_base + kUmABase + as * kUmAStageCols + t * 32, r);
-                ptx::tmem_st_wait();
-                ptx::tc_fence_before_sync();
-                __syncwarp();
-                ptx::mbar_arrive_if(my_full + 8 * as, lane == 0);
-                v += 1 + 2 * second;
-                if (second) {
-                    rs += 2;
-                    if (rs >= kUmRawStages) { rs -= kUmRawStages; rphase ^= 1; }
-                }
+                ptx::mbar_arrive_if(raw_empty + 8 * rs, lane == 0);
+                aphase ^= 1;
+                rs += 2;
+                if (rs >= kUmRawStages) { rs -= kUmRawStages; rphase ^= 1; }
             }
+        }
+        // ------------------------------------------------------------------ accumulators to y, or to the parts of cut tiles
+        // The last tile of a range is emptied by the sixteen warps, which have nothing else left to do, those before it by the four epilogue warps while the
+        // sixteen go on.  Either way a tile is sixteen blocks, of 32 columns x half of the rows: block b has lane quadrant b % 4, column half (b / 4) % 2 and
+        // row half b / 8.  A dequantising warp does one block, an epilogue warp the four of its quadrant.
+        //
+        // A tile cut by range boundaries: each of its CTAs holds a partial sum over a part of K.  A block is finished by whichever CTA gets to it
+        // last.  A ticket is taken first (low half of the block's counter); all but the last then store their part and count it as
+        // written (high half).  The last one waits for those counts: whoever it waits for holds a ticket, so is running,
+        // and the tiles before in their range can only wait for CTAs further down.  It adds the parts in k order whoever it is:
+        // repeated calls agree bit for bit.
+        const uint32_t n_pieces = (u1 - 1) / n_chunks - u0 / n_chunks + 1, n_blocks = dq ? 1 : 4;
+        const uint32_t u_last = n_pieces == 1 ? u0 : (u1 - 1) / n_chunks * n_chunks;
+        const uint32_t row4s = p.rows / 8;                                   // float4s of a block a lane holds, four rows of its column each
+        const size_t piece_f4 = (size_t)p.rows * (kUmBN / 4);
+        uint32_t piece = dq ? n_pieces - 1 : 0;
+        for (uint32_t u = dq ? u_last : u0; ok && u < (dq ? u1 : u_last); ++piece) {
+            const uint32_t item = u / n_chunks, tile_u0 = item * n_chunks, tile_u1 = tile_u0 + n_chunks, u_end = min(u1, tile_u1);
+            const bool cut = u != tile_u0 || u_end != tile_u1;
+            const uint32_t set = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
             u = u_end;
-            // A tile cut by range boundaries: each of its CTAs holds a partial sum over a part of K.  The 32 columns x rows a warp
-            // owns are finished by the same warp of whichever CTA gets to it last, so no warp ever waits for another of its CTA.  A
-            // warp first takes a ticket (low half of the tile's counter); all but the last then store their part and count it as
-            // written (high half).  The last one waits for those counts: the warps it waits for hold a ticket, so they are running,
-            // and the tiles before in their range can only wait for CTAs further down.  It adds the parts in k order whoever it is:
-            // repeated calls agree bit for bit.
-            uint32_t c_first = 0, first_slot = 0, n_parts = 1, ticket = 0;
+            uint32_t c_first = 0, first_slot = 0, n_parts = 1, ticket = 0;   // lane i has the ticket of block i
             uint32_t* counter = nullptr;
-            if (ok && !whole && m_begin < m_end) {
+            if (cut) {
                 c_first = um_owner(tile_u0, p);
                 n_parts = um_owner(tile_u1 - 1, p) - c_first + 1;
-                first_slot = um_begin(c_first, p) < tile_u0 ? 1u : 0u;           // its range began in the tile before: this is not its first piece
-                counter = p.counters + c_first * kUmDqWarps + warp;
-                if (lane == 0) ticket = atomicAdd(counter, 1u) & 0xFFFFu;        // (its round trip passes under the last UMMAs)
+                first_slot = um_begin(c_first, p) < tile_u0 ? 1u : 0u;       // its range began in the tile before: this is not its first piece
+                counter = p.counters + c_first * kUmDqWarps + (dq ? warp : q + 4 * (lane & 3));
+                if (lane < n_blocks) ticket = atomicAdd(counter, 1u) & 0xFFFFu;        // (its round trip passes under the last UMMAs)
             }
-            // ---- epilogue: y[m][n0 + n] = D[lane n][column m]; a warp stores 32 consecutive columns of one row per instruction
-            if (ok && !ptx::mbar_wait(acc_full, piece & 1, abort_flag, p.wait_limit_ns)) {
+            if (!ptx::mbar_wait(acc_full + 8 * set, use & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xC00000);
-                ok = false;
+                break;
             }
-            if (!ok) break;
             ptx::tc_fence_after_sync();
-            ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-            if (ticket + 1 != n_parts) {
-                float4* mine = my_block + ((size_t)blockIdx.x * 2 + (piece == 0 ? 0 : 1)) * piece_f4;
+            __syncwarp();
+            const uint32_t hand_in = __ballot_sync(0xFFFFFFFFu, lane < n_blocks && ticket + 1 != n_parts);
+            // 32 columns of the accumulator (rows m0 .. of y) for this warp's columns of y; a narrow tile's columns beyond its rows are not used
+            auto load_rows = [&](uint32_t b, uint32_t m0, float (&v)[32]) {
+                uint32_t r[32];
+                ptx::tmem_ld_32x32b_x32(tmem_base + lane_base + ((b >> 2) & 1) * 128 + set * 64 + m0, r);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            };
 #pragma unroll 1
-                for (uint32_t i = 0; i < row4s; i += 8) {
+            for (uint32_t i = 0; i < n_blocks; ++i) {
+                if (!(hand_in >> i & 1)) continue;
+                const uint32_t b = dq ? warp : q + 4 * i;
+                float4* mine = (float4*)p.pieces + ((size_t)blockIdx.x * 2 + (piece == 0 ? 0 : 1)) * piece_f4 + (size_t)b * row4s * 32 + lane;
+#pragma unroll 1
+                for (uint32_t r4 = 0; r4 < row4s; r4 += 8) {
                     float v[32];
-                    load_rows(m_begin + 4 * i, v);
+                    load_rows(b, (b >> 3) * (p.rows / 2) + 4 * r4, v);
 #pragma unroll
                     for (uint32_t j = 0; j < 8; ++j)
-                        if (i + j < row4s) __stcg(mine + (i + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
+                        if (r4 + j < row4s) __stcg(mine + (r4 + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
                 }
-                ptx::tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) {
-                    ptx::mbar_arrive(acc_empty);
-                    __threadfence();                       // the warp's part is visible before it is counted
-                    atomicAdd(counter, 0x10000u);
-                }
-                continue;
             }
-            if (n_parts > 1) {
-                uint32_t good = 1;
-                if (lane == 0) {
-                    uint64_t t_start = 0;
-                    for (uint32_t spin = 1; (um_ld_acquire(counter) >> 16) + 1 != n_parts; ++spin) {
-                        if ((spin & 0x3F) == 0) {
-                            const uint64_t now = ptx::globaltimer_ns();
-                            if (t_start == 0) t_start = now;
-                            if (*abort_flag || now - t_start > p.wait_limit_ns) { *abort_flag = 1; good = 0; break; }
-                        }
-                    }
-                    if (good) *counter = 0;                // ready for the next launch
-                    else atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xE00000);
-                }
-                __syncwarp();                              // orders the other lanes' loads of the parts after lane 0's acquire (a shuffle does not)
-                good = __shfl_sync(0xFFFFFFFFu, good, 0);
-                if (!good) { ok = false; break; }
+            __syncwarp();
+            if (hand_in >> lane & 1) {
+                __threadfence();                       // the block is visible before it is counted
+                atomicAdd(counter, 0x10000u);
             }
             const uint32_t prob = item / p.n_tiles;
             float* const y_out = group.y[prob];
-            const uint32_t col = (item - prob * p.n_tiles) * kUmBN + n;
-            // Thirty-two rows at a time, part after part in k order.  What this costs is the round trips of the parts' loads, so eight of a lane's
-            // 16-byte loads are under way together: two problems of M = 128, N = 11008 31.7 us with sixteen rows of two parts at a time, 29.7 so;
-            // M = 40, N = 2560 16.2 and 15.2; M = 64, N = 14336, three problems 40.8 and 39.0.  (Where a warp has eight to sixteen rows the former is
-            // faster, 9.1 against 9.5 us at M = 17, N = 1024; both side by side make the loop above slower than either gains.)
 #pragma unroll 1
-            for (uint32_t i = 0; i < row4s; i += 8) {
-                const uint32_t m0 = m_begin + 4 * i;
-                float sum[32];
-                if (n_parts == 1) load_rows(m0, sum);
+            for (uint32_t i = 0; ok && i < n_blocks; ++i) {
+                if (hand_in >> i & 1) continue;
+                const uint32_t b = dq ? warp : q + 4 * i, m_begin = (b >> 3) * (p.rows / 2), m_end = min(p.M, m_begin + p.rows / 2);
                 if (n_parts > 1) {
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; ++j) sum[j] = 0.0f;
-#pragma unroll 1
-                    for (uint32_t part = 0; part < n_parts; ++part) {
-                        float f[32];
-                        const uint32_t cta = c_first + part;
-                        if (cta == blockIdx.x) {
-                            load_rows(m0, f);
-                        } else {
-                            const float4* theirs = my_block + ((size_t)cta * 2 + (part == 0 ? first_slot : 0u)) * piece_f4;
-#pragma unroll
-                            for (uint32_t j = 0; j < 8; ++j) {
-                                const float4 x = i + j < row4s ? __ldcg(theirs + (i + j) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-                                f[4 * j] = x.x; f[4 * j + 1] = x.y; f[4 * j + 2] = x.z; f[4 * j + 3] = x.w;
+                    uint32_t good = 1;
+                    if (lane == i) {
+                        uint64_t t_start = 0;
+                        for (uint32_t spin = 1; (um_ld_acquire(counter) >> 16) + 1 != n_parts; ++spin) {
+                            if ((spin & 0x3F) == 0) {
+                                const uint64_t now = ptx::globaltimer_ns();
+                                if (t_start == 0) t_start = now;
+                                if (*abort_flag || now - t_start > p.wait_limit_ns) { *abort_flag = 1; good = 0; break; }
                             }
                         }
-#pragma unroll
-                        for (uint32_t j = 0; j < 32; ++j) sum[j] += f[j];
+                        if (good) *counter = 0;            // ready for the next launch
+                        else atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xE00000);
                     }
+                    __syncwarp();                          // orders the other lanes' loads of the parts after that lane's acquire (a shuffle does not)
+                    ok = __shfl_sync(0xFFFFFFFFu, good, i) != 0;
+                    if (!ok) break;
                 }
-                if (col < p.N) {
+                const uint32_t col = (item - prob * p.n_tiles) * kUmBN + ((b >> 2) & 1) * 128 + q * 32 + lane;
+                // Thirty-two rows at a time, part after part in k order.  What this costs is the round trips of the parts' loads, so eight of a lane's
+                // 16-byte loads are under way together.
+#pragma unroll 1
+                for (uint32_t r4 = 0; r4 < row4s; r4 += 8) {
+                    const uint32_t m0 = m_begin + 4 * r4;
+                    float sum[32];
+                    if (n_parts == 1) {
+                        load_rows(b, m0, sum);
+                    } else {
 #pragma unroll
-                    for (uint32_t j = 0; j < 32; ++j)
-                        if (m0 + j < m_end) y_out[(size_t)(m0 + j) * p.N + col] = sum[j];
+                        for (uint32_t j = 0; j < 32; ++j) sum[j] = 0.0f;
+#pragma unroll 1
+                        for (uint32_t part = 0; part < n_parts; ++part) {
+                            float f[32];
+                            const uint32_t cta = c_first + part;
+                            if (cta == blockIdx.x) {
+                                load_rows(b, m0, f);
+                            } else {
+                                const float4* theirs = (const float4*)p.pieces + ((size_t)cta * 2 + (part == 0 ? first_slot : 0u)) * piece_f4 + (size_t)b * row4s * 32 + lane;
+#pragma unroll
+                                for (uint32_t j = 0; j < 8; ++j) {
+                                    const float4 x = r4 + j < row4s ? __ldcg(theirs + (r4 + j) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                                    f[4 * j] = x.x; f[4 * j + 1] = x.y; f[4 * j + 2] = x.z; f[4 * j + 3] = x.w;
+                                }
+                            }
+#pragma unroll
+                            for (uint32_t j = 0; j < 32; ++j) sum[j] += f[j];
+                        }
+                    }
+                    if (col < p.N) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; ++j)
+                            if (m0 + j < m_end) y_out[(size_t)(m0 + j) * p.N + col] = sum[j];
+                    }
                 }
             }
             ptx::tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(acc_empty);
+            if (!dq) ptx::mbar_arrive_if(acc_empty + 8 * set, lane == 0);
         }
     }
 
