@@ -193,6 +193,12 @@ __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, ui
                  ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+__device__ __forceinline__ void bulk_load_if(uint32_t issue, uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+                 "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}"
+                 ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar), "r"(issue)
+                 : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
@@ -308,6 +314,19 @@ __device__ __forceinline__ void umma_bf16_ts_if(uint32_t issue, uint32_t tmem_d,
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %3, p;\n\t"
         "}"
         ::"r"(tmem_d), "r"(tmem_a), "r"(desc_b_lo | (1u << 16)), "r"(idesc), "n"(kAccumulate ? 1 : 0), "n"((1024 >> 4) | (1 << 14) | (2 << 29)), "r"(issue)
+        : "memory");
+}
+__device__ __forceinline__ void umma_bf16_ts_if(uint32_t issue, uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .b64 d;\n\t"
+        "mov.b64 d, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %3, p;\n\t"
+        "}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(desc_b_lo | (1u << 16)), "r"(idesc), "r"(accumulate), "n"((1024 >> 4) | (1 << 14) | (2 << 29)), "r"(issue)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit_if(uint32_t issue, uint32_t bar) {

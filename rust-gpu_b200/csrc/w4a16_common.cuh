@@ -117,13 +117,15 @@ __device__ __forceinline__ void um_dequant_word(uint32_t wd, uint32_t mask, uint
     }
 }
 
-// The four tensor maps (weights, scales, zero points, activations) and the output of up to kProblems problems of one shape, in the kernel parameters:
-// 16.6 KB for a list, 0.5 KB for one problem (a launch copies them: a single call 4.2 us on the host instead of 5.0, 20 x 14336 x 2048 waited for 24.8 instead of 26.0).
+// The tensor maps and outputs of up to kProblems problems of one shape, in the kernel parameters: row layout, four maps each (weights, scales, zero points,
+// activations); tile-major layout, the activations' alone and the buffer, which is copied from without one (4.6 KB for a list).  A launch copies its
+// parameters: a single call in a block of its own size 4.2 us on the host instead of 5.0, 20 x 14336 x 2048 waited for 24.8 instead of 26.0.
 constexpr uint32_t kUmMaxGroup = 32;
-template <uint32_t kProblems>
+template <uint32_t kProblems, bool kTiled>
 struct UmGroup {
-    CUtensorMap maps[4 * kProblems];
+    CUtensorMap maps[(kTiled ? 1 : 4) * kProblems];
     float* y[kProblems];
+    const uint8_t* base[kTiled ? kProblems : 1];
 };
 
 // How a launch shares out its tiles: the parts of a tile's K over the CTAs of a cluster (one problem); whole tiles per CTA; equal ranges of the

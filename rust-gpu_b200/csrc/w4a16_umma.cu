@@ -423,8 +423,9 @@ namespace t0 {
 // w4a16_umma_cut.cu
 int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas);
 uint32_t w4a16_umma_cut_rows(uint32_t M);
-template <uint32_t kProblems>
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems>& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas);
+template <uint32_t kProblems, bool kTiled>
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems, kTiled>& group, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas,
+                          size_t off_scales, size_t off_zeros);
 
 static t0_w4a16_args um_args(uint64_t a, uint64_t packed, uint64_t scales, uint64_t zeros, uint64_t y, uint32_t M, uint32_t N, uint32_t K, uint32_t group) {
     t0_w4a16_args q;
@@ -528,25 +529,40 @@ static UmParams um_params(t0_runtime* rt, uint64_t y, uint32_t M, uint32_t N, ui
     return p;
 }
 
-// The maps and output of problem i of a launch on the kernel that takes whole tiles or cuts them (w4a16_umma_cut.cu).  Tile-major weights, or the row layout.
-template <uint32_t kProblems>
-static int um_group_entry(UmGroup<kProblems>& grp, uint32_t i, const t0_w4a16_args& a, bool tiled) {
+// The maps, buffer and output of problem i of a launch on the kernel that takes whole tiles or cuts them (w4a16_umma_cut.cu).
+template <uint32_t kProblems, bool kTiled>
+static int um_group_entry(UmGroup<kProblems, kTiled>& grp, uint32_t i, const t0_w4a16_args& a) {
     const uint32_t rows = w4a16_umma_cut_rows(a.m);
     grp.y[i] = (float*)a.y;
-    return tiled ? um_maps_tiled(a.a, a.packed, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows)
-                 : um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows);
+    if constexpr (kTiled) {
+        grp.base[i] = (const uint8_t*)a.packed;
+        return gemm::make_map_kmajor(&grp.maps[i], (const void*)a.a, a.m, a.k, a.k, 1, rows);
+    } else {
+        return um_maps(a.a, a.packed, a.scales, a.zeros, a.m, a.n, a.k, a.group, &grp.maps[4 * i], rows);
+    }
 }
 
 // `count` problems of one shape in one launch, which run concurrently.
-static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count, bool tiled, uint32_t cut_ctas) {
-    static UmGroup<kUmMaxGroup> grp;     // 16.6 KB: kept off the stack, filled under the lock, copied by the launch
+template <bool kTiled>
+static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count, uint32_t cut_ctas) {
+    static UmGroup<kUmMaxGroup, kTiled> grp;     // up to 16.6 KB: kept off the stack, filled under the lock, copied by the launch
     static std::mutex grp_mu;
     std::lock_guard<std::mutex> lock(grp_mu);
     for (uint32_t i = 0; i < count; ++i) {
-        int rc = um_group_entry(grp, i, args[i], tiled);
+        int rc = um_group_entry(grp, i, args[i]);
         if (rc != T0_OK) return rc;
     }
-    return launch_w4a16_umma_cut(rt, grp, tiled, args[0].m, args[0].n, args[0].k, args[0].group, count, cut_ctas);
+    const TiledLayout L = tiled_layout(args[0].k, args[0].n, args[0].group);
+    return launch_w4a16_umma_cut(rt, grp, args[0].m, args[0].n, args[0].k, args[0].group, count, cut_ctas, kTiled ? L.off_scales : 0, kTiled ? L.off_zeros : 0);
+}
+
+template <bool kTiled>
+static int um_launch_single(t0_runtime* rt, const t0_w4a16_args& a, uint32_t cut_ctas) {
+    UmGroup<1, kTiled> one;
+    int rc = um_group_entry(one, 0, a);
+    if (rc != T0_OK) return rc;
+    const TiledLayout L = tiled_layout(a.k, a.n, a.group);
+    return launch_w4a16_umma_cut(rt, one, a.m, a.n, a.k, a.group, 1, cut_ctas, kTiled ? L.off_scales : 0, kTiled ? L.off_zeros : 0);
 }
 
 static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
@@ -558,9 +574,8 @@ static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
     if (rc != T0_OK) return rc;
     const int plan = w4a16_umma_plan(rt, a.m, a.n, a.k, 1, split, ceil_div(n_tiles, clusters), &ctas);
     if (plan != kUmClusters) {
-        UmGroup<1> one;
-        rc = um_group_entry(one, 0, a, tiled);
-        return rc != T0_OK ? rc : launch_w4a16_umma_cut(rt, one, tiled, a.m, a.n, a.k, a.group, 1, plan == kUmCut ? ctas : 0);
+        const uint32_t cut_ctas = plan == kUmCut ? ctas : 0;
+        return tiled ? um_launch_single<true>(rt, a, cut_ctas) : um_launch_single<false>(rt, a, cut_ctas);
     }
     UmParams p = um_params(rt, a.y, a.m, a.n, a.k, a.group);
     p.tiled = tiled ? 1 : 0;
@@ -593,7 +608,8 @@ static int um_launch_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_t
     }
     uint32_t ctas;
     const int plan = w4a16_umma_plan(rt, a0.m, a0.n, a0.k, count, 0, 0, &ctas);
-    return um_launch_list(rt, args, count, tiled, plan == kUmCut ? ctas : 0);
+    const uint32_t cut_ctas = plan == kUmCut ? ctas : 0;
+    return tiled ? um_launch_list<true>(rt, args, count, cut_ctas) : um_launch_list<false>(rt, args, count, cut_ctas);
 }
 
 int launch_w4a16_umma_tiled_grouped(t0_runtime* rt, const t0_w4a16_args* args, uint32_t count) { return um_launch_grouped(rt, args, count, true); }

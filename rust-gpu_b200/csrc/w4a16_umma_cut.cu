@@ -36,19 +36,32 @@ constexpr uint32_t kUmDqWarps = 16;
 // (device time of queued launches, as below; the same call takes 34 us by the host's clock in blocks of calls).
 constexpr uint32_t kUmEpWarp0 = kUmDqWarps, kUmEpWarps = 4;  // empty the accumulators of all but the last tile of a range, one per tensor-memory lane quadrant
 constexpr uint32_t kUmIssueWarp = kUmEpWarp0 + kUmEpWarps, kUmLoadWarp = kUmIssueWarp + 2;     // (two issuing warps)
-constexpr uint32_t kUmThreads = (kUmLoadWarp + 1) * 32;
+constexpr uint32_t kUmThreads = (kUmLoadWarp + 1) * 32;     // (a warp more, even an idle one, adds 0.3 us to a launch)
 constexpr uint32_t kUmXBytes = 6 * 128 * kUmBK * 2;         // activations, in stages of two chunks: three at M = 128, four at M <= 96
 constexpr uint32_t kUmMaxXStages = 4;
 // Tensor memory (512 columns): accumulators 2 x 128 columns, then four A stages of 2 halves x 4 k-steps x 8 columns.
 constexpr uint32_t kUmTmemCols = 512;
 constexpr uint32_t kUmABase = 256;                          // first column of the A stages
-constexpr uint32_t kUmAStageCols = 64;
-constexpr uint32_t kUmAStages = 4;
+constexpr uint32_t kUmAStageCols = 128;                     // of two chunks: [chunk][half][k-step] x 8
+constexpr uint32_t kUmAStages = 2;                          // one to a set of eight warps
+constexpr uint32_t kUmScaleOff = 2 * 8 * kUmBN * 4, kUmScaleStride = 1024, kUmRawStage = kUmScaleOff + 2 * kUmScaleStride;      // words of two chunks, then scales and zero points
 constexpr uint32_t kUmRawStages = 6;                        // raw weight stages of two chunks: 106 KB in flight per SM (an even number: a set of warps has every second one)
 // (more than half an SM's shared memory: the kernel takes all 512 tensor-memory columns, so two of its CTAs must never share an SM)
-constexpr uint32_t kUmSmem = kUmRawStages * 2 * kUmRawStride + kUmXBytes + 512 + 1024;
+constexpr uint32_t kUmSmem = kUmRawStages * kUmRawStage + kUmXBytes + 512 + 1024;
 constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long where sums may be: below it the finish costs more than the range
 constexpr size_t kUmCounterBytes = 16 * 1024;               // one word per CTA and dequantisation warp (up to 256 CTAs)
+
+// Division by a number the host knows: the quotient by a product with floor((2^32 - 1) / d), at most two short.  Every CTA divides a few times before its first
+// load, on the way of the whole launch, and a division takes 150 cycles.
+struct UmDiv {
+    uint32_t d, m;
+};
+inline UmDiv um_divisor(uint32_t d) { return {d, 0xFFFFFFFFu / d}; }
+__device__ __forceinline__ uint32_t um_div(uint32_t a, const UmDiv& by) {
+    uint32_t q = __umulhi(a, by.m), r = a - q * by.d;
+    if (r >= by.d) { ++q; r -= by.d; }
+    return r >= by.d ? q + 1 : q;
+}
 
 struct UmParams {
     int* status;
@@ -61,29 +74,34 @@ struct UmParams {
     uint32_t n_tiles, n_chunks;
     uint32_t total;          // chunks of the launch, shared out evenly (less than 2^24)
     uint32_t whole;          // shared out by tiles instead: no tile is cut
+    uint32_t tiles;          // of the launch: total / n_chunks
+    uint32_t per_group;      // chunks per scale / zero-point row
+    uint32_t x_stages;       // stages of activations
+    UmDiv by_grid, by_total, by_chunks, by_tiles, by_group;   // the CTAs, total, n_chunks, n_tiles, per_group
+    uint32_t off_scales, off_zeros;   // tile-major weights: where in a problem's buffer they begin, in units of 16 bytes
 };
 
-// First chunk of a CTA's range, and the CTA whose range holds a chunk: in 32 bits (at most 256 CTAs and 2^24 chunks), since a warp that
-// finishes a cut tile needs a few of these and a 64-bit division takes hundreds of cycles.
+// First chunk of a CTA's range, and the CTA whose range holds a chunk (at most 256 CTAs and 2^24 chunks, so that products fit 32 bits; whole tiles: 2^23 tiles).
 __device__ __forceinline__ uint32_t um_begin(uint32_t cta, const UmParams& p) {
-    return p.whole ? cta * (p.total / p.n_chunks) / gridDim.x * p.n_chunks : cta * p.total / gridDim.x;
+    return p.whole ? um_div(cta * p.tiles, p.by_grid) * p.n_chunks : um_div(cta * p.total, p.by_grid);
 }
-__device__ __forceinline__ uint32_t um_owner(uint32_t chunk, const UmParams& p) { return ((chunk + 1) * gridDim.x - 1) / p.total; }
+__device__ __forceinline__ uint32_t um_owner(uint32_t chunk, const UmParams& p) { return um_div((chunk + 1) * gridDim.x - 1, p.by_total); }
 
 // kTiled: weights in the tile-major layout (3-D maps: column in tile, row, tile), else the row layout; kProblems: room for so many problems
 template <bool kTiled, uint32_t kProblems>
 __global__ void __launch_bounds__(kUmThreads, 1)
-w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblems> group) {
+w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblems, kTiled> group) {
+    constexpr uint32_t kMaps = kTiled ? 1 : 4;                // tensor maps of a problem, the activations' last
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t raw_ring = smem;
-    const uint32_t x_ring = smem + kUmRawStages * 2 * kUmRawStride;           // activations: [rows][64 k] bf16, 128-byte swizzle, per stage
+    const uint32_t x_ring = smem + kUmRawStages * kUmRawStage;           // activations: [rows][64 k] bf16, 128-byte swizzle, per stage
     const uint32_t bars = x_ring + kUmXBytes;
     const uint32_t raw_full = bars, raw_empty = bars + 8 * kUmRawStages;
     const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * 2 * kUmAStages;     // [128-column half][stage]
     const uint32_t x_full = a_empty + 8 * 2 * kUmAStages, x_empty = x_full + 8 * kUmMaxXStages;
     const uint32_t acc_full = x_empty + 8 * kUmMaxXStages, acc_empty = acc_full + 16;                // [accumulator set]
-    const uint32_t x_bytes = p.rows * kUmBK * 2, x_stages = min(kUmMaxXStages, kUmXBytes / (2 * x_bytes));
+    const uint32_t x_bytes = p.rows * kUmBK * 2, x_stages = p.x_stages;
     __shared__ uint32_t tmem_holder;
     __shared__ int s_abort;
     volatile int* abort_flag = &s_abort;
@@ -112,7 +130,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
         s_abort = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
-        for (uint32_t i = 0; i < 4; ++i) ptx::tma_prefetch_desc(&group.maps[4 * (u0 / (n_chunks * p.n_tiles)) + i]);
+        for (uint32_t i = 0; i < kMaps; ++i) ptx::tma_prefetch_desc(&group.maps[kMaps * um_div(um_div(u0, p.by_chunks), p.by_tiles) + i]);
     }
     if (warp == kUmIssueWarp) {
         ptx::tmem_alloc(ptx::smem_u32(&tmem_holder), kUmTmemCols);
@@ -123,98 +141,120 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     ptx::tc_fence_after_sync();
     constexpr uint32_t tmem_base = 0;    // all columns are allocated: tensor-memory addresses are constants
     ptx::grid_launch_dependents();
+    // where the range begins: tile and chunk, problem, row of scales
+    const uint32_t per_group = p.per_group;
+    const uint32_t item0 = um_div(u0, p.by_chunks), c0 = u0 - item0 * n_chunks, prob0 = um_div(item0, p.by_tiles), tile0 = item0 - prob0 * p.n_tiles;
+    const uint32_t at0 = u0 - prob0 * n_chunks * p.n_tiles, row0 = um_div(at0, p.by_group), in_row0 = at0 - row0 * per_group;
     ptx::grid_dependency_wait();
 
+    // The chunks of a range are taken in pairs, an even chunk of a tile and the next one; a pair is short where the range begins or ends inside it, or the tile
+    // with an odd number.  Chunk i of a pair has place i of its stages.  Every role walks the pairs so: n chunks, the first of them i0.
+    struct Pairs {
+        uint32_t u, c, i0, n;                        // chunk of the launch, chunk of the tile
+    };
+    auto first_pair = [&]() { Pairs w; w.u = u0; w.c = c0; w.i0 = w.c & 1; w.n = min(min(2 - w.i0, n_chunks - w.c), u1 - u0); return w; };
+    auto next_pair = [&](Pairs& w) {
+        w.u += w.n; w.c += w.n;
+        if (w.c == n_chunks) w.c = 0;
+        w.i0 = 0;                                    // (all but the first begin at an even chunk)
+        w.n = min(min(2u, n_chunks - w.c), u1 - w.u);
+    };
     // The serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
     if (warp == kUmLoadWarp) {
-        // -------------------------------------------------------------- per two chunks: raw weights, scales, zero points (three TMA boxes a chunk), then activations (one)
-        uint32_t stage = 0, phase = 0, xs = 0, xphase = 0;
-        const uint32_t item = u0 / n_chunks, per_group = p.group / kUmBK;
-        uint32_t c = u0 - item * n_chunks;
-        uint32_t grp = c / per_group, in_group = c - grp * per_group;
-        uint32_t prob = item / p.n_tiles, tile = item - prob * p.n_tiles;
-        for (uint32_t u = u0; u < u1;) {
+        // -------------------------------------------------------------- raw weights, scales and zero points, activations (one box per chunk, rows beyond M are zero)
+        uint32_t stage = 0, phase = 0, xs = 0, xphase = 0, x_dst = x_ring;
+        uint32_t prob = prob0, tile = tile0, at = at0, row = row0, in_row = in_row0;      // at: chunk of the problem, row: its row of scales
+        const uint32_t rows_a_pair = per_group & 1 ? 2 : 1;
+        for (Pairs w = first_pair(); w.u < u1; next_pair(w)) {
             if (!ptx::mbar_wait_warp(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(c & 0xFFFFFF));
+                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w.u & 0xFFFFFF));
                 break;
             }
-            const uint32_t fb = raw_full + 8 * stage, u_stop = min(u1, u + 2), issue = ptx::elect_one();
-            const uint32_t c_x[2] = {c, c + 1 == n_chunks ? 0 : c + 1}, prob_x0 = prob;
-            uint32_t prob_x1 = prob, dst = raw_ring + stage * (2 * kUmRawStride);
-            const uint32_t two = u_stop - u == 2;
+            const uint32_t fb = raw_full + 8 * stage, issue = ptx::elect_one(), dst = raw_ring + stage * kUmRawStage;
             ptx::fence_proxy_async_smem();           // the stage was read through the generic proxy, the copies write it through the async proxy
-            ptx::mbar_arrive_expect_tx_if(issue, fb, (u_stop - u) * kUmRawBytes);
-            for (; u < u_stop; ++u, dst += kUmRawStride) {
-                const CUtensorMap* const mw = &group.maps[4 * prob];
-                prob_x1 = prob;
-                if constexpr (kTiled) {
-                    // tile-major layout: the chunk's 8 KB of words are contiguous, as are its scales and zero points
-                    ptx::tma_load_3d_if(issue, dst, mw, fb, 0, (int32_t)(c * (kUmBK / 8)), (int32_t)tile);
-                    ptx::tma_load_3d_if(issue, dst + 8 * kUmBN * 4, mw + 1, fb, 0, (int32_t)grp, (int32_t)tile);
-                    ptx::tma_load_3d_if(issue, dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, 0, (int32_t)grp, (int32_t)tile);
-                } else {
-                    ptx::tma_load_2d_if(issue, dst, mw, fb, (int32_t)(tile * kUmBN), (int32_t)(c * (kUmBK / 8)));
-                    ptx::tma_load_2d_if(issue, dst + 8 * kUmBN * 4, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)grp);
-                    ptx::tma_load_2d_if(issue, dst + 8 * kUmBN * 4 + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)grp);
+            // a scale row for each chunk, or (group a multiple of two chunks) one for both, in place 0
+            const uint32_t rows = rows_a_pair == 1 ? 1 : w.n, i0 = rows_a_pair == 1 ? 0 : w.i0, step = in_row + 1 == per_group ? 1 : 0;      // to the second chunk's row
+            ptx::mbar_arrive_expect_tx_if(issue, fb, w.n * (8 * kUmBN * 4) + rows * (kUmBN * 2 + kUmBN / 2));
+            if constexpr (kTiled) {
+                // the words of a problem lie one behind the other in the order of its chunks, its scales and zero points likewise
+                const uint8_t* base = group.base[prob];
+                ptx::bulk_load_if(issue, dst + w.i0 * (8 * kUmBN * 4), base + (size_t)at * (8 * kUmBN * 4), w.n * (8 * kUmBN * 4), fb);
+                for (uint32_t j = 0; j < rows; ++j) {
+                    ptx::bulk_load_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride, base + (size_t)p.off_scales * 16 + (size_t)(row + j * step) * (kUmBN * 2), kUmBN * 2, fb);
+                    ptx::bulk_load_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride + kUmBN * 2, base + (size_t)p.off_zeros * 16 + (size_t)(row + j * step) * (kUmBN / 2), kUmBN / 2, fb);
                 }
-                if (++in_group == per_group) { in_group = 0; ++grp; }
-                if (++c == n_chunks) {
-                    c = grp = in_group = 0;
-                    if (++tile == p.n_tiles) { tile = 0; ++prob; }
+            } else {
+                const CUtensorMap* const mw = &group.maps[4 * prob];
+                const uint32_t grp = row - um_div(tile * n_chunks, p.by_group);
+                for (uint32_t j = 0; j < w.n; ++j)
+                    ptx::tma_load_2d_if(issue, dst + (w.i0 + j) * (8 * kUmBN * 4), mw, fb, (int32_t)(tile * kUmBN), (int32_t)((w.c + j) * (kUmBK / 8)));
+                for (uint32_t j = 0; j < rows; ++j) {
+                    ptx::tma_load_2d_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)(grp + j * step));
+                    ptx::tma_load_2d_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)(grp + j * step));
                 }
             }
             if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
             if (!ptx::mbar_wait_warp(x_empty + 8 * xs, xphase ^ 1, abort_flag, p.wait_limit_ns)) {
-                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(c & 0x3FFFFF));
+                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(w.u & 0x3FFFFF));
                 break;
             }
-            const uint32_t xb = x_full + 8 * xs, xd = x_ring + xs * 2 * x_bytes;
-            ptx::mbar_arrive_expect_tx_if(issue, xb, (1 + two) * x_bytes);      // (rows beyond M are zero)
-            ptx::tma_load_3d_if(issue, xd, &group.maps[4 * prob_x0 + 3], xb, (int32_t)(c_x[0] * kUmBK), 0, 0);
-            ptx::tma_load_3d_if(issue & two, xd + x_bytes, &group.maps[4 * prob_x1 + 3], xb, (int32_t)(c_x[1] * kUmBK), 0, 0);
+            const CUtensorMap* const mx = &group.maps[kMaps * prob + kMaps - 1];
+            ptx::mbar_arrive_expect_tx_if(issue, x_full + 8 * xs, w.n * x_bytes);
+            ptx::tma_load_3d_if(issue, x_dst + w.i0 * x_bytes, mx, x_full + 8 * xs, (int32_t)(w.c * kUmBK), 0, 0);
+            ptx::tma_load_3d_if(issue & (w.n >> 1), x_dst + x_bytes, mx, x_full + 8 * xs, (int32_t)((w.c + 1) * kUmBK), 0, 0);
             __syncwarp();
-            if (++xs == x_stages) { xs = 0; xphase ^= 1; }
+            at += w.n;
+            in_row += w.n;
+            while (in_row >= per_group) { in_row -= per_group; ++row; }
+            if (w.c + w.n == n_chunks && ++tile == p.n_tiles) { tile = 0; ++prob; at = row = in_row = 0; }
+            x_dst += 2 * x_bytes;
+            if (++xs == x_stages) { xs = 0; xphase ^= 1; x_dst = x_ring; }
         }
     } else if (warp >= kUmIssueWarp) {
         // -------------------------------------------------------------- UMMA issuers, one per half of the columns: per chunk 4 k-steps of M 128 x N rows x K 16
         const uint32_t idesc = ptx::make_idesc_bf16_f32(128, p.rows, 0u), t = warp - kUmIssueWarp;
         const uint32_t my_full = a_full + 8 * kUmAStages * t, my_empty = a_empty + 8 * kUmAStages * t;
-        uint32_t as = 0, aphase = 0, xs = 0, xphase = 0, piece = 0, second = 0;
-        const uint32_t x_desc = (x_ring & 0x3FFFFu) >> 4;                   // (addresses enter a descriptor in 16-byte units)
-        bool ok = true;
-        for (uint32_t u = u0; ok && u < u1; ++piece) {
-            const uint32_t u_end = min(u1, (u / n_chunks + 1) * n_chunks), set = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
-            const uint32_t acc = t * 128 + set * 64;
-            if (use > 0 && !ptx::mbar_wait_warp(acc_empty + 8 * set, (use - 1) & 1, abort_flag, p.wait_limit_ns)) {
-                if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
+        const uint32_t x0 = (x_ring & 0x3FFFFu) >> 4, a_cols = kUmABase + t * 32;      // (addresses enter a descriptor in 16-byte units)
+        uint32_t set = 0, aphase = 0, xs = 0, xphase = 0, x = x0, piece = 0;           // set: whose A stages, 2 set and 2 set + 1, are next
+        uint32_t acc = t * 128, more = 0;                                              // the piece's accumulator, empty so far or not
+        for (Pairs w = first_pair(); w.u < u1; next_pair(w)) {
+            if (!ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns) ||
+                !ptx::mbar_wait_warp(my_full + 8 * set, aphase, abort_flag, p.wait_limit_ns)) {
+                if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(w.u & 0x7FFFFF));
                 break;
             }
-            for (uint32_t first = 1; u < u_end; ++u, first = 0) {
-                if ((!second && !ptx::mbar_wait_warp(x_full + 8 * xs, xphase, abort_flag, p.wait_limit_ns)) ||
-                    !ptx::mbar_wait_warp(my_full + 8 * as, aphase, abort_flag, p.wait_limit_ns)) {
-                    if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | (int)(u & 0x7FFFFF));
-                    ok = false;
+            ptx::tc_fence_after_sync();
+            const uint32_t issue = ptx::elect_one();
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) {
+                if (i < w.i0 || i >= w.i0 + w.n) continue;
+                const uint32_t a = a_cols + set * kUmAStageCols + i * 64, xi = x + i * (x_bytes / 16);
+                ptx::umma_bf16_ts_if(issue, acc, a, xi, idesc, more);
+#pragma unroll
+                for (uint32_t k4 = 1; k4 < kUmBK / 16; ++k4) ptx::umma_bf16_ts_if<true>(issue, acc, a + k4 * 8, xi + k4 * 2, idesc);
+                more = 1;
+            }
+            ptx::umma_commit_if(issue, my_empty + 8 * set);
+            ptx::umma_commit_if(issue, x_empty + 8 * xs);
+            if (w.c + w.n == n_chunks || w.u + w.n == u1) {
+                // the piece is complete; on to the next one's accumulators, which the epilogue warps must have emptied
+                ptx::umma_commit_if(issue, acc_full + 8 * (acc_sets == 2 ? piece & 1 : 0));
+                __syncwarp();
+                ++piece;
+                const uint32_t s = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
+                if (w.u + w.n < u1 && use > 0 && !ptx::mbar_wait_warp(acc_empty + 8 * s, (use - 1) & 1, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000);
                     break;
                 }
                 ptx::tc_fence_after_sync();
-                const uint32_t x = x_desc + (2 * xs + second) * (x_bytes / 16), a_cols = kUmABase + as * kUmAStageCols + t * 32, issue = ptx::elect_one();
-                if (first)
-                    ptx::umma_bf16_ts_if<false>(issue, acc, a_cols, x, idesc);
-                else
-                    ptx::umma_bf16_ts_if<true>(issue, acc, a_cols, x, idesc);
-#pragma unroll
-                for (uint32_t k4 = 1; k4 < kUmBK / 16; ++k4) ptx::umma_bf16_ts_if<true>(issue, acc, a_cols + k4 * 8, x + k4 * 2, idesc);
-                ptx::umma_commit_if(issue, my_empty + 8 * as);
-                if (second) {
-                    ptx::umma_commit_if(issue, x_empty + 8 * xs);
-                    if (++xs == x_stages) { xs = 0; xphase ^= 1; }
-                }
-                __syncwarp();
-                second ^= 1;
-                if (++as == kUmAStages) { as = 0; aphase ^= 1; }
+                acc = t * 128 + s * 64;
+                more = 0;
             }
-            if (ok) ptx::umma_commit_if(ptx::elect_one(), acc_full + 8 * set);
             __syncwarp();
+            aphase ^= set;
+            set ^= 1;
+            x += 2 * (x_bytes / 16);
+            if (++xs == x_stages) { xs = 0; xphase ^= 1; x = x0; }
         }
     } else {
         const uint32_t q = warp & 3, lane_base = (q * 32) << 16;             // lane quadrant
@@ -229,24 +269,31 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
             uint32_t mask, magic;
             asm volatile("mov.b32 %0, 0x000F000F;" : "=r"(mask));
             asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
-            const uint32_t my_full = a_full + 8 * (kUmAStages * t + 2 * h), my_empty = a_empty + 8 * (kUmAStages * t + 2 * h);
-            const uint32_t lane_w = raw_ring + n * 4, lane_s = raw_ring + 8 * kUmBN * 4 + n * 2, lane_z = raw_ring + 8 * kUmBN * 4 + kUmBN * 2 + (n >> 3) * 4;
-            const uint32_t a_col = tmem_base + lane_base + kUmABase + 2 * h * kUmAStageCols + t * 32;
+            const uint32_t my_full = a_full + 8 * (kUmAStages * t + h), my_empty = a_empty + 8 * (kUmAStages * t + h);
+            const uint32_t lane_w = raw_ring + n * 4, lane_s = raw_ring + kUmScaleOff + n * 2, lane_z = raw_ring + kUmScaleOff + kUmBN * 2 + (n >> 3) * 4;
+            const uint32_t a_col = tmem_base + lane_base + kUmABase + h * kUmAStageCols + t * 32;
+            const uint32_t second = per_group & 1 ? kUmScaleStride : 0;      // where the second chunk's scales and zero points are: its own, or the first one's
             uint32_t rs = h, rphase = 0, aphase = 0;
-            for (uint32_t v = u0 + 2 * h; v < u1; v += 4) {
-                ok = ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns);
-#pragma unroll 1
-                for (uint32_t i = 0; ok && i < min(2u, u1 - v); ++i) {
-                    const uint32_t off = rs * (2 * kUmRawStride) + i * kUmRawStride;
+            Pairs w = first_pair();
+            if (h) next_pair(w);
+            for (; w.u < u1; next_pair(w), next_pair(w)) {
+                // The A stage is free once the UMMAs of this set's pair before have read it.  (Waited for here and not before the stores: values that
+                // live across a wait are moved once more to where the store takes them.)
+                ok = ptx::mbar_wait(raw_full + 8 * rs, rphase, abort_flag, p.wait_limit_ns) &&
+                     ptx::mbar_wait(my_empty, aphase ^ 1, abort_flag, p.wait_limit_ns);
+                if (!ok) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(w.u & 0x3FFFFF));
+                    break;
+                }
+                ptx::tc_fence_after_sync();
+                const uint32_t off = rs * kUmRawStage;
+                // (both chunks, also where a pair is short: what comes of the bytes that happen to be there is not used)
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
                     uint32_t words[8];
 #pragma unroll
-                    for (uint32_t j = 0; j < 8; ++j) words[j] = um_lds32(lane_w + off + j * (kUmBN * 4));
-                    const uint32_t sbits = um_lds16(lane_s + off), zword = um_lds32(lane_z + off);
-                    // The A stage is free once the UMMAs of four chunks ago have read it.  (Waited for here and not before the store: values that live across
-                    // a wait are moved once more to where the store takes them.)
-                    ok = ptx::mbar_wait(my_empty + 8 * i, aphase ^ 1, abort_flag, p.wait_limit_ns);
-                    if (!ok) break;
-                    ptx::tc_fence_after_sync();
+                    for (uint32_t j = 0; j < 8; ++j) words[j] = um_lds32(lane_w + off + (8 * i + j) * (kUmBN * 4));
+                    const uint32_t sbits = um_lds16(lane_s + off + i * second), zword = um_lds32(lane_z + off + i * second);
                     const uint32_t zz = ((zword >> ((n & 7) * 4)) & 0xFu) * 0x00010001u + 0x43004300u;     // bf16x2 (128+z, 128+z)
                     const uint32_t ss = sbits * 0x00010001u;                                               // (s, s)
                     uint32_t r[32];                            // k order: (0,1) (2,3) ..., two consecutive k per tensor-memory column
@@ -257,16 +304,12 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
 #pragma unroll
                         for (uint32_t e = 0; e < 4; ++e) r[4 * j + e] = d[e];
                     }
-                    ptx::tmem_st_32x32b_x32(a_col + i * kUmAStageCols, r);
-                    ptx::tmem_st_wait();
-                    ptx::tc_fence_before_sync();
-                    __syncwarp();
-                    ptx::mbar_arrive_if(my_full + 8 * i, lane == 0);
+                    ptx::tmem_st_32x32b_x32(a_col + i * 64, r);
                 }
-                if (!ok) {
-                    if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | (int)(v & 0x3FFFFF));
-                    break;
-                }
+                ptx::tmem_st_wait();
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                ptx::mbar_arrive_if(my_full, lane == 0);
                 ptx::mbar_arrive_if(raw_empty + 8 * rs, lane == 0);
                 aphase ^= 1;
                 rs += 2;
@@ -283,13 +326,13 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
         // written (high half).  The last one waits for those counts: whoever it waits for holds a ticket, so is running,
         // and the tiles before in their range can only wait for CTAs further down.  It adds the parts in k order whoever it is:
         // repeated calls agree bit for bit.
-        const uint32_t n_pieces = (u1 - 1) / n_chunks - u0 / n_chunks + 1, n_blocks = dq ? 1 : 4;
-        const uint32_t u_last = n_pieces == 1 ? u0 : (u1 - 1) / n_chunks * n_chunks;
+        const uint32_t last_item = um_div(u1 - 1, p.by_chunks), n_pieces = last_item - item0 + 1, n_blocks = dq ? 1 : 4;
+        const uint32_t u_last = n_pieces == 1 ? u0 : last_item * n_chunks;
         const uint32_t row4s = p.rows / 8;                                   // float4s of a block a lane holds, four rows of its column each
         const size_t piece_f4 = (size_t)p.rows * (kUmBN / 4);
         uint32_t piece = dq ? n_pieces - 1 : 0;
         for (uint32_t u = dq ? u_last : u0; ok && u < (dq ? u1 : u_last); ++piece) {
-            const uint32_t item = u / n_chunks, tile_u0 = item * n_chunks, tile_u1 = tile_u0 + n_chunks, u_end = min(u1, tile_u1);
+            const uint32_t item = item0 + piece, tile_u0 = item * n_chunks, tile_u1 = tile_u0 + n_chunks, u_end = min(u1, tile_u1);
             const bool cut = u != tile_u0 || u_end != tile_u1;
             const uint32_t set = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
             u = u_end;
@@ -331,12 +374,15 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
                         if (r4 + j < row4s) __stcg(mine + (r4 + j) * 32, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
                 }
             }
+            ptx::tc_fence_before_sync();
             __syncwarp();
+            const bool all_in = hand_in == (1u << n_blocks) - 1;
+            if (!dq && all_in) ptx::mbar_arrive_if(acc_empty + 8 * set, lane == 0);        // nothing is left to read: the UMMAs may go on
             if (hand_in >> lane & 1) {
                 __threadfence();                       // the block is visible before it is counted
                 atomicAdd(counter, 0x10000u);
             }
-            const uint32_t prob = item / p.n_tiles;
+            const uint32_t prob = um_div(item, p.by_tiles);
             float* const y_out = group.y[prob];
 #pragma unroll 1
             for (uint32_t i = 0; ok && i < n_blocks; ++i) {
@@ -399,7 +445,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
             }
             ptx::tc_fence_before_sync();
             __syncwarp();
-            if (!dq) ptx::mbar_arrive_if(acc_empty + 8 * set, lane == 0);
+            if (!dq && !all_in) ptx::mbar_arrive_if(acc_empty + 8 * set, lane == 0);
         }
     }
 
@@ -491,16 +537,17 @@ int w4a16_umma_plan(t0_runtime* rt, uint32_t M, uint32_t N, uint32_t K, uint32_t
 
 uint32_t w4a16_umma_cut_rows(uint32_t M) { return (M + 15) & ~15u; }
 
-// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows) and outputs of `count` problems of one shape.  `cut_ctas`: tiles cut between so
-// many CTAs, w4a16_umma_plan has made room for their parts; 0: every CTA takes whole tiles.
-template <uint32_t kProblems>
-int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems>& group, bool tiled, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas) {
-    auto kern = tiled ? w4a16_umma_cut_kernel<true, kProblems> : w4a16_umma_cut_kernel<false, kProblems>;
-    static bool attr_set[2][64] = {};
+// `group` holds the maps (activation boxes of w4a16_umma_cut_rows(M) rows), buffers and outputs of `count` problems of one shape.  `cut_ctas`: tiles cut between so
+// many CTAs, w4a16_umma_plan has made room for their parts; 0: every CTA takes whole tiles.  Tile-major weights: `off_scales` and `off_zeros` are the offsets of these.
+template <uint32_t kProblems, bool kTiled>
+int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems, kTiled>& group, uint32_t M, uint32_t N, uint32_t K, uint32_t group_size, uint32_t count, uint32_t cut_ctas,
+                          size_t off_scales, size_t off_zeros) {
+    auto kern = w4a16_umma_cut_kernel<kTiled, kProblems>;
+    static bool attr_set[64] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
-    if (!attr_set[tiled][rt->device]) {
+    if (!attr_set[rt->device]) {
         T0_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUmSmem));
-        attr_set[tiled][rt->device] = true;
+        attr_set[rt->device] = true;
     }
     UmParams p;
     memset(&p, 0, sizeof p);
@@ -516,6 +563,13 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems>& group, bool 
     const uint32_t grid = cut_ctas ? cut_ctas : (uint32_t)std::min<uint64_t>(items, std::min(rt->sm_count, 256));
     p.total = (uint32_t)(items * p.n_chunks);
     p.whole = cut_ctas ? 0 : 1;
+    p.tiles = (uint32_t)items;
+    p.per_group = group_size / kUmBK;
+    p.x_stages = std::min(kUmMaxXStages, kUmXBytes / (2 * p.rows * kUmBK * 2));
+    p.by_grid = um_divisor(grid); p.by_total = um_divisor(p.total); p.by_chunks = um_divisor(p.n_chunks); p.by_tiles = um_divisor(p.n_tiles);
+    p.by_group = um_divisor(p.per_group);
+    if (off_zeros / 16 > 0xFFFFFFFFull) return fail(T0_ERR_UNSUPPORTED, "weights too large");
+    p.off_scales = (uint32_t)(off_scales / 16); p.off_zeros = (uint32_t)(off_zeros / 16);
     if (cut_ctas) {
         p.counters = (uint32_t*)rt->scratch_um.ptr;
         p.pieces = (float*)((uint8_t*)rt->scratch_um.ptr + kUmCounterBytes);
@@ -537,7 +591,9 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems>& group, bool 
     return T0_OK;
 }
 
-template int launch_w4a16_umma_cut<1>(t0_runtime*, const UmGroup<1>&, bool, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t);
-template int launch_w4a16_umma_cut<kUmMaxGroup>(t0_runtime*, const UmGroup<kUmMaxGroup>&, bool, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t);
+template int launch_w4a16_umma_cut<1, false>(t0_runtime*, const UmGroup<1, false>&, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, size_t, size_t);
+template int launch_w4a16_umma_cut<1, true>(t0_runtime*, const UmGroup<1, true>&, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, size_t, size_t);
+template int launch_w4a16_umma_cut<kUmMaxGroup, false>(t0_runtime*, const UmGroup<kUmMaxGroup, false>&, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, size_t, size_t);
+template int launch_w4a16_umma_cut<kUmMaxGroup, true>(t0_runtime*, const UmGroup<kUmMaxGroup, true>&, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, size_t, size_t);
 
 }  // namespace t0
