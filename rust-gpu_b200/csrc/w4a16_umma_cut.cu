@@ -161,54 +161,66 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     };
     // The serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
     if (warp == kUmLoadWarp) {
-        // -------------------------------------------------------------- raw weights, scales and zero points, activations (one box per chunk, rows beyond M are zero)
+        // -------------------------------------------------------------- raw weights, scales and zero points; activations (one box per chunk, rows beyond M are zero)
+        // Weights have six stages, activations three or four.  With three (M > 96) the activations follow the weights at that distance once these are full, so
+        // that weights are not asked for late: 2 x (128 x 11008 x 4096) 25.7 us in step, 24.7 so.  With four the longer chain of this warp costs more: 2 x (64 x
+        // 1024 x 4096) 12.6 and 12.8.
         uint32_t stage = 0, phase = 0, xs = 0, xphase = 0, x_dst = x_ring;
         uint32_t prob = prob0, tile = tile0, at = at0, row = row0, in_row = in_row0;      // at: chunk of the problem, row: its row of scales
+        uint32_t x_prob = prob0, x_tile = tile0;
         const uint32_t rows_a_pair = per_group & 1 ? 2 : 1;
-        for (Pairs w = first_pair(); w.u < u1; next_pair(w)) {
-            if (!ptx::mbar_wait_warp(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) {
-                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w.u & 0xFFFFFF));
-                break;
-            }
-            const uint32_t fb = raw_full + 8 * stage, issue = ptx::elect_one(), dst = raw_ring + stage * kUmRawStage;
-            ptx::fence_proxy_async_smem();           // the stage was read through the generic proxy, the copies write it through the async proxy
-            // a scale row for each chunk, or (group a multiple of two chunks) one for both, in place 0
-            const uint32_t rows = rows_a_pair == 1 ? 1 : w.n, i0 = rows_a_pair == 1 ? 0 : w.i0, step = in_row + 1 == per_group ? 1 : 0;      // to the second chunk's row
-            ptx::mbar_arrive_expect_tx_if(issue, fb, w.n * (8 * kUmBN * 4) + rows * (kUmBN * 2 + kUmBN / 2));
-            if constexpr (kTiled) {
-                // the words of a problem lie one behind the other in the order of its chunks, its scales and zero points likewise
-                const uint8_t* base = group.base[prob];
-                ptx::bulk_load_if(issue, dst + w.i0 * (8 * kUmBN * 4), base + (size_t)at * (8 * kUmBN * 4), w.n * (8 * kUmBN * 4), fb);
-                for (uint32_t j = 0; j < rows; ++j) {
-                    ptx::bulk_load_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride, base + (size_t)p.off_scales * 16 + (size_t)(row + j * step) * (kUmBN * 2), kUmBN * 2, fb);
-                    ptx::bulk_load_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride + kUmBN * 2, base + (size_t)p.off_zeros * 16 + (size_t)(row + j * step) * (kUmBN / 2), kUmBN / 2, fb);
+        Pairs w = first_pair(), wx = w;
+        for (uint32_t j = 0; wx.u < u1; ++j) {
+            const uint32_t issue = ptx::elect_one();
+            if (w.u < u1) {
+                if (!ptx::mbar_wait_warp(raw_empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                    if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w.u & 0xFFFFFF));
+                    break;
                 }
-            } else {
-                const CUtensorMap* const mw = &group.maps[4 * prob];
-                const uint32_t grp = row - um_div(tile * n_chunks, p.by_group);
-                for (uint32_t j = 0; j < w.n; ++j)
-                    ptx::tma_load_2d_if(issue, dst + (w.i0 + j) * (8 * kUmBN * 4), mw, fb, (int32_t)(tile * kUmBN), (int32_t)((w.c + j) * (kUmBK / 8)));
-                for (uint32_t j = 0; j < rows; ++j) {
-                    ptx::tma_load_2d_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)(grp + j * step));
-                    ptx::tma_load_2d_if(issue, dst + kUmScaleOff + (i0 + j) * kUmScaleStride + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)(grp + j * step));
+                const uint32_t fb = raw_full + 8 * stage, dst = raw_ring + stage * kUmRawStage;
+                ptx::fence_proxy_async_smem();       // the stage was read through the generic proxy, the copies write it through the async proxy
+                // a scale row for each chunk, or (group a multiple of two chunks) one for both, in place 0
+                const uint32_t rows = rows_a_pair == 1 ? 1 : w.n, i0 = rows_a_pair == 1 ? 0 : w.i0, step = in_row + 1 == per_group ? 1 : 0;      // to the second chunk's row
+                ptx::mbar_arrive_expect_tx_if(issue, fb, w.n * (8 * kUmBN * 4) + rows * (kUmBN * 2 + kUmBN / 2));
+                if constexpr (kTiled) {
+                    // the words of a problem lie one behind the other in the order of its chunks, its scales and zero points likewise
+                    const uint8_t* base = group.base[prob];
+                    ptx::bulk_load_if(issue, dst + w.i0 * (8 * kUmBN * 4), base + (size_t)at * (8 * kUmBN * 4), w.n * (8 * kUmBN * 4), fb);
+                    for (uint32_t k = 0; k < rows; ++k) {
+                        ptx::bulk_load_if(issue, dst + kUmScaleOff + (i0 + k) * kUmScaleStride, base + (size_t)p.off_scales * 16 + (size_t)(row + k * step) * (kUmBN * 2), kUmBN * 2, fb);
+                        ptx::bulk_load_if(issue, dst + kUmScaleOff + (i0 + k) * kUmScaleStride + kUmBN * 2, base + (size_t)p.off_zeros * 16 + (size_t)(row + k * step) * (kUmBN / 2), kUmBN / 2, fb);
+                    }
+                } else {
+                    const CUtensorMap* const mw = &group.maps[4 * prob];
+                    const uint32_t grp = row - um_div(tile * n_chunks, p.by_group);
+                    for (uint32_t k = 0; k < w.n; ++k)
+                        ptx::tma_load_2d_if(issue, dst + (w.i0 + k) * (8 * kUmBN * 4), mw, fb, (int32_t)(tile * kUmBN), (int32_t)((w.c + k) * (kUmBK / 8)));
+                    for (uint32_t k = 0; k < rows; ++k) {
+                        ptx::tma_load_2d_if(issue, dst + kUmScaleOff + (i0 + k) * kUmScaleStride, mw + 1, fb, (int32_t)(tile * kUmBN), (int32_t)(grp + k * step));
+                        ptx::tma_load_2d_if(issue, dst + kUmScaleOff + (i0 + k) * kUmScaleStride + kUmBN * 2, mw + 2, fb, (int32_t)(tile * (kUmBN / 8)), (int32_t)(grp + k * step));
+                    }
                 }
+                at += w.n;
+                in_row += w.n;
+                while (in_row >= per_group) { in_row -= per_group; ++row; }
+                if (w.c + w.n == n_chunks && ++tile == p.n_tiles) { tile = 0; ++prob; at = row = in_row = 0; }
+                if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
+                next_pair(w);
+                if (x_stages < kUmMaxXStages && j >= x_stages && j < kUmRawStages) continue;
             }
-            if (++stage == kUmRawStages) { stage = 0; phase ^= 1; }
             if (!ptx::mbar_wait_warp(x_empty + 8 * xs, xphase ^ 1, abort_flag, p.wait_limit_ns)) {
-                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(w.u & 0x3FFFFF));
+                if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | 0x400000 | (int)(wx.u & 0x3FFFFF));
                 break;
             }
-            const CUtensorMap* const mx = &group.maps[kMaps * prob + kMaps - 1];
-            ptx::mbar_arrive_expect_tx_if(issue, x_full + 8 * xs, w.n * x_bytes);
-            ptx::tma_load_3d_if(issue, x_dst + w.i0 * x_bytes, mx, x_full + 8 * xs, (int32_t)(w.c * kUmBK), 0, 0);
-            ptx::tma_load_3d_if(issue & (w.n >> 1), x_dst + x_bytes, mx, x_full + 8 * xs, (int32_t)((w.c + 1) * kUmBK), 0, 0);
+            const CUtensorMap* const mx = &group.maps[kMaps * x_prob + kMaps - 1];
+            ptx::mbar_arrive_expect_tx_if(issue, x_full + 8 * xs, wx.n * x_bytes);
+            ptx::tma_load_3d_if(issue, x_dst + wx.i0 * x_bytes, mx, x_full + 8 * xs, (int32_t)(wx.c * kUmBK), 0, 0);
+            ptx::tma_load_3d_if(issue & (wx.n >> 1), x_dst + x_bytes, mx, x_full + 8 * xs, (int32_t)((wx.c + 1) * kUmBK), 0, 0);
             __syncwarp();
-            at += w.n;
-            in_row += w.n;
-            while (in_row >= per_group) { in_row -= per_group; ++row; }
-            if (w.c + w.n == n_chunks && ++tile == p.n_tiles) { tile = 0; ++prob; at = row = in_row = 0; }
+            if (wx.c + wx.n == n_chunks && ++x_tile == p.n_tiles) { x_tile = 0; ++x_prob; }
             x_dst += 2 * x_bytes;
             if (++xs == x_stages) { xs = 0; xphase ^= 1; x_dst = x_ring; }
+            next_pair(wx);
         }
     } else if (warp >= kUmIssueWarp) {
         // -------------------------------------------------------------- UMMA issuers, one per half of the columns: per chunk 4 k-steps of M 128 x N rows x K 16
