@@ -101,6 +101,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
     const uint32_t a_full = raw_empty + 8 * kUmRawStages, a_empty = a_full + 8 * 2 * kUmAStages;     // [128-column half][stage]
     const uint32_t x_full = a_empty + 8 * 2 * kUmAStages, x_empty = x_full + 8 * kUmMaxXStages;
     const uint32_t acc_full = x_empty + 8 * kUmMaxXStages, acc_empty = acc_full + 16;                // [accumulator set]
+    const uint32_t tail_full = acc_empty + 16;               // the range's last piece is complete
     const uint32_t x_bytes = p.rows * kUmBK * 2, x_stages = p.x_stages;
     __shared__ uint32_t tmem_holder;
     __shared__ int s_abort;
@@ -127,6 +128,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
             ptx::mbar_init(acc_full + 8 * s, 2);
             ptx::mbar_init(acc_empty + 8 * s, kUmEpWarps);
         }
+        ptx::mbar_init(tail_full, 2);
         s_abort = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
@@ -250,7 +252,9 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
             ptx::umma_commit_if(issue, x_empty + 8 * xs);
             if (w.c + w.n == n_chunks || w.u + w.n == u1) {
                 // the piece is complete; on to the next one's accumulators, which the epilogue warps must have emptied
-                ptx::umma_commit_if(issue, acc_full + 8 * (acc_sets == 2 ? piece & 1 : 0));
+                // (the last one has a barrier of its own: the dequantising warps come to it without having waited for the pieces before, so that the phase of a
+                // shared one would not tell them which piece is complete)
+                ptx::umma_commit_if(issue, w.u + w.n == u1 ? tail_full : acc_full + 8 * (acc_sets == 2 ? piece & 1 : 0));
                 __syncwarp();
                 ++piece;
                 const uint32_t s = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
@@ -357,7 +361,7 @@ w4a16_umma_cut_kernel(const UmParams p, const __grid_constant__ UmGroup<kProblem
                 counter = p.counters + c_first * kUmDqWarps + (dq ? warp : q + 4 * (lane & 3));
                 if (lane < n_blocks) ticket = atomicAdd(counter, 1u) & 0xFFFFu;        // (its round trip passes under the last UMMAs)
             }
-            if (!ptx::mbar_wait(acc_full + 8 * set, use & 1, abort_flag, p.wait_limit_ns)) {
+            if (!ptx::mbar_wait(dq ? tail_full : acc_full + 8 * set, dq ? 0 : use & 1, abort_flag, p.wait_limit_ns)) {
                 if (lane == 0) atomicCAS(p.status, 0, kStatusEpilogueTimeout | 0xC00000);
                 break;
             }

@@ -646,3 +646,39 @@ def test_streaming_kernel_edges(t0, oracle, rt, shapes):
             assert np.array_equal(again[i], outs[0][i])
     for b in bufs:
         b.free()
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("M,K,N,G,count", [
+    (128, 4096, 14336, 128, 1),                                   # ranges that end one chunk into a tile, and begin at an odd chunk
+    (100, 4096, 2560, 64, 1), (64, 576, 9024, 192, 1),            # scales of every chunk; an odd number of chunks, a group of three
+    (33, 128, 9504, 128, 3), (128, 192, 8192, 64, 4), (17, 320, 9024, 320, 5),      # tiles of one to three pairs, several to a range
+    (48, 1088, 6176, 64, 2), (128, 1024, 11008, 256, 4), (65, 2048, 4128, 512, 7),
+])
+def test_cut_tiles_whatever_a_range_begins_and_ends_with(t0, oracle, rt, M, K, N, G, count, tiled):
+    rng = np.random.default_rng(M * 7 + N)
+    probs, bufs, calls = [], [], []
+    for i in range(count):
+        a = oracle.fill_normal_bf16(M * K, 40 + i)
+        packed, scales, zeros = make_w4(oracle, K, N, G, seed=60 + i)
+        up = [rt.upload(x) for x in (a, packed, scales, zeros)]
+        w = rt.w4_to_tiled(*(b.gpu_addr() for b in up[1:]), K, N, G) if tiled else None
+        y = rt.alloc(M * N * 4 + 4096)
+        y.write(np.full(M * N + 1024, -9999.0, np.float32))
+        calls.append(t0.W4A16Args(up[0].gpu_addr(), (w or up[1]).gpu_addr(), 0 if tiled else up[2].gpu_addr(), 0 if tiled else up[3].gpu_addr(), y.gpu_addr(), M, N, K, G))
+        probs.append((a, packed, scales, zeros, y))
+        bufs += up + [y] + ([w] if tiled else [])
+    outs = []
+    for _ in range(3):
+        (rt.w4a16_gemm_tiled_grouped if tiled else rt.w4a16_gemm_grouped)(calls)
+        rt.synchronize()
+        outs.append([p[4].read(M * N * 4, np.float32).reshape(M, N) for p in probs])
+    rows = sorted(set(rng.integers(0, M, 6).tolist() + [0, M // 2, M - 1]))      # the oracle multiplies one row at a time
+    for i, (a, packed, scales, zeros, y) in enumerate(probs):
+        assert np.all(y.read_bytes(M * N * 4, 4096, np.float32) == -9999.0), "wrote past the output"
+        ref = oracle.w4a16_gemm(np.ascontiguousarray(a.reshape(M, K)[rows]).reshape(-1), packed, scales, zeros, len(rows), N, K, G)
+        assert_close(outs[0][i][rows], ref, K)
+        for again in outs[1:]:
+            assert np.array_equal(again[i], outs[0][i])
+    for b in bufs:
+        b.free()
