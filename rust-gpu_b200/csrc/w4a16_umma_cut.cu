@@ -5,21 +5,25 @@
 // src/t0/quant_kernels.rs:53-171).  y[m,n] = sum_k a[m,k] * w[k,n],  w = RNE_bf16((q - z) * s),  fp32 accumulate.
 //
 // The work is a list of chunks, 256 columns x 64 k, problem by problem, tile by tile, k last; every CTA (one per SM) takes an
-// equal contiguous range of it.  Per chunk:
-//   * one warp fetches the packed words (8 rows x 256 columns), scales and zero points with three TMA boxes each into a ring of
-//     raw stages of two chunks, another warp's the activations (rows up to M rounded to 16; rows beyond M are zero-filled);
-//   * sixteen warps turn the words into bf16 (one LOP3 per nibble pair: 0x4300 | q is the bf16 128+q, minus 128+z, times s -
+// equal contiguous range of it, and its warps go through that in pairs of chunks:
+//   * one warp fetches the packed words, scales and zero points of a pair into a ring of raw stages (tile-major weights: a 16 KiB piece, plain copies; row
+//     layout: TMA boxes) and its activations into another (two boxes; rows up to M rounded to 16; rows beyond M are zero-filled);
+//   * sixteen warps, eight to a pair in turn, turn the words into bf16 (one LOP3 per nibble pair: 0x4300 | q is the bf16 128+q, minus 128+z, times s -
 //     bit-identical to the oracle because (q-z)*s is rounded once) and put them straight into tensor memory (tcgen05.st): the
 //     weights are the 128-row A operand, two halves of 128 columns of y;
-//   * a third serial warp issues 2 x 4 tcgen05.mma (128 x M' x 16, M' = M rounded to 16) with the activations as the B operand in shared
-//     memory.  The accumulator is y transposed: lane = column of y, tensor-memory column = row of y.
+//   * two warps, one per half, issue 8 tcgen05.mma (128 x M' x 16, M' = M rounded to 16) a pair with the activations as the B operand in shared
+//     memory.  The accumulator is y transposed: lane = column of y, tensor-memory column = row of y;
+//   * four warps empty the accumulators of the tiles that end inside the range (two sets where M <= 64, so that the next tile goes on meanwhile); the
+//     last tile is emptied by the sixteen.
 // A tile that lies wholly in one range is stored from tensor memory.  A tile cut by range boundaries is finished by the warps that
-// reach it last: see the epilogue.
+// reach it last: see there.
 //
 // Whole tiles per CTA leave SMs idle where the tiles are few or just over a multiple of them: two problems of N = 11008 are 86 tiles on 148
 // SMs.  A launch takes its tiles whole or cut, or leaves a single problem to the clusters of w4a16_umma.cu: `w4a16_umma_plan` weighs them.
-// What bounds it is the dequantising warps' instructions and the waits around them (0.4 us a chunk, 0.5 at M = 128; the UMMAs of a chunk take
-// 0.27 there), and per launch with cut tiles 2 to 10 us for handing in and adding their parts.
+// What bounds it is the dequantisation's instructions (0.28 us a chunk up to M = 64; two pipes that take one per two cycles are half busy, the schedulers two
+// thirds) and at M = 128 the UMMAs beside them (0.34; 0.27 of tensor work), and per launch with cut tiles 3 to 7 us for handing in and adding their parts.
+// Two problems of N = 11008, K = 4096 at M = 32 / 128: 24.4 / 29.1 us with one issuing warp, one loading by boxes and the sixteen emptying every
+// tile; 20.9 / 26.6 with two issuing warps, predicated; 18.8 / 26.3 with warps that empty the accumulators; 18.4 / 24.7 in pairs.
 #include "w4a16_common.cuh"
 
 using namespace t0;
@@ -28,12 +32,8 @@ using namespace t0::w4;
 namespace {
 
 constexpr uint32_t kUmDqWarps = 16;
-// + the warps that fetch weights and activations and the one that issues the UMMAs.  Each works through a serial chain of instructions per
-// chunk, at several cycles an instruction, so the chains are kept short (running counters, no divisions, descriptors stepped by addition,
-// one barrier for both operands of a chunk) and apart.  The issuer's chain took 1190 cycles a chunk as one diverged lane with a barrier per
-// operand, which the sixteen dequantising warps spent waiting: two problems of M = 128, N = 11008, K = 4096 39.7 us, 33.3 with the warp
-// converged, 31.7 with one barrier
-// (device time of queued launches, as below; the same call takes 34 us by the host's clock in blocks of calls).
+// + the warps that empty accumulators, issue and load.  The serial ones share a scheduler with dequantising warps and work through a chain of instructions per
+// pair, so the chains are kept short: predicated instructions on uniform values, running addresses, no divisions.
 constexpr uint32_t kUmEpWarp0 = kUmDqWarps, kUmEpWarps = 4;  // empty the accumulators of all but the last tile of a range, one per tensor-memory lane quadrant
 constexpr uint32_t kUmIssueWarp = kUmEpWarp0 + kUmEpWarps, kUmLoadWarp = kUmIssueWarp + 2;     // (two issuing warps)
 constexpr uint32_t kUmThreads = (kUmLoadWarp + 1) * 32;     // (a warp more, even an idle one, adds 0.3 us to a launch)
@@ -512,12 +512,16 @@ static uint32_t cut_grid(uint32_t sms, uint64_t items, uint32_t n_chunks) {
     return grid;
 }
 
-// How to share out the tiles of `count` problems: the fastest form, by times in microseconds fitted to M = 17 ... 128, 4 ... 516 tiles and
-// K = 1024 ... 8192.  A chunk takes 0.42 us at small M and 0.52 at M = 128 in either form of this kernel; handing in and adding parts adds 2 to 10 us
-// with M.  Measured, whole tiles / cut: 2 x (128 x 11008 x 4096) 36.6 / 34.1, 12 of them 142 / 140, 4 x (64 x 1024 x 2048) 18.0 / 13.1; one problem
-// as clusters / cut: 128 x 11008 x 4096 21.8 / 22.7, 32 x 11008 x 4096 21.3 / 15.6, 100 x 1024 x 2048 14.1 / 16.5, 20 x 14336 x 2048 19.6 / 13.1.
+// How to share out the tiles of `count` problems: the fastest form, by times in microseconds fitted to 402 launches of M = 17 ... 128, 4 ... 224 tiles and
+// K = 768 ... 8192, each timed in both forms (the choice is within 0.3 % of the better one in the mean; the fit of before the last changes to this kernel was 2.6 %
+// off).  A chunk takes 0.28 us up to M = 64 and 0.34 (cut) or 0.32 (whole) at M = 128; handing in and adding parts adds 3 to 7 us with M.  Measured, whole tiles /
+// cut: 4 x (17 x 14336 x 2048) 21.5 / 22.4, 4 x (64 x 4096 x 2048) 13.5 / 12.5; one problem as clusters / cut: 17 x 16384 x 8192 46.8 / 24.3, 100 x 14336 x 1024
+// 13.4 / 15.5, 128 x 16384 x 2048 17.8 / 16.2.  (4 x (17 x 14336 x 2048): cut all the same, for the shorter sums.)
 // `cluster_split`: into how many parts the cluster form would cut K (1: one problem that has tiles enough; 0: a list); `cluster_rounds`: in how many rounds
 // its clusters fit on the GPU (the GPCs hold 33 of four CTAs, not 37: 128 x 9472 x 4096 36.4 us in two rounds of clusters, 20.7 cut).
+//
+// Clusters are left only for a gain of more than 8 % (they share no memory between launches, so that a recorded launch gives the same bits), whole tiles for
+// none at all, nor for a loss of up to 3 % (their sums are the longest).
 //
 // The times choose only among forms whose sums are no longer than the library has made them for the problem, since the tensor cores' error grows with
 // the length of an accumulation.  One problem: its pieces are no longer than the parts of the clusters (K = 768: four of 3 chunks, where the grid
@@ -535,10 +539,11 @@ int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t c
     const double per_cta = (double)items * n_chunks / grid;
     const double rounds = (double)((items + sms - 1) / sms);
     if (cluster_split == 0 && per_cta * 0.67 + 14.4 <= 0.97 * (rounds * n_chunks * 0.63 + 4.0)) return kUmCut;
-    const double chunk = 0.42 + 0.0008 * M;
-    const double cut = per_cta * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0);
-    const double without = other == kUmClusters ? cluster_rounds * (ceil_div(n_chunks, cluster_split) * 0.495 + 8.2) + 2.0 : rounds * n_chunks * chunk + 4.2;
-    return cut > 0.97 * without ? other : kUmCut;
+    const double wide = M > 64 ? M - 64.0 : 0.0;
+    const double cut = per_cta * (0.288 - 0.00037 * M + 0.00176 * wide) + 6.0 + 0.049 * M + (grid >= sms ? 1.35 : 0.0);
+    const double without = other == kUmClusters ? cluster_rounds * (ceil_div(n_chunks, cluster_split) * 0.497 + 5.1 + 0.0018 * M) + 5.1
+                                                : rounds * n_chunks * (0.285 - 0.0001 * M + 0.0008 * wide) + 3.3 + 0.021 * M;
+    return cut > (other == kUmClusters ? 0.92 : 1.03) * without ? other : kUmCut;
 }
 
 // The form of a launch.  Cut tiles need room for their parts, and run only in launches of the runtime's own stream, whose launches run one after the
