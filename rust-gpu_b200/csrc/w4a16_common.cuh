@@ -100,6 +100,18 @@ __device__ __forceinline__ uint32_t um_ld_acquire(const uint32_t* p) {
     return v;
 }
 
+// Division by a number the host knows: the quotient by a product with floor((2^32 - 1) / d), at most two short.  Every CTA divides a few times before its first
+// load, on the way of the whole launch, and a division takes 150 cycles.
+struct UmDiv {
+    uint32_t d, m;
+};
+inline UmDiv um_divisor(uint32_t d) { return {d, 0xFFFFFFFFu / d}; }
+__device__ __forceinline__ uint32_t um_div(uint32_t a, const UmDiv& by) {
+    uint32_t q = __umulhi(a, by.m), r = a - q * by.d;
+    if (r >= by.d) { ++q; r -= by.d; }
+    return r >= by.d ? q + 1 : q;
+}
+
 // The eight codes of a packed word as bf16x2 pairs in k order, (0,1) (2,3) (4,5) (6,7): (code | 0x4300) is the bf16 128 + code, so minus (128 + z),
 // times s, is (q - z) * s rounded once.  zz = (128 + z) and ss = s, both halves alike.
 __device__ __forceinline__ void um_dequant_word(uint32_t wd, uint32_t mask, uint32_t magic, uint32_t zz, uint32_t ss, bool tiled, uint32_t (&o)[4]) {

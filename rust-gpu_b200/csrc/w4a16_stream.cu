@@ -21,7 +21,7 @@
 //     they were on mma.sync (two warps with two accumulators each);
 //   * four warps empty the accumulators: a band that lies wholly inside a range is stored directly; a band shared by several CTAs is finished by
 //     whichever CTA arrives last (per-band arrival counter, partial pieces in scratch, added in k order: deterministic, repeated calls agree bit
-//     for bit); no CTA ever waits for another.  A spare warp counts a range's leading partial band in meanwhile.
+//     for bit); no CTA ever waits for another.  The loading warp counts a range's leading partial band in meanwhile.
 // What bounds the loop is the pipes of the dequantisation (15 instructions per packed word, on two pipes that take one per two cycles; a step is 512 cycles
 // of theirs at the least and takes about 940), then HBM (710).  Everything else was taken off the dequantising warps' schedulers: with mma.sync the
 // products and the activation fragments were theirs as well.  Two problems of M = 1, N = 11008, K = 4096: 18.6 us with mma.sync, 17.2 so; four of M = 16,
@@ -37,11 +37,10 @@ using namespace t0::w4;
 
 namespace {
 
-constexpr int kStDqWarps = 16;                        // dequantising warps: warp w owns columns 32 (w % 8) .. + 31 of the band in every second step, w / 8 saying which
+constexpr int kStDqWarps = 16;                        // dequantising warps: eight to a step in turn, each with 32 columns of the band
 constexpr int kStEpWarps = 4;                         // empty the accumulators (one per tensor-memory lane quadrant)
 constexpr int kStProducerWarp = 0, kStIssueWarp0 = 1; // two warps issue the UMMAs, one per 128-column half of the band
-constexpr int kStHeadWarp = 3;                        // counts in the first piece of a range
-constexpr int kStEpWarp0 = 4, kStDqWarp0 = 8;
+constexpr int kStEpWarp0 = 3, kStDqWarp0 = kStEpWarp0 + kStEpWarps;      // (a warp more, even an idle one, adds 0.3 us to a launch)
 constexpr int kStThreads = (kStDqWarp0 + kStDqWarps) * 32;
 constexpr int kStMRows = 16;                          // rows of the activations the UMMAs take
 constexpr int kStSzOff = kWeightBytes;                // in a stage: the tile, scales and zero points, activations
@@ -67,6 +66,7 @@ struct StProblem {
     uint32_t ksteps, groups, units_per_group, n_bands;
     uint32_t unit_begin;       // first unit of this problem in the launch's list
     uint32_t band_begin;       // first arrival counter of this problem
+    UmDiv by_ksteps, by_group; // ksteps, units_per_group
 };
 
 template <uint32_t kProblems>
@@ -81,6 +81,7 @@ struct StParams {
     uint32_t n_problems, total_units;
     uint32_t per_cta, rest;    // total_units = grid * per_cta + rest
     float cta_per_unit;        // grid / total_units
+    UmDiv by_grid;
 };
 constexpr uint32_t kStMaxProblems = 32;               // problems per launch (the table travels as a kernel parameter) ...
 constexpr uint32_t kStFewProblems = 4;                // ... or as a parameter of a seventh of the size
@@ -88,7 +89,7 @@ constexpr uint32_t kStFewProblems = 4;                // ... or as a parameter o
 // First unit of a CTA's range, floor(cta * total / grid), and the CTA whose range holds a unit: without the 64-bit divisions, which take hundreds of cycles
 // where a band is finished.
 template <class Params>
-__device__ __forceinline__ uint32_t st_begin(const Params& P, uint32_t cta) { return cta * P.per_cta + cta * P.rest / gridDim.x; }
+__device__ __forceinline__ uint32_t st_begin(const Params& P, uint32_t cta) { return cta * P.per_cta + um_div(cta * P.rest, P.by_grid); }
 template <class Params>
 __device__ __forceinline__ uint32_t st_owner(const Params& P, uint32_t unit) {
     uint32_t c = (uint32_t)((float)unit * P.cta_per_unit);     // off by a CTA at most
@@ -104,9 +105,9 @@ __device__ __forceinline__ Cursor locate(const Params& P, uint32_t unit) {
     Cursor c;
     c.p = 0;
     while (c.p + 1 < P.n_problems && P.prob[c.p + 1].unit_begin <= unit) ++c.p;
-    const uint32_t r = unit - P.prob[c.p].unit_begin, ks = P.prob[c.p].ksteps;
-    c.band = r / ks;
-    c.ks = r - c.band * ks;
+    const uint32_t r = unit - P.prob[c.p].unit_begin;
+    c.band = um_div(r, P.prob[c.p].by_ksteps);
+    c.ks = r - c.band * P.prob[c.p].ksteps;
     return c;
 }
 
@@ -283,45 +284,56 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
     ptx::tc_fence_after_sync();
     constexpr uint32_t tmem_base = 0;    // all columns are allocated: tensor-memory addresses are constants
     ptx::grid_launch_dependents();
-    const Cursor c0 = locate(P, U0);
-    Cursor c = c0;
+    Cursor c = locate(P, U0);
     if (warp == kStProducerWarp && lane == 0) ptx::tma_prefetch_desc(&P.x[c.p]);
     ptx::grid_dependency_wait();      // global memory is read and written only after the previous grid in the stream is done
     if (tid == 0) stamp(0);
-    // the last piece of the range (the steps of one band this CTA owns) goes on in the next CTA, or began in the one before
-    const Cursor c_end = locate(P, U1 - 1);
-    const uint32_t end_first = P.prob[c_end.p].unit_begin + c_end.band * P.prob[c_end.p].ksteps;
-    const bool tail_cut = end_first < U0 || end_first + P.prob[c_end.p].ksteps > U1;
-    // A head piece: the range starts inside a band and goes on into the next one.  Counting it in (fence, atomic round trip) is a spare warp's job, so
-    // that the epilogue warps are there for the last piece, which may come soon.
-    const uint32_t head_first = U0 - c0.ks, head_ksteps = P.prob[c0.p].ksteps;
-    const bool has_head = c0.ks != 0 && head_first + head_ksteps < U1;
+    // What is cut at the ends of the range.  Worked out where it is needed, after a warp's loop (the empty statement keeps it there: it would take registers
+    // that the loops have none of).
+    struct Ends {
+        Cursor first, last;
+        uint32_t head_first, head_ksteps;   // first unit and steps of the first band
+        bool has_head;           // A head piece: the range starts inside a band and goes on into the next one.  Counting it in (fence, atomic round trip) is the loading
+                                 // warp's job, so that the epilogue warps are there for the last piece, which may come soon.
+        bool tail_cut;           // the last piece (the steps of one band this CTA owns) goes on in the next CTA, or began in the one before
+    };
+    auto range_ends = [&]() {
+        uint32_t lo = U0, hi = U1;
+        asm volatile("" : "+r"(lo), "+r"(hi));
+        Ends e;
+        e.first = locate(P, lo);
+        e.last = locate(P, hi - 1);
+        e.head_first = lo - e.first.ks;
+        e.head_ksteps = P.prob[e.first.p].ksteps;
+        e.has_head = e.first.ks != 0 && e.head_first + e.head_ksteps < hi;
+        const uint32_t end_first = P.prob[e.last.p].unit_begin + e.last.band * P.prob[e.last.p].ksteps;
+        e.tail_cut = end_first < lo || end_first + P.prob[e.last.p].ksteps > hi;
+        return e;
+    };
     // The serial roles walk with their whole warp and let one elected lane issue: see ptx::mbar_wait_warp.
-    if (warp == kStHeadWarp) {
-        if (lane == 0 && has_head) {
-            int last = 0;
-            if (ptx::mbar_wait(head_written, 0, abort_flag, P.wait_limit_ns)) {
-                const StShare h = st_share(P, head_first, head_ksteps);
-                __threadfence();                       // the piece is visible before this CTA is counted
-                last = atomicAdd(&P.counters[P.prob[c0.p].band_begin + c0.band], 1) == (int)(h.last - h.first);
-                if (last) __threadfence();
-            } else {
-                atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xD00000);
-            }
-            s_head_last = last;
-            ptx::mbar_arrive(head_counted);
-        }
-    } else if (warp == kStProducerWarp) {
+    if (warp == kStProducerWarp) {
         // (A problem's tiles lie one behind the other in the order of its units, its rows of scales and zero points likewise: running addresses.  The chain of
         // this warp is kept short: with a division per step it took 800 cycles a step from the four dequantising warps it shares a scheduler with.)
+        // It counts the head piece in as soon as that is written: the ring holds several steps, which the fence and the atomic's round trip do not take.
+        const uint32_t head_left = P.prob[c.p].ksteps - c.ks, first_p = c.p, first_band = c.band;
+        bool head_pending = c.ks != 0 && head_left < U1 - U0;
+        auto count_head = [&]() {
+            if (lane == 0) {
+                const StShare h = st_share(P, U0 + head_left - P.prob[first_p].ksteps, P.prob[first_p].ksteps);
+                __threadfence();                       // the piece is visible before this CTA is counted
+                const int last = atomicAdd(&P.counters[P.prob[first_p].band_begin + first_band], 1) == (int)(h.last - h.first);
+                if (last) __threadfence();
+                s_head_last = last;
+            }
+        };
         uint32_t stage = 0, phase = 0;
         for (uint32_t u = U0; u < U1; ++c.p) {
             const StProblem& pr = P.prob[c.p];
-            const uint32_t at = u - pr.unit_begin, row = at / pr.units_per_group, u_stop = min(U1, pr.unit_begin + pr.ksteps * pr.n_bands);
+            const uint32_t at = u - pr.unit_begin, row = um_div(at, pr.by_group), u_stop = min(U1, pr.unit_begin + pr.ksteps * pr.n_bands);
             const uint8_t* tile = pr.tiles + (size_t)at * kWeightBytes;
             const uint8_t* scales = pr.scales_t + (size_t)row * kScaleBytes;
             const uint8_t* zeros = pr.zeros_t + (size_t)row * kZeroBytes;
-            uint32_t in_row = at - row * pr.units_per_group, k = (at % pr.ksteps) * kUnitK;
+            uint32_t in_row = at - row * pr.units_per_group, k = (at - um_div(at, pr.by_ksteps) * pr.ksteps) * kUnitK;
             bool ok = true;
             for (; u < u_stop; ++u) {
                 ok = ptx::mbar_wait_warp(empty_bar + stage * 8, phase ^ 1, abort_flag, P.wait_limit_ns);
@@ -337,6 +349,12 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
                     ptx::tma_load_3d(dst + kStXOff + kStXChunk, &P.x[c.p], fb, (int32_t)k + 64, 0, 0);
                 }
                 __syncwarp();
+                if (head_pending && ptx::mbar_test_wait(head_written, 0)) {
+                    count_head();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(head_counted);
+                    head_pending = false;
+                }
                 if (++stage == kStStages) { stage = 0; phase ^= 1; }
                 tile += kWeightBytes;
                 if (++in_row == pr.units_per_group) { in_row = 0; scales += kScaleBytes; zeros += kZeroBytes; }
@@ -348,7 +366,12 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
                 break;
             }
         }
-    } else if (warp < kStHeadWarp) {
+        if (head_pending) {
+            if (ptx::mbar_wait(head_written, 0, abort_flag, P.wait_limit_ns)) count_head(); else if (lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xD00000);
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(head_counted);       // (counted or not: nobody waits for what does not come)
+        }
+    } else if (warp < kStEpWarp0) {
         // -------------------------------------------------------------- UMMA issuers: per 64 k four k steps of M 128 x N 16 x K 16
         constexpr uint32_t idesc = ptx::make_idesc_bf16_f32(128, kStMRows, 0u);
         const uint32_t t = warp - kStIssueWarp0;
@@ -394,7 +417,8 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
         }
     } else if (warp >= kStDqWarp0) {
         // -------------------------------------------------------------- sixteen warps: dequantise into tensor memory
-        const uint32_t set = (warp - kStDqWarp0) >> 3, pair = warp & 7, g = lane >> 2;      // every second step; columns 32 pair .. + 31; a lane has columns g + 8 i of these
+        const uint32_t set = (warp - kStDqWarp0) >> 3, g = lane >> 2;              // every second step; a lane has columns g + 8 i of the warp's 32
+        const uint32_t pair = ((warp - kStDqWarp0) & 4) | (warp & 3);            // columns 32 pair .. + 31, those of its tensor-memory lane quadrant
         const uint32_t a_lane = (((pair & 3) * 32) << 16) + kStAccCols + (pair >> 2) * 64;
         const uint32_t my_full = a_full + (pair >> 2) * kStAStages * 8, my_empty = a_empty + (pair >> 2) * kStAStages * 8;
         uint32_t mask, magic;
@@ -467,21 +491,22 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
         // Finish the bands of the last and the first piece, where this CTA turned out to be the last to contribute to them.  (The last step is done with by
         // then, so the ring is free.)
         const uint32_t ft = tid - kStDqWarp0 * 32;
-        if (tail_cut) {
-            const StFinish f = st_finish(P, c_end.p, c_end.band, ft);
+        const Ends e = range_ends();
+        if (e.tail_cut) {
+            const StFinish f = st_finish(P, e.last.p, e.last.band, ft);
             st_tail_sync();
             if (s_last) st_reduce_band(P, f, ft, ring);
         }
-        if (has_head) {
-            const StFinish f = st_finish(P, c0.p, c0.band, ft);
+        if (e.has_head) {
+            const StFinish f = st_finish(P, e.first.p, e.first.band, ft);
             if (ft == 0) s_head_go = ptx::mbar_wait(head_counted, 0, abort_flag, P.wait_limit_ns) && s_head_last;
-            if (tail_cut) st_finishers_sync();
+            if (e.tail_cut) st_finishers_sync();
             else st_tail_sync();
             if (s_head_go) st_reduce_band(P, f, ft, ring);
         }
     } else {
         // -------------------------------------------------------------- four warps: accumulators to y, or to a piece
-        const uint32_t quad = warp - kStEpWarp0, et = tid - kStEpWarp0 * 32;
+        const uint32_t quad = warp & 3, et = tid - kStEpWarp0 * 32;
         bool ok = true;
         uint32_t piece = 0;
         for (uint32_t u = U0; u < U1; ++piece) {
@@ -571,7 +596,8 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
             c.ks = 0;
             if (++c.band == pr.n_bands) { c.band = 0; ++c.p; }
         }
-        if (tail_cut || has_head) st_tail_sync();
+        const Ends e = range_ends();
+        if (e.tail_cut || e.has_head) st_tail_sync();
     }
 
     __syncwarp();
@@ -681,6 +707,7 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
         q.M = a.m; q.N = a.n;
         q.ksteps = L.ksteps; q.groups = L.groups; q.units_per_group = a.group / kUnitK; q.n_bands = L.bands;
         q.unit_begin = (uint32_t)total; q.band_begin = (uint32_t)bands;
+        q.by_ksteps = um_divisor(q.ksteps); q.by_group = um_divisor(q.units_per_group);
         total += (uint64_t)L.bands * L.ksteps;
         bands += L.bands;
     }
@@ -699,7 +726,7 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
     const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
     P.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
     P.n_problems = (uint32_t)count; P.total_units = (uint32_t)total;
-    P.per_cta = (uint32_t)total / grid; P.rest = (uint32_t)total % grid; P.cta_per_unit = (float)grid / (float)total;
+    P.per_cta = (uint32_t)total / grid; P.rest = (uint32_t)total % grid; P.cta_per_unit = (float)grid / (float)total; P.by_grid = um_divisor(grid);
     static bool attr_set[64] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");
     if (!attr_set[rt->device]) {

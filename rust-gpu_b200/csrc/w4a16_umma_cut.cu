@@ -51,18 +51,6 @@ constexpr uint32_t kUmSmem = kUmRawStages * kUmRawStage + kUmXBytes + 512 + 1024
 constexpr uint32_t kUmMinChunks = 4;                        // a CTA's range is at least this long where sums may be: below it the finish costs more than the range
 constexpr size_t kUmCounterBytes = 16 * 1024;               // one word per CTA and dequantisation warp (up to 256 CTAs)
 
-// Division by a number the host knows: the quotient by a product with floor((2^32 - 1) / d), at most two short.  Every CTA divides a few times before its first
-// load, on the way of the whole launch, and a division takes 150 cycles.
-struct UmDiv {
-    uint32_t d, m;
-};
-inline UmDiv um_divisor(uint32_t d) { return {d, 0xFFFFFFFFu / d}; }
-__device__ __forceinline__ uint32_t um_div(uint32_t a, const UmDiv& by) {
-    uint32_t q = __umulhi(a, by.m), r = a - q * by.d;
-    if (r >= by.d) { ++q; r -= by.d; }
-    return r >= by.d ? q + 1 : q;
-}
-
 struct UmParams {
     int* status;
     uint32_t* counters;      // [grid][16]: arrivals at the tile that CTA begins and does not complete; zero between launches
