@@ -163,7 +163,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint32_t* tmem_holder = (uint32_t*)(bars + 2 * kStages + 5);
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
 
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);     // (the shuffle tells the compiler that a role is the whole warp's)
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t work_per_problem = p.tiles_m * p.tiles_n * p.split_k;
     uint32_t total_work = work_per_problem;                 // a grouped launch walks the tiles of all its problems, problem-major
@@ -194,7 +194,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     __syncthreads();
     if constexpr (kCluster) ptx::cluster_sync_all();          // every CTA's barriers exist before anyone signals across the cluster
     ptx::tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_holder;
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *tmem_holder, 0);
+    const uint32_t a_smem = ptx::smem_u32(a_tiles), b_smem = ptx::smem_u32(b_tiles), full = ptx::smem_u32(full_bar), empty = ptx::smem_u32(empty_bar);
     // everything above touched only shared and tensor memory; global memory comes after the previous grid is done
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
@@ -215,35 +216,30 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 if constexpr (kGrouped) { ma = &group.maps[3 * prob]; mb = &group.maps[3 * prob + 1]; }
                 const KRange kr = k_range<kCluster>(wi.split, p);
                 for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
-                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag, p.wait_limit_ns)) {
+                    if (!ptx::mbar_wait_warp(empty + 8 * stage, phase ^ 1, abort_flag, p.wait_limit_ns)) {
                         if (lane == 0) atomicCAS(p.status, 0, kStatusProducerTimeout | (int)(w & 0xFFFFFF));
                         ok = false;
                         break;
                     }
-                    const uint32_t fb = ptx::smem_u32(&full_bar[stage]);
+                    const uint32_t fb = full + 8 * stage, a_dst = a_smem + stage * kAStageBytes, b_dst = b_smem + stage * kBStageBytes;
                     // self-test of the failure path: this stage is never filled, so the issuer's bounded wait must run out
                     if (p.drop_load && blockIdx.x == 0 && w == 0 && kb == 0) { if (++stage == kStages) { stage = 0; phase ^= 1; } continue; }
-                    if (ptx::elect_one()) {
-                        ptx::mbar_arrive_expect_tx(fb, kStageBytes);
-                        if constexpr (!A_MN) {
-                            ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes), ma, fb,
-                                             (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)kr.z);
-                        } else {
+                    const uint32_t issue = ptx::elect_one();
+                    ptx::mbar_arrive_expect_tx_if(issue, fb, kStageBytes);
+                    if constexpr (!A_MN) {
+                        ptx::tma_load_3d_if(issue, a_dst, ma, fb, (int32_t)(kb * BK), (int32_t)(wi.m_blk * BM), (int32_t)kr.z);
+                    } else {
 #pragma unroll
-                            for (uint32_t j = 0; j < BM / 64; ++j)
-                                ptx::tma_load_3d(ptx::smem_u32(a_tiles + stage * kAStageBytes + j * (BK * 128)), ma, fb,
-                                                 (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
-                        }
-                        if constexpr (!B_MN) {
-                            ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes), mb, fb,
-                                             (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)kr.z);
-                        } else {
-                            // B[K,N]: one 64(k) x 64(n) box per 64 columns; each box is an [k][128 B] block
+                        for (uint32_t j = 0; j < BM / 64; ++j)
+                            ptx::tma_load_3d_if(issue, a_dst + j * (BK * 128), ma, fb, (int32_t)(wi.m_blk * BM + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
+                    }
+                    if constexpr (!B_MN) {
+                        ptx::tma_load_3d_if(issue, b_dst, mb, fb, (int32_t)(kb * BK), (int32_t)(wi.n_blk * BN), (int32_t)kr.z);
+                    } else {
+                        // B[K,N]: one 64(k) x 64(n) box per 64 columns; each box is an [k][128 B] block
 #pragma unroll
-                            for (uint32_t j = 0; j < BN / 64; ++j)
-                                ptx::tma_load_3d(ptx::smem_u32(b_tiles + stage * kBStageBytes + j * (BK * 128)), mb, fb,
-                                                 (int32_t)(wi.n_blk * BN + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
-                        }
+                        for (uint32_t j = 0; j < BN / 64; ++j)
+                            ptx::tma_load_3d_if(issue, b_dst + j * (BK * 128), mb, fb, (int32_t)(wi.n_blk * BN + j * 64), (int32_t)(kb * BK), (int32_t)kr.z);
                     }
                     __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -254,6 +250,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         // ------------------------------------------------------------ UMMA issuer: the whole warp walks, one lane issues
         {
             uint32_t stage = 0, phase = 0, iter = 0;
+            const uint32_t a_desc = ptx::smem_desc_lo(a_smem, A_MN ? BK * 128 : 16), b_desc = ptx::smem_desc_lo(b_smem, B_MN ? BK * 128 : 16);
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < total_work; w += gridDim.x, ++iter) {
                 const uint32_t buf = iter & 1, acc_phase = (iter >> 1) & 1;
@@ -266,28 +263,20 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const uint32_t kb_mid = k_mid<kAccs>(kr, p);
                 uint32_t tmem_d = tmem_base + buf * BN * kAccs;
                 for (uint32_t kb = kr.first; kb < kr.end; ++kb) {
-                    if (!ptx::mbar_wait_warp(ptx::smem_u32(&full_bar[stage]), phase, abort_flag, p.wait_limit_ns)) {
+                    if (!ptx::mbar_wait_warp(full + 8 * stage, phase, abort_flag, p.wait_limit_ns)) {
                         if (lane == 0) atomicCAS(p.status, 0, kStatusMmaTimeout | 0x800000 | (int)(w & 0x7FFFFF));
                         ok = false;
                         break;
                     }
                     ptx::tc_fence_after_sync();
                     if (kb == kb_mid) tmem_d += BN;
-                    if (ptx::elect_one()) {
-                        const uint32_t a_addr = ptx::smem_u32(a_tiles + stage * kAStageBytes);
-                        const uint32_t b_addr = ptx::smem_u32(b_tiles + stage * kBStageBytes);
+                    // K-major, 128B swizzle: 8-row groups 1024 B apart; a 16-element K step is 32 B.  MN-major: 64-column atoms 8 KiB apart, 8-row k
+                    // groups 1024 B apart; a K step is two groups.
+                    const uint32_t issue = ptx::elect_one(), a = a_desc + stage * (kAStageBytes / 16), b = b_desc + stage * (kBStageBytes / 16);
+                    ptx::umma_bf16_ss_if(issue, tmem_d, a, b, kIdesc, kb != kr.first && kb != kb_mid);
 #pragma unroll
-                        for (uint32_t k4 = 0; k4 < BK / 16; ++k4) {
-                            // K-major, 128B swizzle: 8-row groups 1024 B apart; a 16-element K step is 32 B
-                            const uint64_t da = A_MN ? ptx::make_smem_desc(a_addr + k4 * 2048, BK * 128, 1024)
-                                                     : ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024);
-                            // N-major B: 64-column atoms 8 KiB apart, 8-row k groups 1024 B apart; a K step is two groups
-                            const uint64_t db = B_MN ? ptx::make_smem_desc(b_addr + k4 * 2048, BK * 128, 1024)
-                                                     : ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024);
-                            ptx::umma_bf16_ss(tmem_d, da, db, kIdesc, ((kb != kr.first && kb != kb_mid) || k4 != 0) ? 1u : 0u);
-                        }
-                        ptx::umma_commit(ptx::smem_u32(&empty_bar[stage]));
-                    }
+                    for (uint32_t k4 = 1; k4 < BK / 16; ++k4) ptx::umma_bf16_ss_if(issue, tmem_d, a + k4 * (A_MN ? 128 : 2), b + k4 * (B_MN ? 128 : 2), kIdesc, 1u);
+                    ptx::umma_commit_if(issue, empty + 8 * stage);
                     __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1; }
                 }

@@ -329,6 +329,23 @@ __device__ __forceinline__ void umma_bf16_ts_if(uint32_t issue, uint32_t tmem_d,
         ::"r"(tmem_d), "r"(tmem_a), "r"(desc_b_lo | (1u << 16)), "r"(idesc), "r"(accumulate), "n"((1024 >> 4) | (1 << 14) | (2 << 29)), "r"(issue)
         : "memory");
 }
+// Low word of a descriptor of make_smem_desc with groups of eight rows 1024 bytes apart: start address and leading offset, in 16-byte units.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16); }
+// D[tmem] (+)= A[smem] * B[smem], issued where `issue` holds, both descriptors given by their low words.
+__device__ __forceinline__ void umma_bf16_ss_if(uint32_t issue, uint32_t tmem_d, uint32_t desc_a_lo, uint32_t desc_b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .b64 a, b;\n\t"
+        "mov.b64 a, {%1, %5};\n\t"
+        "mov.b64 b, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+        "}"
+        ::"r"(tmem_d), "r"(desc_a_lo), "r"(desc_b_lo), "r"(idesc), "r"(accumulate), "n"((1024 >> 4) | (1 << 14) | (2 << 29)), "r"(issue)
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit_if(uint32_t issue, uint32_t bar) {
     asm volatile(
         "{\n\t"
