@@ -124,24 +124,6 @@ __device__ __forceinline__ bool elect_one() {
     return is != 0;
 }
 
-// The same wait for a role that runs well ahead of the roles it waits on (a producer that fills a deep ring, a helper
-// that prepares later steps): between polls the thread sleeps, so that its polling takes no issue slots from the warps
-// that do the arithmetic.  In the W4A16 kernel five such lanes polling back to back executed a quarter of all instructions.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns, uint32_t sleep_ns) {
-    if (mbar_try_wait(bar, parity)) return true;
-    uint64_t t_start = 0;
-    for (uint32_t spin = 1;; ++spin) {
-        __nanosleep(sleep_ns);
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 0x1F) == 0) {
-            if (*abort_flag) return false;
-            uint64_t now = globaltimer_ns();
-            if (t_start == 0) t_start = now;
-            else if (now - t_start > limit_ns) { *abort_flag = 1; return false; }
-        }
-    }
-}
-
 // ------------------------------------------------------------------ programmatic dependent launch
 // With the launch attribute set, the next grid in the stream may start its CTAs (and run its prologue)
 // while this grid drains; `grid_dependency_wait` then blocks until the previous grid has completed and
@@ -253,22 +235,9 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-                   "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                  : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
