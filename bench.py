@@ -464,7 +464,7 @@ def run_aux_workload(args, name, rt=None, brief=False):
         ok = err <= tol
         tf = 2.0 * M * N * K / sec / 1e12
         line.update({"metric": "matmul_f32_tflops", "value": tf, "unit": "TFLOP/s", "ms_per_step": sec * 1e3, "dtype": "f32 in, bf16 multiply, f32 accumulate and out",
-                     "config": {"workload": name, "m": M, "n": N, "k": K, "kernel": "cvt_operands_kernel + gemm (B[K,N] layout)",
+                     "config": {"workload": name, "m": M, "n": N, "k": K, "kernel": "cvt_dense_kernel + gemm (B[K,N] layout)",
                                 "extra_bytes": "two conversion passes: 2 x (64 MiB read + 32 MiB written)"},
                      "roofline": {"bound": "tensor", "achieved": tf, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s", "frac": tf / peaks["bf16_tflops"],
                                   "traffic": ncu_traffic(name), "peak_source": f"{peaks['source']} (burst cuBLAS bf16)"},

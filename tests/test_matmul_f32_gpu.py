@@ -128,3 +128,25 @@ def test_f32_entries_reject_bad_arguments(t0, rt):
     assert lib.t0_blas_gemv_f32(rt._h, 4, 4, 1.0, p, 4, p, 0, 0.0, p, 1) == 1        # incx == 0
     assert lib.t0_matmul_f32(rt._h, p, p, p, 0, 4, 4) == 0                           # empty M is a no-op
     buf.free()
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 8, 8), (3, 40, 24), (2048, 2400, 16), (4000, 4096, 32), (4032, 4096, 32)])
+def test_dense_operands_convert_as_strided_ones_do(t0, rt, m, k, n):
+    # one unit; operands that meet inside a block; more units than threads; just below and above the size from which sources are not kept in L2.
+    # An x that begins four bytes into its buffer goes through the kernel for any stride and alignment: the same bf16 operands, so the same bytes.
+    rng = np.random.default_rng(k)
+    x, w = rng.standard_normal((m, k), np.float32), rng.standard_normal((k, n), np.float32)
+    x.ravel()[[0, 1, -1]] = np.inf, np.float32(-3.4e38), np.nan
+    w[-1, -1] = -np.inf
+    wd, y = rt.upload(w), rt.alloc(m * n * 4)
+    got = []
+    for skip in (0, 1):
+        xd = rt.upload(np.concatenate([np.zeros(skip, np.float32), x.ravel()]))
+        y.write(np.full(m * n * 4, 0xA5, np.uint8))
+        rt.matmul_f32(xd.gpu_addr() + 4 * skip, wd.gpu_addr(), y.gpu_addr(), m, k, n)
+        rt.synchronize()
+        got.append(y.read(m * n * 4, np.uint8))
+        xd.free()
+    assert np.array_equal(got[0], got[1])
+    for b in (wd, y):
+        b.free()
