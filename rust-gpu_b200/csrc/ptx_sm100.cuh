@@ -60,8 +60,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Whether the phase is over, without waiting for it.
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+// Whether the phase is over, without waiting for it: one answer for a whole converged warp, as mbar_wait_warp below.  (The instruction may answer lanes
+// differently; a branch on that would part a warp whose roles meet in __syncwarp and votes.)
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
@@ -72,7 +73,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
-    return ok != 0;
+    return __all_sync(0xFFFFFFFFu, ok != 0);
 }
 
 // Wait limit for any single barrier wait.  The longest legitimate wait in these kernels is one

@@ -349,7 +349,7 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
                     ptx::tma_load_3d(dst + kStXOff + kStXChunk, &P.x[c.p], fb, (int32_t)k + 64, 0, 0);
                 }
                 __syncwarp();
-                if (head_pending && ptx::mbar_test_wait(head_written, 0)) {
+                if (head_pending && ptx::mbar_test_warp(head_written, 0)) {
                     count_head();
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(head_counted);
@@ -367,7 +367,7 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
             }
         }
         if (head_pending) {
-            if (ptx::mbar_wait(head_written, 0, abort_flag, P.wait_limit_ns)) count_head(); else if (lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xD00000);
+            if (ptx::mbar_wait_warp(head_written, 0, abort_flag, P.wait_limit_ns)) count_head(); else if (lane == 0) atomicCAS(P.status, 0, kStatusEpilogueTimeout | 0xD00000);
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(head_counted);       // (counted or not: nobody waits for what does not come)
         }
