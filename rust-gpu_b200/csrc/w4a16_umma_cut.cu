@@ -501,8 +501,8 @@ static uint32_t cut_grid(uint32_t sms, uint64_t items, uint32_t n_chunks) {
 }
 
 // How to share out the tiles of `count` problems: the fastest form, by times in microseconds fitted to 402 launches of M = 17 ... 128, 4 ... 224 tiles and
-// K = 768 ... 8192, each timed in both forms (the choice is within 0.3 % of the better one in the mean; the fit of before the last changes to this kernel was 2.6 %
-// off).  A chunk takes 0.28 us up to M = 64 and 0.34 (cut) or 0.32 (whole) at M = 128; handing in and adding parts adds 3 to 7 us with M.  Measured, whole tiles /
+// K = 768 ... 8192, each timed in both forms (the faster one by the times is within 0.3 % of the better one in the mean; the fit of before the last changes to this
+// kernel was 2.6 % off).  A chunk takes 0.28 us up to M = 64 and 0.34 (cut) or 0.32 (whole) at M = 128; handing in and adding parts adds 3 to 7 us with M.  Measured, whole tiles /
 // cut: 4 x (17 x 14336 x 2048) 21.5 / 22.4, 4 x (64 x 4096 x 2048) 13.5 / 12.5; one problem as clusters / cut: 17 x 16384 x 8192 46.8 / 24.3, 100 x 14336 x 1024
 // 13.4 / 15.5, 128 x 16384 x 2048 17.8 / 16.2.  (4 x (17 x 14336 x 2048): cut all the same, for the shorter sums.)
 // `cluster_split`: into how many parts the cluster form would cut K (1: one problem that has tiles enough; 0: a list); `cluster_rounds`: in how many rounds
@@ -513,8 +513,11 @@ static uint32_t cut_grid(uint32_t sms, uint64_t items, uint32_t n_chunks) {
 //
 // The times choose only among forms whose sums are no longer than the library has made them for the problem, since the tensor cores' error grows with
 // the length of an accumulation.  One problem: its pieces are no longer than the parts of the clusters (K = 768: four of 3 chunks, where the grid
-// above would make three of 4; 39 x 3264 x 768 12.4 us as clusters, 9.2 so).  Lists: whole tiles, all of K in a sum, only where the kernels of before their roles walked converged were no faster
-// cut; that fit (0.63 us a chunk whole, 0.67 cut, 14.4 us for the parts) is kept for this alone.  2 x (114 x 4680 x 1664): 26 chunks in one sum whole, 7 cut.
+// above would make three of 4; 39 x 3264 x 768 12.4 us as clusters, 9.2 so).  Tiles that would be cut by the times of the kernel as it was before two warps
+// issued its UMMAs (0.42 to 0.52 us a chunk either way), and lists that would be by those of before its roles walked converged (0.63 us a chunk whole, 0.67 cut, 14.4 us
+// for the parts), stay cut where that makes their sums shorter: both fits are kept for this alone.
+// Three of 70 x 2320 x 1280, whole / cut: 10.7 / 13.1 us, 1.06e-6 / 2.4e-7 off the exact result with sums of 20 / 5 chunks; two of 84 x 4352 x 1280
+// 11.0 / 13.6 us; 120 x 19352 x 2944 21.3 / 20.9 us, 2.7e-6 / 1.1e-6.
 // Gives the form, and for cut tiles the number of CTAs in *ctas.
 int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t count, uint32_t cluster_split, uint32_t cluster_rounds, uint32_t* ctas) {
     const uint64_t items = (uint64_t)ceil_div(N, kUmBN) * count;
@@ -526,12 +529,19 @@ int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t c
     if (items % grid == 0 || items * n_chunks >= (1u << 24)) return other;
     const double per_cta = (double)items * n_chunks / grid;
     const double rounds = (double)((items + sms - 1) / sms);
+    const bool cluster_form = other == kUmClusters;
+    const uint32_t parts = std::max(1u, cluster_split);
     if (cluster_split == 0 && per_cta * 0.67 + 14.4 <= 0.97 * (rounds * n_chunks * 0.63 + 4.0)) return kUmCut;
+    if (ceil_div(n_chunks, parts) > items * n_chunks / grid) {       // (the first CTA's range begins with a tile: cut, no sum needs to be longer than that range)
+        const double chunk = 0.42 + 0.0008 * M;
+        const double uncut = cluster_form ? cluster_rounds * (ceil_div(n_chunks, parts) * 0.495 + 8.2) + 2.0 : rounds * n_chunks * chunk + 4.2;
+        if (per_cta * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0) <= 0.97 * uncut) return kUmCut;
+    }
     const double wide = M > 64 ? M - 64.0 : 0.0;
     const double cut = per_cta * (0.288 - 0.00037 * M + 0.00176 * wide) + 6.0 + 0.049 * M + (grid >= sms ? 1.35 : 0.0);
-    const double without = other == kUmClusters ? cluster_rounds * (ceil_div(n_chunks, cluster_split) * 0.497 + 5.1 + 0.0018 * M) + 5.1
+    const double without = cluster_form ? cluster_rounds * (ceil_div(n_chunks, parts) * 0.497 + 5.1 + 0.0018 * M) + 5.1
                                                 : rounds * n_chunks * (0.285 - 0.0001 * M + 0.0008 * wide) + 3.3 + 0.021 * M;
-    return cut > (other == kUmClusters ? 0.92 : 1.03) * without ? other : kUmCut;
+    return cut > (cluster_form ? 0.92 : 1.03) * without ? other : kUmCut;
 }
 
 // The form of a launch.  Cut tiles need room for their parts, and run only in launches of the runtime's own stream, whose launches run one after the

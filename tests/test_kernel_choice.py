@@ -1,6 +1,8 @@
 """What the library chooses when the caller fixes nothing, asked on the CPU: a small C++ program linked against the library calls the rules.  The
 numbers are those of a B200 (148 SMs, clusters of 2 to 8 CTAs that fit at once)."""
+import math
 import os
+import random
 import subprocess
 
 import pytest
@@ -77,30 +79,77 @@ def test_sums_are_no_longer_than_they_have_been(ask):
 CLUSTERS, WHOLE, CUT = 0, 1, 2
 
 
-def w4a16_form(ask, m, n, k, count):
-    """How `count` problems (0: one that is not given as a list, whose K clusters would cut into at most four parts) are shared out, and the 64-deep chunks of
-    the longest accumulation."""
+def w4a16_split(n, k, count):
+    """The tiles and 64-deep chunks of `count` problems (0: one that is not given as a list), and for such a one into how many parts clusters would cut its K and
+    in how many rounds they run."""
     tiles, chunks = -(-n // 256) * (count or 1), k // 64
     split = 0 if count else min(max(1, min(4, 148 // tiles)), chunks)
     at_once = {0: tiles, 1: tiles, 2: 74, 3: 48, 4: 33}[split]                                                # clusters of `split` CTAs that fit at once
-    form, ctas = ask([("w4a16", m, n, k, count or 1, split, -(-tiles // at_once))])[0]
+    return tiles, chunks, split, -(-tiles // at_once)
+
+
+def w4a16_longest(form, ctas, tiles, chunks, split):
+    """The chunks of the longest accumulation."""
     if form != CUT:
-        return form, -(-chunks // max(split, 1))
-    ends = [c * tiles * chunks // ctas for c in range(ctas + 1)] + [t * chunks for t in range(tiles)]      # of the CTAs' ranges, and of the tiles
-    ends = sorted(set(ends))
-    return form, max(b - a for a, b in zip(ends, ends[1:]))
+        return -(-chunks // max(split, 1))
+    ends = sorted({c * tiles * chunks // ctas for c in range(ctas + 1)} | {t * chunks for t in range(tiles)})      # of the CTAs' ranges, and of the tiles
+    return max(b - a for a, b in zip(ends, ends[1:]))
+
+
+def w4a16_forms(ask, problems):
+    """How each (m, n, k, count) is shared out, and the 64-deep chunks of the longest accumulation."""
+    splits = [w4a16_split(n, k, count) for _, n, k, count in problems]
+    answers = ask([("w4a16", m, n, k, count or 1, split, rounds) for (m, n, k, count), (_, _, split, rounds) in zip(problems, splits)])
+    return [(form, w4a16_longest(form, ctas, tiles, chunks, split)) for (form, ctas), (tiles, chunks, split, _) in zip(answers, splits)]
+
+
+def w4a16_form(ask, m, n, k, count):
+    return w4a16_forms(ask, [(m, n, k, count)])[0]
 
 
 # lists whose tiles have been cut, and single problems, with the chunks of the longest accumulation the library has given them
 W4A16_LONGEST = [((113, 4456, 1920, 3), 11), ((125, 9800, 2944, 2), 25), ((114, 4680, 1664, 2), 7), ((128, 1632, 2240, 8), 14), ((121, 5144, 3008, 4), 27),
                  ((58, 592, 960, 0), 4), ((50, 4840, 576, 0), 3), ((36, 304, 576, 0), 3), ((20, 3200, 768, 0), 3), ((50, 7736, 832, 0), 4), ((128, 256, 64, 0), 1),
-                 ((17, 1024, 256, 0), 1), ((52, 8968, 576, 0), 3), ((128, 11008, 4096, 0), 22), ((20, 14336, 2048, 0), 16), ((100, 28672, 1024, 0), 16)]
+                 ((17, 1024, 256, 0), 1), ((52, 8968, 576, 0), 3), ((128, 11008, 4096, 0), 22), ((20, 14336, 2048, 0), 16), ((100, 28672, 1024, 0), 16),
+                 ((70, 2320, 1280, 3), 5), ((84, 4352, 1280, 2), 5), ((77, 6024, 1408, 2), 8), ((42, 3488, 1024, 2), 4), ((28, 8224, 1408, 2), 11),
+                 ((17, 2408, 832, 4), 5), ((39, 9776, 1152, 1), 6), ((25, 22296, 2368, 0), 22), ((120, 19352, 2944, 0), 24)]
 
 
 def test_w4a16_sums_are_no_longer_than_they_have_been(ask):
     for (m, n, k, count), longest in W4A16_LONGEST:
         form, chunks = w4a16_form(ask, m, n, k, count)
         assert chunks <= longest, (m, n, k, count, form, chunks)
+
+
+def w4a16_bound(m, n, k, count):
+    """The longest accumulation by the rule that these kernels were first given, its grid and its times."""
+    tiles, chunks, split, rounds = w4a16_split(n, k, count)
+    total = tiles * chunks
+    ctas = min(max(1, total // 4), 148)
+    if tiles * 2 <= 148:
+        parts = max(1, min(4, 148 // tiles, chunks // 4))
+        if parts == 4 or parts * 8 > chunks or tiles * parts * 5 >= 148 * 4:
+            ctas = tiles * parts
+    other = CLUSTERS if split > 1 else WHOLE
+    if other == CLUSTERS and -(-total // ctas) > -(-chunks // split):
+        ctas = tiles * split
+    form = other
+    if tiles % ctas:
+        waves, chunk = -(-tiles // 148), 0.42 + 0.0008 * m
+        whole = rounds * (-(-chunks // split) * 0.495 + 8.2) + 2.0 if other == CLUSTERS else waves * chunks * chunk + 4.2
+        if total / ctas * chunk + 6.2 + 0.055 * m + (2.0 if ctas >= 148 else 0.0) <= 0.97 * whole or \
+                (split == 0 and total / ctas * 0.67 + 14.4 <= 0.97 * (waves * chunks * 0.63 + 4.0)):
+            form = CUT
+    return w4a16_longest(form, ctas, tiles, chunks, split)
+
+
+def test_w4a16_sums_are_no_longer_over_the_range(ask):
+    rng = random.Random(11)
+    def size(low, high, step):
+        return max(low, round(math.exp(rng.uniform(math.log(low), math.log(high))) / step) * step)
+    problems = [(rng.randint(17, 128), size(256, 32768, 8), size(128, 8192, 64), rng.choice([0, 0, 1, 2, 2, 3, 4, 8, 16])) for _ in range(20000)]
+    longer = [(p, got, w4a16_bound(*p)) for p, got in zip(problems, w4a16_forms(ask, problems)) if got[1] > w4a16_bound(*p)]
+    assert not longer, (len(longer), longer[:5])
 
 
 def test_w4a16_clusters_in_two_rounds_are_weighed_as_such(ask):
