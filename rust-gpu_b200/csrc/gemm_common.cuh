@@ -340,6 +340,22 @@ inline int make_map_kmajor(CUtensorMap* map, const void* base, uint32_t rows, ui
     return T0_OK;
 }
 
+// The map `like` over another base address: a tenth of the time an encoding takes.  False where the driver has no such call, or refuses.
+inline bool make_map_like(CUtensorMap* map, const CUtensorMap& like, const void* base) {
+    typedef CUresult (*ReplaceAddressFn)(CUtensorMap*, void*);
+    static ReplaceAddressFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapReplaceAddress", &p, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+            fn = (ReplaceAddressFn)p;
+    });
+    if (!fn) return false;
+    *map = like;
+    return fn(map, const_cast<void*>(base)) == CUDA_SUCCESS;
+}
+
 // Plain 2-D row-major view [rows][cols] of 16- or 32-bit elements, no swizzle, box = box_cols x box_rows.
 inline int make_map_2d_plain(CUtensorMap* map, const void* base, uint32_t elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_cols,
                              uint32_t box_rows) {

@@ -63,16 +63,13 @@ struct StProblem {
     const uint8_t* scales_t;   // [band][K/G][256] bf16
     const uint8_t* zeros_t;    // [band][K/G][32] u32
     uint32_t M, N;
-    uint32_t ksteps, groups, units_per_group, n_bands;
-    uint32_t unit_begin;       // first unit of this problem in the launch's list
+    uint32_t ksteps, units_per_group, n_bands;
     uint32_t band_begin;       // first arrival counter of this problem
     UmDiv by_ksteps, by_group; // ksteps, units_per_group
 };
 
 template <uint32_t kProblems>
 struct StParams {
-    CUtensorMap x[kProblems];  // activations, boxes of 16 rows x 64 k
-    StProblem prob[kProblems];
     float* partials;           // [grid][2][16*256]
     int* counters;             // one per band of the launch, zero between launches
     int* status;               // error word of the runtime (bounded waits)
@@ -82,9 +79,12 @@ struct StParams {
     uint32_t per_cta, rest;    // total_units = grid * per_cta + rest
     float cta_per_unit;        // grid / total_units
     UmDiv by_grid;
+    uint32_t unit_begin[kProblems];   // first unit of a problem in the launch's list; beyond the last problem 2^32 - 1
+    StProblem prob[kProblems];
+    CUtensorMap x[kProblems];  // activations, boxes of 16 rows x 64 k (last: what every launch reads first lies together)
 };
 constexpr uint32_t kStMaxProblems = 32;               // problems per launch (the table travels as a kernel parameter) ...
-constexpr uint32_t kStFewProblems = 4;                // ... or as a parameter of a seventh of the size
+constexpr uint32_t kStFewProblems = 8;                // ... or as a parameter of a fourth of the size: 0.4 us less on the host (5 x 512 x 512: 5.2 us of host time a launch, 4.85)
 
 // First unit of a CTA's range, floor(cta * total / grid), and the CTA whose range holds a unit: without the 64-bit divisions, which take hundreds of cycles
 // where a band is finished.
@@ -100,12 +100,14 @@ __device__ __forceinline__ uint32_t st_owner(const Params& P, uint32_t unit) {
 
 struct Cursor { uint32_t p, band, ks; };
 
-template <class Params>
-__device__ __forceinline__ Cursor locate(const Params& P, uint32_t unit) {
+// By a converged warp, of which each lane looks at a problem.  (Walking the list problem by problem, three times a launch, missed the constant cache at each:
+// 32 of 1024 x 1024 at M = 1 15.1 us, 11.5 so.)
+template <uint32_t kProblems>
+__device__ __forceinline__ Cursor locate(const StParams<kProblems>& P, uint32_t unit) {
+    static_assert(kProblems <= 32, "a lane looks at a problem");
     Cursor c;
-    c.p = 0;
-    while (c.p + 1 < P.n_problems && P.prob[c.p + 1].unit_begin <= unit) ++c.p;
-    const uint32_t r = unit - P.prob[c.p].unit_begin;
+    c.p = __popc(__ballot_sync(0xFFFFFFFFu, P.unit_begin[min(threadIdx.x & 31, kProblems - 1)] <= unit && (threadIdx.x & 31) < kProblems)) - 1;
+    const uint32_t r = unit - P.unit_begin[c.p];
     c.band = um_div(r, P.prob[c.p].by_ksteps);
     c.ks = r - c.band * P.prob[c.p].ksteps;
     return c;
@@ -165,7 +167,7 @@ template <class Params>
 __device__ __forceinline__ StFinish st_finish(const Params& P, uint32_t p, uint32_t band, uint32_t t) {
     StFinish f;
     const StProblem& pr = P.prob[p];
-    f.h = st_share(P, pr.unit_begin + band * pr.ksteps, pr.ksteps);
+    f.h = st_share(P, P.unit_begin[p] + band * pr.ksteps, pr.ksteps);
     f.p = p; f.band = band;
     f.items = pr.M * (kBandCols / 4);
     const uint32_t count = f.h.last - f.h.first + 1;
@@ -300,13 +302,14 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
     auto range_ends = [&]() {
         uint32_t lo = U0, hi = U1;
         asm volatile("" : "+r"(lo), "+r"(hi));
+        __syncwarp();
         Ends e;
         e.first = locate(P, lo);
         e.last = locate(P, hi - 1);
         e.head_first = lo - e.first.ks;
         e.head_ksteps = P.prob[e.first.p].ksteps;
         e.has_head = e.first.ks != 0 && e.head_first + e.head_ksteps < hi;
-        const uint32_t end_first = P.prob[e.last.p].unit_begin + e.last.band * P.prob[e.last.p].ksteps;
+        const uint32_t end_first = P.unit_begin[e.last.p] + e.last.band * P.prob[e.last.p].ksteps;
         e.tail_cut = end_first < lo || end_first + P.prob[e.last.p].ksteps > hi;
         return e;
     };
@@ -329,11 +332,12 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
         uint32_t stage = 0, phase = 0;
         for (uint32_t u = U0; u < U1; ++c.p) {
             const StProblem& pr = P.prob[c.p];
-            const uint32_t at = u - pr.unit_begin, row = um_div(at, pr.by_group), u_stop = min(U1, pr.unit_begin + pr.ksteps * pr.n_bands);
+            const uint32_t begin = P.unit_begin[c.p], at = u - begin, row = um_div(at, pr.by_group), u_stop = min(U1, begin + pr.ksteps * pr.n_bands);
             const uint8_t* tile = pr.tiles + (size_t)at * kWeightBytes;
             const uint8_t* scales = pr.scales_t + (size_t)row * kScaleBytes;
             const uint8_t* zeros = pr.zeros_t + (size_t)row * kZeroBytes;
             uint32_t in_row = at - row * pr.units_per_group, k = (at - um_div(at, pr.by_ksteps) * pr.ksteps) * kUnitK;
+            if (u_stop < U1 && lane == 0) ptx::tma_prefetch_desc(&P.x[c.p + 1]);
             bool ok = true;
             for (; u < u_stop; ++u) {
                 ok = ptx::mbar_wait_warp(empty_bar + stage * 8, phase ^ 1, abort_flag, P.wait_limit_ns);
@@ -511,7 +515,7 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
         uint32_t piece = 0;
         for (uint32_t u = U0; u < U1; ++piece) {
             const StProblem& pr = P.prob[c.p];
-            const uint32_t first_unit = pr.unit_begin + c.band * pr.ksteps, last_unit = first_unit + pr.ksteps;   // [first, last)
+            const uint32_t first_unit = P.unit_begin[c.p] + c.band * pr.ksteps, last_unit = first_unit + pr.ksteps;   // [first, last)
             const bool whole = first_unit >= U0 && last_unit <= U1, tail = last_unit >= U1;
             const StShare h = st_share(P, first_unit, pr.ksteps);
             int* const counter = P.counters + pr.band_begin + c.band;
@@ -691,26 +695,35 @@ uint32_t prepack_grid_for(uint64_t n, uint32_t block) {
 // One launch for up to kProblems problems (already validated).
 template <uint32_t kProblems>
 int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count) {
-    StParams<kProblems> P;
-    memset(&P, 0, sizeof P);
+    StParams<kProblems> P;                            // (up to 6.7 KB: what the kernel reads is filled in, nothing is cleared first)
+    P.stamps = nullptr;
     uint64_t total = 0, bands = 0;
+    PrepackLayout L = {};
     for (size_t i = 0; i < count; ++i) {
         const t0_w4a16_args& a = args[i];
-        const PrepackLayout L = prepack_layout(a.k, a.n, a.group);
-        int rc = gemm::make_map_kmajor(&P.x[i], (const void*)a.a, a.m, a.k, a.k, 1, kStMRows);
+        // A list is mostly of one shape: what that decides is taken from the problem before, since divisions and the encoding of a map are most of a problem's time
+        // here (32 of 512 x 512: 12.6 us of host time a launch without, 11.1 so).
+        const bool same_x = i > 0 && a.m == args[i - 1].m && a.k == args[i - 1].k && gemm::make_map_like(&P.x[i], P.x[i - 1], (const void*)a.a);
+        int rc = same_x ? T0_OK : gemm::make_map_kmajor(&P.x[i], (const void*)a.a, a.m, a.k, a.k, 1, kStMRows);
         if (rc != T0_OK) return rc;
+        if (i == 0 || a.k != args[i - 1].k || a.n != args[i - 1].n || a.group != args[i - 1].group) L = prepack_layout(a.k, a.n, a.group);
         StProblem& q = P.prob[i];
+        if (i > 0 && a.k == args[i - 1].k && a.group == args[i - 1].group) {
+            q = P.prob[i - 1];
+        } else {
+            q.ksteps = L.ksteps; q.units_per_group = a.group / kUnitK;
+            q.by_ksteps = um_divisor(q.ksteps); q.by_group = um_divisor(q.units_per_group);
+        }
         q.y = (float*)a.y;
         q.tiles = (const uint8_t*)a.packed + L.off_tiles;
         q.scales_t = (const uint8_t*)a.packed + L.off_scales;
         q.zeros_t = (const uint8_t*)a.packed + L.off_zeros;
-        q.M = a.m; q.N = a.n;
-        q.ksteps = L.ksteps; q.groups = L.groups; q.units_per_group = a.group / kUnitK; q.n_bands = L.bands;
-        q.unit_begin = (uint32_t)total; q.band_begin = (uint32_t)bands;
-        q.by_ksteps = um_divisor(q.ksteps); q.by_group = um_divisor(q.units_per_group);
+        q.M = a.m; q.N = a.n; q.n_bands = L.bands;
+        P.unit_begin[i] = (uint32_t)total; q.band_begin = (uint32_t)bands;
         total += (uint64_t)L.bands * L.ksteps;
         bands += L.bands;
     }
+    for (size_t i = count; i < kProblems; ++i) P.unit_begin[i] = 0xFFFFFFFFu;
     if (total == 0) return T0_OK;
     if (total > 0x7FFFFFFFull || bands * sizeof(int) > kCounterRegion) return fail(T0_ERR_UNSUPPORTED, "batch too large: %llu steps, %llu bands", (unsigned long long)total, (unsigned long long)bands);
     const uint32_t grid = (uint32_t)std::min<uint64_t>(total, (uint64_t)rt->sm_count);
@@ -752,7 +765,8 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, w4a16_stream_kernel<kProblems>, P);
+    void* launch_args[] = {&P};                       // (not by value, which would copy them once more)
+    cudaError_t le = cudaLaunchKernelExC(&cfg, (const void*)w4a16_stream_kernel<kProblems>, launch_args);
     if (le != cudaSuccess) return fail(T0_ERR_CUDA, "W4A16 kernel launch failed: %s", cudaGetErrorString(le));
     rt->launches.fetch_add(1);
     if (trace) {

@@ -629,7 +629,9 @@ def test_tiled_grouped_random_shapes(t0, oracle, rt):
     [(1, 14336, 40, 128)], [(2, 7168, 256, 1024)], [(16, 3584, 136, 3584)],        # one band, a CTA per step: contributors added in groups of threads (M = 1, 2) and by one (M = 16)
     [(8, 4096, 18944, 128)], [(9, 4096, 18944, 128)],                              # 74 bands on 148 CTAs: two contributors each, the edge of eight rows
     [(16, 1024, 33000, 128), (3, 1024, 4736, 256)],                                # whole bands, cut ones, and a range across two problems
-    [(m, 512, 1000, 512) for m in (1, 7, 16, 9)], [(m, 512, 1000, 512) for m in (1, 7, 16, 9, 8)],   # the two sizes of parameter block
+    [(m, 512, 1000, 512) for m in (1, 7, 16, 9)], [(m, 512, 1000, 512) for m in (1, 7, 16, 9, 8)],   # short lists
+    [(m, 256, 264, 256) for m in (1, 1, 7, 16, 16, 9, 8, 8)], [(m, 256, 264, 256) for m in (1, 1, 7, 16, 16, 9, 8, 8, 8)],   # the edge between them
+    [(1 + i // 2, 128 * (1 + i // 7 % 3), 8 + 248 * (i % 2), 128) for i in range(31)] + [(3, 1024, 40000, 128)],   # a full launch: ranges over several problems of one to three units
 ])
 def test_streaming_kernel_edges(t0, oracle, rt, shapes):
     probs, bufs = _batch_problems(oracle, rt, shapes, 700)
