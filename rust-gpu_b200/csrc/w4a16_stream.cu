@@ -54,7 +54,7 @@ constexpr uint32_t kStTmemCols = 512;
 constexpr uint32_t kStAccCols = 128;
 constexpr uint32_t kStAStages = 3;
 constexpr uint32_t kStAStageCols = 128;
-constexpr uint32_t kStBars = 2 * kStStages + 4 * kStAStages + 4;
+constexpr uint32_t kStBars = 2 * kStStages + 4 * kStAStages + 5;
 constexpr size_t kStSmem = 1024 + (size_t)kStStages * kStStageBytes + kStBars * 8;      // (more than half an SM's: two CTAs must never share its tensor memory)
 
 struct StProblem {
@@ -249,6 +249,7 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
     const uint32_t acc_empty = acc_full + 8;
     const uint32_t head_written = acc_empty + 8;                         // the epilogue warps have stored the head piece
     const uint32_t head_counted = head_written + 8;                      // it is counted in and s_head_last is valid
+    const uint32_t end_near = head_counted + 8;                          // one step of the range is left to dequantise
     __shared__ uint32_t tmem_holder;
     __shared__ int s_abort, s_last, s_all, s_head_last, s_head_go;
     volatile int* abort_flag = &s_abort;
@@ -272,6 +273,7 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
         ptx::mbar_init(acc_empty, kStEpWarps);
         ptx::mbar_init(head_written, kStEpWarps);
         ptx::mbar_init(head_counted, 1);
+        ptx::mbar_init(end_near, 1);
         s_abort = 0;
         s_last = s_all = s_head_last = 0;
         ptx::fence_barrier_init();
@@ -491,6 +493,8 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
             stage += 2;
             if (stage >= kStStages) { stage -= kStStages; phase ^= 1; }
         }
+        // The set that does not have the last step is through first, one step before the end.
+        ptx::mbar_arrive_if(end_near, tid == (kStDqWarp0 + ((U1 - U0) & 1) * 8) * 32);
         if (tid == kStDqWarp0 * 32) stamp(2);
         // Finish the bands of the last and the first piece, where this CTA turned out to be the last to contribute to them.  (The last step is done with by
         // then, so the ring is free.)
@@ -521,12 +525,13 @@ w4a16_stream_kernel(const __grid_constant__ StParams<kProblems> P) {
             int* const counter = P.counters + pr.band_begin + c.band;
             float* const part = P.partials + ((size_t)blockIdx.x * 2 + (first_unit <= U0 ? 0u : 1u)) * kPieceFloats;   // slot 0: the piece with this CTA's first unit
             // The last piece is on the way of everything behind the launch.  Where its band has one more part, that lies as a rule in a range that began with it,
-            // and is long there: looked for as the last step's bytes land, it is fetched and added to the accumulators at once, with no hand-in, fence and atomic.
+            // and is long there: looked for as the last step is dequantised, it is fetched and added to the accumulators at once, with no hand-in, fence and atomic.
+            // (On a barrier that completes once.  These warps follow none of the ring's barriers, whose parity an earlier phase answers as well.)
             bool rest_there = false;
             float other[2][16];
             if (!whole && tail && h.last - h.first == 1) {      // (barriers are met whether or not a wait has run out)
-                const uint32_t i = U1 - 1 - U0, cta = h.first == blockIdx.x ? h.last : h.first;
-                ok = ok && ptx::mbar_wait(full_bar + (i % kStStages) * 8, (i / kStStages) & 1, abort_flag, P.wait_limit_ns);
+                const uint32_t cta = h.first == blockIdx.x ? h.last : h.first;
+                ok = ok && ptx::mbar_wait(end_near, 0, abort_flag, P.wait_limit_ns);
                 if (et == 0) s_all = ok && um_ld_acquire((const uint32_t*)counter) != 0;
                 st_epilogue_sync();
                 rest_there = s_all != 0;

@@ -15,3 +15,13 @@ def test_barriers_are_polled_once_only_by_whole_warps(t0):
     looks = re.findall(r"__device__ __forceinline__ bool (\w+)\([^)]*\) \{\n(.*?)\n\}", helpers, flags=re.S)
     single = [(name, body) for name, body in looks if "mbarrier.test_wait" in body]
     assert single and all("return __all_sync(0xFFFFFFFFu" in body for _, body in single), [name for name, _ in single]
+
+
+def test_the_streaming_epilogue_follows_no_ring(t0):
+    # A wait asks for a parity, which every second phase of a barrier answers: a role may wait on a ring's barrier only if it waits for every phase.  The epilogue
+    # warps of the streaming kernel come by once per piece of a range.
+    csrc = os.path.join(os.path.dirname(os.path.dirname(t0.HEADER_PATH)), "rust-gpu_b200", "csrc")
+    text = open(os.path.join(csrc, "w4a16_stream.cu")).read()
+    role = text[text.index("four warps: accumulators to y"):text.index("give copies and UMMAs already in flight")]
+    waits = re.findall(r"mbar_wait\w*\((\w+)", role)
+    assert sorted(set(waits)) == ["acc_full", "end_near"], waits

@@ -628,6 +628,7 @@ def test_tiled_grouped_random_shapes(t0, oracle, rt):
     [(1, 128, 8, 128)],                                                            # one step, one CTA
     [(1, 14336, 40, 128)], [(2, 7168, 256, 1024)], [(16, 3584, 136, 3584)],        # one band, a CTA per step: contributors added in groups of threads (M = 1, 2) and by one (M = 16)
     [(8, 4096, 18944, 128)], [(9, 4096, 18944, 128)],                              # 74 bands on 148 CTAs: two contributors each, the edge of eight rows
+    [(9, 2048, 40448, 128)],                                                       # ranges one step and a bit longer than a band: short last pieces, whose other part is counted long before
     [(16, 1024, 33000, 128), (3, 1024, 4736, 256)],                                # whole bands, cut ones, and a range across two problems
     [(m, 512, 1000, 512) for m in (1, 7, 16, 9)], [(m, 512, 1000, 512) for m in (1, 7, 16, 9, 8)],   # short lists
     [(m, 256, 264, 256) for m in (1, 1, 7, 16, 16, 9, 8, 8)], [(m, 256, 264, 256) for m in (1, 1, 7, 16, 16, 9, 8, 8, 8)],   # the edge between them
