@@ -131,22 +131,32 @@ def test_f32_entries_reject_bad_arguments(t0, rt):
 
 
 @pytest.mark.parametrize("m,k,n", [(1, 8, 8), (3, 40, 24), (2048, 2400, 16), (4000, 4096, 32), (4032, 4096, 32)])
-def test_dense_operands_convert_as_strided_ones_do(t0, rt, m, k, n):
+def test_dense_operands_convert_as_strided_ones_do(t0, oracle, rt, m, k, n):
     # one unit; operands that meet inside a block; more units than threads; just below and above the size from which sources are not kept in L2.
     # An x that begins four bytes into its buffer goes through the kernel for any stride and alignment: the same bf16 operands, so the same bytes.
+    # Finite operands first, against the product of the rounded operands as well (f32 sums of exact products, whose error grows by 1e-9 of the result per k: four times that);
+    # then with an infinity, a value that rounds to one and a NaN in x and an infinity in w, each in a row or column of its own where there is one.
     rng = np.random.default_rng(k)
     x, w = rng.standard_normal((m, k), np.float32), rng.standard_normal((k, n), np.float32)
-    x.ravel()[[0, 1, -1]] = np.inf, np.float32(-3.4e38), np.nan
-    w[-1, -1] = -np.inf
-    wd, y = rt.upload(w), rt.alloc(m * n * 4)
-    got = []
-    for skip in (0, 1):
-        xd = rt.upload(np.concatenate([np.zeros(skip, np.float32), x.ravel()]))
-        y.write(np.full(m * n * 4, 0xA5, np.uint8))
-        rt.matmul_f32(xd.gpu_addr() + 4 * skip, wd.gpu_addr(), y.gpu_addr(), m, k, n)
-        rt.synchronize()
-        got.append(y.read(m * n * 4, np.uint8))
-        xd.free()
-    assert np.array_equal(got[0], got[1])
+    xs, ws = x.copy(), w.copy()
+    xs[0, 0], xs[m // 2, 1], xs[-1, -1] = np.inf, np.float32(-3.4e38), np.nan
+    ws[-1, -1] = -np.inf
+    wd, y = rt.alloc(k * n * 4), rt.alloc(m * n * 4)
+    for xv, wv in ((x, w), (xs, ws)):
+        wd.write(wv)
+        got = []
+        for skip in (0, 1):
+            xd = rt.upload(np.concatenate([np.zeros(skip, np.float32), xv.ravel()]))
+            y.write(np.full(m * n * 4, 0xA5, np.uint8))
+            rt.matmul_f32(xd.gpu_addr() + 4 * skip, wd.gpu_addr(), y.gpu_addr(), m, k, n)
+            rt.synchronize()
+            got.append(y.read(m * n * 4, np.uint8))
+            xd.free()
+        assert np.array_equal(got[0], got[1])
+        if xv is x:
+            rounded = [oracle.bf16_to_f32(oracle.f32_to_bf16_rne(v.ravel())).astype(np.float64).reshape(v.shape) for v in (x, w)]
+            some = sorted({0, m // 3, m // 2, m - 1})
+            out, ref = got[0].view(np.float32).reshape(m, n)[some], rounded[0][some] @ rounded[1]
+            assert np.linalg.norm(out - ref) <= max(4e-6, 4e-9 * k) * np.linalg.norm(ref)
     for b in (wd, y):
         b.free()

@@ -710,3 +710,29 @@ def test_lists_keep_their_sums_short(t0, oracle, rt, M, N, K, count, longest):
         assert err <= 2 * 7.5e-10 * 64 * longest, err
     for b in bufs:
         b.free()
+
+
+@pytest.mark.parametrize("M,K,N", [(16, 1024, 1000), (3, 4096, 520), (9, 384, 40000)])      # cut bands, many contributors, whole bands
+def test_streaming_rows_of_infinities_and_nans_leave_the_others_alone(t0, oracle, rt, M, K, N):
+    # The rows of the activations share one UMMA.  An infinity in the last row and a NaN in the first but one: those rows follow IEEE, the others keep their bits.
+    probs, bufs = _batch_problems(oracle, rt, [(M, K, N, 128)], 900)
+    p = probs[0]
+    call = t0.W4A16Args(p["xa"].gpu_addr(), p["pre"].gpu_addr(), 0, 0, p["y"].gpu_addr(), M, N, K, 128)
+
+    def run(a):
+        p["xa"].write(a)
+        rt.w4a16_gemm_prepacked_batch([call])
+        rt.synchronize()
+        return p["y"].read(M * N * 4, np.float32).reshape(M, N)
+
+    finite = run(p["a"])
+    a = p["a"].copy().reshape(M, K)
+    a[1, K - 3], a[M - 1, K // 2 + 1] = 0x7FC0, 0x7F80
+    got = run(a.reshape(-1))
+    w = oracle.bf16_to_f32(oracle.dequant_w4_b200(p["packed"], p["scales"], p["zeros"], K, N, 128)).reshape(K, N)[K // 2 + 1]
+    assert np.all(np.isnan(got[1]))
+    assert np.array_equal(got[M - 1], np.where(w == 0, np.float32(np.nan), np.copysign(np.float32(np.inf), w)), equal_nan=True)
+    others = [m for m in range(M) if m not in (1, M - 1)]
+    assert np.array_equal(got[others], finite[others]) and np.all(np.isfinite(finite))
+    for b in bufs:
+        b.free()
