@@ -58,7 +58,6 @@ struct UmParams {
     uint64_t wait_limit_ns;
     uint32_t M, N;
     uint32_t rows;           // M rounded up to 16: width of the UMMAs and height of the activation boxes
-    uint32_t group;          // k per scale / zero-point row (a multiple of 64)
     uint32_t n_tiles, n_chunks;
     uint32_t total;          // chunks of the launch, shared out evenly (less than 2^24)
     uint32_t whole;          // shared out by tiles instead: no tile is cut
@@ -508,6 +507,10 @@ static uint32_t cut_grid(uint32_t sms, uint64_t items, uint32_t n_chunks) {
 // `cluster_split`: into how many parts the cluster form would cut K (1: one problem that has tiles enough; 0: a list); `cluster_rounds`: in how many rounds
 // its clusters fit on the GPU (the GPCs hold 33 of four CTAs, not 37: 128 x 9472 x 4096 36.4 us in two rounds of clusters, 20.7 cut).
 //
+// Cut tiles of more than 64 rows whose parts are not the same number to each (56 tiles on 148 CTAs) take 2.0 to 2.7 us more than that, which matters beside clusters: a chunk
+// of one accumulator set, and up to four parts to a tile.  260 single problems that the times without it would move from clusters to cut tiles, weights not in
+// L2: 9 were slower so, by up to 7 % (93 x 14112 x 1536 16.8 us cut, 15.6 as clusters; 85 x 14784 x 1152 16.1 and 14.1), with it 2 of 247, by up to 2 %.
+//
 // Clusters are left only for a gain of more than 8 % (they share no memory between launches, so that a recorded launch gives the same bits), whole tiles for
 // none at all, nor for a loss of up to 3 % (their sums are the longest).
 //
@@ -538,7 +541,8 @@ int w4a16_umma_form(uint32_t sms, uint32_t M, uint32_t N, uint32_t K, uint32_t c
         if (per_cta * chunk + 6.2 + 0.055 * M + (grid >= sms ? 2.0 : 0.0) <= 0.97 * uncut) return kUmCut;
     }
     const double wide = M > 64 ? M - 64.0 : 0.0;
-    const double cut = per_cta * (0.288 - 0.00037 * M + 0.00176 * wide) + 6.0 + 0.049 * M + (grid >= sms ? 1.35 : 0.0);
+    const double uneven = cluster_form && M > 64 && grid % items ? 2.3 : 0.0;
+    const double cut = per_cta * (0.288 - 0.00037 * M + 0.00176 * wide) + 6.0 + 0.049 * M + (grid >= sms ? 1.35 : 0.0) + uneven;
     const double without = cluster_form ? cluster_rounds * (ceil_div(n_chunks, parts) * 0.497 + 5.1 + 0.0018 * M) + 5.1
                                                 : rounds * n_chunks * (0.285 - 0.0001 * M + 0.0008 * wide) + 3.3 + 0.021 * M;
     return cut > (cluster_form ? 0.92 : 1.03) * without ? other : kUmCut;
@@ -573,7 +577,7 @@ int launch_w4a16_umma_cut(t0_runtime* rt, const UmGroup<kProblems, kTiled>& grou
     p.status = rt->d_status;
     const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
     p.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
-    p.M = M; p.N = N; p.group = group_size;
+    p.M = M; p.N = N;
     p.rows = w4a16_umma_cut_rows(M);
     p.n_tiles = ceil_div(N, kUmBN);
     p.n_chunks = K / kUmBK;

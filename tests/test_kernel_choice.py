@@ -152,6 +152,14 @@ def test_w4a16_sums_are_no_longer_over_the_range(ask):
     assert not longer, (len(longer), longer[:5])
 
 
+def test_w4a16_uneven_parts_of_many_rows_leave_clusters_alone(ask):
+    # measured slower cut than as clusters (56, 53, 38, 58 tiles on 148 CTAs); even parts, few rows, or more of K: cut
+    for m, n, k in [(93, 14112, 1536), (81, 13416, 1536), (66, 9720, 1664), (85, 14784, 1152)]:
+        assert w4a16_form(ask, m, n, k, 0)[0] == CLUSTERS, (m, n, k)
+    for m, n, k in [(92, 3232, 6272), (49, 14112, 1536), (96, 15312, 2816), (121, 12128, 7424)]:
+        assert w4a16_form(ask, m, n, k, 0)[0] == CUT, (m, n, k)
+
+
 def test_w4a16_clusters_in_two_rounds_are_weighed_as_such(ask):
     # 33 clusters of four CTAs fit at once: 33 tiles take one round, 34 take two and are cut in their place
     assert w4a16_form(ask, 128, 33 * 256, 4096, 0)[0] == CLUSTERS
