@@ -39,10 +39,6 @@ struct W4Params {
     uint32_t units_per_group;   // group / 128: steps that share one row of scales and zero points
     uint32_t n_bands, ksteps, total_units;
     uint32_t a_units;    // steps of activations the shared-memory area holds (max steps of one CTA)
-    const uint8_t* tiles;      // streaming layout only: [band][kstep][16][256] u32
-    const uint8_t* scales_t;   //   [band][K/G][256] bf16
-    const uint8_t* zeros_t;    //   [band][K/G][32] u32
-    uint32_t groups;           //   K / G
     unsigned long long* stamps;   // optional trace: 4 nanosecond stamps per CTA (entry, staged, loop done, exit)
 };
 

@@ -75,9 +75,8 @@ struct StParams {
     int* status;               // error word of the runtime (bounded waits)
     unsigned long long* stamps;   // optional trace: 4 nanosecond stamps per CTA (entry, first step landed, loop done, exit)
     uint64_t wait_limit_ns;
-    uint32_t n_problems, total_units;
-    uint32_t per_cta, rest;    // total_units = grid * per_cta + rest
-    float cta_per_unit;        // grid / total_units
+    uint32_t per_cta, rest;    // the launch's units = grid * per_cta + rest
+    float cta_per_unit;        // grid / units
     UmDiv by_grid;
     uint32_t unit_begin[kProblems];   // first unit of a problem in the launch's list; beyond the last problem 2^32 - 1
     StProblem prob[kProblems];
@@ -743,7 +742,6 @@ int launch_stream_chunk(t0_runtime* rt, const t0_w4a16_args* args, size_t count)
     P.status = rt->d_status;
     const uint64_t limit = rt->wait_limit_ns.load(std::memory_order_relaxed);
     P.wait_limit_ns = limit ? limit : ptx::kWaitLimitNs;
-    P.n_problems = (uint32_t)count; P.total_units = (uint32_t)total;
     P.per_cta = (uint32_t)total / grid; P.rest = (uint32_t)total % grid; P.cta_per_unit = (float)grid / (float)total; P.by_grid = um_divisor(grid);
     static bool attr_set[64] = {};
     if (rt->device >= 64) return fail(T0_ERR_INVALID, "device ordinal out of range");

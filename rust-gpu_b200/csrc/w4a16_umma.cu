@@ -552,8 +552,9 @@ static int um_launch_list(t0_runtime* rt, const t0_w4a16_args* args, uint32_t co
         int rc = um_group_entry(grp, i, args[i]);
         if (rc != T0_OK) return rc;
     }
-    const TiledLayout L = tiled_layout(args[0].k, args[0].n, args[0].group);
-    return launch_w4a16_umma_cut(rt, grp, args[0].m, args[0].n, args[0].k, args[0].group, count, cut_ctas, kTiled ? L.off_scales : 0, kTiled ? L.off_zeros : 0);
+    TiledLayout L = {};                              // (the row layout's scales and zero points have maps)
+    if constexpr (kTiled) L = tiled_layout(args[0].k, args[0].n, args[0].group);
+    return launch_w4a16_umma_cut(rt, grp, args[0].m, args[0].n, args[0].k, args[0].group, count, cut_ctas, L.off_scales, L.off_zeros);
 }
 
 template <bool kTiled>
@@ -561,8 +562,9 @@ static int um_launch_single(t0_runtime* rt, const t0_w4a16_args& a, uint32_t cut
     UmGroup<1, kTiled> one;
     int rc = um_group_entry(one, 0, a);
     if (rc != T0_OK) return rc;
-    const TiledLayout L = tiled_layout(a.k, a.n, a.group);
-    return launch_w4a16_umma_cut(rt, one, a.m, a.n, a.k, a.group, 1, cut_ctas, kTiled ? L.off_scales : 0, kTiled ? L.off_zeros : 0);
+    TiledLayout L = {};
+    if constexpr (kTiled) L = tiled_layout(a.k, a.n, a.group);
+    return launch_w4a16_umma_cut(rt, one, a.m, a.n, a.k, a.group, 1, cut_ctas, L.off_scales, L.off_zeros);
 }
 
 static int um_launch_one(t0_runtime* rt, const t0_w4a16_args& a, bool tiled) {
