@@ -107,7 +107,9 @@ static std::vector<Candidate> schedule(uint32_t m, uint32_t n, uint32_t k) {
 // per round what of its epilogue stays exposed.  With K in parts there is one round, and instead the exchange in the clusters: longer with
 // the rows and columns of a tile, a little with every part, and a launch that leaves half of the SMs to the next one's prologue is
 // shorter.  The pair's 256 x 128 tile takes in 24 KB a k block where the 128 x 128 tiles of two CTAs take 32: 2048 x 1024 x 4096 22.1 -> 20.3 us,
-// 1664 x 1056 x 3248 18.6 -> 17.4 (that tile alone, converged roles on both sides, one box).  The search above
+// 1664 x 1056 x 3248 18.6 -> 17.4 (that tile alone, converged roles on both sides, one box).  The single tiles and parts have become faster since (predicated
+// issue: a k block of the 64- and 32-wide ones 0.15 and 0.11 us), the pair tiles have not; the times are not refitted to that, so single tiles and parts are taken
+// somewhat more seldom than they pay.  The search above
 // scores whole configurations for the public entry points; its split-K entries stand for the two-launch and cluster forms.
 struct Fit { uint32_t tile_n; double fixed, kblock, round, exchange; };
 struct ChoiceFit {

@@ -13,7 +13,8 @@
 //   warps 2..5  epilogue: tcgen05.ld the finished accumulator, apply the epilogue, store to global,
 //               while the issuer already fills the other accumulator buffer
 // The producer and the issuer walk with their whole warp and one elected lane issues (see ptx::mbar_wait_warp): nanoseconds per 64-deep k block at
-// BN = 128 / 64 / 32: 310 / 302 / 298 as a single diverged lane, 255 / 242 / 234 so.
+// BN = 128 / 64 / 32: 310 / 302 / 298 as a single diverged lane, 255 / 242 / 234 so.  With copies and UMMAs predicated instead of branched around 204 / 152 / 108,
+// where the same measurement (the slope from K = 2048 to 8192, 144 tiles) gives 227 / 234 / 232 for the branch.
 // All inter-role hand-offs are mbarriers; every wait is bounded and a wait that expires writes an
 // error word the host turns into an error (no trap, no unbounded spin).
 #include "kernels.h"

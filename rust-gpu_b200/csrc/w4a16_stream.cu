@@ -22,10 +22,10 @@
 //   * four warps empty the accumulators: a band that lies wholly inside a range is stored directly; a band shared by several CTAs is finished by
 //     whichever CTA arrives last (per-band arrival counter, partial pieces in scratch, added in k order: deterministic, repeated calls agree bit
 //     for bit); no CTA ever waits for another.  The loading warp counts a range's leading partial band in meanwhile.
-// What bounds the loop is the pipes of the dequantisation (15 instructions per packed word, on two pipes that take one per two cycles; a step is 512 cycles
-// of theirs at the least and takes about 940), then HBM (710).  Everything else was taken off the dequantising warps' schedulers: with mma.sync the
-// products and the activation fragments were theirs as well.  Two problems of M = 1, N = 11008, K = 4096: 18.6 us with mma.sync, 17.2 so; four of M = 16,
-// N = 14336: 53.2 and 35.6.  On the way there: one issuing warp, its instructions behind a branch and not predicated, a division per step in
+// What bounds the loop is instructions: a step takes about 940 cycles, of which its 2975 warp instructions need 744 to issue (1920 are the dequantisation, 15 per packed
+// word, on two pipes that take one per two cycles: 512 cycles of theirs at the least), then HBM (710).  Everything else was taken off the dequantising warps' schedulers: with mma.sync the
+// products and the activation fragments were theirs as well.  Two problems of M = 1, N = 11008, K = 4096: 18.6 us with mma.sync, 16.8 so; four of M = 16,
+// N = 14336: 53.3 and 35.9.  On the way there: one issuing warp, its instructions behind a branch and not predicated, a division per step in
 // the producer, waits between the arithmetic and its stores: 38.3 at M = 16.  Tried and taken back: three groups of eight dequantising warps (35.8),
 // a warp that prepares scales and zero points for them (35.9), barriers tested a step ahead (36.7).
 // Every barrier wait is bounded; a wait that runs out raises the CTA's abort flag, the roles unwind, the status word is

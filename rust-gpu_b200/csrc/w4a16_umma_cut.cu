@@ -22,8 +22,9 @@
 // SMs.  A launch takes its tiles whole or cut, or leaves a single problem to the clusters of w4a16_umma.cu: `w4a16_umma_plan` weighs them.
 // What bounds it is the dequantisation's instructions (0.28 us a chunk up to M = 64; two pipes that take one per two cycles are half busy, the schedulers two
 // thirds) and at M = 128 the UMMAs beside them (0.34; 0.27 of tensor work), and per launch with cut tiles 3 to 7 us for handing in and adding their parts.
-// Two problems of N = 11008, K = 4096 at M = 32 / 128: 24.4 / 29.1 us with one issuing warp, one loading by boxes and the sixteen emptying every
-// tile; 20.9 / 26.6 with two issuing warps, predicated; 18.8 / 26.3 with warps that empty the accumulators; 18.4 / 24.7 in pairs.
+// Two problems of N = 11008, K = 4096 at M = 32 / 128, in bursts of a few milliseconds: 24.4 / 29.1 us with one issuing warp, one loading by boxes and the sixteen
+// emptying every tile; 20.9 / 26.6 with two issuing warps, predicated; 18.8 / 26.3 with warps that empty the accumulators; 18.4 / 24.7 in pairs, and with
+// activations three pairs behind at M = 128 (25.7 in step).  In long blocks, where the clock settles, M = 128 takes 31.9 us (34.6 with one issuing warp).
 #include "w4a16_common.cuh"
 
 using namespace t0;
