@@ -122,7 +122,7 @@ def test_w4a16_sums_are_no_longer_than_they_have_been(ask):
 
 
 def w4a16_bound(m, n, k, count):
-    """The longest accumulation by the rule that these kernels were first given, its grid and its times."""
+    """The longest accumulation by the rule whose lengths the library keeps: the times of the kernels as they were before two warps issued, with the grid of cut tiles."""
     tiles, chunks, split, rounds = w4a16_split(n, k, count)
     total = tiles * chunks
     ctas = min(max(1, total // 4), 148)
